@@ -73,9 +73,10 @@ __device__ inline void pmat_one(const PmatArgs &a, unsigned idx, unsigned q) {
         for (int mk = 0; mk < 16; ++mk) tt[(size_t)mk * a.kact * 4] = T[mk];
     }
     if (a.precision == CXG_FP32) {
-        float *o = reinterpret_cast<float *>(dst) + (size_t)k * 16 + i * 4;
+        // By columns.
+        float *o = reinterpret_cast<float *>(dst) + (size_t)k * 16 + i;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) o[j] = (float)P[j];
+        for (int j = 0; j < 4; ++j) o[j * 4] = (float)P[j];
     } else {
         double *o = reinterpret_cast<double *>(dst) + (size_t)k * 16 + i * 4;
 #pragma unroll

@@ -25,18 +25,25 @@ struct NvtxRange {
 // Patterns are padded to a multiple of this on the device, so that every
 // plane of a CL buffer starts on a 512-byte boundary.
 constexpr unsigned kPatternQuantum = 128;
-// Most patterns per tile.
+// Most patterns per tile a caller may tune (cxgTune), and of a CTA whose
+// patterns have several threads each.
 constexpr unsigned kBlock = 128;
-// Largest CTA of the plan walkers: tile patterns x threads per pattern.
-constexpr unsigned kMaxThreads = 256;
+// Largest CTA a caller may tune: tile patterns x threads per pattern.
+constexpr unsigned kTuneThreads = 256;
+// Largest CTA of the plan walkers.  18 warps: 80,000 patterns on 152 SMs are
+// 17 warps an SM, which one CTA of 112 registers a thread holds.
+constexpr unsigned kMaxThreads = 576;
 // Largest CTA of the op-lane walker: 2 lanes x tile patterns (tile <= 64).
 constexpr unsigned kLaneThreads = 128;
 // Default patterns per tile.
 constexpr unsigned kTile = 64;
 // Most shared-memory stack slots per tile.
 constexpr unsigned kMaxSlots = 16;
-// Op records in flight per CTA (bulk-copy ring depth).
+// Op records in flight per CTA of the two-pattern and op-lane walkers
+// (bulk-copy ring depth).
 constexpr unsigned kRing = 4;
+// Stages of the plan walker's ring, each a group of ops.
+constexpr unsigned kStages = 3;
 // Default iteration bound of every spin on an mbarrier (the record waits
 // take theirs from set_spin_limit).
 constexpr unsigned kSpinLimit = 1u << 26;
@@ -63,8 +70,11 @@ enum : uint32_t {
 //
 //   RecHead | RecChild[nchild] | one area per child, at RecChild.off
 //
-// A child's area is filled in place by the P-matrix kernel of each run:
-// the P matrices T P[kact][16], or for a leaf child of an FP32 plan its
+// (the areas follow the descriptors in child order).  A child's area is
+// filled in place by the P-matrix kernel of each run: the P matrices
+// T P[kact][16] (FP64 by rows; FP32 by columns, so that one 16-byte read
+// gives the walker two packed pairs of rows), or for a leaf child of an FP32
+// plan its
 // message table float[kact][16 masks][4] (the message P x indicator(mask)
 // of every state mask, summed in FP64 and rounded once).
 struct RecHead {
@@ -75,7 +85,7 @@ struct RecHead {
     uint32_t flags;    // REC_NO_HBM: the result is not written to HBM
     // Bytes of the record `ring` positions later, which refills this ring
     // stage after this op (a multiple of 16); 0: the whole record stride.
-    // Read by the one-lane walker with staged leaves; others copy whole
+    // Read by the two-pattern walker with staged leaves; others copy whole
     // strides.
     uint32_t next_bytes;
 };
@@ -84,9 +94,8 @@ struct RecHead {
 // root) and is not kept as a cache, so the walker skips its HBM write.
 enum : uint32_t { REC_NO_HBM = 1 };
 
-// RecHead.flags bits 8-10: the kind of a two-child op of an FP32 plan run
-// one op at a time, one thread per pattern, named by where its children
-// come from (F: the previous op's result, still in registers; L: a leaf;
+// RecHead.flags bits 8-10: the kind of a two-child op of a plan run one op
+// at a time, named by where its children come from (F: the previous op's result, still in registers; L: a leaf;
 // I: an internal CL in HBM or a stack slot).  The walker then runs
 // straight-line code for that kind.  Bit 12 gives the record index of
 // child A (the first letter); child B is the other.  A product of two
@@ -171,7 +180,7 @@ struct PlanArgs {
     const uint8_t *const *leaves;
     uint32_t nleaf;
     uint32_t rstride;
-    uint32_t ring;        // records in flight per CTA
+    uint32_t ring;        // WalkShape::ring
     uint32_t nops;
     uint32_t nslot;       // shared-memory stack slots per tile
     uint32_t tile;        // patterns per CTA (blockDim.x / tpp)
@@ -190,7 +199,7 @@ struct PlanArgs {
     double *total;        // [2] final (sum, compensation)
     uint32_t *err;        // nonzero: a bounded wait gave up
     const double *ltab;   // FP64 plans: [ntab][16 masks][kact][4]
-    uint32_t ntiles;      // tiles of this job (ppad / tile)
+    uint32_t ntiles;      // tiles of this job (ppad / tile, rounded up)
     uint32_t no_root;     // 1: stop after the ops (per-node launches)
     uint32_t tpp;         // threads per pattern (each holds kact / tpp
                           // components); 0 is read as 1
@@ -199,9 +208,9 @@ struct PlanArgs {
 
 // Threads per pattern and patterns per thread a walker is built for with
 // `kact` components: one of each for every shape; 2 or 4 threads per
-// pattern for the FP32 form when they divide kact; 2 patterns per thread
-// for the FP32 form with one thread per pattern and at most 5 components.
-// Op lanes (two independent ops per step, walk_tile's L) exist for the
+// pattern when they divide kact; 2 patterns per thread for the FP32 form
+// with one thread per pattern and at most 5 components.
+// Op lanes (two independent ops per step, walk_tile_lanes) exist for the
 // FP32 form with one thread and one pattern per thread, kact <= 5.
 inline bool lanes_shape_ok(int precision, unsigned kact, unsigned tpp, unsigned ppt) {
     return precision == CXG_FP32 && tpp == 1 && ppt == 1 && kact >= 1 && kact <= 5;
@@ -213,30 +222,49 @@ inline bool walker_shape_ok(int precision, unsigned kact, unsigned tpp,
         return precision == CXG_FP32 && tpp == 1 && kact >= 1 && kact <= 5;
     if (ppt != 1) return false;
     if (tpp == 1) return kact >= 1 && kact <= kMaxComps;
-    if (precision != CXG_FP32 || (tpp != 2 && tpp != 4)) return false;
-    return kact % tpp == 0 && kact / tpp <= (tpp == 2 ? 4u : 2u);
+    if (tpp != 2 && tpp != 4) return false;
+    return kact != 0 && kact % tpp == 0 && kact / tpp <= (tpp == 2 ? 4u : 2u);
 }
 
-// Threads per pattern for a new plan: the tuned value where the walker is
-// built for it (walker_shape_ok, tile x tpp <= kMaxThreads), else 1.
-inline unsigned tuned_tpp(int precision, unsigned kact, unsigned tile) {
-    unsigned t = 0, tpp = 1, ppt = 1;
-    size_t b = 0;
-    cxgTuneGet(&t, &tpp, &ppt, &b);
-    if (!walker_shape_ok(precision, kact, tpp) || tile * tpp > kMaxThreads) tpp = 1;
-    return tpp;
+// Launch shape of a walker: patterns per CTA, threads per pattern, patterns
+// per thread, op lanes; `ring` is ops per stage of the lean walker's ring
+// (one pattern per thread, one lane), records in flight of the others.
+struct WalkShape {
+    int precision = CXG_FP64;
+    unsigned kact = 1, tile = kTile, tpp = 1, ppt = 1, lanes = 1, ring = kRing;
+    bool lean() const { return ppt == 1 && lanes == 1; }
+};
+
+// Largest CTA the walker of KT components a thread, G threads per pattern is
+// built for.  The wide FP32 walkers are held to 112 registers (one CTA of
+// 576 threads), the others to 128 (two of 256).
+__host__ __device__ constexpr unsigned walker_threads(int precision, unsigned KT, unsigned G) {
+    return precision == CXG_FP32 && G == 1 && KT <= 5 ? kMaxThreads : kTuneThreads;
 }
 
-// Patterns per thread for a new plan with `tpp` threads per pattern: the
-// tuned value where the walker is built for it (and the tile keeps at
-// least one warp), else 1.
-inline unsigned tuned_ppt(int precision, unsigned kact, unsigned tile, unsigned tpp) {
-    unsigned t = 0, tq = 1, ppt = 1;
-    size_t b = 0;
-    cxgTuneGet(&t, &tq, &ppt, &b);
-    if (!walker_shape_ok(precision, kact, tpp, ppt) || tile / ppt < 32) ppt = 1;
-    return ppt;
-}
+// The lean walker's shared memory: barriers and counts, the ring's stages,
+// the CL stack and its scalers.
+struct LeanLayout {
+    size_t stage0, stage, slots, slot_sc, total;
+};
+
+// Launch shape for new work of `kact` components over `patterns` padded
+// patterns in all: the caller's (cxgTune), or when none was set the one that
+// suits the size (choose_shape, cxg_lik.cu).  `lanes_ok`: op lanes may be
+// used.
+WalkShape choose_shape(int precision, unsigned kact, size_t patterns, bool lanes_ok);
+// Ring of a shape for records of `rstride` bytes with up to `lmax` leaf
+// children: sets w.ring.
+void fit_ring(WalkShape &w, unsigned rstride, unsigned lmax);
+// Whether a job's leaves are staged once per tile (the two-pattern and
+// op-lane walkers, when they fit) rather than streamed with the records.
+bool stages_leaves(const WalkShape &w, unsigned nleaf);
+// Shared-memory stack slots of the walk within the tuned budget.
+unsigned stack_slots(const WalkShape &w, unsigned rstride, unsigned lmax, unsigned nleaf);
+size_t walk_smem_bytes(const WalkShape &w, unsigned nslot, unsigned rstride, unsigned lmax,
+                       unsigned nleaf);
+size_t lean_smem_bytes(int precision, unsigned kact, unsigned tile, unsigned nslot,
+                       unsigned grp, unsigned rstride, unsigned lmax);
 
 // One (job, tile) work item of a batched launch.
 struct WalkItem {
@@ -282,8 +310,7 @@ constexpr size_t kLeafStageBytes = 16 * 1024;
 cudaError_t launch_batch(int precision, const BatchArgs &b, unsigned grid,
                          cudaStream_t s);
 // Resident CTAs per SM of the batched walker for this shape.
-int batch_ctas_per_sm(int precision, unsigned kact, unsigned tile,
-                      unsigned tpp, unsigned ppt, bool staged, size_t smem);
+int batch_ctas_per_sm(const WalkShape &w, bool staged, size_t smem);
 
 // Inputs of the P-matrix kernel: one thread per (child, active comp); the
 // P matrix (FP64 arithmetic, stored as the plan's precision) goes into the

@@ -419,6 +419,7 @@ struct Plan {
     double updates = 0.0;     // pattern-node updates of one run
     unsigned tile = kTile, tpp = 1, ppt = 1, nslot = 0, nleaf = 0;
     unsigned lanes = 1;       // op lanes of the walker (records per step)
+    WalkShape shape;
     // Where the per-call values sit in the program (byte offsets): branch
     // lengths [stepsLen], cmult, rmult, model index [kact], cube and
     // eigenvalues [models], root weights pn [kact][4]; and what they are
@@ -482,9 +483,62 @@ static unsigned g_tpp = 1;
 static unsigned g_ppt = 1;
 static unsigned g_lanes = 1;
 static size_t g_smem_budget = 24 * 1024;
+static bool g_tuned = false;  // cxgTune was called: its shape is used as it is
 
+WalkShape choose_shape(int precision, unsigned kact, size_t patterns, bool lanes_ok) {
+    WalkShape w;
+    w.precision = precision;
+    w.kact = kact;
+    w.tile = g_tile;
+    // The caller's shape, each part where a walker is built for it.
+    if (precision == CXG_FP32 && walker_shape_ok(precision, kact, g_tpp) &&
+        g_tile * g_tpp <= kTuneThreads)
+        w.tpp = g_tpp;
+    if (walker_shape_ok(precision, kact, w.tpp, g_ppt) && g_tile / g_ppt >= 32) w.ppt = g_ppt;
+    if (lanes_ok && g_lanes == 2 && lanes_shape_ok(precision, kact, w.tpp, w.ppt) &&
+        g_tile * 2 <= kLaneThreads)
+        w.lanes = 2;
+    (void)patterns;
+    return w;
+}
+
+void fit_ring(WalkShape &w, unsigned rstride, unsigned lmax) {
+    if (!w.lean()) {
+        // A stage of the op-lane walker holds two records: half the stages
+        // keep as many records in flight.
+        w.ring = w.lanes == 2 ? kRing / 2 : kRing;
+        return;
+    }
+    const size_t bytes = w.tile * w.tpp >= 128 ? 48 * 1024 : 28 * 1024;
+    size_t n = bytes / (kStages * ((size_t)rstride + (size_t)lmax * w.tile));
+    if (n > 16) n = 16;
+    if (lmax && n > 32 / lmax) n = 32 / lmax;
+    w.ring = n ? (unsigned)n : 1;
+}
+
+bool stages_leaves(const WalkShape &w, unsigned nleaf) {
+    return !w.lean() && (size_t)nleaf * w.tile <= kLeafStageBytes;
+}
+
+unsigned stack_slots(const WalkShape &w, unsigned rstride, unsigned lmax, unsigned nleaf) {
+    const size_t base = walk_smem_bytes(w, 0, rstride, lmax, nleaf);
+    const size_t slot = walk_smem_bytes(w, 1, rstride, lmax, nleaf) - base;
+    size_t cap = 0;
+    if (w.lean()) {
+        // The budget is the stack's; the CTA as a whole stays launchable.
+        cap = g_smem_budget / slot;
+        const size_t most = 200 * 1024;
+        if (base + cap * slot > most) cap = base < most ? (most - base) / slot : 0;
+    } else if (g_smem_budget > base) {
+        cap = (g_smem_budget - base) / slot;
+    }
+    return cap > kMaxSlots ? kMaxSlots : (unsigned)cap;
+}
+
+// `patterns`: padded patterns of all the jobs this plan is launched with (0:
+// its own).
 static int translate(State &S, CxtLik *lik, int prec, Plan &P,
-                     bool use_slots = true, bool allow_lanes = false) {
+                     bool use_slots = true, bool allow_lanes = false, size_t patterns = 0) {
     int rc;
     if (lik == nullptr) return fail(CXG_EINVAL, "lik is NULL");
     if (lik->dim != 4)
@@ -615,7 +669,9 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
     // Leaves: staged once per tile (each distinct leaf one row, named by
     // kids[c].idx) when they fit kLeafStageBytes, else each op's mask
     // arrays (kids[c].data) travel with its record (lmax rows per stage).
-    const unsigned tile = g_tile;
+    WalkShape w = choose_shape(prec, kact, patterns ? patterns : ppad,
+                               allow_lanes && ops.size() >= 2);
+    const unsigned tile = w.tile;
     std::vector<const uint8_t *> leaf_ptrs;
     unsigned lmax = 0;
     {
@@ -637,7 +693,9 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
         }
     }
     const unsigned nleaf = (unsigned)leaf_ptrs.size();
-    const bool stage_leaves = (size_t)nleaf * tile <= kLeafStageBytes;
+    // (Op lanes need staged leaves.)
+    if (w.lanes == 2 && !stages_leaves(w, nleaf)) w.lanes = 1;
+    const bool stage_leaves = stages_leaves(w, nleaf);
     const unsigned s_lmax = stage_leaves ? 0 : lmax;
     const unsigned s_nleaf = stage_leaves ? nleaf : 0;
 
@@ -657,14 +715,7 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
         if (b > rstride) rstride = b;
     }
     const bool root_last = !ops.empty() && P.parents.back() == P.root;
-    const unsigned tpp = tuned_tpp(prec, kact, tile);
-    const unsigned ppt = tuned_ppt(prec, kact, tile, tpp);
-    // Op lanes: two mutually independent ops per step (single plans of the
-    // FP32 form with staged leaves, when tuned so).
-    const unsigned lanes =
-        (allow_lanes && g_lanes == 2 && stage_leaves && ops.size() >= 2 &&
-         lanes_shape_ok(prec, kact, tpp, ppt) && tile * 2 <= kLaneThreads)
-            ? 2u : 1u;
+    const unsigned lanes = w.lanes;
     // order[r]: the op in record position r, or -1 for an empty lane.  With
     // lanes, each op goes to the earliest step after those of the ops that
     // produce its children (ops in post-order, steps filled in that order),
@@ -701,19 +752,9 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
             order[st * lanes + n_in[st]++] = (int)o;
         }
     }
-    // A stage of the lane walker holds two records: half the stages keep
-    // as many records in flight.
-    const unsigned ring = lanes == 2 ? kRing / 2 : kRing;
-    const unsigned sbytes = (unsigned)rstride * lanes;  // one ring stage
-    const size_t base_bytes = plan_smem_bytes(prec, kact, tile, 0, ring,
-                                              sbytes, s_lmax, s_nleaf);
-    const size_t slot_bytes =
-        plan_smem_bytes(prec, kact, tile, 1, ring, sbytes, s_lmax, s_nleaf) -
-        base_bytes;
-    unsigned cap = 0;
-    if (g_smem_budget > base_bytes)
-        cap = (unsigned)((g_smem_budget - base_bytes) / slot_bytes);
-    if (cap > kMaxSlots) cap = kMaxSlots;
+    fit_ring(w, (unsigned)rstride, s_lmax);
+    const unsigned ring = w.ring;
+    unsigned cap = stack_slots(w, (unsigned)rstride, s_lmax, s_nleaf);
     if (!use_slots) cap = 0;
     unsigned used = 0;
     {
@@ -818,13 +859,13 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
             continue;
         }
         const size_t o = (size_t)order[pos];
-        if (lanes == 1 && pos + ring < order.size())
+        if (!w.lean() && lanes == 1 && pos + ring < order.size())
             hd.next_bytes = (uint32_t)rec_bytes[order[pos + ring]];
         hd.data = ops[o].data;
         hd.scaler = ops[o].scaler;
         hd.nchild = ops[o].nchild;
         hd.slot = ops[o].slot;
-        if (prec == CXG_FP32 && lanes == 1 && ops[o].nchild == 2) {
+        if (lanes == 1 && ops[o].nchild == 2) {
             const HostChild &k0 = kids[ops[o].child0], &k1 = kids[ops[o].child0 + 1];
             hd.flags |= op_kind_flags(k0.src, k0.data, k1.src, k1.data,
                                       pos > 0 ? ops[order[pos - 1]].data : nullptr);
@@ -922,8 +963,8 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
     a.ring = ring;
     a.nslot = nslot;
     a.tile = tile;
-    a.tpp = tpp;
-    a.ppt = ppt;
+    a.tpp = w.tpp;
+    a.ppt = w.ppt;
     a.root_last = root_last ? 1u : 0u;
     a.nops = (uint32_t)order.size();  // records, empty lanes included
     a.kact = kact;
@@ -954,6 +995,7 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
     P.tpp = a.tpp;
     P.ppt = a.ppt;
     P.lanes = lanes;
+    P.shape = w;
     P.nslot = nslot;
     P.nleaf = nleaf;
     return 0;
@@ -1037,6 +1079,7 @@ static void plan_key(const State &S, const CxtLik *lik, int prec,
     k.push_back(g_ppt);
     k.push_back(g_smem_budget);
     k.push_back(g_lanes);
+    k.push_back(g_tuned);
     k.push_back(S.epoch);
     k.push_back((uintptr_t)lik);
     k.push_back(lik->dim);
@@ -1214,7 +1257,7 @@ int cxgTune(unsigned tile, unsigned tpp, unsigned ppt, size_t smem_budget) {
         return fail(CXG_EINVAL, "cxgTune: tile must be 32, 64 or 128");
     if (tpp != 1 && tpp != 2 && tpp != 4)
         return fail(CXG_EINVAL, "cxgTune: threads per pattern must be 1, 2 or 4");
-    if (tile * tpp > kMaxThreads)
+    if (tile * tpp > kTuneThreads)
         return fail(CXG_EINVAL, "cxgTune: tile x threads per pattern above 256");
     if (ppt != 1 && ppt != 2)
         return fail(CXG_EINVAL, "cxgTune: patterns per thread must be 1 or 2");
@@ -1229,6 +1272,7 @@ int cxgTune(unsigned tile, unsigned tpp, unsigned ppt, size_t smem_budget) {
     g_tpp = tpp;
     g_ppt = ppt;
     g_smem_budget = smem_budget;
+    g_tuned = true;
     return 0;
 }
 
@@ -1555,10 +1599,13 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
     b->prec = precision;
     b->per_node = (flags & CXG_BATCH_PER_NODE) != 0;
     unsigned kact = 0;
+    size_t patterns = 0;  // of all the jobs
+    for (unsigned j = 0; j < n; ++j)
+        if (liks[j] != nullptr) patterns += pad_patterns(liks[j]->mschars);
     for (unsigned j = 0; j < n; ++j) {
         Plan *P = new Plan();
         b->plans.push_back(P);
-        rc = translate(S, liks[j], precision, *P, !b->per_node);
+        rc = translate(S, liks[j], precision, *P, !b->per_node, false, patterns);
         if (rc) {
             free_batch(b);
             return rc;
@@ -1602,11 +1649,15 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
         prefix[j + 1] = prefix[j] + pm[j].nchild * pm[j].kact;
         for (unsigned t = 0; t < a.ntiles; ++t) items.push_back(WalkItem{j, t});
     }
-    // Staged-leaf jobs first, then streamed ones (the two launches); each
-    // group longest jobs first, so its persistent grid ends together.
+    // The two-pattern walker is built for staged or streamed leaves: jobs
+    // that stage them first, then the others (two launches; the lean walker
+    // takes all in the second).  Each group longest jobs first, so its
+    // persistent grid ends together.
+    const bool lean = b->plans[0]->ppt == 1;
+    auto streams = [&](const WalkItem &x) { return lean || jobs[x.job].lmax != 0; };
     std::stable_sort(items.begin(), items.end(),
                      [&](const WalkItem &x, const WalkItem &y) {
-                         const bool sx = jobs[x.job].lmax != 0, sy = jobs[y.job].lmax != 0;
+                         const bool sx = streams(x), sy = streams(y);
                          if (sx != sy) return sy;
                          return jobs[x.job].nops > jobs[y.job].nops;
                      });
@@ -1629,7 +1680,7 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
         return cuda_fail(e, "cxgBatchCreate upload");
     }
     unsigned nstaged = 0;
-    while (nstaged < items.size() && jobs[items[nstaged].job].lmax == 0) ++nstaged;
+    while (nstaged < items.size() && !streams(items[nstaged])) ++nstaged;
     for (int gi = 0; gi < 2; ++gi) {
         BatchArgs &ba = b->args[gi];
         memset(&ba, 0, sizeof(ba));
@@ -1652,6 +1703,10 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
             ba.max_lmax = std::max(ba.max_lmax, a.lmax);
             ba.max_nleaf = std::max(ba.max_nleaf, a.nleaf);
         }
+        // One ring for all: every job's group fits the stage of the widest.
+        WalkShape w = b->plans[0]->shape;
+        fit_ring(w, ba.max_rstride, ba.max_lmax);
+        ba.ring = w.ring;
     }
     if (!b->per_node) {
         int dev = 0, nsm = 0;
@@ -1661,11 +1716,11 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
         for (int gi = 0; gi < 2; ++gi) {
             const BatchArgs &ba = b->args[gi];
             if (ba.nitems == 0) continue;
-            const size_t smem =
-                plan_smem_bytes(precision, kact, ba.tile, ba.max_nslot, kRing,
-                                ba.max_rstride, ba.max_lmax, ba.max_nleaf);
-            const int per =
-                batch_ctas_per_sm(precision, kact, ba.tile, ba.tpp, ba.ppt, gi == 0, smem);
+            WalkShape w = b->plans[0]->shape;
+            w.ring = ba.ring;
+            const size_t smem = walk_smem_bytes(w, ba.max_nslot, ba.max_rstride, ba.max_lmax,
+                                                ba.max_nleaf);
+            const int per = batch_ctas_per_sm(w, gi == 0, smem);
             if (per <= 0 || nsm <= 0) {
                 free_batch(b);
                 return fail(CXG_EINVAL, "cxgBatchCreate: walker does not fit an SM");

@@ -1544,7 +1544,7 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
             ++ci;
         }
         for (unsigned j = nl; j < 3; ++j) lr[j] = nullptr;
-        if (d.prec == CXG_FP32 && nch == 2) hd.flags |= op_kind_of_classes(kcls[0], kcls[1]);
+        if (nch == 2) hd.flags |= op_kind_of_classes(kcls[0], kcls[1]);
         memcpy(r, &hd, sizeof(hd));
     }
     // The tree (moved) and the dirty list back to HBM; an eTBR result goes
@@ -1845,25 +1845,15 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
                                           child_area_bytes(cfg->precision, K, false))) +
                             15) &
                            ~(size_t)15);
-    unsigned tile = 0, tpp_q = 1;
-    size_t budget = 0;
-    unsigned ppt_q = 1;
-    cxgTuneGet(&tile, &tpp_q, &ppt_q, &budget);
-    const unsigned tpp = tuned_tpp(cfg->precision, K, tile);
-    const unsigned ppt = tuned_ppt(cfg->precision, K, tile, tpp);
-    d.ntiles = d.ppad / tile;
-    {
-        // Leaves staged per tile when they fit, else streamed with the op
-        // records; stack slots within the tuned shared-memory budget.
-        d.staged = (size_t)N * tile <= kLeafStageBytes;
-        const unsigned lm = d.staged ? 0 : 3, nl = d.staged ? N : 0;
-        const size_t base_b =
-            plan_smem_bytes(cfg->precision, K, tile, 0, kRing, d.rstride, lm, nl);
-        const size_t slot_b =
-            plan_smem_bytes(cfg->precision, K, tile, 1, kRing, d.rstride, lm, nl) - base_b;
-        size_t cap = budget > base_b ? (budget - base_b) / slot_b : 0;
-        d.nslot_cap = (uint32_t)(cap > kMaxSlots ? kMaxSlots : cap);
-    }
+    WalkShape w = choose_shape(cfg->precision, K, (size_t)C * d.ppad, false);
+    const unsigned tile = w.tile;
+    d.ntiles = plan_blocks(d.ppad, tile);
+    // Leaves staged per tile or streamed with the op records; stack slots
+    // within the tuned shared-memory budget.
+    d.staged = stages_leaves(w, N);
+    const unsigned lm = d.staged ? 0 : 3, nl = d.staged ? N : 0;
+    fit_ring(w, d.rstride, lm);
+    d.nslot_cap = stack_slots(w, d.rstride, lm, nl);
     d.seed = cfg->seed;
     d.swap_stride = cfg->swap_stride ? cfg->swap_stride : 1;
     // Without a +I component the +I weight move has nothing to change
@@ -2076,12 +2066,12 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
         a.leaves = d.staged ? d.leafmask : nullptr;
         a.nleaf = d.staged ? N : 0;
         a.rstride = d.rstride;
-        a.ring = kRing;
+        a.ring = w.ring;
         a.nops = 0;
         a.nslot = d.nslot_cap;
         a.tile = tile;
-        a.tpp = tpp;
-        a.ppt = ppt;
+        a.tpp = w.tpp;
+        a.ppt = w.ppt;
         a.kact = K;
         a.npat = d.npat;
         a.ppad = d.ppad;
@@ -2111,21 +2101,20 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
     ba.nitems = (uint32_t)items.size();
     ba.counter = d.counter;
     ba.tile = tile;
-    ba.tpp = tpp;
-    ba.ppt = ppt;
-    ba.ring = kRing;
+    ba.tpp = w.tpp;
+    ba.ppt = w.ppt;
+    ba.ring = w.ring;
     ba.kact = K;
     ba.max_nslot = d.nslot_cap;
     ba.max_rstride = d.rstride;
     ba.max_lmax = d.staged ? 0 : 3;
     ba.max_nleaf = d.staged ? N : 0;
-    const size_t smem = plan_smem_bytes(cfg->precision, K, tile, d.nslot_cap, kRing,
-                                        d.rstride, ba.max_lmax, ba.max_nleaf);
+    const size_t smem =
+        walk_smem_bytes(w, d.nslot_cap, d.rstride, ba.max_lmax, ba.max_nleaf);
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const int per =
-        batch_ctas_per_sm(cfg->precision, K, tile, tpp, ppt, d.staged != 0, smem);
+    const int per = batch_ctas_per_sm(w, d.staged != 0, smem);
     if (per <= 0) {
         mc3_free(h);
         return fail(CXG_EINVAL, "cxgMc3Create: walker does not fit an SM");

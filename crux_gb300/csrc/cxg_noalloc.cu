@@ -218,14 +218,9 @@ extern "C" int cxgLikExecuteNoAlloc(const CxtLik *lik, int precision,
             return fail(CXG_EINVAL, "cxgLikExecuteNoAlloc: leaf tables above 1.5 MiB");
     }
     const size_t o_part = al16(o_ltab + (ltab_bytes ? ltab_bytes : 16));
-    unsigned tile = kTile;
-    size_t budget = 0;
-    {
-        unsigned tpp_q = 1;
-        unsigned ppt_q = 1;
-        cxgTuneGet(&tile, &tpp_q, &ppt_q, &budget);
-    }
-    const unsigned tpp = tuned_tpp(prec, kact, tile);
+    WalkShape w = choose_shape(prec, kact, ppad, false);
+    const unsigned tile = w.tile;
+    fit_ring(w, (unsigned)rstride, lmax);
     const unsigned nb = plan_blocks(ppad, tile);
     if (o_part + (size_t)nb * 16 > kNaScratchBytes)
         return fail(CXG_EINVAL, "cxgLikExecuteNoAlloc: scratch too small");
@@ -242,18 +237,12 @@ extern "C" int cxgLikExecuteNoAlloc(const CxtLik *lik, int precision,
     // Shared-memory stack slots (LIFO, oldest holder loses its slot), as in
     // the allocating path.
     // (Leaves always stream here: no leaf table in the fixed scratch.)
-    const size_t base_b =
-        plan_smem_bytes(prec, kact, tile, 0, kRing, (unsigned)rstride, lmax, 0);
-    const size_t slot_b =
-        plan_smem_bytes(prec, kact, tile, 1, kRing, (unsigned)rstride, lmax, 0) - base_b;
+    const unsigned cap = stack_slots(w, (unsigned)rstride, lmax, 0);
     const void **lrows = reinterpret_cast<const void **>(h + o_lrow);
     int owner[kMaxSlots];
     for (unsigned k = 0; k < kMaxSlots; ++k) owner[k] = -1;
     unsigned used = 0;
     unsigned o = 0, kid = 0, ntab = 0;
-    unsigned cap = 0;
-    if (budget > base_b) cap = (unsigned)((budget - base_b) / slot_b);
-    if (cap > kMaxSlots) cap = kMaxSlots;
     uint64_t *dsts = reinterpret_cast<uint64_t *>(h + o_dst);
     int32_t *tabs = reinterpret_cast<int32_t *>(h + o_tab);
     double *elens = reinterpret_cast<double *>(h + o_elen);
@@ -334,7 +323,7 @@ extern "C" int cxgLikExecuteNoAlloc(const CxtLik *lik, int precision,
             hd.slot = sl;
             if ((unsigned)sl + 1 > used) used = (unsigned)sl + 1;
         }
-        if (prec == CXG_FP32 && n == 2) {
+        if (n == 2) {
             RecChild k0, k1;
             memcpy(&k0, r + sizeof(RecHead), sizeof(k0));
             memcpy(&k1, r + sizeof(RecHead) + sizeof(RecChild), sizeof(k1));
@@ -389,12 +378,12 @@ extern "C" int cxgLikExecuteNoAlloc(const CxtLik *lik, int precision,
     a.lrows = reinterpret_cast<const uint8_t *const *>(dev + o_lrow);
     a.lmax = lmax;
     a.rstride = (uint32_t)rstride;
-    a.ring = kRing;
+    a.ring = w.ring;
     a.nops = nops;
     a.nslot = used;
     a.tile = tile;
-    a.tpp = tpp;
-    a.ppt = tuned_ppt(prec, kact, tile, tpp);
+    a.tpp = w.tpp;
+    a.ppt = w.ppt;
     a.kact = kact;
     a.npat = npat;
     a.ppad = ppad;

@@ -28,6 +28,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <condition_variable>
 #include <deque>
@@ -130,7 +131,8 @@ struct HostKid {
 struct HostPlan {
     bool ready = false;
     unsigned K = 0, ppad = 0, ntiles = 0, nops = 0, nk = 0, nslot = 0, nhbm = 0;
-    unsigned tile = kTile, tpp = 1, ppt = 1, lmax = 0;
+    WalkShape w;
+    unsigned lmax = 0;
     bool staged = false;  // leaves staged per tile (else streamed)
     size_t rstride = 0, job_bytes = 0, data_bytes = 0;
     size_t up_bytes = 0;  // records .. model: the job's one upload
@@ -326,13 +328,8 @@ void plan_request(SrvRequest &rq, int prec) {
     const unsigned N = r.ntaxa, NN = 2 * N - 2;
     P.K = r.ncat + (r.pinv > 0.0 ? 1 : 0);
     P.ppad = pad_patterns(r.npat);
-    unsigned tq = 0;
-    size_t budget = 0;
-    unsigned pq = 1;
-    cxgTuneGet(&P.tile, &tq, &pq, &budget);
-    P.tpp = tuned_tpp(prec, P.K, P.tile);
-    P.ppt = tuned_ppt(prec, P.K, P.tile, P.tpp);
-    P.ntiles = P.ppad / P.tile;
+    P.w = choose_shape(prec, P.K, P.ppad, false);
+    P.ntiles = plan_blocks(P.ppad, P.w.tile);
     const size_t elt = prec == CXG_FP32 ? 4 : 8;
     const unsigned K = P.K;
     // Record stride: up to three children, each with the larger area (an
@@ -367,15 +364,10 @@ void plan_request(SrvRequest &rq, int prec) {
         for (int j = 0; j < 3; ++j) n += (child[v * 3 + j] >= 0 && child[v * 3 + j] < (int)N);
         if (n > P.lmax) P.lmax = n;
     }
-    P.staged = (size_t)N * P.tile <= kLeafStageBytes;
+    P.staged = stages_leaves(P.w, N);
     const unsigned s_lmax = P.staged ? 0 : P.lmax, s_nleaf = P.staged ? N : 0;
-    const size_t base_b =
-        plan_smem_bytes(prec, K, P.tile, 0, kRing, (unsigned)P.rstride, s_lmax, s_nleaf);
-    const size_t slot_b =
-        plan_smem_bytes(prec, K, P.tile, 1, kRing, (unsigned)P.rstride, s_lmax, s_nleaf) -
-        base_b;
-    unsigned cap = budget > base_b ? (unsigned)((budget - base_b) / slot_b) : 0;
-    if (cap > kMaxSlots) cap = kMaxSlots;
+    fit_ring(P.w, (unsigned)P.rstride, s_lmax);
+    const unsigned cap = stack_slots(P.w, (unsigned)P.rstride, s_lmax, s_nleaf);
     std::vector<int> owner(cap, -1), op_of(NN, -1);
     std::vector<char> need_hbm(nops, 0);
     P.slot.assign(nops, -1);
@@ -679,7 +671,7 @@ int prepare_job(cxgServer *S, SrvJob &J, char *stage) {
             area += child_area_bytes(prec, K, k.src == SRC_LEAF);
             ++nk;
         }
-        if (prec == CXG_FP32 && nch == 2) {
+        if (nch == 2) {
             hd.flags |= op_kind_of_classes(kcls[0], kcls[1]);
             memcpy(rr, &hd, sizeof(hd));
         }
@@ -704,12 +696,12 @@ int prepare_job(cxgServer *S, SrvJob &J, char *stage) {
     a.leaves = P.staged ? J.ds->leaves : nullptr;
     a.nleaf = P.staged ? N : 0;
     a.rstride = (uint32_t)rstride;
-    a.ring = kRing;
+    a.ring = P.w.ring;
     a.nops = P.nops;
     a.nslot = P.nslot;
-    a.tile = P.tile;
-    a.tpp = P.tpp;
-    a.ppt = P.ppt;
+    a.tile = P.w.tile;
+    a.tpp = P.w.tpp;
+    a.ppt = P.w.ppt;
     a.kact = K;
     a.npat = r.npat;
     a.ppad = J.ppad;
@@ -809,20 +801,21 @@ int launch_batch_of(cxgServer *S, SrvBatch &B, cudaStream_t st) {
     ba.tile = B.jobs[0]->a.tile;
     ba.tpp = B.jobs[0]->a.tpp;
     ba.ppt = B.jobs[0]->a.ppt;
-    ba.ring = kRing;
     ba.kact = B.jobs[0]->kact;
     ba.max_nslot = max_nslot;
     ba.max_rstride = max_rstride;
     ba.max_lmax = max_lmax;
     ba.max_nleaf = max_nleaf;
     const int prec = S->cfg.precision;
-    const size_t smem = plan_smem_bytes(prec, ba.kact, ba.tile, max_nslot,
-                                        kRing, max_rstride, max_lmax, max_nleaf);
+    // One ring for all: every job's group fits the stage of the widest.
+    WalkShape w = B.jobs[0]->rq->plan.w;
+    fit_ring(w, max_rstride, max_lmax);
+    ba.ring = w.ring;
+    const size_t smem = walk_smem_bytes(w, max_nslot, max_rstride, max_lmax, max_nleaf);
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const int per =
-        batch_ctas_per_sm(prec, ba.kact, ba.tile, ba.tpp, ba.ppt, max_lmax == 0, smem);
+    const int per = batch_ctas_per_sm(w, max_lmax == 0, smem);
     if (per <= 0) return fail(CXG_EINVAL, "server: walker does not fit an SM");
     cudaError_t e = launch_batch(prec, ba, (unsigned)(per * nsm), st);
     if (e != cudaSuccess) return cuda_fail(e, "walk_batch_kernel (server)");
@@ -1026,10 +1019,9 @@ void lnl_loop(cxgServer *S) {
             // A failed launch must give its slot back.
             // One launch per walker shape: components, tile, threads per
             // pattern, staged or streamed leaves.
-            std::map<unsigned, std::vector<SrvJob *>> byk;
+            std::map<std::array<unsigned, 5>, std::vector<SrvJob *>> byk;
             for (SrvJob *J : ready)
-                byk[J->kact | J->a.tile << 8 | J->a.tpp << 16 | J->a.ppt << 20 |
-                    (J->a.lmax ? 1u : 0u) << 24]
+                byk[{J->kact, J->a.tile, J->a.tpp, J->a.ppt, J->rq->plan.staged ? 0u : 1u}]
                     .push_back(J);
             ready.clear();
             for (auto &kv : byk) {
