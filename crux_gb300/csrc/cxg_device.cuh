@@ -15,8 +15,7 @@ namespace cxg {
 // message table instead: row mask = sum over the allowed states j of
 // P[i][j], in j order (P times the reference's 0/1 row, CxLik.c:357-374
 // with Lik.pyx:1466-1475), in the FP64 table for FP64 plans ([16 masks]
-// [kact][4]) and in the record, rounded once to FP32, for FP32 plans
-// ([kact][16 masks][4]).
+// [kact][4]) and in the record, rounded once to FP32, for FP32 plans.
 //
 // Four consecutive lanes (q = lane & 3, all four active) share one idx:
 // lane q computes exp(lambda_q t) and row i = q, so each lane runs a
@@ -60,10 +59,13 @@ __device__ inline void pmat_one(const PmatArgs &a, unsigned idx, unsigned q) {
             T[mk] = __dadd_rn(T[mk ^ (1 << h)], P[h]);
         }
         if (a.precision == CXG_FP32) {
-            // Component-major, [kact][16 masks][4 states]: the walker's
-            // threads read one component's rows at once, so rows of
-            // different masks sit in different shared-memory banks.
-            float *o = reinterpret_cast<float *>(dst) + (size_t)k * 64 + i;
+            // Units of four floats by mask, so that rows of different masks
+            // sit in different shared-memory banks: components go in pairs
+            // (see Rows in cxg_kernels.cu), the last of an odd number alone.
+            const bool lone = (a.kact & 1u) && k + 1 == a.kact;
+            float *o = reinterpret_cast<float *>(dst) +
+                       (lone ? (size_t)k * 64 + i
+                             : (size_t)(k >> 1) * 128 + (i >> 1) * 64 + (i & 1) * 2 + (k & 1u));
 #pragma unroll
             for (int mk = 0; mk < 16; ++mk) o[(size_t)mk * 4] = (float)T[mk];
             return;
@@ -73,10 +75,14 @@ __device__ inline void pmat_one(const PmatArgs &a, unsigned idx, unsigned q) {
         for (int mk = 0; mk < 16; ++mk) tt[(size_t)mk * a.kact * 4] = T[mk];
     }
     if (a.precision == CXG_FP32) {
-        // By columns.
-        float *o = reinterpret_cast<float *>(dst) + (size_t)k * 16 + i;
+        // By columns, components in pairs (see Rows in cxg_kernels.cu), the
+        // last of an odd number alone.
+        const bool lone = (a.kact & 1u) && k + 1 == a.kact;
+        const unsigned step = lone ? 4 : 8;
+        float *o = reinterpret_cast<float *>(dst) +
+                   (lone ? (size_t)k * 16 + i : (size_t)(k >> 1) * 32 + i * 2 + (k & 1u));
 #pragma unroll
-        for (int j = 0; j < 4; ++j) o[j * 4] = (float)P[j];
+        for (int j = 0; j < 4; ++j) o[j * step] = (float)P[j];
     } else {
         double *o = reinterpret_cast<double *>(dst) + (size_t)k * 16 + i * 4;
 #pragma unroll

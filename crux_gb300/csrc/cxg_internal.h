@@ -32,7 +32,7 @@ constexpr unsigned kBlock = 128;
 constexpr unsigned kTuneThreads = 256;
 // Largest CTA of the plan walkers.  18 warps: 80,000 patterns on 152 SMs are
 // 17 warps an SM, which one CTA of 112 registers a thread holds.
-constexpr unsigned kMaxThreads = 576;
+constexpr unsigned kMaxThreads = 640;
 // Largest CTA of the op-lane walker: 2 lanes x tile patterns (tile <= 64).
 constexpr unsigned kLaneThreads = 128;
 // Default patterns per tile.
@@ -55,6 +55,12 @@ constexpr unsigned kMaxChildren = 16;
 inline unsigned pad_patterns(unsigned p) {
     return (p + kPatternQuantum - 1) / kPatternQuantum * kPatternQuantum;
 }
+
+// A job's result words, cleared before its walk: ticket, -inf count, error
+// word, pad (4 bytes each), total [2 doubles], sum limbs [4 x 8].
+constexpr size_t kResultBytes = 64;
+// Those read back.
+constexpr size_t kResultRead = 32;
 
 // Where a child's CL comes from during a plan walk.
 enum : uint32_t {
@@ -83,11 +89,7 @@ struct RecHead {
     uint32_t nchild;
     int32_t slot;      // stack slot keeping the result for a later op, or -1
     uint32_t flags;    // REC_NO_HBM: the result is not written to HBM
-    // Bytes of the record `ring` positions later, which refills this ring
-    // stage after this op (a multiple of 16); 0: the whole record stride.
-    // Read by the two-pattern walker with staged leaves; others copy whole
-    // strides.
-    uint32_t next_bytes;
+    uint32_t pad;
 };
 
 // RecHead.flags: the parent is consumed from its stack slot (or is the
@@ -174,9 +176,9 @@ struct PlanArgs {
     // stage (a plan with no leaf children may use lmax 0).
     const uint8_t *const *lrows;
     uint32_t lmax;
-    // A job whose leaves fit the staging budget stages them instead: nleaf
-    // mask arrays, each loaded once per tile; leaf children then name their
-    // staged row by RecChild.idx (lmax is 0).  nleaf 0: leaves stream.
+    // The op-lane walker stages its leaves instead: nleaf mask arrays, each
+    // loaded once per tile; leaf children then name their staged row by
+    // RecChild.idx (lmax is 0).
     const uint8_t *const *leaves;
     uint32_t nleaf;
     uint32_t rstride;
@@ -193,10 +195,10 @@ struct PlanArgs {
     const void *rootsc;   // root scaler
     const uint32_t *freqs;// [npat] pattern weights (charFreqs + cbase)
     double *site;         // [npat] site lnL out (may be null)
-    double *partial;      // [nblocks][2] compensated partial sums
+    uint64_t *acc;        // [4] limbs of the sum of site lnLs, cleared before
     uint32_t *ninf;       // count of -inf sites
     unsigned *ticket;     // last-block counter
-    double *total;        // [2] final (sum, compensation)
+    double *total;        // [2] the sum: integer and fraction part
     uint32_t *err;        // nonzero: a bounded wait gave up
     const double *ltab;   // FP64 plans: [ntab][16 masks][kact][4]
     uint32_t ntiles;      // tiles of this job (ppad / tile, rounded up)
@@ -227,44 +229,40 @@ inline bool walker_shape_ok(int precision, unsigned kact, unsigned tpp,
 }
 
 // Launch shape of a walker: patterns per CTA, threads per pattern, patterns
-// per thread, op lanes; `ring` is ops per stage of the lean walker's ring
-// (one pattern per thread, one lane), records in flight of the others.
+// per thread, op lanes; `ring` is ops per stage of the walker's ring (steps
+// in flight of the op-lane walker).
 struct WalkShape {
     int precision = CXG_FP64;
     unsigned kact = 1, tile = kTile, tpp = 1, ppt = 1, lanes = 1, ring = kRing;
-    bool lean() const { return ppt == 1 && lanes == 1; }
+    size_t budget = 0;  // bytes of the CL stack
 };
 
-// Largest CTA the walker of KT components a thread, G threads per pattern is
-// built for.  The wide FP32 walkers are held to 112 registers (one CTA of
-// 576 threads), the others to 128 (two of 256).
-__host__ __device__ constexpr unsigned walker_threads(int precision, unsigned KT, unsigned G) {
-    return precision == CXG_FP32 && G == 1 && KT <= 5 ? kMaxThreads : kTuneThreads;
+// Largest CTA the walker of KT components a thread, G threads per pattern and
+// N patterns per thread is built for.  The wide FP32 walkers are held to the
+// registers of one CTA of 576 threads, the others to 128 (two of 256).
+__host__ __device__ constexpr unsigned walker_threads(int precision, unsigned KT, unsigned G,
+                                                      unsigned N) {
+    return precision == CXG_FP32 && G == 1 && N == 1 && KT <= 5 ? kMaxThreads : kTuneThreads;
 }
 
-// The lean walker's shared memory: barriers and counts, the ring's stages,
+// The walker's shared memory: barriers and counts, the ring's stages,
 // the CL stack and its scalers.
 struct LeanLayout {
     size_t stage0, stage, slots, slot_sc, total;
 };
 
 // Launch shape for new work of `kact` components over `patterns` padded
-// patterns in all: the caller's (cxgTune), or when none was set the one that
-// suits the size (choose_shape, cxg_lik.cu).  `lanes_ok`: op lanes may be
-// used.
-WalkShape choose_shape(int precision, unsigned kact, size_t patterns, bool lanes_ok);
+// patterns in all of `jobs` jobs: the caller's (cxgTune), or when none was set
+// the one that suits the size.  `lanes_ok`: op lanes may be used.
+WalkShape choose_shape(int precision, unsigned kact, size_t patterns, unsigned jobs,
+                       bool lanes_ok);
 // Ring of a shape for records of `rstride` bytes with up to `lmax` leaf
 // children: sets w.ring.
 void fit_ring(WalkShape &w, unsigned rstride, unsigned lmax);
-// Whether a job's leaves are staged once per tile (the two-pattern and
-// op-lane walkers, when they fit) rather than streamed with the records.
-bool stages_leaves(const WalkShape &w, unsigned nleaf);
-// Shared-memory stack slots of the walk within the tuned budget.
+// Shared-memory stack slots of the walk within the shape's budget.
 unsigned stack_slots(const WalkShape &w, unsigned rstride, unsigned lmax, unsigned nleaf);
 size_t walk_smem_bytes(const WalkShape &w, unsigned nslot, unsigned rstride, unsigned lmax,
                        unsigned nleaf);
-size_t lean_smem_bytes(int precision, unsigned kact, unsigned tile, unsigned nslot,
-                       unsigned grp, unsigned rstride, unsigned lmax);
 
 // One (job, tile) work item of a batched launch.
 struct WalkItem {
@@ -282,16 +280,13 @@ struct BatchArgs {
     uint32_t nitems;
     unsigned *counter;
     uint32_t tile, ring, kact;
-    uint32_t max_nslot, max_rstride, max_lmax, max_nleaf;
+    uint32_t max_nslot, max_rstride, max_lmax;
     uint32_t tpp;         // threads per pattern (all jobs); 0 is read as 1
     uint32_t ppt;         // patterns per thread (all jobs); 0 is read as 1
     uint32_t direct;      // 1: CTA i walks item i (grid = nitems), no
                           // counter; launch_batch sets it
 };
 
-size_t plan_smem_bytes(int precision, unsigned kact, unsigned tile, unsigned nslot,
-                       unsigned ring, unsigned rstride, unsigned lmax,
-                       unsigned nleaf);
 // Pattern compression on the device (cxg_compact.cu): scratch bytes, and
 // the compaction of rows [ntaxa][nsites] (device, 16-byte aligned) into rows_out / masks
 // (row strides rstride / mstride; mask pad patterns up to mstride get
@@ -304,13 +299,12 @@ int compact_device(const uint8_t *rows, unsigned ntaxa, unsigned nsites,
                    uint8_t *masks, unsigned mstride, uint32_t *freq_out, uint32_t *npat_dev,
                    void *work, size_t work_bytes, cudaStream_t s);
 
-// Largest staged leaf rows per CTA: jobs whose leaves take more stream
-// them with their records instead.
+// Largest staged leaf rows per CTA of the op-lane walker.
 constexpr size_t kLeafStageBytes = 16 * 1024;
 cudaError_t launch_batch(int precision, const BatchArgs &b, unsigned grid,
                          cudaStream_t s);
 // Resident CTAs per SM of the batched walker for this shape.
-int batch_ctas_per_sm(const WalkShape &w, bool staged, size_t smem);
+int batch_ctas_per_sm(const WalkShape &w, size_t smem);
 
 // Inputs of the P-matrix kernel: one thread per (child, active comp); the
 // P matrix (FP64 arithmetic, stored as the plan's precision) goes into the
@@ -332,7 +326,7 @@ struct PmatArgs {
     const double *wnorm_dev;   // if set, wNorm is read here (model built on the GPU)
     unsigned char *rec;
     double *ltab;              // FP64 plans: leaf-message tables
-    uint64_t *zero = nullptr;  // pmat_kernel: four words cleared before the
+    uint64_t *zero = nullptr;  // pmat_kernel: kResultBytes cleared before the
                                // walker that follows it runs (its result)
 };
 

@@ -52,7 +52,8 @@ __global__ void pmat_kernel(PmatArgs a) {
     pdl_launch_dependents();
     // The walker's result words (ticket, counts, sum): it reads them only
     // after this grid has completed (stream order, or griddepcontrol.wait).
-    if (a.zero != nullptr && blockIdx.x == 0 && threadIdx.x < 4) a.zero[threadIdx.x] = 0;
+    if (a.zero != nullptr && blockIdx.x == 0 && threadIdx.x < kResultBytes / 8)
+        a.zero[threadIdx.x] = 0;
     const unsigned idx = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
     if (idx >= a.nchild * a.kact) return;  // the same for all four lanes
     pmat_one(a, idx, threadIdx.x & 3u);
@@ -87,85 +88,100 @@ cudaError_t launch_pmat(const PmatArgs &a, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------
-// Compensated (Neumaier two-sum) reduction helpers.
+// The sum of a job's site lnLs, in 128-bit fixed point with 64 fraction
+// bits.  Integer addition is associative, so the sum is the same for every
+// tile and launch shape, and it is exact but for what each value has below
+// 2^-64.  (The FP64 unit adds one warp instruction in 64 cycles: a
+// compensated FP64 sum, six dependent adds a step, took 3 to 8 us at the end
+// of every walk -- shuffles, a serial fold per CTA and one per job.)
 // ---------------------------------------------------------------------------
-struct Comp {
-    double s, c;
-};
+typedef unsigned __int128 fixed128;
 
-__device__ __forceinline__ Comp comp_add(Comp a, Comp b) {
-    const double s = a.s + b.s;
-    const double bb = s - a.s;
-    const double err = (a.s - (s - bb)) + (b.s - bb);
-    return Comp{s, a.c + b.c + err};
+// |v| < 2^63; NaN and infinities do not come here.
+__device__ __forceinline__ fixed128 to_fixed(double v) {
+    const uint64_t bits = (uint64_t)__double_as_longlong(v);
+    const int e = (int)(bits >> 52) & 0x7ff;
+    uint64_t m = bits & 0xfffffffffffffull;
+    if (e != 0) m |= 1ull << 52;
+    const int sh = (e != 0 ? e : 1) - 1075 + 64;  // v = m 2^(sh - 64)
+    fixed128 f = 0;
+    if (sh >= 0)
+        f = (fixed128)m << (sh < 127 ? sh : 127);
+    else if (sh > -64)
+        f = m >> -sh;
+    return (long long)bits < 0 ? (fixed128)0 - f : f;
 }
 
-__device__ __forceinline__ Comp warp_comp(Comp v) {
+__device__ __forceinline__ fixed128 warp_sum(fixed128 f) {
+    uint64_t lo = (uint64_t)f, hi = (uint64_t)(f >> 64);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
-        Comp o;
-        o.s = __shfl_down_sync(0xffffffffu, v.s, off);
-        o.c = __shfl_down_sync(0xffffffffu, v.c, off);
-        v = comp_add(v, o);
+        const uint64_t l = __shfl_xor_sync(0xffffffffu, lo, off);
+        const uint64_t h = __shfl_xor_sync(0xffffffffu, hi, off);
+        const fixed128 t = (((fixed128)hi << 64) | lo) + (((fixed128)h << 64) | l);
+        lo = (uint64_t)t;
+        hi = (uint64_t)(t >> 64);
     }
-    return v;
+    return ((fixed128)hi << 64) | lo;
 }
 
-// Tile sum of site values (finite values; -inf sites are counted
-// separately) into a.partial[tile]; the last tile of the job to finish
-// folds all of the job's partials into a.total.  Thread t holds the values
-// of patterns t + h * blockDim (h < NV): every group of 32 consecutive
-// patterns reduces by the same shuffle tree and the groups add in pattern
-// order, and warp 0 alone folds the partials, so the sums do not depend
-// on the launch shape.
+// Add the CTA's site values (finite ones; -inf sites are counted) to the
+// job's sum, four 32-bit limbs in 64-bit accumulators a.acc (cleared with the
+// job's result words); the last tile of the job to finish writes the total.
 template <int NV>
-__device__ void reduce_sites_n(const PlanArgs &a, unsigned tile_idx, const double *v,
-                               const bool *neg_inf) {
-    __shared__ Comp warp_part[kMaxThreads / 32];
-    __shared__ unsigned ninf_block;
-    __shared__ bool last;
+__device__ void reduce_sites(const PlanArgs &a, const double (&v)[NV],
+                             const bool (&neg_inf)[NV]) {
+    __shared__ uint64_t s_limb[kMaxThreads / 32][4];
+    __shared__ unsigned s_ninf[kMaxThreads / 32];
     const unsigned nwarp = blockDim.x / 32;
-    if (threadIdx.x == 0) ninf_block = 0;
-    __syncthreads();
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    fixed128 f = 0;
+    unsigned ninf = 0;
 #pragma unroll
     for (int h = 0; h < NV; ++h) {
-        if (neg_inf[h]) atomicAdd(&ninf_block, 1u);
-        const Comp c = warp_comp(Comp{v[h], 0.0});
-        if (lane == 0) warp_part[h * nwarp + warp] = c;
+        f += to_fixed(v[h]);
+        ninf += __popc(__ballot_sync(0xffffffffu, neg_inf[h]));
+    }
+    f = warp_sum(f);
+    if (lane < 4) {
+        // The top limb keeps the sign.
+        const uint64_t w = (uint64_t)(f >> (32 * lane));
+        s_limb[warp][lane] = lane == 3 ? (uint64_t)(long long)(int)(uint32_t)w : (uint32_t)w;
+        if (lane == 0) s_ninf[warp] = ninf;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        Comp b = warp_part[0];
-        for (unsigned w = 1; w < NV * nwarp; ++w) b = comp_add(b, warp_part[w]);
-        a.partial[2 * tile_idx] = b.s;
-        a.partial[2 * tile_idx + 1] = b.c;
-        if (ninf_block) atomicAdd(a.ninf, ninf_block);
+    if (warp == 0) {
+        uint64_t sum = 0;
+        ninf = 0;
+        if (lane < 4)
+            for (unsigned w = 0; w < nwarp; ++w) sum += s_limb[w][lane];
+        if (lane == 4)
+            for (unsigned w = 0; w < nwarp; ++w) ninf += s_ninf[w];
+        if (lane < 4) atomicAdd(reinterpret_cast<unsigned long long *>(a.acc) + lane, sum);
+        if (lane == 4 && ninf) atomicAdd(a.ninf, ninf);
         __threadfence();
-        const unsigned t = atomicAdd(a.ticket, 1u);
-        last = (t == a.ntiles - 1);
-    }
-    __syncthreads();
-    if (last && warp == 0) {
-        __threadfence();
-        Comp acc{0.0, 0.0};
-        for (unsigned b = lane; b < a.ntiles; b += 32) {
-            const volatile double *pp = a.partial;
-            acc = comp_add(acc, Comp{pp[2 * b], pp[2 * b + 1]});
+        __syncwarp();
+        unsigned t = 0;
+        if (lane == 0) t = atomicAdd(a.ticket, 1u);
+        if (__shfl_sync(0xffffffffu, t, 0) == a.ntiles - 1) {
+            __threadfence();
+            if (lane == 0) {
+                const volatile uint64_t *q = a.acc;
+                fixed128 T = 0;
+                for (int i = 0; i < 4; ++i)
+                    T += (i == 3 ? (fixed128)(__int128)(long long)q[i] : (fixed128)q[i])
+                         << (32 * i);
+                const bool neg = (T >> 127) != 0;
+                if (neg) T = (fixed128)0 - T;
+                const double hi = (double)(uint64_t)(T >> 64);
+                const double lo = (double)(uint64_t)T * 5.421010862427522e-20;  // 2^-64
+                a.total[0] = neg ? -hi : hi;
+                a.total[1] = neg ? -lo : lo;
+                *a.ticket = 0;
+            }
         }
-        acc = warp_comp(acc);
-        if (lane == 0) {
-            a.total[0] = acc.s;
-            a.total[1] = acc.c;
-            *a.ticket = 0;  // ready for the next launch
-        }
     }
-    __syncthreads();  // warp_part / last are reused by the next item
-}
-
-__device__ __forceinline__ void reduce_sites(const PlanArgs &a, unsigned tile_idx, double v,
-                                             bool neg_inf) {
-    reduce_sites_n<1>(a, tile_idx, &v, &neg_inf);
+    __syncthreads();  // s_limb is reused by the next item
 }
 
 // ---------------------------------------------------------------------------
@@ -193,9 +209,6 @@ struct Prec<float> {
 
 __device__ __forceinline__ void unpack(const float4 v, float *x) {
     x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
-}
-__device__ __forceinline__ float4 pack4(const float *x) {
-    return make_float4(x[0], x[1], x[2], x[3]);
 }
 
 __device__ __forceinline__ float pow2f(int n) {  // n in [-126, 127]
@@ -228,11 +241,6 @@ static __host__ __device__ SmemLayout smem_layout(int precision, unsigned kact,
     L.masks = L.slot_sc + (((size_t)nslot * tile * sc + 15) & ~(size_t)15);
     L.total = L.masks + (size_t)nleaf * tile;
     return L;
-}
-
-size_t plan_smem_bytes(int precision, unsigned kact, unsigned tile, unsigned nslot,
-                       unsigned ring, unsigned rstride, unsigned lmax, unsigned nleaf) {
-    return smem_layout(precision, kact, tile, nslot, ring, rstride, lmax, nleaf).total;
 }
 
 // --- mbarrier and bulk-copy primitives (PTX) --------------------------------
@@ -275,42 +283,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Leaf-row pointers of op q that thread 0 reads ahead (the first
-// kLeafPre; rows past them are read when the stage is issued).  Indexed
-// with constants only, so they stay in registers.
-constexpr int kLeafPre = 4;
-__device__ __forceinline__ void read_rows(const PlanArgs &a, unsigned q,
-                                          const uint8_t *(&pre)[kLeafPre]) {
-    const uint8_t *const *rows = a.lrows + (size_t)q * a.lmax;
-#pragma unroll
-    for (int j = 0; j < kLeafPre; ++j) pre[j] = (unsigned)j < a.lmax ? rows[j] : nullptr;
-}
-
-// Start op q's stage: its record and this tile's mask rows of its leaf
-// children (a.lrows[q][0..lmax), null-terminated, in the record's child
-// order), all completing on the stage's mbarrier.
-__device__ __forceinline__ void issue_stage(const PlanArgs &a, unsigned q,
-                                            unsigned char *st, uint64_t *bar,
-                                            unsigned tile_idx, unsigned tile,
-                                            const uint8_t *const (&pre)[kLeafPre]) {
-    const uint8_t *const *rows = a.lrows + (size_t)q * a.lmax;
-    unsigned n = 0;
-#pragma unroll
-    for (int j = 0; j < kLeafPre; ++j)
-        if (n == (unsigned)j && pre[j] != nullptr) n = j + 1;
-    if (n == kLeafPre)
-        while (n < a.lmax && rows[n] != nullptr) ++n;
-    fence_proxy_async();
-    mbar_expect_tx(bar, a.rstride + n * tile);
-    bulk_g2s(st, a.rec + (size_t)q * a.rstride, a.rstride, bar);
-    const size_t off = (size_t)tile_idx * tile;
-#pragma unroll
-    for (int j = 0; j < kLeafPre; ++j)
-        if ((unsigned)j < n) bulk_g2s(st + a.rstride + (size_t)j * tile, pre[j] + off, tile, bar);
-    for (unsigned j = kLeafPre; j < n; ++j)
-        bulk_g2s(st + a.rstride + (size_t)j * tile, rows[j] + off, tile, bar);
-}
-
 // Attempts of mbarrier.try_wait per record wait (set_spin_limit; the
 // default is kSpinLimit, 0 gives up without waiting).  Read once per tile
 // by the thread that waits.
@@ -350,189 +322,6 @@ __device__ __forceinline__ bool cta_hand_off(bool ok, unsigned nthr) {
     return __syncthreads_and(ok) != 0;
 }
 
-// Max of n values as a balanced tree (the same value as a left-to-right
-// chain: fmax is exact and ignores NaN operands either way), so the
-// dependent chain is log2(n) long instead of n.
-template <int N, typename X>
-__device__ __forceinline__ X tree_max(const X *v) {
-    if constexpr (N == 1) {
-        return v[0];
-    } else {
-        constexpr int H = N / 2;
-        return fmax(tree_max<H>(v), tree_max<N - H>(v + H));
-    }
-}
-
-// --- FP32 two-child ops by kind (one thread per pattern) --------------------
-// One component's message m = P x: P comes as its four columns c (column j
-// holds P[0..3][j]), every entry as a product, then three fused adds, in
-// column order.
-__device__ __forceinline__ void pcol(const float4 (&c)[4], const float *x, float *m) {
-    m[0] = c[0].x * x[0];
-    m[1] = c[0].y * x[0];
-    m[2] = c[0].z * x[0];
-    m[3] = c[0].w * x[0];
-#pragma unroll
-    for (int j = 1; j < 4; ++j) {
-        m[0] = fmaf(c[j].x, x[j], m[0]);
-        m[1] = fmaf(c[j].y, x[j], m[1]);
-        m[2] = fmaf(c[j].z, x[j], m[2]);
-        m[3] = fmaf(c[j].w, x[j], m[3]);
-    }
-}
-
-// An internal child's rows and exponent: from its stack slot, or from HBM
-// through L2 (the rows were written by this same thread earlier in the
-// walk, or by an earlier launch).
-template <int KT>
-__device__ __forceinline__ int load_internal(const RecChild &c, const float4 *slots,
-                                             const int *slot_sc, unsigned tile,
-                                             unsigned pl, unsigned p, size_t ppad,
-                                             float *x) {
-    if (c.src == SRC_SLOT) {
-        const float4 *s = slots + (size_t)c.idx * KT * tile + pl;
-#pragma unroll
-        for (int k = 0; k < KT; ++k) unpack(s[(size_t)k * tile], x + 4 * k);
-        return slot_sc[(size_t)c.idx * tile + pl];
-    }
-    const float4 *g = static_cast<const float4 *>(c.data) + p;
-#pragma unroll
-    for (int k = 0; k < KT; ++k) unpack(__ldcg(g + (size_t)k * ppad), x + 4 * k);
-    return __ldcg(static_cast<const int *>(c.scaler) + p);
-}
-
-// One two-child op of kind `kind` (OPK_*) for the NP patterns pl[h] (in
-// the tile) / p[h] (in the CL buffers) a thread owns: acc[h] becomes the
-// product of the two children's messages and lns[h] the sum of their
-// exponents.  acc holds the previous op's result on entry (child A of the
-// F kinds), with its exponents in lns.  `ia` is child A's record index; a
-// streamed leaf's row is its rank among the op's leaf children.  Each P
-// row is read from shared memory once for all NP patterns.
-template <int KT, bool STAGED, int NP>
-__device__ __forceinline__ void op2_kind(uint32_t kind, const unsigned char *rec,
-                                         const RecChild *kids, unsigned ia,
-                                         float (&acc)[NP][KT * 4], int (&lns)[NP],
-                                         const uint8_t *masks, const uint8_t *lrow,
-                                         const float4 *slots, const int *slot_sc,
-                                         unsigned tile, const unsigned (&pl)[NP],
-                                         const unsigned (&p)[NP], size_t ppad) {
-    const RecChild &cA = kids[ia];
-    const RecChild &cB = kids[ia ^ 1u];
-    const float4 *PA = reinterpret_cast<const float4 *>(rec + cA.off);
-    const float4 *PB = reinterpret_cast<const float4 *>(rec + cB.off);
-    auto mask = [&](const RecChild &c, unsigned rank, unsigned q) -> unsigned {
-        return STAGED ? masks[(size_t)c.idx * tile + q] : lrow[(size_t)rank * tile + q];
-    };
-    // y = a * b, one component (states 0..3) at a time.
-    auto mul4 = [](float *y, const float *a, const float4 b) {
-        y[0] = a[0] * b.x;
-        y[1] = a[1] * b.y;
-        y[2] = a[2] * b.z;
-        y[3] = a[3] * b.w;
-    };
-    switch (kind) {
-    case OPK_LL: {
-        unsigned mA[NP], mB[NP];
-#pragma unroll
-        for (int h = 0; h < NP; ++h) {
-            mA[h] = mask(cA, ia, pl[h]);
-            mB[h] = mask(cB, ia ^ 1u, pl[h]);
-        }
-#pragma unroll
-        for (int k = 0; k < KT; ++k)
-#pragma unroll
-            for (int h = 0; h < NP; ++h) {
-                const float4 a = PA[k * 16 + mA[h]];
-                const float ax[4] = {a.x, a.y, a.z, a.w};
-                mul4(acc[h] + 4 * k, ax, PB[k * 16 + mB[h]]);
-            }
-#pragma unroll
-        for (int h = 0; h < NP; ++h) lns[h] = 0;
-        return;
-    }
-    case OPK_FL:
-    case OPK_IL: {
-        // A's rows: the previous result (FL) or loaded (IL); B a leaf.
-        float xA[NP][KT * 4];
-        int lA[NP];
-#pragma unroll
-        for (int h = 0; h < NP; ++h) {
-            if (kind == OPK_IL) {
-                lA[h] = load_internal<KT>(cA, slots, slot_sc, tile, pl[h], p[h], ppad, xA[h]);
-            } else {
-#pragma unroll
-                for (int q = 0; q < KT * 4; ++q) xA[h][q] = acc[h][q];
-                lA[h] = lns[h];
-            }
-        }
-        unsigned mB[NP];
-#pragma unroll
-        for (int h = 0; h < NP; ++h) mB[h] = mask(cB, 0, pl[h]);
-#pragma unroll
-        for (int k = 0; k < KT; ++k) {
-            const float4 ca[4] = {PA[k * 4], PA[k * 4 + 1], PA[k * 4 + 2], PA[k * 4 + 3]};
-#pragma unroll
-            for (int h = 0; h < NP; ++h) {
-                float m[4];
-                pcol(ca, xA[h] + 4 * k, m);
-                mul4(acc[h] + 4 * k, m, PB[k * 16 + mB[h]]);
-            }
-        }
-#pragma unroll
-        for (int h = 0; h < NP; ++h) lns[h] = lA[h];
-        return;
-    }
-    case OPK_FI: {
-        float xB[NP][KT * 4];
-        int lB[NP];
-#pragma unroll
-        for (int h = 0; h < NP; ++h)
-            lB[h] = load_internal<KT>(cB, slots, slot_sc, tile, pl[h], p[h], ppad, xB[h]);
-#pragma unroll
-        for (int k = 0; k < KT; ++k) {
-            const float4 ca[4] = {PA[k * 4], PA[k * 4 + 1], PA[k * 4 + 2], PA[k * 4 + 3]};
-            const float4 cb[4] = {PB[k * 4], PB[k * 4 + 1], PB[k * 4 + 2], PB[k * 4 + 3]};
-#pragma unroll
-            for (int h = 0; h < NP; ++h) {
-                float ma[4], mb[4];
-                pcol(ca, acc[h] + 4 * k, ma);
-                pcol(cb, xB[h] + 4 * k, mb);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) acc[h][4 * k + i] = ma[i] * mb[i];
-            }
-        }
-#pragma unroll
-        for (int h = 0; h < NP; ++h) lns[h] = lns[h] + lB[h];
-        return;
-    }
-    default: {  // OPK_II
-        float xA[NP][KT * 4], xB[NP][KT * 4];
-        int lA[NP], lB[NP];
-#pragma unroll
-        for (int h = 0; h < NP; ++h) {
-            lA[h] = load_internal<KT>(cA, slots, slot_sc, tile, pl[h], p[h], ppad, xA[h]);
-            lB[h] = load_internal<KT>(cB, slots, slot_sc, tile, pl[h], p[h], ppad, xB[h]);
-        }
-#pragma unroll
-        for (int k = 0; k < KT; ++k) {
-            const float4 ca[4] = {PA[k * 4], PA[k * 4 + 1], PA[k * 4 + 2], PA[k * 4 + 3]};
-            const float4 cb[4] = {PB[k * 4], PB[k * 4 + 1], PB[k * 4 + 2], PB[k * 4 + 3]};
-#pragma unroll
-            for (int h = 0; h < NP; ++h) {
-                float ma[4], mb[4];
-                pcol(ca, xA[h] + 4 * k, ma);
-                pcol(cb, xB[h] + 4 * k, mb);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) acc[h][4 * k + i] = ma[i] * mb[i];
-            }
-        }
-#pragma unroll
-        for (int h = 0; h < NP; ++h) lns[h] = lA[h] + lB[h];
-        return;
-    }
-    }
-}
-
 // ---------------------------------------------------------------------------
 // The plan walker (one pattern per thread, or G threads per pattern).
 //
@@ -560,16 +349,20 @@ __host__ __device__ inline LeanLayout lean_layout(int precision, unsigned kact, 
     LeanLayout L;
     L.stage0 = 128;  // mbarriers, counts and flags before it
     L.stage = (size_t)grp * (rstride + (size_t)lmax * tile);
-    L.slots = L.stage0 + kStages * L.stage;
+    // (An op reads the next one's header and two mask rows ahead; past the
+    // last stage those lie in this gap.)
+    L.slots = L.stage0 + kStages * L.stage + ((64 + 2 * (size_t)tile + 15) & ~(size_t)15);
     L.slot_sc = L.slots + (size_t)nslot * kact * U * tile * 16;
     L.total = L.slot_sc + (((size_t)nslot * tile * sc + 15) & ~(size_t)15);
     return L;
 }
 
-size_t lean_smem_bytes(int precision, unsigned kact, unsigned tile, unsigned nslot,
-                       unsigned grp, unsigned rstride, unsigned lmax) {
-    return lean_layout(precision, kact, tile, nslot, grp, rstride, lmax).total;
-}
+// A header's slot in the word the walker keeps of it: above the flags, plus
+// one.
+constexpr unsigned kSlotShift = 16;
+// Set where a result is not simply written to HBM (kept in a slot, or not
+// written).
+constexpr uint32_t kPlainMask = 0xffffu << kSlotShift | REC_NO_HBM;
 
 // Shared words before the stages.
 struct LeanHead {
@@ -634,7 +427,9 @@ __device__ __forceinline__ uint32_t count_done(uint32_t *p) {
     return old;
 }
 
-// Two packed FP32 values (a register pair).
+// Two packed FP32 values (a register pair): the FP32 products run on two of
+// a pattern's components at a time (fma.rn.f32x2, each half rounded as a
+// scalar fused multiply-add).
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 pack2f(float lo, float hi) {
     f32x2 r;
@@ -659,148 +454,382 @@ __device__ __forceinline__ float max3f(float a, float b, float c) {
     asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
 }
-
-// The four states of one component: FP32 two pairs, FP64 four doubles; and
-// this thread's KT components of one pattern.
-template <typename T>
-struct Quad;
-template <>
-struct Quad<float> {
-    f32x2 v[2];
-};
-template <>
-struct Quad<double> {
-    double v[4];
-};
-template <typename T, int KT>
-struct Rows {
-    Quad<T> q[KT];
-};
-
-__device__ __forceinline__ Quad<float> quad(const float4 x) {
-    return Quad<float>{{pack2f(x.x, x.y), pack2f(x.z, x.w)}};
+// base + a * b bytes, one instruction; 16-byte loads through L2 (rows may
+// have been written by this walk) and stores, at global addresses.
+__device__ __forceinline__ uint64_t addr_at(uint64_t base, uint32_t a, uint32_t b) {
+    uint64_t r;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(base));
+    return r;
 }
-__device__ __forceinline__ Quad<double> quad(const double2 x, const double2 y) {
-    return Quad<double>{{x.x, x.y, y.x, y.y}};
+template <typename X>
+__device__ __forceinline__ X ld_l2(uint64_t at) {
+    return __ldcg(reinterpret_cast<const X *>(at));
 }
-__device__ __forceinline__ void unquad(const Quad<float> &q, float *x) {
-    unpack2f(q.v[0], x[0], x[1]);
-    unpack2f(q.v[1], x[2], x[3]);
+// (Units of packed pairs move as two 64-bit words: taken apart to four
+// floats and packed again, each pair cost two register moves.)
+typedef ulonglong2 pairs;
+__device__ __forceinline__ void st_global(uint64_t at, const pairs v) {
+    asm volatile("st.global.v2.b64 [%0], {%1, %2};" ::"l"(at), "l"(v.x), "l"(v.y) : "memory");
 }
-__device__ __forceinline__ void unquad(const Quad<double> &q, double *x) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) x[i] = q.v[i];
+__device__ __forceinline__ void st_global(uint64_t at, const float4 v) {
+    asm volatile("st.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(at), "f"(v.x), "f"(v.y),
+                 "f"(v.z), "f"(v.w)
+                 : "memory");
 }
-__device__ __forceinline__ Quad<float> operator*(const Quad<float> &a, const Quad<float> &b) {
-    return Quad<float>{{mul2(a.v[0], b.v[0]), mul2(a.v[1], b.v[1])}};
+__device__ __forceinline__ void st_global(uint64_t at, const double2 v) {
+    asm volatile("st.global.v2.f64 [%0], {%1, %2};" ::"l"(at), "d"(v.x), "d"(v.y) : "memory");
 }
-__device__ __forceinline__ Quad<double> operator*(const Quad<double> &a, const Quad<double> &b) {
-    return Quad<double>{
-        {a.v[0] * b.v[0], a.v[1] * b.v[1], a.v[2] * b.v[2], a.v[3] * b.v[3]}};
+__device__ __forceinline__ void st_global(uint64_t at, float v) {
+    asm volatile("st.global.f32 [%0], %1;" ::"l"(at), "f"(v) : "memory");
 }
-
-// Rows from HBM (through L2: they may have been written by this walk) and
-// from the stack in shared memory; unit stride `stride`.
-template <int KT>
-__device__ __forceinline__ void load_l2(const float4 *p, size_t stride, Rows<float, KT> &r) {
-#pragma unroll
-    for (int k = 0; k < KT; ++k) r.q[k] = quad(__ldcg(p + (size_t)k * stride));
+__device__ __forceinline__ void st_global(uint64_t at, int v) {
+    asm volatile("st.global.s32 [%0], %1;" ::"l"(at), "r"(v) : "memory");
 }
-template <int KT>
-__device__ __forceinline__ void load_l2(const double2 *p, size_t stride, Rows<double, KT> &r) {
-#pragma unroll
-    for (int k = 0; k < KT; ++k)
-        r.q[k] = quad(__ldcg(p + (size_t)(2 * k) * stride),
-                      __ldcg(p + (size_t)(2 * k + 1) * stride));
-}
-template <int KT>
-__device__ __forceinline__ void load_smem(const float4 *p, unsigned stride, Rows<float, KT> &r) {
-#pragma unroll
-    for (int k = 0; k < KT; ++k) r.q[k] = quad(p[k * stride]);
-}
-template <int KT>
-__device__ __forceinline__ void load_smem(const double2 *p, unsigned stride,
-                                          Rows<double, KT> &r) {
-#pragma unroll
-    for (int k = 0; k < KT; ++k) r.q[k] = quad(p[2 * k * stride], p[(2 * k + 1) * stride]);
-}
-template <int KT>
-__device__ __forceinline__ void store_rows(float4 *p, size_t stride, const Rows<float, KT> &r) {
-#pragma unroll
-    for (int k = 0; k < KT; ++k) {
-        float x[4];
-        unquad(r.q[k], x);
-        p[(size_t)k * stride] = pack4(x);
-    }
-}
-template <int KT>
-__device__ __forceinline__ void store_rows(double2 *p, size_t stride,
-                                           const Rows<double, KT> &r) {
-#pragma unroll
-    for (int k = 0; k < KT; ++k) {
-        p[(size_t)(2 * k) * stride] = make_double2(r.q[k].v[0], r.q[k].v[1]);
-        p[(size_t)(2 * k + 1) * stride] = make_double2(r.q[k].v[2], r.q[k].v[3]);
-    }
-}
-
-// One component's message of an internal child, P x (P in shared memory:
-// FP32 by columns, FP64 by rows), every entry a product and three fused adds
-// in column order.
-__device__ __forceinline__ Quad<float> matvec(const float4 *P, const Quad<float> &x) {
-    float s[4];
-    unquad(x, s);
-    Quad<float> m;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const Quad<float> c = quad(P[j]);
-        const f32x2 d = pack2f(s[j], s[j]);
-        m.v[0] = j == 0 ? mul2(c.v[0], d) : fma2(c.v[0], d, m.v[0]);
-        m.v[1] = j == 0 ? mul2(c.v[1], d) : fma2(c.v[1], d, m.v[1]);
-    }
-    return m;
-}
-__device__ __forceinline__ Quad<double> matvec(const double2 *P, const Quad<double> &x) {
-    Quad<double> m;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const double2 a = P[2 * i], b = P[2 * i + 1];
-        double v = a.x * x.v[0];
-        v = fma(a.y, x.v[1], v);
-        v = fma(b.x, x.v[2], v);
-        m.v[i] = fma(b.y, x.v[3], v);
-    }
-    return m;
-}
-
-// Largest entry of a pattern's rows.  FP32: the value (operands that are
-// NaN are passed over, as fmax does).  FP64: the exponent word of the
-// largest of entries that are >= 0 (the sign bit is clear, so the high words
-// order as the values; a NaN orders above infinity), on the integer pipe.
-template <int KT>
-__device__ __forceinline__ float rows_max(const Rows<float, KT> &r) {
-    float m = 0.0f;
-#pragma unroll
-    for (int k = 0; k < KT; ++k) {
-        float x[4];
-        unquad(r.q[k], x);
-        m = max3f(max3f(x[0], x[1], x[2]), x[3], m);
-    }
-    return m;
-}
-template <int KT>
-__device__ __forceinline__ int rows_max(const Rows<double, KT> &r) {
-    int m = 0;
-#pragma unroll
-    for (int k = 0; k < KT; ++k) {
-        const double *x = r.q[k].v;
-        const int a = max(__double2hiint(x[0]), __double2hiint(x[1]));
-        const int b = max(__double2hiint(x[2]), __double2hiint(x[3]));
-        m = max(m, max(a, b));
-    }
-    return m;
+__device__ __forceinline__ void st_global(uint64_t at, double v) {
+    asm volatile("st.global.f64 [%0], %1;" ::"l"(at), "d"(v) : "memory");
 }
 __device__ __forceinline__ float vmax(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ int vmax(int a, int b) { return max(a, b); }
+
+// ---------------------------------------------------------------------------
+// One pattern's rows: the KT components (of KT * G) that a thread holds, the
+// first being component k0, a multiple of KT.
+//
+// FP32 layouts (CL rows in HBM and in the stack, P matrices and leaf tables
+// in the op records): components go in pairs, 2m and 2m + 1, the two values
+// of a state side by side, so that a 16-byte unit is two register pairs and
+// the packed products need no moves; the last of an odd number of components
+// stands alone.
+//   CL row     unit 2m + h: (s = 2h: k = 2m, 2m + 1; s = 2h + 1: same)
+//              unit of a lone component: its four states
+//   P          pair block at m * 128 bytes: column j, row i: two floats
+//              lone block at k * 64 bytes, by columns
+//   leaf table pair block at m * 512 bytes: [h][16 masks] units as a CL row's
+//              lone block at k * 256 bytes: [16 masks] of its four states
+// A thread whose odd KT splits pairs between threads (G > 1) holds single
+// components and reads and writes single floats of those units.
+//
+// FP64: component by component, two units (double2) of a CL row each; P by
+// rows; leaf tables in HBM, [16 masks][K][4].
+// ---------------------------------------------------------------------------
+template <typename T, int KT, int G>
+struct Rows;
+
+template <int KT, int G>
+struct Rows<float, KT, G> {
+    typedef float4 V;
+    static constexpr int NP = (G == 1 || KT % 2 == 0) ? KT / 2 : 0;  // pairs
+    static constexpr int NS = KT - 2 * NP;                           // single components
+    static constexpr bool split = NS > 0 && G > 1;  // singles are halves of pairs
+    f32x2 pr[NP ? NP : 1][4];
+    float sg[NS ? NS : 1][4];
+
+    // A row's units in HBM (`at`: the pattern's place in unit 0; units are
+    // `pitch` bytes apart) and in shared memory (`stride` units apart).  A
+    // split single's state s is one float of unit (k & ~1) + s / 2.
+    __device__ static __forceinline__ unsigned part(unsigned k, int s) {
+        return ((s & 1) * 2 + (k & 1u)) * 4;
+    }
+    __device__ __forceinline__ void set(int u, const pairs x) {
+        pr[u / 2][(u & 1) * 2] = x.x;
+        pr[u / 2][(u & 1) * 2 + 1] = x.y;
+    }
+    __device__ __forceinline__ pairs unit(int u) const {
+        return pairs{pr[u / 2][(u & 1) * 2], pr[u / 2][(u & 1) * 2 + 1]};
+    }
+    __device__ __forceinline__ void load_l2(uint64_t at, uint32_t pitch, unsigned k0) {
+#pragma unroll
+        for (int u = 0; u < 2 * NP; ++u) set(u, ld_l2<pairs>(addr_at(at, pitch, k0 + u)));
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {
+            const unsigned k = k0 + 2 * NP + i;
+            if (split) {
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+                    sg[i][s] = __ldcg(reinterpret_cast<const float *>(
+                        addr_at(at, pitch, (k & ~1u) + (s >> 1)) + part(k, s)));
+            } else {
+                unpack(ld_l2<float4>(addr_at(at, pitch, k)), sg[i]);
+            }
+        }
+    }
+    __device__ __forceinline__ void store_global(uint64_t at, uint32_t pitch,
+                                                 unsigned k0) const {
+#pragma unroll
+        for (int u = 0; u < 2 * NP; ++u) st_global(addr_at(at, pitch, k0 + u), unit(u));
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {
+            const unsigned k = k0 + 2 * NP + i;
+            if (split) {
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+                    st_global(addr_at(at, pitch, (k & ~1u) + (s >> 1)) + part(k, s), sg[i][s]);
+            } else {
+                st_global(addr_at(at, pitch, k),
+                          make_float4(sg[i][0], sg[i][1], sg[i][2], sg[i][3]));
+            }
+        }
+    }
+    __device__ __forceinline__ void load_smem(const float4 *p, unsigned stride, unsigned k0) {
+#pragma unroll
+        for (int u = 0; u < 2 * NP; ++u)
+            set(u, *reinterpret_cast<const pairs *>(p + (k0 + u) * stride));
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {
+            const unsigned k = k0 + 2 * NP + i;
+            if (split) {
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+                    sg[i][s] = reinterpret_cast<const float *>(
+                        p + ((k & ~1u) + (s >> 1)) * stride)[part(k, s) / 4];
+            } else {
+                unpack(p[k * stride], sg[i]);
+            }
+        }
+    }
+    __device__ __forceinline__ void store_smem(float4 *p, unsigned stride, unsigned k0) const {
+#pragma unroll
+        for (int u = 0; u < 2 * NP; ++u)
+            *reinterpret_cast<pairs *>(p + (k0 + u) * stride) = unit(u);
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {
+            const unsigned k = k0 + 2 * NP + i;
+            if (split) {
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+                    reinterpret_cast<float *>(p + ((k & ~1u) + (s >> 1)) *
+                                                      stride)[part(k, s) / 4] = sg[i][s];
+            } else {
+                p[k * stride] = make_float4(sg[i][0], sg[i][1], sg[i][2], sg[i][3]);
+            }
+        }
+    }
+    // Component q of this thread's, state s.
+    __device__ __forceinline__ float get(int q, int s) const {
+        if (q >= 2 * NP) return sg[q - 2 * NP][s];
+        float a, b;
+        unpack2f(pr[q / 2][s], a, b);
+        return (q & 1) ? b : a;
+    }
+    // Largest entry (operands that are NaN are passed over, as fmax does).
+    __device__ __forceinline__ float top() const {
+        float m = 0.0f;
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+            float a[4], b[4];
+#pragma unroll
+            for (int s = 0; s < 4; ++s) unpack2f(pr[i][s], a[s], b[s]);
+            m = max3f(max3f(max3f(a[0], b[0], a[1]), b[1], a[2]), max3f(b[2], a[3], b[3]), m);
+        }
+#pragma unroll
+        for (int i = 0; i < NS; ++i)
+            m = max3f(max3f(sg[i][0], sg[i][1], sg[i][2]), sg[i][3], m);
+        return m;
+    }
+    __device__ __forceinline__ void scale(float f) {
+        const f32x2 ff = pack2f(f, f);
+#pragma unroll
+        for (int i = 0; i < NP; ++i)
+#pragma unroll
+            for (int s = 0; s < 4; ++s) pr[i][s] = mul2(pr[i][s], ff);
+#pragma unroll
+        for (int i = 0; i < NS; ++i)
+#pragma unroll
+            for (int s = 0; s < 4; ++s) sg[i][s] *= f;
+    }
+    __device__ __forceinline__ void mul(const Rows &b) {
+#pragma unroll
+        for (int i = 0; i < NP; ++i)
+#pragma unroll
+            for (int s = 0; s < 4; ++s) pr[i][s] = mul2(pr[i][s], b.pr[i][s]);
+#pragma unroll
+        for (int i = 0; i < NS; ++i)
+#pragma unroll
+            for (int s = 0; s < 4; ++s) sg[i][s] *= b.sg[i][s];
+    }
+};
+
+template <int KT, int G>
+struct Rows<double, KT, G> {
+    typedef double2 V;
+    double v[KT][4];
+
+    __device__ __forceinline__ void set(int u, const double2 x) {
+        v[u / 2][(u & 1) * 2] = x.x;
+        v[u / 2][(u & 1) * 2 + 1] = x.y;
+    }
+    __device__ __forceinline__ double2 unit(int u) const {
+        return make_double2(v[u / 2][(u & 1) * 2], v[u / 2][(u & 1) * 2 + 1]);
+    }
+    __device__ __forceinline__ void load_l2(uint64_t at, uint32_t pitch, unsigned k0) {
+#pragma unroll
+        for (int u = 0; u < 2 * KT; ++u)
+            set(u, ld_l2<double2>(addr_at(at, pitch, 2 * k0 + u)));
+    }
+    __device__ __forceinline__ void store_global(uint64_t at, uint32_t pitch,
+                                                 unsigned k0) const {
+#pragma unroll
+        for (int u = 0; u < 2 * KT; ++u) st_global(addr_at(at, pitch, 2 * k0 + u), unit(u));
+    }
+    __device__ __forceinline__ void load_smem(const double2 *p, unsigned stride, unsigned k0) {
+#pragma unroll
+        for (int u = 0; u < 2 * KT; ++u) set(u, p[(2 * k0 + u) * stride]);
+    }
+    __device__ __forceinline__ void store_smem(double2 *p, unsigned stride, unsigned k0) const {
+#pragma unroll
+        for (int u = 0; u < 2 * KT; ++u) p[(2 * k0 + u) * stride] = unit(u);
+    }
+    __device__ __forceinline__ double get(int q, int s) const { return v[q][s]; }
+    // Exponent word of the largest of entries that are >= 0: the sign bit is
+    // clear, so the high words order as the values (a NaN above infinity),
+    // on the integer pipe.
+    __device__ __forceinline__ int top() const {
+        int m = 0;
+#pragma unroll
+        for (int k = 0; k < KT; ++k) {
+            const int a = max(__double2hiint(v[k][0]), __double2hiint(v[k][1]));
+            const int b = max(__double2hiint(v[k][2]), __double2hiint(v[k][3]));
+            m = max(m, max(a, b));
+        }
+        return m;
+    }
+    __device__ __forceinline__ void scale(double f) {
+#pragma unroll
+        for (int k = 0; k < KT; ++k)
+#pragma unroll
+            for (int s = 0; s < 4; ++s) v[k][s] *= f;
+    }
+    __device__ __forceinline__ void mul(const Rows &b) {
+#pragma unroll
+        for (int k = 0; k < KT; ++k)
+#pragma unroll
+            for (int s = 0; s < 4; ++s) v[k][s] *= b.v[k][s];
+    }
+};
+
+// r[h] = P r[h] for the NP patterns of a thread (each unit of P, at `area` in
+// the record, is read once for all of them): every entry a product and
+// three fused adds, in column order.
+template <int KT, int G, int N>
+__device__ __forceinline__ void apply_p(const unsigned char *area, unsigned k0,
+                                        Rows<float, KT, G> (&r)[N]) {
+    typedef Rows<float, KT, G> R;
+#pragma unroll
+    for (int i = 0; i < R::NP; ++i) {
+        const pairs *P = reinterpret_cast<const pairs *>(area + (k0 / 2 + i) * 128);
+        f32x2 y[N][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const pairs a = P[2 * j], b = P[2 * j + 1];
+            const f32x2 c[4] = {a.x, a.y, b.x, b.y};
+#pragma unroll
+            for (int h = 0; h < N; ++h)
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+                    y[h][s] = j == 0 ? mul2(c[s], r[h].pr[i][0])
+                                     : fma2(c[s], r[h].pr[i][j], y[h][s]);
+        }
+#pragma unroll
+        for (int h = 0; h < N; ++h)
+#pragma unroll
+            for (int s = 0; s < 4; ++s) r[h].pr[i][s] = y[h][s];
+    }
+#pragma unroll
+    for (int i = 0; i < R::NS; ++i) {
+        float y[N][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float c[4];
+            if (R::split) {
+                const unsigned k = k0 + i;
+                const float *f = reinterpret_cast<const float *>(area + (k / 2) * 128) + (k & 1u);
+#pragma unroll
+                for (int s = 0; s < 4; ++s) c[s] = f[(j * 4 + s) * 2];
+            } else {
+                unpack(reinterpret_cast<const float4 *>(area + (k0 + 2 * R::NP) * 64)[j], c);
+            }
+#pragma unroll
+            for (int h = 0; h < N; ++h)
+#pragma unroll
+                for (int s = 0; s < 4; ++s)
+                    y[h][s] = j == 0 ? c[s] * r[h].sg[i][0]
+                                     : fmaf(c[s], r[h].sg[i][j], y[h][s]);
+        }
+#pragma unroll
+        for (int h = 0; h < N; ++h)
+#pragma unroll
+            for (int s = 0; s < 4; ++s) r[h].sg[i][s] = y[h][s];
+    }
+}
+template <int KT, int G, int N>
+__device__ __forceinline__ void apply_p(const unsigned char *area, unsigned k0,
+                                        Rows<double, KT, G> (&r)[N]) {
+#pragma unroll
+    for (int k = 0; k < KT; ++k) {
+        const double2 *P = reinterpret_cast<const double2 *>(area) + (k0 + k) * 8;
+        double y[N][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const double2 a = P[2 * i], b = P[2 * i + 1];
+#pragma unroll
+            for (int h = 0; h < N; ++h) {
+                const double *x = r[h].v[k];
+                y[h][i] = fma(b.y, x[3], fma(b.x, x[2], fma(a.y, x[1], a.x * x[0])));
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < N; ++h)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) r[h].v[k][i] = y[h][i];
+    }
+}
+
+// The message of a leaf child with state mask m: r = it, or r *= it.  FP32:
+// from the table in the record at `area`; FP64: from table `tab` of `ltab`.
+template <bool MUL, int KT, int G>
+__device__ __forceinline__ void leaf_message(const unsigned char *area, unsigned,
+                                             const double *, unsigned m, unsigned k0,
+                                             Rows<float, KT, G> &r) {
+    typedef Rows<float, KT, G> R;
+#pragma unroll
+    for (int i = 0; i < R::NP; ++i) {
+        const pairs *t = reinterpret_cast<const pairs *>(area + (k0 / 2 + i) * 512) + m;
+        const pairs a = t[0], b = t[16];
+        const f32x2 c[4] = {a.x, a.y, b.x, b.y};
+#pragma unroll
+        for (int s = 0; s < 4; ++s) r.pr[i][s] = MUL ? mul2(r.pr[i][s], c[s]) : c[s];
+    }
+#pragma unroll
+    for (int i = 0; i < R::NS; ++i) {
+        float c[4];
+        if (R::split) {
+            const unsigned k = k0 + i;
+            const float *f =
+                reinterpret_cast<const float *>(area + (k / 2) * 512) + m * 4 + (k & 1u);
+#pragma unroll
+            for (int s = 0; s < 4; ++s) c[s] = f[(s >> 1) * 64 + (s & 1) * 2];
+        } else {
+            unpack(reinterpret_cast<const float4 *>(area + (k0 + 2 * R::NP) * 256)[m], c);
+        }
+#pragma unroll
+        for (int s = 0; s < 4; ++s) r.sg[i][s] = MUL ? r.sg[i][s] * c[s] : c[s];
+    }
+}
+template <bool MUL, int KT, int G>
+__device__ __forceinline__ void leaf_message(const unsigned char *, unsigned tab,
+                                             const double *ltab, unsigned m, unsigned k0,
+                                             Rows<double, KT, G> &r) {
+    const double2 *t =
+        reinterpret_cast<const double2 *>(ltab + (((size_t)tab * 16 + m) * (KT * G) + k0) * 4);
+#pragma unroll
+    for (int k = 0; k < KT; ++k) {
+        const double2 a = __ldg(t + 2 * k), b = __ldg(t + 2 * k + 1);
+        r.v[k][0] = MUL ? r.v[k][0] * a.x : a.x;
+        r.v[k][1] = MUL ? r.v[k][1] * a.y : a.y;
+        r.v[k][2] = MUL ? r.v[k][2] * b.x : b.x;
+        r.v[k][3] = MUL ? r.v[k][3] * b.y : b.y;
+    }
+}
 
 // Max over the G consecutive lanes that share a pattern.
 template <int G, typename X>
@@ -813,51 +842,40 @@ __device__ __forceinline__ X group_max(X x) {
 // Rescale a pattern's rows by an exact power of two when their largest
 // entry has fallen low.
 //
-// FP32: below 2^-16 (or after a product of more than two messages): to
-// [0.5, 1), the exponent added to the integer scaler.  Every entry is at
-// most 1, a binary op's result then keeps its largest entry far above the
-// FP32 normal range's floor, and the scaling is exact, so a rescale that is
-// skipped changes no mantissa.
+// FP32: when the largest entry of any pattern of the warp has left
+// [2^-16, 2^44), every pattern of it goes to [2^19, 2^20), the exponent added
+// to the integer scaler.  So a warp's patterns fall together and it
+// rescales about once in ten ops; pattern by pattern, at below 2^-16 to
+// [0.5, 1), nearly every op had some lane in the branch.  P has entries of
+// at most 1, so a product of two rows stays far inside the FP32 range, the
+// scaling is exact, and a rescale sooner or later changes no mantissa: the
+// root takes rows and exponent together.  Called by whole warps.
 template <int KT, int G>
-__device__ __forceinline__ void rescale(Rows<float, KT> &r, int &lns, bool always) {
-    const float mx = group_max<G>(rows_max(r));
-    if (!(mx > 0.0f && mx <= 3.0e38f && (always || mx < 1.52587890625e-05f))) return;
-    const int e0 = __float_as_int(mx) >> 23;  // biased exponent (0: subnormal)
-    if (e0 >= 1 && e0 <= 252) {
-        // 2^n with n = 126 - e0: the exponent frexp gives is e0 - 126.
-        const float s = __int_as_float((253 - e0) << 23);
-        const f32x2 ss = pack2f(s, s);
-#pragma unroll
-        for (int k = 0; k < KT; ++k) {
-            r.q[k].v[0] = mul2(r.q[k].v[0], ss);
-            r.q[k].v[1] = mul2(r.q[k].v[1], ss);
-        }
-        lns += e0 - 126;
-        return;
-    }
+__device__ __forceinline__ void rescale(Rows<float, KT, G> &r, int &lns, bool always) {
+    constexpr uint32_t kLow = (127 - 16) << 23, kHigh = (127 + 44) << 23;
+    const float mx = group_max<G>(r.top());
+    if (!__any_sync(0xffffffffu, (__float_as_uint(mx) - kLow >= kHigh - kLow) | always)) return;
+    if (!(mx > 0.0f && mx <= 3.0e38f)) return;
     int e;
     frexpf(mx, &e);
-    const int n = -e, n1 = n / 2, n2 = n - n1;
-    const f32x2 s1 = pack2f(pow2f(n1), pow2f(n1)), s2 = pack2f(pow2f(n2), pow2f(n2));
-#pragma unroll
-    for (int k = 0; k < KT; ++k) {
-        r.q[k].v[0] = mul2(mul2(r.q[k].v[0], s1), s2);
-        r.q[k].v[1] = mul2(mul2(r.q[k].v[1], s1), s2);
-    }
-    lns += e;
+    const int n = 20 - e;
+    r.scale(pow2f(n < 127 ? n : 127));
+    if (n > 127) r.scale(pow2f(n - 127));
+    lns -= n;
 }
-// FP64: below 2^-256 (or at 2^256), to [1, 2), and its exponent times ln 2 joins the log
-// scaler.  The reference divides by the largest child message and adds its
-// log on every op (CxLik.c:390-403, 577-588); the product of rows and scale
-// is the same, the power of two is exact, and the FP64 pipe, which bounds
-// this form, is spared a reciprocal, 4 K products and a log per op (134 to
-// about 80 FP64 instructions per update).  Two children at or above 2^-256
-// give products far above the normal range's floor.  Rows of zeros stay, and
-// a pattern with an infinite entry ends with NaN rows, as dividing by an
-// infinite scaler leaves it: its site lnL is -inf either way.
+// FP64: below 2^-256 (or at 2^256), to [1, 2), and its exponent times ln 2
+// joins the log scaler.  The reference divides by the largest child message
+// and adds its log on every op (CxLik.c:390-403, 577-588); the product of
+// rows and scale is the same, the power of two is exact, and the FP64 pipe,
+// which bounds this form, is spared a reciprocal, 4 K products and a log per
+// op (134 to about 80 FP64 instructions per update).  Two children at or
+// above 2^-256 give products far above the normal range's floor.  Rows of
+// zeros stay zeros, and a pattern with an infinite entry ends with NaN rows,
+// as dividing by an infinite scaler leaves it: its site lnL is -inf either
+// way.
 template <int KT, int G>
-__device__ __forceinline__ void rescale(Rows<double, KT> &r, double &lns, bool) {
-    const int hi = group_max<G>(rows_max(r));
+__device__ __forceinline__ void rescale(Rows<double, KT, G> &r, double &lns, bool) {
+    const int hi = group_max<G>(r.top());
     constexpr int kLow = (1023 - 256) << 20, kHigh = (1023 + 256) << 20;
     if (hi >= kLow && hi < kHigh) return;
     double s;
@@ -872,13 +890,19 @@ __device__ __forceinline__ void rescale(Rows<double, KT> &r, double &lns, bool) 
         s = __hiloint2double((1023 - e) << 20, 0);
         lns = fma((double)e, 0.69314718055994530942, lns);
     }
-#pragma unroll
-    for (int k = 0; k < KT; ++k)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) r.q[k].v[i] *= s;
+    r.scale(s);
 }
 
-// A warp's view of the tile it walks.
+// ln(L 2^e): the exponent of L joins e, so that the sum does not depend on
+// how rows and scaler shared it.
+__device__ __forceinline__ double site_log(double L, int e) {
+    int f;
+    const double m = frexp(L, &f);
+    return log(m) + (double)(e + f) * 0.69314718055994530942;
+}
+
+// A thread's view of the tile it walks: N patterns `nthr` apart (G = 1), the
+// first at pl in the tile and p in the CL buffers.
 template <typename T>
 struct TileView {
     typedef typename Prec<T>::V V;
@@ -886,70 +910,61 @@ struct TileView {
     V *slots;
     S *slot_sc;
     const double *ltab;  // FP64: leaf-message tables
-    size_t ppad;
+    uint32_t pitch;      // bytes between a CL's units
     unsigned tile, pl, p, k0;
 };
 
 // An internal child's rows and scaler: from its stack slot, or from HBM
 // through L2 (rows this same thread wrote earlier in the walk, or an
 // earlier launch did).  `cr` is the child's descriptor in the record.
-template <typename T, int KT, int G>
-__device__ __forceinline__ typename Prec<T>::S child_rows(const unsigned char *cr,
-                                                          const TileView<T> &w,
-                                                          Rows<T, KT> &x) {
+template <typename T, int KT, int G, int N>
+__device__ __forceinline__ void child_rows(const unsigned char *cr, const TileView<T> &w,
+                                           Rows<T, KT, G> (&x)[N],
+                                           typename Prec<T>::S (&l)[N]) {
     typedef typename Prec<T>::V V;
     typedef typename Prec<T>::S S;
-    constexpr int U = Prec<T>::U;
-    const RecChild *c = reinterpret_cast<const RecChild *>(cr);
+    constexpr unsigned U = Prec<T>::U;
     const ulonglong2 ptr = *reinterpret_cast<const ulonglong2 *>(cr);
-    const uint2 si = *reinterpret_cast<const uint2 *>(&c->src);
+    const uint2 si = *reinterpret_cast<const uint2 *>(cr + 16);  // src, idx
+    const unsigned step = w.tile / N;
     if (si.x == SRC_SLOT) {
-        load_smem<KT>(w.slots + (si.y * (KT * G) + w.k0) * U * w.tile + w.pl, w.tile, x);
-        return w.slot_sc[si.y * w.tile + w.pl];
+        const V *q = w.slots + si.y * (KT * G * U) * w.tile + w.pl;
+#pragma unroll
+        for (int h = 0; h < N; ++h) {
+            x[h].load_smem(q + h * step, w.tile, w.k0);
+            l[h] = w.slot_sc[si.y * w.tile + w.pl + h * step];
+        }
+    } else {
+        const uint64_t q = addr_at(ptr.x, w.p, sizeof(V)), ql = addr_at(ptr.y, w.p, sizeof(S));
+#pragma unroll
+        for (int h = 0; h < N; ++h) {
+            x[h].load_l2(q + h * step * sizeof(V), w.pitch, w.k0);
+            l[h] = __ldcg(reinterpret_cast<const S *>(ql + h * step * sizeof(S)));
+        }
     }
-    load_l2<KT>(reinterpret_cast<const V *>(ptr.x) + (size_t)w.k0 * U * w.ppad + w.p, w.ppad, x);
-    return __ldcg(reinterpret_cast<const S *>(ptr.y) + w.p);
-}
-
-// Component k (of this thread's) of the message of a leaf child with state
-// mask m.  FP32: from the table in the record at `area`; FP64: from table
-// `tab` in HBM.
-template <int KA>
-__device__ __forceinline__ Quad<float> leaf_message(const unsigned char *area, unsigned,
-                                                    unsigned m, const TileView<float> &w,
-                                                    int k) {
-    return quad(reinterpret_cast<const float4 *>(area)[(w.k0 + k) * 16 + m]);
-}
-template <int KA>
-__device__ __forceinline__ Quad<double> leaf_message(const unsigned char *, unsigned tab,
-                                                     unsigned m, const TileView<double> &w,
-                                                     int k) {
-    const double2 *t = reinterpret_cast<const double2 *>(
-        w.ltab + (((size_t)tab * 16 + m) * KA + w.k0 + k) * 4);
-    return quad(__ldg(t), __ldg(t + 1));
 }
 
 // One op.  `acc` and `lns` hold the previous op's result on entry and this
 // op's on return; m0 and m1 are the state masks of its first two leaf
-// children, `rows` this pattern's mask of the op's leaf children (one per
-// `tile` bytes).  Two-child ops run the code of their kind (an op's kind and
-// the child that plays A are in its flags), others a loop over children.
+// children, `rows` this pattern's masks of the op's leaf children (one row
+// per `tile` bytes).  Two-child ops run the code of their kind (an op's kind
+// and the child that plays A are in its flags), others a loop over children.
 // The product of two messages and the sum of two scalers are the same in
 // either order, so every path gives the same bits.
-template <typename T, int KT, int G>
-__device__ __forceinline__ void walk_op(const unsigned char *rec, unsigned nchild, uint32_t flags,
-                                        bool first, unsigned m0, unsigned m1,
+template <typename T, int KT, int G, int N>
+__device__ __forceinline__ void walk_op(const unsigned char *rec, uint32_t flags, bool first,
+                                        const unsigned (&m0)[N], const unsigned (&m1)[N],
                                         const uint8_t *rows, const TileView<T> &w,
-                                        Rows<T, KT> &acc, typename Prec<T>::S &lns) {
-    typedef typename Prec<T>::V V;
+                                        Rows<T, KT, G> (&acc)[N],
+                                        typename Prec<T>::S (&lns)[N]) {
     typedef typename Prec<T>::S S;
-    constexpr int KA = KT * G;
-    constexpr unsigned PB = KA * 16 * sizeof(T);                       // bytes of a P area
-    constexpr unsigned LB = sizeof(T) == 4 ? KA * 16 * 4 * 4 : PB;     // of a leaf's area
-    constexpr unsigned PU = 16 * sizeof(T) / 16;                       // P units per component
-    constexpr unsigned A0 = sizeof(RecHead) + 2 * sizeof(RecChild);
-    const unsigned ia = (flags & kOpKindA) ? 1u : 0u;
+    typedef Rows<T, KT, G> R;
+    constexpr unsigned KA = KT * G;
+    constexpr unsigned PB = KA * 16 * sizeof(T);                    // bytes of a P area
+    constexpr unsigned LB = sizeof(T) == 4 ? KA * 16 * 4 * 4 : PB;  // of a leaf's area
     const unsigned char *kid0 = rec + sizeof(RecHead);
+    const unsigned char *area = kid0 + 2 * sizeof(RecChild);
+    const unsigned ia = (flags & kOpKindA) ? 1u : 0u;
     uint32_t kind = (flags >> kOpKindShift) & 7u;
     // A walk that starts inside a plan (one launch per node) holds no
     // previous result.
@@ -957,100 +972,107 @@ __device__ __forceinline__ void walk_op(const unsigned char *rec, unsigned nchil
     auto tab_of = [&](unsigned c) -> unsigned {
         return sizeof(T) == 8 ? reinterpret_cast<const RecChild *>(kid0)[c].tab : 0u;
     };
-    auto pmat = [&](const unsigned char *area) {
-        return reinterpret_cast<const V *>(area) + (size_t)w.k0 * PU;
-    };
     if (kind == OPK_FL || kind == OPK_IL) {
-        const unsigned char *aA = rec + A0 + (ia ? LB : 0u), *aB = rec + A0 + (ia ? 0u : PB);
-        if (kind == OPK_IL) lns = child_rows<T, KT, G>(kid0 + ia * sizeof(RecChild), w, acc);
-        const V *P = pmat(aA);
+        if (kind == OPK_IL)
+            child_rows<T, KT, G, N>(kid0 + ia * sizeof(RecChild), w, acc, lns);
         const unsigned tab = tab_of(ia ^ 1u);
+        apply_p<KT, G, N>(area + (ia ? LB : 0u), w.k0, acc);
 #pragma unroll
-        for (int k = 0; k < KT; ++k)
-            acc.q[k] = matvec(P + k * PU, acc.q[k]) * leaf_message<KA>(aB, tab, m0, w, k);
+        for (int h = 0; h < N; ++h)
+            leaf_message<true, KT, G>(area + (ia ? 0u : PB), tab, w.ltab, m0[h], w.k0, acc[h]);
     } else if (kind == OPK_LL) {
-        lns = S(0);
         const unsigned t0 = tab_of(0), t1 = tab_of(1);
 #pragma unroll
-        for (int k = 0; k < KT; ++k)
-            acc.q[k] = leaf_message<KA>(rec + A0, t0, m0, w, k) *
-                       leaf_message<KA>(rec + A0 + LB, t1, m1, w, k);
+        for (int h = 0; h < N; ++h) {
+            leaf_message<false, KT, G>(area, t0, w.ltab, m0[h], w.k0, acc[h]);
+            leaf_message<true, KT, G>(area + LB, t1, w.ltab, m1[h], w.k0, acc[h]);
+            lns[h] = S(0);
+        }
     } else if (kind == OPK_FI || kind == OPK_II) {
-        const unsigned char *aA = rec + A0 + (ia ? PB : 0u), *aB = rec + A0 + (ia ? 0u : PB);
-        Rows<T, KT> xb;
-        const S lb = child_rows<T, KT, G>(kid0 + (ia ^ 1u) * sizeof(RecChild), w, xb);
-        if (kind == OPK_II) lns = child_rows<T, KT, G>(kid0 + ia * sizeof(RecChild), w, acc);
-        const V *PA = pmat(aA), *PX = pmat(aB);
-        // (The previous result's products come first: the sibling's rows
-        // are on their way from L2.)
+        R xb[N];
+        S lb[N];
+        child_rows<T, KT, G, N>(kid0 + (ia ^ 1u) * sizeof(RecChild), w, xb, lb);
+        if (kind == OPK_II)
+            child_rows<T, KT, G, N>(kid0 + ia * sizeof(RecChild), w, acc, lns);
+        // (A's products come first: B's rows are on their way from L2.)
+        apply_p<KT, G, N>(area + (ia ? PB : 0u), w.k0, acc);
+        apply_p<KT, G, N>(area + (ia ? 0u : PB), w.k0, xb);
 #pragma unroll
-        for (int k = 0; k < KT; ++k) acc.q[k] = matvec(PA + k * PU, acc.q[k]);
-#pragma unroll
-        for (int k = 0; k < KT; ++k) acc.q[k] = acc.q[k] * matvec(PX + k * PU, xb.q[k]);
-        lns = lns + lb;
+        for (int h = 0; h < N; ++h) {
+            acc[h].mul(xb[h]);
+            lns[h] = lns[h] + lb[h];
+        }
     } else {
         // Any number of children, each read from where its record says.
-        lns = S(0);
+        const unsigned nchild = reinterpret_cast<const RecHead *>(rec)->nchild;
         unsigned nl = 0;
 #pragma unroll 1
         for (unsigned ci = 0; ci < nchild; ++ci) {
             const unsigned char *cr = kid0 + ci * sizeof(RecChild);
             const uint4 d = *reinterpret_cast<const uint4 *>(cr + 16);  // src idx tab off
-            Rows<T, KT> x;
+            R x[N];
+            S l[N];
             if (d.x == SRC_LEAF) {
-                const unsigned m = rows[(nl++) * w.tile];
 #pragma unroll
-                for (int k = 0; k < KT; ++k) x.q[k] = leaf_message<KA>(rec + d.w, d.z, m, w, k);
+                for (int h = 0; h < N; ++h) {
+                    const unsigned m = rows[nl * w.tile + h * (w.tile / N)];
+                    leaf_message<false, KT, G>(rec + d.w, d.z, w.ltab, m, w.k0, x[h]);
+                    l[h] = S(0);
+                }
+                ++nl;
             } else {
-                lns = lns + child_rows<T, KT, G>(cr, w, x);
-                const V *P = pmat(rec + d.w);
-#pragma unroll
-                for (int k = 0; k < KT; ++k) x.q[k] = matvec(P + k * PU, x.q[k]);
+                child_rows<T, KT, G, N>(cr, w, x, l);
+                apply_p<KT, G, N>(rec + d.w, w.k0, x);
             }
-            if (ci == 0) {
-                acc = x;
-            } else {
 #pragma unroll
-                for (int k = 0; k < KT; ++k) acc.q[k] = acc.q[k] * x.q[k];
+            for (int h = 0; h < N; ++h) {
+                if (ci == 0) {
+                    acc[h] = x[h];
+                    lns[h] = l[h];
+                } else {
+                    acc[h].mul(x[h]);
+                    lns[h] = lns[h] + l[h];
+                }
+                // A long product stays inside the range.
+                if (ci >= 1 && ci + 1 < nchild) rescale<KT, G>(acc[h], lns[h], true);
             }
-            // (The FP64 form keeps a long product inside the range.)
-            if (sizeof(T) == 8 && ci >= 1 && ci + 1 < nchild) rescale<KT, G>(acc, lns, false);
         }
     }
 }
 
 // Walk every op of job `a` for tile `tile_idx`, aggregate the root and
 // reduce.  G consecutive threads share a pattern, each holding KT of its
-// KT*G components; with G = 1 one thread owns a pattern.  Every G and every
-// tile gives the same bits: scalers are maxima over the group, and the root
-// sum and the tile reduction run in the G = 1 order.  Returns false if a
-// bounded wait gave up.
-template <typename T, int KT, int G>
+// KT*G components; with G = 1 a thread owns N patterns, blockDim apart.
+// Every G, N and tile gives the same bits: scalers are maxima over the
+// group, the root sum runs in one order and the sum over sites in any.
+// Returns false if a bounded wait gave up.
+template <typename T, int KT, int G, int N>
 __device__ bool walk_tile(const PlanArgs &a, unsigned tile_idx, const LeanLayout &Lay,
                           unsigned grp, RingPos &ring) {
+    static_assert(G == 1 || N == 1, "several threads a pattern or several patterns a thread");
     typedef typename Prec<T>::S S;
     typedef typename Prec<T>::V V;
-    constexpr int U = Prec<T>::U;
+    typedef Rows<T, KT, G> R;
     extern __shared__ __align__(128) unsigned char smem[];
     LeanHead &hd = *reinterpret_cast<LeanHead *>(smem);
     const unsigned nthr = blockDim.x, nwarp = nthr / 32;
     const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const unsigned tile = nthr / G;
+    const unsigned tile = nthr / G * N;
     const unsigned p0 = tile_idx * tile;
     const unsigned g = tid % G;
     TileView<T> w;
     w.slots = reinterpret_cast<V *>(smem + Lay.slots);
     w.slot_sc = reinterpret_cast<S *>(smem + Lay.slot_sc);
     w.ltab = a.ltab;
-    w.ppad = a.ppad;
+    w.pitch = a.ppad * 16u;
     w.tile = tile;
     w.pl = tid / G;
     w.p = p0 + w.pl;
     w.k0 = g * KT;
-    const unsigned p = w.p;
     // The last tile of a job may pass its padded patterns by whole warps
-    // (32 / G patterns each, and the padding is to 128).
-    const bool on = p < a.ppad;
+    // (32 / G patterns each, and the padding is to 128); a tile of the
+    // two-pattern walker divides them.
+    const bool on = w.p < a.ppad;
     const unsigned rowb = min(tile, a.ppad - p0);
     const unsigned ngrp = (a.nops + grp - 1) / grp;
     const unsigned lmax = a.lmax;
@@ -1069,8 +1091,8 @@ __device__ bool walk_tile(const PlanArgs &a, unsigned tile_idx, const LeanLayout
         if (lane == 0) hd.issued = n;
     }
 
-    Rows<T, KT> acc;
-    S lns = S(0);
+    R acc[N];
+    S lns[N];
     bool ok = true;
     for (unsigned q = 0; q < ngrp; ++q) {
         unsigned char *st = smem + Lay.stage0 + ring.stage * Lay.stage;
@@ -1093,42 +1115,71 @@ __device__ bool walk_tile(const PlanArgs &a, unsigned tile_idx, const LeanLayout
             const unsigned n = min(grp, a.nops - q * grp);
             const unsigned char *rec = st;
             const uint8_t *rows = st + (size_t)grp * a.rstride + w.pl;
-            // The first record's header and masks; then each op reads the
-            // next one's ahead.
-            ulonglong2 h0 = *reinterpret_cast<const ulonglong2 *>(rec);
-            uint4 h1 = *reinterpret_cast<const uint4 *>(rec + 16);
-            unsigned m0 = lmax > 0 ? rows[0] : 0u, m1 = lmax > 1 ? rows[tile] : 0u;
+            // What an op needs from its header, and its first two leaf
+            // children's masks, are read while the op before it runs (past
+            // a group's last op the words read are not used).
+            uint64_t y, ysc;
+            uint32_t word;
+            unsigned m0[N], m1[N];
+            auto head = [&](const unsigned char *r, uint64_t &hy, uint64_t &hs, uint32_t &hw) {
+                const ulonglong2 h0 = *reinterpret_cast<const ulonglong2 *>(r);
+                const uint4 h1 = *reinterpret_cast<const uint4 *>(r + 16);
+                hy = addr_at(h0.x, w.p, sizeof(V));
+                hs = addr_at(h0.y, w.p, sizeof(S));
+                // (In a uniform register: the branches on it are the warp's.)
+                hw = __reduce_or_sync(0xffffffffu, h1.z | (h1.y + 1u) << kSlotShift);
+            };
+            auto masks = [&](const uint8_t *rw, unsigned (&a0)[N], unsigned (&a1)[N]) {
+#pragma unroll
+                for (int h = 0; h < N; ++h) {
+                    a0[h] = rw[h * nthr];
+                    a1[h] = rw[tile + h * nthr];
+                }
+            };
+            head(rec, y, ysc, word);
+            masks(rows, m0, m1);
             for (unsigned b = 0; b < n; ++b) {
-                const unsigned char *nrec = rec + a.rstride;
-                const uint8_t *nrows = rows + (size_t)lmax * tile;
-                ulonglong2 n0 = h0;
-                uint4 n1 = h1;
-                unsigned nm0 = 0u, nm1 = 0u;
-                if (b + 1 < n) {
-                    n0 = *reinterpret_cast<const ulonglong2 *>(nrec);
-                    n1 = *reinterpret_cast<const uint4 *>(nrec + 16);
-                    if (lmax > 0) nm0 = nrows[0];
-                    if (lmax > 1) nm1 = nrows[tile];
-                }
-                walk_op<T, KT, G>(rec, h1.x, h1.z, (q | b) == 0u, m0, m1, rows, w, acc, lns);
-                rescale<KT, G>(acc, lns, h1.x > 2u);
-                if (!(h1.z & REC_NO_HBM)) {
-                    store_rows<KT>(reinterpret_cast<V *>(h0.x) + (size_t)w.k0 * U * w.ppad + p,
-                                   w.ppad, acc);
-                    if (g == 0) reinterpret_cast<S *>(h0.y)[p] = lns;
-                }
-                if ((int)h1.y >= 0) {
-                    store_rows<KT>(w.slots + (h1.y * (KT * G) + w.k0) * U * tile + w.pl, tile,
-                                   acc);
-                    if (g == 0) w.slot_sc[h1.y * tile + w.pl] = lns;
+                walk_op<T, KT, G, N>(rec, word, (q | b) == 0u, m0, m1, rows, w, acc, lns);
+                rec += a.rstride;
+                rows += lmax * tile;
+                uint64_t ny, nysc;
+                uint32_t nword;
+                unsigned nm0[N], nm1[N];
+                head(rec, ny, nysc, nword);
+                masks(rows, nm0, nm1);
+#pragma unroll
+                for (int h = 0; h < N; ++h) rescale<KT, G>(acc[h], lns[h], false);
+                if ((word & kPlainMask) == 0) {
+#pragma unroll
+                    for (int h = 0; h < N; ++h) {
+                        acc[h].store_global(y + h * nthr * sizeof(V), w.pitch, w.k0);
+                        if (g == 0) st_global(ysc + h * nthr * sizeof(S), lns[h]);
+                    }
+                } else {
+                    const unsigned slot = word >> kSlotShift;
+#pragma unroll
+                    for (int h = 0; h < N; ++h) {
+                        if (!(word & REC_NO_HBM)) {
+                            acc[h].store_global(y + h * nthr * sizeof(V), w.pitch, w.k0);
+                            if (g == 0) st_global(ysc + h * nthr * sizeof(S), lns[h]);
+                        }
+                        if (slot != 0) {
+                            const unsigned at = (slot - 1) * tile, q0 = w.pl + h * nthr;
+                            acc[h].store_smem(w.slots + at * (KT * G * Prec<T>::U) + q0, tile,
+                                              w.k0);
+                            if (g == 0) w.slot_sc[at + q0] = lns[h];
+                        }
+                    }
                 }
                 if (G > 1) __syncwarp();  // lane g = 0's scaler is read by the group
-                rec = nrec;
-                rows = nrows;
-                h0 = n0;
-                h1 = n1;
-                m0 = nm0;
-                m1 = nm1;
+                y = ny;
+                ysc = nysc;
+                word = nword;
+#pragma unroll
+                for (int h = 0; h < N; ++h) {
+                    m0[h] = nm0[h];
+                    m1[h] = nm1[h];
+                }
             }
         }
         if (refill) {
@@ -1163,55 +1214,47 @@ __device__ bool walk_tile(const PlanArgs &a, unsigned tile_idx, const LeanLayout
     }
 
     if (a.no_root) return true;
-    // Root aggregation (CxLik.c:598-632): L = sum_k sum_i pn[k][i] root.
-    if (!a.root_last && on) {
-        load_l2<KT>(static_cast<const V *>(a.root) + (size_t)w.k0 * U * w.ppad + p, w.ppad, acc);
-        lns = static_cast<const S *>(a.rootsc)[p];
-    }
-    T x[KT * 4];
+    double v[N];
+    bool ninf[N];
 #pragma unroll
-    for (int k = 0; k < KT; ++k) unquad(acc.q[k], x + 4 * k);
-    // Lsum = sum over components and states in one sequential order; every
-    // lane of the group gathers the others' entries and sums them all.
-    double Lsum = 0.0;
-    const unsigned lead = lane - g;
+    for (int h = 0; h < N; ++h) {
+        const unsigned p = w.p + h * nthr;
+        // Root aggregation (CxLik.c:598-632): L = sum_k sum_i pn[k][i] root.
+        if (!a.root_last && on) {
+            acc[h].load_l2(addr_at(reinterpret_cast<uint64_t>(a.root), p, sizeof(V)), w.pitch,
+                           w.k0);
+            lns[h] = static_cast<const S *>(a.rootsc)[p];
+        }
+        // L = sum over components and states in one sequential order; every
+        // lane of the group gathers the others' entries and sums them all.
+        double L = 0.0;
+        const unsigned lead = lane - g;
 #pragma unroll
-    for (int gg = 0; gg < G; ++gg) {
+        for (int gg = 0; gg < G; ++gg) {
 #pragma unroll
-        for (int q = 0; q < KT * 4; ++q) {
-            const T y = G > 1 ? __shfl_sync(0xffffffffu, x[q], lead + gg) : x[q];
-            Lsum = fma(__ldg(a.pn + gg * KT * 4 + q), (double)y, Lsum);
+            for (int i = 0; i < KT * 4; ++i) {
+                T x = acc[h].get(i / 4, i % 4);
+                if (G > 1) x = __shfl_sync(0xffffffffu, x, lead + gg);
+                L = fma(__ldg(a.pn + gg * KT * 4 + i), (double)x, L);
+            }
+        }
+        v[h] = 0.0;
+        ninf[h] = false;
+        if (g == 0 && p < a.npat) {
+            v[h] = (sizeof(T) == 8 ? log(L) + (double)lns[h] : site_log(L, (int)lns[h])) *
+                   (double)a.freqs[p];
+            if (isnan(v[h])) v[h] = -INFINITY;
+            if (a.site) a.site[p] = v[h];
+            if (isinf(v[h])) {
+                ninf[h] = (v[h] < 0.0);
+                v[h] = 0.0;
+            }
         }
     }
-    double v = 0.0;
-    bool ninf = false;
-    if (g == 0 && p < a.npat) {
-        const double lsc = (sizeof(T) == 8) ? (double)lns
-                                           : (double)lns * 0.69314718055994530942;
-        v = (log(Lsum) + lsc) * (double)a.freqs[p];
-        if (isnan(v)) v = -INFINITY;
-        if (a.site) a.site[p] = v;
-        if (isinf(v)) {
-            ninf = (v < 0.0);
-            v = 0.0;
-        }
-    }
-    if (G > 1) {
-        // Pattern pl's value moves to thread pl, so the tile reduces in the
-        // one-thread-per-pattern order (the extra threads add exact zeros).
-        __shared__ double s_v[kBlock];
-        __shared__ unsigned char s_inf[kBlock];
-        if (g == 0) {
-            s_v[w.pl] = v;
-            s_inf[w.pl] = ninf;
-        }
-        __syncthreads();
-        v = tid < tile ? s_v[tid] : 0.0;
-        ninf = tid < tile ? s_inf[tid] != 0 : false;
-    }
-    reduce_sites(a, tile_idx, v, ninf);
+    reduce_sites<N>(a, v, ninf);
     return true;
 }
+
 // The walker with two op lanes (FP32, one thread per pattern, staged
 // leaves): the CTA is two groups of `tile` threads over the same patterns.
 // The host schedules the plan in steps of two mutually independent ops (a
@@ -1225,7 +1268,6 @@ __device__ bool walk_tile(const PlanArgs &a, unsigned tile_idx, const LeanLayout
 template <int KT>
 __device__ bool walk_tile_lanes(const PlanArgs &a, unsigned tile_idx, const SmemLayout &Lay,
                                 unsigned ring_depth, uint32_t &phase) {
-    typedef float T;
     constexpr unsigned L = 2;
     extern __shared__ __align__(128) unsigned char smem[];
     const unsigned nthr = blockDim.x;
@@ -1234,21 +1276,20 @@ __device__ bool walk_tile_lanes(const PlanArgs &a, unsigned tile_idx, const Smem
     const unsigned lane = tid / tile;  // op lane of this thread
     const unsigned pl = tid % tile;    // pattern within the tile
     const unsigned p = tile_idx * tile + pl;
-    const size_t ppad = a.ppad;
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + Lay.bars);
     unsigned char *ring = smem + Lay.ring;
     float4 *slots = reinterpret_cast<float4 *>(smem + Lay.slots);
     int *slot_sc = reinterpret_cast<int *>(smem + Lay.slot_sc);
     const size_t sstride = (size_t)a.rstride * L;
     uint8_t *masks = smem + Lay.masks;
-    const unsigned R = ring_depth;
+    const unsigned R_ = ring_depth;
     const unsigned nsteps = a.nops / L;  // the host pads nops to a multiple
 
     pdl_wait();  // the records hold the P kernel's matrices
     // Start streaming the job's first R steps of op records.
     if (tid == 0) {
         fence_proxy_async();
-        for (unsigned o = 0; o < R && o < nsteps; ++o) {
+        for (unsigned o = 0; o < R_ && o < nsteps; ++o) {
             mbar_expect_tx(&bars[o], (uint32_t)sstride);
             bulk_g2s(ring + (size_t)o * sstride, a.rec + (size_t)o * sstride,
                      (uint32_t)sstride, &bars[o]);
@@ -1264,11 +1305,13 @@ __device__ bool walk_tile_lanes(const PlanArgs &a, unsigned tile_idx, const Smem
     }
     __syncthreads();
 
-    T acc[KT * 4];
-    int lns = 0;
+    typedef Rows<float, KT, 1> R;
+    R acc[1];
+    int lns[1] = {0};
+    const TileView<float> w{slots, slot_sc, nullptr, a.ppad * 16u, tile, pl, p, 0u};
     const uint32_t spin = g_spin_limit;
     for (unsigned o = 0, stage = 0; o < nsteps;
-         ++o, stage = (stage + 1 == R) ? 0u : stage + 1) {
+         ++o, stage = (stage + 1 == R_) ? 0u : stage + 1) {
         // Every thread waits for the step's records itself (one block
         // barrier per step, the hand-off below); a warp computes only if all
         // its threads saw the records arrive.
@@ -1286,58 +1329,42 @@ __device__ bool walk_tile_lanes(const PlanArgs &a, unsigned tile_idx, const Smem
             const RecHead *hd = reinterpret_cast<const RecHead *>(rec);
             const RecChild *kids = reinterpret_cast<const RecChild *>(rec + sizeof(RecHead));
             nchild = hd->nchild;
-            lns = 0;
-            // A child's inputs: its state rows (internal) with its scaler, or
-            // its leaf's state mask.  Loading them is split from computing
-            // the message so that an op with two children issues both
-            // children's loads before it waits on either.
-            struct In {
-                T x[KT * 4];
-                int l;
-                unsigned m;
+            // A child's message: the rows of an internal child (a leaf has
+            // none) are loaded first, so that an op with two children issues
+            // both children's loads before it waits on either.
+            auto load_in = [&](unsigned c, R (&x)[1], int (&l)[1]) {
+                l[0] = 0;
+                if (kids[c].src != SRC_LEAF)
+                    child_rows<float, KT, 1, 1>(reinterpret_cast<const unsigned char *>(kids + c),
+                                                w, x, l);
             };
-            auto load_in = [&](const RecChild &ch, In &in) {
-                in.m = 0u;
-                if (ch.src == SRC_LEAF)
-                    in.m = masks[(size_t)ch.idx * tile + pl];
+            auto message = [&](unsigned c, R (&x)[1]) {
+                if (kids[c].src == SRC_LEAF)
+                    leaf_message<false, KT, 1>(rec + kids[c].off, 0u, nullptr,
+                                               masks[(size_t)kids[c].idx * tile + pl], 0u, x[0]);
                 else
-                    in.l = load_internal<KT>(ch, slots, slot_sc, tile, pl, p, ppad, in.x);
+                    apply_p<KT, 1, 1>(rec + kids[c].off, 0u, x);
             };
-            auto message = [&](const RecChild &ch, const In &in, T *msg) {
-                const float4 *P = reinterpret_cast<const float4 *>(rec + ch.off);
-#pragma unroll
-                for (int k = 0; k < KT; ++k) {
-                    if (ch.src == SRC_LEAF) {
-                        unpack(P[k * 16 + in.m], msg + 4 * k);
-                    } else {
-                        const float4 c[4] = {P[k * 4], P[k * 4 + 1], P[k * 4 + 2],
-                                             P[k * 4 + 3]};
-                        pcol(c, in.x + 4 * k, msg + 4 * k);
-                    }
-                }
-            };
-            auto fold = [&](unsigned ci, const RecChild &ch, const In &in, const T *msg) {
-                if (ch.src != SRC_LEAF) lns = lns + in.l;
-#pragma unroll
-                for (int q = 0; q < KT * 4; ++q) acc[q] = ci == 0 ? msg[q] : acc[q] * msg[q];
-            };
-            T msg[KT * 4];
+            R x[1];
+            int l[1];
             if (nchild == 2) {
-                const RecChild c0 = kids[0], c1 = kids[1];
-                In in0, in1;
-                load_in(c0, in0);
-                load_in(c1, in1);
-                message(c0, in0, msg);
-                fold(0, c0, in0, msg);
-                message(c1, in1, msg);
-                fold(1, c1, in1, msg);
+                load_in(0, acc, lns);
+                load_in(1, x, l);
+                message(0, acc);
+                message(1, x);
+                acc[0].mul(x[0]);
+                lns[0] += l[0];
             } else {
                 for (unsigned ci = 0; ci < nchild; ++ci) {
-                    const RecChild ch = kids[ci];
-                    In in;
-                    load_in(ch, in);
-                    message(ch, in, msg);
-                    fold(ci, ch, in, msg);
+                    load_in(ci, x, l);
+                    message(ci, x);
+                    if (ci == 0) {
+                        acc[0] = x[0];
+                        lns[0] = l[0];
+                    } else {
+                        acc[0].mul(x[0]);
+                        lns[0] += l[0];
+                    }
                 }
             }
             ydata = hd->data;
@@ -1345,47 +1372,36 @@ __device__ bool walk_tile_lanes(const PlanArgs &a, unsigned tile_idx, const Smem
             yslot = hd->slot;
             yhbm = !(hd->flags & REC_NO_HBM);
         }
-        // Every thread has read the stage: hand it to step o + R.  A record
+        // Every thread has read the stage: hand it to the step a ring on.  A record
         // wait that gave up in any warp ends the tile for all: thread 0
         // waits for the copies still in flight into the ring.
         if (!cta_hand_off(ok, nthr)) {
             if (tid == 0) {
                 atomicOr(a.err, 1u);
-                drain_ring(bars, phase ^ (1u << stage), o, nsteps, R);
+                drain_ring(bars, phase ^ (1u << stage), o, nsteps, R_);
             }
             return false;
         }
-        if (tid == 0 && o + R < nsteps) {
+        if (tid == 0 && o + R_ < nsteps) {
             fence_proxy_async();
             mbar_expect_tx(&bars[stage], (uint32_t)sstride);
-            bulk_g2s(ring + (size_t)stage * sstride, a.rec + (size_t)(o + R) * sstride,
+            bulk_g2s(ring + (size_t)stage * sstride, a.rec + (size_t)(o + R_) * sstride,
                      (uint32_t)sstride, &bars[stage]);
         }
-        // An empty lane of a step (no children) computes and stores nothing.
-        if (nchild == 0) continue;
-        const T mx = fmax(T(0), tree_max<KT * 4>(acc));
-        // The rescale rule of walk_tile (same bits).
-        if (mx > T(0) && mx <= (T)3.0e38 && (nchild > 2 || mx < (T)1.52587890625e-05f)) {
-            int e;
-            frexpf(mx, &e);
-            const int n = -e, n1 = n / 2, n2 = n - n1;
-            const float s1 = pow2f(n1), s2 = pow2f(n2);
-#pragma unroll
-            for (int q = 0; q < KT * 4; ++q) acc[q] = (acc[q] * s1) * s2;
-            lns = lns + e;
+        // (An empty lane of a step, with no children, stores nothing.)
+        if (nchild != 0) {
+            rescale<KT, 1>(acc[0], lns[0], nchild > 2);
+            if (yhbm) {
+                acc[0].store_global(reinterpret_cast<uint64_t>(static_cast<float4 *>(ydata) + p),
+                                    w.pitch, 0u);
+                static_cast<int *>(yscaler)[p] = lns[0];
+            }
+            if (yslot >= 0) {
+                acc[0].store_smem(slots + (unsigned)yslot * KT * tile + pl, tile, 0u);
+                slot_sc[(unsigned)yslot * tile + pl] = lns[0];
+            }
         }
-        if (yhbm) {
-            float4 *y = static_cast<float4 *>(ydata) + p;
-#pragma unroll
-            for (int k = 0; k < KT; ++k) y[(size_t)k * ppad] = pack4(acc + k * 4);
-            static_cast<int *>(yscaler)[p] = lns;
-        }
-        if (yslot >= 0) {
-            float4 *ys = slots + (size_t)yslot * KT * tile + pl;
-#pragma unroll
-            for (int k = 0; k < KT; ++k) ys[(size_t)k * tile] = pack4(acc + k * 4);
-            slot_sc[(size_t)yslot * tile + pl] = lns;
-        }
+        __syncthreads();  // the other lane may read these results next step
     }
 
     if (a.no_root) {
@@ -1394,260 +1410,26 @@ __device__ bool walk_tile_lanes(const PlanArgs &a, unsigned tile_idx, const Smem
     }
     // Root aggregation (CxLik.c:598-632), lane 0's.
     if (!a.root_last) {
-        const float4 *r = static_cast<const float4 *>(a.root) + p;
-#pragma unroll
-        for (int k = 0; k < KT; ++k) unpack(r[(size_t)k * ppad], acc + k * 4);
-        lns = static_cast<const int *>(a.rootsc)[p];
+        acc[0].load_l2(reinterpret_cast<uint64_t>(static_cast<const float4 *>(a.root) + p),
+                       w.pitch, 0u);
+        lns[0] = static_cast<const int *>(a.rootsc)[p];
     }
     double Lsum = 0.0;
 #pragma unroll
-    for (int q = 0; q < KT * 4; ++q) Lsum = fma(__ldg(a.pn + q), (double)acc[q], Lsum);
-    double v = 0.0;
-    bool ninf = false;
+    for (int q = 0; q < KT * 4; ++q)
+        Lsum = fma(__ldg(a.pn + q), (double)acc[0].get(q / 4, q % 4), Lsum);
+    double v[1] = {0.0};
+    bool ninf[1] = {false};
     if (lane == 0 && p < a.npat) {
-        v = (log(Lsum) + (double)lns * 0.69314718055994530942) * (double)a.freqs[p];
-        if (isnan(v)) v = -INFINITY;
-        if (a.site) a.site[p] = v;
-        if (isinf(v)) {
-            ninf = (v < 0.0);
-            v = 0.0;
+        v[0] = site_log(Lsum, lns[0]) * (double)a.freqs[p];
+        if (isnan(v[0])) v[0] = -INFINITY;
+        if (a.site) a.site[p] = v[0];
+        if (isinf(v[0])) {
+            ninf[0] = (v[0] < 0.0);
+            v[0] = 0.0;
         }
     }
-    reduce_sites(a, tile_idx, v, ninf);
-    return true;
-}
-
-// The FP32 walker with two patterns per thread (one thread per pattern
-// pair, components not split): thread t owns patterns t and t + blockDim
-// of the tile, so loads stay coalesced, and every P row, record field and
-// loop step serves both.  The arithmetic of each pattern is that of
-// walk_tile<float, K, 1, STAGED>, and the tile reduction runs in its order,
-// so the bits are the same.
-template <int K, bool STAGED>
-__device__ bool walk_tile2(const PlanArgs &a, unsigned tile_idx, const SmemLayout &Lay,
-                           unsigned ring_depth, uint32_t &phase) {
-    typedef float T;
-    extern __shared__ __align__(128) unsigned char smem[];
-    const unsigned nthr = blockDim.x;
-    const unsigned tile = 2 * nthr;
-    const unsigned tid = threadIdx.x;
-    const unsigned pl[2] = {tid, tid + nthr};
-    const unsigned p[2] = {tile_idx * tile + tid, tile_idx * tile + tid + nthr};
-    const size_t ppad = a.ppad;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + Lay.bars);
-    unsigned char *ring = smem + Lay.ring;
-    float4 *slots = reinterpret_cast<float4 *>(smem + Lay.slots);
-    int *slot_sc = reinterpret_cast<int *>(smem + Lay.slot_sc);
-    const size_t sstride = STAGED ? (size_t)a.rstride : Lay.stage;
-    uint8_t *masks = smem + Lay.masks;
-    const unsigned R = ring_depth;
-
-    if (STAGED) {
-        pdl_wait();
-        if (tid == 0) {
-            fence_proxy_async();
-            for (unsigned o = 0; o < R && o < a.nops; ++o) {
-                mbar_expect_tx(&bars[o], a.rstride);
-                bulk_g2s(ring + (size_t)o * a.rstride, a.rec + (size_t)o * a.rstride,
-                         a.rstride, &bars[o]);
-            }
-        }
-        const unsigned chunks = tile / 16;
-        for (unsigned i = tid; i < a.nleaf * chunks; i += nthr) {
-            const unsigned l = i / chunks, c = i % chunks;
-            const uint4 *src =
-                reinterpret_cast<const uint4 *>(a.leaves[l] + (size_t)tile_idx * tile) + c;
-            reinterpret_cast<uint4 *>(masks + (size_t)l * tile)[c] = __ldg(src);
-        }
-        __syncthreads();
-    } else {
-        pdl_wait();
-        if (tid == 0)
-            for (unsigned o = 0; o < R && o < a.nops; ++o) {
-                const uint8_t *rows0[kLeafPre];
-                read_rows(a, o, rows0);
-                issue_stage(a, o, ring + (size_t)o * sstride, &bars[o], tile_idx, tile, rows0);
-            }
-    }
-
-    T acc[2][K * 4];
-    int lns[2] = {0, 0};
-    const uint32_t spin = g_spin_limit;
-    for (unsigned o = 0, stage = 0; o < a.nops;
-         ++o, stage = (stage + 1 == R) ? 0u : stage + 1) {
-        const uint8_t *pre[kLeafPre] = {nullptr, nullptr, nullptr, nullptr};
-        if (!STAGED && tid == 0 && o + R < a.nops) read_rows(a, o + R, pre);
-        // Every thread waits for the record (walk_tile's hand-off).
-        const bool ok =
-            __all_sync(0xffffffffu, mbar_wait_bounded(&bars[stage], (phase >> stage) & 1u,
-                                                      spin));
-        phase ^= 1u << stage;
-        void *ydata = nullptr, *yscaler = nullptr;
-        int yslot = -1;
-        bool yhbm = false;
-        unsigned nchild = 0;
-        uint32_t nbytes = (uint32_t)sstride;
-        if (ok) {
-        const unsigned char *rec = ring + (size_t)stage * sstride;
-        const uint8_t *lrow = rec + a.rstride;
-        unsigned nlk = 0;
-        const RecHead *hd = reinterpret_cast<const RecHead *>(rec);
-        const RecChild *kids = reinterpret_cast<const RecChild *>(rec + sizeof(RecHead));
-        nchild = hd->nchild;
-        const uint32_t fl = hd->flags;
-        uint32_t kind = (fl >> kOpKindShift) & 7u;
-        if ((kind == OPK_FL || kind == OPK_FI) && o == 0) kind = OPK_GENERIC;
-        if (kind != OPK_GENERIC) {
-            op2_kind<K, STAGED, 2>(kind, rec, kids, (fl & kOpKindA) ? 1u : 0u, acc, lns, masks,
-                                   lrow, slots, slot_sc, tile, pl, p, ppad);
-        } else {
-        lns[0] = lns[1] = 0;
-        for (unsigned ci = 0; ci < nchild; ++ci) {
-            const RecChild ch = kids[ci];
-            const float *area = reinterpret_cast<const float *>(rec + ch.off);
-            T msg[2][K * 4];
-            if (ch.src == SRC_LEAF) {
-                unsigned m[2];
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    m[h] = STAGED ? masks[(size_t)ch.idx * tile + pl[h]]
-                                  : lrow[(size_t)nlk * tile + pl[h]];
-                if (!STAGED) ++nlk;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const float4 *t = reinterpret_cast<const float4 *>(area) + m[h];
-#pragma unroll
-                    for (int k = 0; k < K; ++k) {
-                        const float4 v = t[k * 16];
-                        msg[h][k * 4 + 0] = v.x;
-                        msg[h][k * 4 + 1] = v.y;
-                        msg[h][k * 4 + 2] = v.z;
-                        msg[h][k * 4 + 3] = v.w;
-                    }
-                }
-            } else {
-                const bool in_slot = (ch.src == SRC_SLOT);
-                const float4 *P = reinterpret_cast<const float4 *>(area);
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    const float4 c[4] = {P[k * 4], P[k * 4 + 1], P[k * 4 + 2], P[k * 4 + 3]};
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const float4 v =
-                            in_slot ? slots[((size_t)ch.idx * K + k) * tile + pl[h]]
-                                    : static_cast<const float4 *>(ch.data)[(size_t)k * ppad + p[h]];
-                        float x[4];
-                        unpack(v, x);
-                        pcol(c, x, msg[h] + k * 4);
-                    }
-                }
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    lns[h] += in_slot ? slot_sc[(size_t)ch.idx * tile + pl[h]]
-                                      : static_cast<const int *>(ch.scaler)[p[h]];
-            }
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                if (ci == 0) {
-#pragma unroll
-                    for (int q = 0; q < K * 4; ++q) acc[h][q] = msg[h][q];
-                } else {
-#pragma unroll
-                    for (int q = 0; q < K * 4; ++q) acc[h][q] *= msg[h][q];
-                }
-            }
-        }
-        }  // generic
-        ydata = hd->data;
-        yscaler = hd->scaler;
-        yslot = hd->slot;
-        yhbm = !(fl & REC_NO_HBM);
-        nbytes = (hd->next_bytes != 0u && hd->next_bytes <= (uint32_t)sstride)
-                     ? hd->next_bytes : (uint32_t)sstride;
-        }  // ok
-        if (!cta_hand_off(ok, nthr)) {
-            if (tid == 0) {
-                atomicOr(a.err, 1u);
-                drain_ring(bars, phase ^ (1u << stage), o, a.nops, R);
-            }
-            return false;
-        }
-        if (tid == 0 && o + R < a.nops) {
-            if (STAGED) {
-                fence_proxy_async();
-                mbar_expect_tx(&bars[stage], nbytes);
-                bulk_g2s(ring + (size_t)stage * a.rstride,
-                         a.rec + (size_t)(o + R) * a.rstride, nbytes, &bars[stage]);
-            } else {
-                issue_stage(a, o + R, ring + (size_t)stage * sstride, &bars[stage], tile_idx,
-                            tile, pre);
-            }
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            T mx = T(0);
-#pragma unroll
-            for (int q = 0; q < K * 4; ++q) mx = fmax(mx, acc[h][q]);
-            // The rescale rule of walk_tile (same bits).
-            if (mx > T(0) && mx <= (T)3.0e38 && (nchild > 2 || mx < 1.52587890625e-05f)) {
-                int e;
-                frexpf(mx, &e);
-                const int n = -e;
-                if (n >= -126 && n <= 127) {
-                    const float s1 = pow2f(n);
-#pragma unroll
-                    for (int q = 0; q < K * 4; ++q) acc[h][q] *= s1;
-                } else {
-                    const int n1 = n / 2, n2 = n - n1;
-                    const float s1 = pow2f(n1), s2 = pow2f(n2);
-#pragma unroll
-                    for (int q = 0; q < K * 4; ++q) acc[h][q] = (acc[h][q] * s1) * s2;
-                }
-                lns[h] += e;
-            }
-            if (yhbm) {
-                float4 *y = static_cast<float4 *>(ydata) + p[h];
-#pragma unroll
-                for (int k = 0; k < K; ++k) y[(size_t)k * ppad] = pack4(acc[h] + k * 4);
-                static_cast<int *>(yscaler)[p[h]] = lns[h];
-            }
-            if (yslot >= 0) {
-                float4 *ys = slots + (size_t)yslot * K * tile + pl[h];
-#pragma unroll
-                for (int k = 0; k < K; ++k) ys[(size_t)k * tile] = pack4(acc[h] + k * 4);
-                slot_sc[(size_t)yslot * tile + pl[h]] = lns[h];
-            }
-        }
-    }
-
-    if (a.no_root) {
-        __syncthreads();
-        return true;
-    }
-    double v[2] = {0.0, 0.0};
-    bool ninf[2] = {false, false};
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        if (!a.root_last) {
-            const float4 *r = static_cast<const float4 *>(a.root) + p[h];
-#pragma unroll
-            for (int k = 0; k < K; ++k) unpack(r[(size_t)k * ppad], acc[h] + k * 4);
-            lns[h] = static_cast<const int *>(a.rootsc)[p[h]];
-        }
-        double L = 0.0;
-#pragma unroll
-        for (int q = 0; q < K * 4; ++q) L = fma(__ldg(a.pn + q), (double)acc[h][q], L);
-        if (p[h] < a.npat) {
-            v[h] = (log(L) + (double)lns[h] * 0.69314718055994530942) * (double)a.freqs[p[h]];
-            if (isnan(v[h])) v[h] = -INFINITY;
-            if (a.site) a.site[p[h]] = v[h];
-            if (isinf(v[h])) {
-                ninf[h] = (v[h] < 0.0);
-                v[h] = 0.0;
-            }
-        }
-    }
-    reduce_sites_n<2>(a, tile_idx, v, ninf);
+    reduce_sites<1>(a, v, ninf);
     return true;
 }
 
@@ -1690,22 +1472,23 @@ __device__ __forceinline__ void init_lean() {
 }
 
 // Launch bounds of the walkers (see walker_threads).
-template <typename T, int KT, int G>
+template <typename T, int KT, int G, int N>
 struct CtaOf {
     static constexpr int threads =
-        walker_threads(sizeof(T) == 4 ? CXG_FP32 : CXG_FP64, KT, G);
-    static constexpr int per_sm = threads > 512 ? 1 : 2;
+        walker_threads(sizeof(T) == 4 ? CXG_FP32 : CXG_FP64, KT, G, N);
+    static constexpr int per_sm = 1;
 };
 
 // One plan: one CTA per tile.
-template <typename T, int KT, int G>
-__global__ void __launch_bounds__(CtaOf<T, KT, G>::threads, CtaOf<T, KT, G>::per_sm)
+template <typename T, int KT, int G, int N>
+__global__ void __launch_bounds__(CtaOf<T, KT, G, N>::threads, CtaOf<T, KT, G, N>::per_sm)
     walk_kernel(PlanArgs a) {
     const LeanLayout Lay = lean_layout(sizeof(T) == 4 ? CXG_FP32 : CXG_FP64, KT * G,
-                                       blockDim.x / G, a.nslot, a.ring, a.rstride, a.lmax);
+                                       blockDim.x / G * N, a.nslot, a.ring, a.rstride,
+                                       a.lmax);
     init_lean();
     RingPos ring{0, 0};
-    walk_tile<T, KT, G>(a, blockIdx.x, Lay, a.ring, ring);
+    walk_tile<T, KT, G, N>(a, blockIdx.x, Lay, a.ring, ring);
 }
 
 // One plan with L = 2 op lanes (FP32, one thread per pattern, staged
@@ -1724,13 +1507,13 @@ __global__ void __launch_bounds__(NT, MINB) walk_kernel_lanes(PlanArgs a) {
 
 // Many jobs: a persistent grid claims (job, tile) items in the host's order
 // (longest first).
-template <typename T, int KT, int G>
-__global__ void __launch_bounds__(CtaOf<T, KT, G>::threads, CtaOf<T, KT, G>::per_sm)
+template <typename T, int KT, int G, int N>
+__global__ void __launch_bounds__(CtaOf<T, KT, G, N>::threads, CtaOf<T, KT, G, N>::per_sm)
     walk_batch_kernel(BatchArgs b) {
     __shared__ unsigned s_item;
     __shared__ __align__(16) PlanArgs s_job;
     const LeanLayout Lay = lean_layout(sizeof(T) == 4 ? CXG_FP32 : CXG_FP64, KT * G,
-                                       blockDim.x / G, b.max_nslot, b.ring, b.max_rstride,
+                                       blockDim.x / G * N, b.max_nslot, b.ring, b.max_rstride,
                                        b.max_lmax);
     init_lean();
     RingPos ring{0, 0};
@@ -1751,46 +1534,7 @@ __global__ void __launch_bounds__(CtaOf<T, KT, G>::threads, CtaOf<T, KT, G>::per
             load_job(s_job, b.jobs + it.job);
             job = it.job;
         }
-        if (!walk_tile<T, KT, G>(s_job, it.tile, Lay, b.ring, ring)) break;
-    }
-}
-
-// Two patterns per thread (FP32, one thread per pattern pair).
-template <int K, bool STAGED>
-__global__ void __launch_bounds__(kBlock) walk_kernel2(PlanArgs a) {
-    const SmemLayout Lay = smem_layout(CXG_FP32, K, blockDim.x * 2, a.nslot, a.ring,
-                                       a.rstride, a.lmax, a.nleaf);
-    init_ring(Lay, a.ring);
-    uint32_t phase = 0;
-    walk_tile2<K, STAGED>(a, blockIdx.x, Lay, a.ring, phase);
-}
-
-template <int K, bool STAGED>
-__global__ void __launch_bounds__(kBlock) walk_batch_kernel2(BatchArgs b) {
-    __shared__ unsigned s_item;
-    __shared__ __align__(16) PlanArgs s_job;
-    unsigned job = ~0u;
-    const SmemLayout Lay = smem_layout(CXG_FP32, K, blockDim.x * 2, b.max_nslot, b.ring,
-                                       b.max_rstride, b.max_lmax, b.max_nleaf);
-    init_ring(Lay, b.ring);
-    uint32_t phase = 0;
-    for (unsigned n = 0;; ++n) {
-        unsigned item;
-        if (b.direct) {
-            item = n == 0 ? blockIdx.x : b.nitems;
-        } else {
-            if (threadIdx.x == 0) s_item = atomicAdd(b.counter, 1u);
-            __syncthreads();
-            item = s_item;
-            __syncthreads();
-        }
-        if (item >= b.nitems) break;
-        const WalkItem it = b.items[item];
-        if (it.job != job) {
-            load_job(s_job, b.jobs + it.job);
-            job = it.job;
-        }
-        if (!walk_tile2<K, STAGED>(s_job, it.tile, Lay, b.ring, phase)) break;
+        if (!walk_tile<T, KT, G, N>(s_job, it.tile, Lay, b.ring, ring)) break;
     }
 }
 
@@ -1815,22 +1559,25 @@ static cudaError_t ensure_smem(Kern k, size_t sm, size_t &optin) {
 }
 
 // Instantiated walker shapes (per-thread components KT, threads per
-// pattern G): every kact with G = 1, and a pattern's components split over 2
-// or 4 threads (walker_shape_ok).
-#define CXG_SHAPES_G1(X) X(1, 1) X(2, 1) X(3, 1) X(4, 1) X(5, 1) X(6, 1) X(7, 1) X(8, 1)
-#define CXG_SHAPES_GN(X) X(1, 2) X(2, 2) X(3, 2) X(4, 2) X(1, 4) X(2, 4)
+// pattern G, patterns per thread N): every kact with one of each, a
+// pattern's components split over 2 or 4 threads, and the FP32 form with two
+// patterns a thread (walker_shape_ok).
+#define CXG_SHAPES_1(X) \
+    X(1, 1, 1) X(2, 1, 1) X(3, 1, 1) X(4, 1, 1) X(5, 1, 1) X(6, 1, 1) X(7, 1, 1) X(8, 1, 1)
+#define CXG_SHAPES_G(X) X(1, 2, 1) X(2, 2, 1) X(3, 2, 1) X(4, 2, 1) X(1, 4, 1) X(2, 4, 1)
+#define CXG_SHAPES_N(X) X(1, 1, 2) X(2, 1, 2) X(3, 1, 2) X(4, 1, 2) X(5, 1, 2)
 
-template <typename T, int KT, int G>
+template <typename T, int KT, int G, int N>
 static cudaError_t walk_fn(size_t sm, void (**fn)(PlanArgs)) {
     static size_t optin = 0;
-    *fn = walk_kernel<T, KT, G>;
-    return ensure_smem(walk_kernel<T, KT, G>, sm, optin);
+    *fn = walk_kernel<T, KT, G, N>;
+    return ensure_smem(walk_kernel<T, KT, G, N>, sm, optin);
 }
-template <typename T, int KT, int G>
+template <typename T, int KT, int G, int N>
 static cudaError_t batch_fn(size_t sm, void (**fn)(BatchArgs)) {
     static size_t optin = 0;
-    *fn = walk_batch_kernel<T, KT, G>;
-    return ensure_smem(walk_batch_kernel<T, KT, G>, sm, optin);
+    *fn = walk_batch_kernel<T, KT, G, N>;
+    return ensure_smem(walk_batch_kernel<T, KT, G, N>, sm, optin);
 }
 template <int K, int NT, int MINB>
 static cudaError_t lanes_fn(size_t sm, void (**fn)(PlanArgs)) {
@@ -1838,46 +1585,19 @@ static cudaError_t lanes_fn(size_t sm, void (**fn)(PlanArgs)) {
     *fn = walk_kernel_lanes<K, NT, MINB>;
     return ensure_smem(walk_kernel_lanes<K, NT, MINB>, sm, optin);
 }
-template <int K, bool ST>
-static cudaError_t walk2_fn(size_t sm, void (**fn)(PlanArgs)) {
-    static size_t optin = 0;
-    *fn = walk_kernel2<K, ST>;
-    return ensure_smem(walk_kernel2<K, ST>, sm, optin);
-}
-template <int K, bool ST>
-static cudaError_t batch2_fn(size_t sm, void (**fn)(BatchArgs)) {
-    static size_t optin = 0;
-    *fn = walk_batch_kernel2<K, ST>;
-    return ensure_smem(walk_batch_kernel2<K, ST>, sm, optin);
-}
-
-// The two-patterns-per-thread walker for kact (FP32), with its dynamic
-// shared memory limit raised to `sm` bytes.
-template <typename Fn>
-static cudaError_t pick_walker2(unsigned kact, bool staged, size_t sm, Fn *fn, bool batch) {
-#define CXG_X2(K)                                                                       \
-    if (kact == (K)) {                                                                  \
-        if (batch)                                                                      \
-            return staged ? batch2_fn<K, true>(sm, reinterpret_cast<void (**)(BatchArgs)>(fn)) \
-                          : batch2_fn<K, false>(sm, reinterpret_cast<void (**)(BatchArgs)>(fn)); \
-        return staged ? walk2_fn<K, true>(sm, reinterpret_cast<void (**)(PlanArgs)>(fn))       \
-                      : walk2_fn<K, false>(sm, reinterpret_cast<void (**)(PlanArgs)>(fn));     \
-    }
-    CXG_X2(1) CXG_X2(2) CXG_X2(3) CXG_X2(4) CXG_X2(5)
-#undef CXG_X2
-    return cudaErrorInvalidValue;
-}
-
-// The walker for (kact, G), with its dynamic shared memory limit raised to
-// `sm` bytes.
+// The walker of shape w, with its dynamic shared memory limit raised to `sm`
+// bytes.
 template <typename T, typename Fn>
-static cudaError_t pick_walker(unsigned kact, unsigned G, size_t sm, Fn *fn, bool batch) {
-#define CXG_X(KT, GG)                                                                     \
-    if (kact == (KT) * (GG) && G == (GG))                                                 \
-        return batch ? batch_fn<T, KT, GG>(sm, reinterpret_cast<void (**)(BatchArgs)>(fn)) \
-                     : walk_fn<T, KT, GG>(sm, reinterpret_cast<void (**)(PlanArgs)>(fn));
-    CXG_SHAPES_G1(CXG_X)
-    CXG_SHAPES_GN(CXG_X)
+static cudaError_t pick_walker(const WalkShape &w, size_t sm, Fn *fn, bool batch) {
+#define CXG_X(KT, GG, NN)                                                                     \
+    if (w.kact == (KT) * (GG) && w.tpp == (GG) && w.ppt == (NN))                              \
+        return batch ? batch_fn<T, KT, GG, NN>(sm, reinterpret_cast<void (**)(BatchArgs)>(fn)) \
+                     : walk_fn<T, KT, GG, NN>(sm, reinterpret_cast<void (**)(PlanArgs)>(fn));
+    CXG_SHAPES_1(CXG_X)
+    CXG_SHAPES_G(CXG_X)
+    if constexpr (sizeof(T) == 4) {
+        CXG_SHAPES_N(CXG_X)
+    }
 #undef CXG_X
     return cudaErrorInvalidValue;
 }
@@ -1895,21 +1615,26 @@ static cudaError_t pick_walker_lanes(unsigned kact, unsigned tile, size_t sm,
 }
 
 // Dynamic shared memory of a walker launch: the lean layout (its ring counts
-// ops per stage) for one pattern per thread and one op lane, else the layout
-// of the two-pattern and op-lane walkers (its ring counts records).
+// ops per stage), or that of the op-lane walker (its ring counts steps).
 size_t walk_smem_bytes(const WalkShape &w, unsigned nslot, unsigned rstride, unsigned lmax,
                        unsigned nleaf) {
-    return w.lean() ? lean_smem_bytes(w.precision, w.kact, w.tile, nslot, w.ring, rstride, lmax)
-                    : plan_smem_bytes(w.precision, w.kact, w.tile, nslot, w.ring,
-                                      rstride * w.lanes, lmax, nleaf);
+    return w.lanes == 1
+               ? lean_layout(w.precision, w.kact, w.tile, nslot, w.ring, rstride, lmax).total
+               : smem_layout(w.precision, w.kact, w.tile, nslot, w.ring, rstride * w.lanes, lmax,
+                             nleaf).total;
 }
 
 static bool shape_launches(const WalkShape &w) {
-    return w.tile != 0 && w.tile % 32 == 0 && w.ring != 0 &&
-           walker_shape_ok(w.precision, w.kact, w.tpp, w.ppt) &&
-           (w.lean() ? w.tile * w.tpp <= walker_threads(w.precision, w.kact / w.tpp, w.tpp) &&
-                           (w.tpp == 1 || w.tile <= kBlock)
-                     : w.tile <= kBlock && w.tile / w.ppt >= 32 && w.ring <= 8);
+    if (w.tile == 0 || w.tile % 32 || w.ring == 0 ||
+        !walker_shape_ok(w.precision, w.kact, w.tpp, w.ppt))
+        return false;
+    if (w.lanes == 2)
+        return lanes_shape_ok(w.precision, w.kact, w.tpp, w.ppt) && w.ring <= 8 &&
+               w.tile * 2 <= kLaneThreads;
+    return w.lanes == 1 && w.tile / w.ppt >= 32 &&
+           w.tile / w.ppt * w.tpp <=
+               walker_threads(w.precision, w.kact / w.tpp, w.tpp, w.ppt) &&
+           (w.tpp == 1 || w.tile <= kBlock) && (w.ppt == 1 || kPatternQuantum % w.tile == 0 || w.tile % 64 == 0);
 }
 
 static WalkShape shape_of(int precision, unsigned kact, unsigned tile, unsigned tpp,
@@ -1929,20 +1654,14 @@ cudaError_t launch_plan(int precision, const PlanArgs &a, cudaStream_t s, unsign
                         bool pdl) {
     const WalkShape w = shape_of(precision, a.kact, a.tile, a.tpp, a.ppt, lanes, a.ring);
     if (!shape_launches(w) || a.rstride % 16 || a.rstride == 0 ||
-        a.ntiles != plan_blocks(a.ppad, a.tile) || (!w.lean() && a.ppad % a.tile) ||
-        (w.lean() && w.ring * a.lmax > 32))
-        return cudaErrorInvalidValue;
-    if (lanes != 1 && !(lanes == 2 && lanes_shape_ok(precision, a.kact, w.tpp, w.ppt) &&
-                        a.lmax == 0 && a.tile * lanes <= kLaneThreads &&
-                        a.nops % lanes == 0))
+        a.ntiles != plan_blocks(a.ppad, a.tile) || (lanes == 1 && w.ring * a.lmax > 32) ||
+        (lanes == 2 && (a.lmax != 0 || a.nops % 2 || a.ppad % a.tile)))
         return cudaErrorInvalidValue;
     const size_t sm = walk_smem_bytes(w, a.nslot, a.rstride, a.lmax, a.nleaf);
     void (*fn)(PlanArgs) = nullptr;
-    cudaError_t e = lanes == 2      ? pick_walker_lanes(a.kact, a.tile, sm, &fn)
-                    : w.ppt == 2    ? pick_walker2(a.kact, a.lmax == 0, sm, &fn, false)
-                    : precision == CXG_FP32
-                        ? pick_walker<float>(a.kact, w.tpp, sm, &fn, false)
-                        : pick_walker<double>(a.kact, w.tpp, sm, &fn, false);
+    cudaError_t e = lanes == 2              ? pick_walker_lanes(a.kact, a.tile, sm, &fn)
+                    : precision == CXG_FP32 ? pick_walker<float>(w, sm, &fn, false)
+                                            : pick_walker<double>(w, sm, &fn, false);
     if (e != cudaSuccess) return e;
     const unsigned nb = a.ntiles, nt = a.tile * w.tpp * lanes / w.ppt;
     if (pdl) {
@@ -1963,11 +1682,9 @@ cudaError_t launch_plan(int precision, const PlanArgs &a, cudaStream_t s, unsign
     return cudaGetLastError();
 }
 
-static cudaError_t pick_batch(const WalkShape &w, bool staged, size_t sm,
-                              void (**fn)(BatchArgs)) {
-    return w.ppt == 2 ? pick_walker2(w.kact, staged, sm, fn, true)
-           : w.precision == CXG_FP32 ? pick_walker<float>(w.kact, w.tpp, sm, fn, true)
-                                     : pick_walker<double>(w.kact, w.tpp, sm, fn, true);
+static cudaError_t pick_batch(const WalkShape &w, size_t sm, void (**fn)(BatchArgs)) {
+    return w.precision == CXG_FP32 ? pick_walker<float>(w, sm, fn, true)
+                                   : pick_walker<double>(w, sm, fn, true);
 }
 
 cudaError_t launch_batch(int precision, const BatchArgs &b_in, unsigned grid,
@@ -1982,20 +1699,20 @@ cudaError_t launch_batch(int precision, const BatchArgs &b_in, unsigned grid,
     }
     const WalkShape w = shape_of(precision, b.kact, b.tile, b.tpp, b.ppt, 1, b.ring);
     if (!shape_launches(w) || b.max_rstride % 16 || b.max_rstride == 0 || grid == 0 ||
-        (w.lean() && w.ring * b.max_lmax > 32))
+        w.ring * b.max_lmax > 32)
         return cudaErrorInvalidValue;
-    const size_t sm = walk_smem_bytes(w, b.max_nslot, b.max_rstride, b.max_lmax, b.max_nleaf);
+    const size_t sm = walk_smem_bytes(w, b.max_nslot, b.max_rstride, b.max_lmax, 0);
     void (*fn)(BatchArgs) = nullptr;
-    const cudaError_t e = pick_batch(w, b.max_lmax == 0, sm, &fn);
+    const cudaError_t e = pick_batch(w, sm, &fn);
     if (e != cudaSuccess) return e;
     fn<<<grid, b.tile * w.tpp / w.ppt, sm, s>>>(b);
     return cudaGetLastError();
 }
 
-int batch_ctas_per_sm(const WalkShape &w, bool staged, size_t smem) {
+int batch_ctas_per_sm(const WalkShape &w, size_t smem) {
     if (!shape_launches(w)) return 0;
     void (*fn)(BatchArgs) = nullptr;
-    cudaError_t e = pick_batch(w, staged, smem, &fn);
+    cudaError_t e = pick_batch(w, smem, &fn);
     int n = 0;
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, (int)(w.tile * w.tpp / w.ppt),

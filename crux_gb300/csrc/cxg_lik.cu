@@ -409,7 +409,7 @@ static int internal_child(State &S, const CxtLik *lik, const CxtLikCL *cl,
 struct Plan {
     int prec = CXG_FP64;
     unsigned npat = 0, ppad = 0, kact = 0, nops = 0, nchild = 0;
-    DevBuf prog, partial, misc, ltab;
+    DevBuf prog, misc, ltab;
     HostBuf out;
     DevCL *root = nullptr;
     std::vector<DevCL *> parents;
@@ -485,60 +485,117 @@ static unsigned g_lanes = 1;
 static size_t g_smem_budget = 24 * 1024;
 static bool g_tuned = false;  // cxgTune was called: its shape is used as it is
 
-WalkShape choose_shape(int precision, unsigned kact, size_t patterns, bool lanes_ok) {
+// SMs of the GPU these kernels are built for.
+constexpr unsigned kSMs = 152;
+
+// Shape for work no caller has tuned.  Measured on the 128-taxon tree over
+// 81,664 patterns (2,552 warps), the 32-job batch and the small trees:
+//
+// FP32.  A walker of 96 registers keeps 20 warps on an SM, and a warp that
+// starts late ends late (65 us of latency for 127 ops): so a plan whose warps
+// all fit gets one wave of equal CTAs, two to an SM (tile 288: 144 us; 128,
+// 4.2 CTAs to an SM: 155; 32, which streams the records 9 times as often: 267),
+// and a larger one as few equal waves.  Below four warps an SM the walk is
+// bound by one warp's op after op; two warps a CTA spread it (64: 41.5 us, 32:
+// 44, 128: 42 on 17,018 patterns of 8 components).  Many jobs take tiles of
+// 128 (525 us; 64: 562).
+//
+// FP64.  Each SM quarter issues one FP64 instruction a warp in 64 cycles and a
+// pattern's components are independent, so two threads a pattern halve the
+// unit in which quarters are loaded (1,511 us against 1,681 with one and
+// 1,535 with four), and four serve a walk of few patterns (27 us against 57
+// on 522).
+//
+// No shape takes stack slots: a result is stored to HBM anyway, and reading
+// it back through L2 costs less than storing it twice.
+static WalkShape auto_shape(int precision, unsigned kact, size_t patterns, unsigned jobs) {
     WalkShape w;
     w.precision = precision;
     w.kact = kact;
-    w.tile = g_tile;
-    // The caller's shape, each part where a walker is built for it.
-    if (precision == CXG_FP32 && walker_shape_ok(precision, kact, g_tpp) &&
-        g_tile * g_tpp <= kTuneThreads)
-        w.tpp = g_tpp;
-    if (walker_shape_ok(precision, kact, w.tpp, g_ppt) && g_tile / g_ppt >= 32) w.ppt = g_ppt;
+    const size_t warps = (patterns + 31) / 32;
+    if (precision == CXG_FP64) {
+        const bool few = warps * 4 <= (size_t)kSMs * 16;
+        w.tile = 32;
+        if (few && walker_shape_ok(precision, kact, 4)) w.tpp = 4;
+        else if (walker_shape_ok(precision, kact, 2)) w.tpp = 2;
+        else w.tile = 64;
+        return w;
+    }
+    if (jobs > 1) {
+        w.tile = 128;
+        return w;
+    }
+    const unsigned most = walker_threads(precision, kact, 1, 1) / 32;  // warps an SM holds
+    if (warps <= 4 * (size_t)kSMs) {
+        w.tile = 64;
+    } else {
+        const size_t waves = (warps + (size_t)kSMs * most - 1) / ((size_t)kSMs * most);
+        const size_t ctas = 2 * kSMs * waves;
+        w.tile = 32 * (unsigned)std::min<size_t>((warps + ctas - 1) / ctas, most / 2);
+    }
+    return w;
+}
+
+WalkShape choose_shape(int precision, unsigned kact, size_t patterns, unsigned jobs,
+                       bool lanes_ok) {
+    WalkShape w = auto_shape(precision, kact, patterns, jobs);
+    if (g_tuned) {
+        // The caller's shape, each part where a walker is built for it.
+        w = WalkShape();
+        w.precision = precision;
+        w.kact = kact;
+        w.tile = g_tile;
+        w.budget = g_smem_budget;
+        if (precision == CXG_FP32 && walker_shape_ok(precision, kact, g_tpp) &&
+            g_tile * g_tpp <= kTuneThreads)
+            w.tpp = g_tpp;
+        if (walker_shape_ok(precision, kact, w.tpp, g_ppt) && g_tile / g_ppt >= 32)
+            w.ppt = g_ppt;
+    }
     if (lanes_ok && g_lanes == 2 && lanes_shape_ok(precision, kact, w.tpp, w.ppt) &&
-        g_tile * 2 <= kLaneThreads)
+        g_tile * 2 <= kLaneThreads) {
         w.lanes = 2;
-    (void)patterns;
+        w.tile = g_tile;
+        w.budget = g_smem_budget;
+    }
     return w;
 }
 
 void fit_ring(WalkShape &w, unsigned rstride, unsigned lmax) {
-    if (!w.lean()) {
-        // A stage of the op-lane walker holds two records: half the stages
-        // keep as many records in flight.
-        w.ring = w.lanes == 2 ? kRing / 2 : kRing;
+    if (w.lanes == 2) {
+        w.ring = kRing / 2;  // a stage holds a step's two records
         return;
     }
-    const size_t bytes = w.tile * w.tpp >= 128 ? 48 * 1024 : 28 * 1024;
+    // Ring bytes: shared by the CTA's warps, so that the CTAs an SM's
+    // registers hold fit its shared memory (five of 128 threads, two of 288).
+    const unsigned threads = w.tile * w.tpp / w.ppt;
+    size_t bytes = threads > 128 ? 60 * 1024 : 42 * 1024;
     size_t n = bytes / (kStages * ((size_t)rstride + (size_t)lmax * w.tile));
     if (n > 16) n = 16;
     if (lmax && n > 32 / lmax) n = 32 / lmax;
     w.ring = n ? (unsigned)n : 1;
 }
 
-bool stages_leaves(const WalkShape &w, unsigned nleaf) {
-    return !w.lean() && (size_t)nleaf * w.tile <= kLeafStageBytes;
-}
-
 unsigned stack_slots(const WalkShape &w, unsigned rstride, unsigned lmax, unsigned nleaf) {
     const size_t base = walk_smem_bytes(w, 0, rstride, lmax, nleaf);
     const size_t slot = walk_smem_bytes(w, 1, rstride, lmax, nleaf) - base;
     size_t cap = 0;
-    if (w.lean()) {
+    if (w.lanes == 1) {
         // The budget is the stack's; the CTA as a whole stays launchable.
-        cap = g_smem_budget / slot;
+        cap = w.budget / slot;
         const size_t most = 200 * 1024;
         if (base + cap * slot > most) cap = base < most ? (most - base) / slot : 0;
-    } else if (g_smem_budget > base) {
-        cap = (g_smem_budget - base) / slot;
+    } else if (w.budget > base) {
+        cap = (w.budget - base) / slot;
     }
     return cap > kMaxSlots ? kMaxSlots : (unsigned)cap;
 }
 
-// `patterns`: padded patterns of all the jobs this plan is launched with (0:
-// its own).
+// `patterns`: padded patterns of all the njobs jobs this plan is launched
+// with (0: its own).
 static int translate(State &S, CxtLik *lik, int prec, Plan &P,
-                     bool use_slots = true, bool allow_lanes = false, size_t patterns = 0) {
+                     bool use_slots = true, bool allow_lanes = false, size_t patterns = 0,
+                     unsigned njobs = 1) {
     int rc;
     if (lik == nullptr) return fail(CXG_EINVAL, "lik is NULL");
     if (lik->dim != 4)
@@ -669,7 +726,7 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
     // Leaves: staged once per tile (each distinct leaf one row, named by
     // kids[c].idx) when they fit kLeafStageBytes, else each op's mask
     // arrays (kids[c].data) travel with its record (lmax rows per stage).
-    WalkShape w = choose_shape(prec, kact, patterns ? patterns : ppad,
+    WalkShape w = choose_shape(prec, kact, patterns ? patterns : ppad, njobs,
                                allow_lanes && ops.size() >= 2);
     const unsigned tile = w.tile;
     std::vector<const uint8_t *> leaf_ptrs;
@@ -693,9 +750,9 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
         }
     }
     const unsigned nleaf = (unsigned)leaf_ptrs.size();
-    // (Op lanes need staged leaves.)
-    if (w.lanes == 2 && !stages_leaves(w, nleaf)) w.lanes = 1;
-    const bool stage_leaves = stages_leaves(w, nleaf);
+    // Op lanes stage the leaves, and run where they fit.
+    if ((size_t)nleaf * tile > kLeafStageBytes) w.lanes = 1;
+    const bool stage_leaves = w.lanes == 2;
     const unsigned s_lmax = stage_leaves ? 0 : lmax;
     const unsigned s_nleaf = stage_leaves ? nleaf : 0;
 
@@ -859,8 +916,6 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
             continue;
         }
         const size_t o = (size_t)order[pos];
-        if (!w.lean() && lanes == 1 && pos + ring < order.size())
-            hd.next_bytes = (uint32_t)rec_bytes[order[pos + ring]];
         hd.data = ops[o].data;
         hd.scaler = ops[o].scaler;
         hd.nchild = ops[o].nchild;
@@ -945,12 +1000,10 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
     pa.ltab = (double *)P.ltab.p;
 
     const unsigned nb = plan_blocks(ppad, tile);
-    rc = P.partial.ensure((size_t)nb * 16);
+    // misc: result words | site
+    rc = P.misc.ensure(kResultBytes + (size_t)ppad * 8);
     if (rc) return rc;
-    // misc: ticket (4) | ninf (4) | err (4) | pad (4) | total (16) | site
-    rc = P.misc.ensure(32 + (size_t)ppad * 8);
-    if (rc) return rc;
-    rc = P.out.ensure(32);
+    rc = P.out.ensure(kResultRead);
     if (rc) return rc;
     char *mp = static_cast<char *>(P.misc.p);
     PlanArgs &a = P.a;
@@ -975,7 +1028,7 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
     a.rootsc = P.root->scaler;
     a.freqs = (const uint32_t *)dfreqs;
     a.site = nullptr;
-    a.partial = (double *)P.partial.p;
+    a.acc = (uint64_t *)(mp + 32);
     a.ticket = (unsigned *)mp;
     a.ninf = (uint32_t *)(mp + 4);
     a.err = (uint32_t *)(mp + 8);
@@ -1009,24 +1062,24 @@ static int enqueue(State &S, Plan &P, bool want_site,
                    cudaEvent_t e0 = nullptr, cudaEvent_t e1 = nullptr,
                    bool pdl = false) {
     char *mp = static_cast<char *>(P.misc.p);
-    P.a.site = want_site ? (double *)(mp + 32) : nullptr;
-    // The P kernel clears the walker's 32 result bytes; a plan with no P
+    P.a.site = want_site ? (double *)(mp + kResultBytes) : nullptr;
+    // The P kernel clears the walker's result words; a plan with no P
     // matrices clears them with a memset.
     const bool pmat = P.pa.nchild * P.pa.kact > 0;
     P.pa.zero = pmat ? reinterpret_cast<uint64_t *>(mp) : nullptr;
-    if (!pmat) CXG_CUDA(cudaMemsetAsync(mp, 0, 32, S.stream));
+    if (!pmat) CXG_CUDA(cudaMemsetAsync(mp, 0, kResultBytes, S.stream));
     CXG_CUDA(launch_pmat(P.pa, S.stream));
     if (e0) CXG_CUDA(cudaEventRecord(e0, S.stream));
     CXG_CUDA(launch_plan(P.prec, P.a, S.stream, P.lanes,
                          pdl && e0 == nullptr && P.pa.nchild > 0));
     if (e1) CXG_CUDA(cudaEventRecord(e1, S.stream));
-    CXG_CUDA(cudaMemcpyAsync(P.out.p, mp, 32, cudaMemcpyDeviceToHost, S.stream));
+    CXG_CUDA(cudaMemcpyAsync(P.out.p, mp, kResultRead, cudaMemcpyDeviceToHost, S.stream));
     return 0;
 }
 
 static int finish(State &S, Plan &P, double *lnL, double *site) {
     if (site)
-        CXG_CUDA(cudaMemcpyAsync(site, static_cast<char *>(P.misc.p) + 32,
+        CXG_CUDA(cudaMemcpyAsync(site, static_cast<char *>(P.misc.p) + kResultBytes,
                                  (size_t)P.npat * 8, cudaMemcpyDeviceToHost,
                                  S.stream));
     CXG_CUDA(cudaStreamSynchronize(S.stream));
@@ -1049,12 +1102,10 @@ static int finish(State &S, Plan &P, double *lnL, double *site) {
 static void free_plan(Plan &P) {
     if (P.prog.p) dev_free(P.prog.p);
     if (P.ltab.p) dev_free(P.ltab.p);
-    if (P.partial.p) dev_free(P.partial.p);
     if (P.misc.p) dev_free(P.misc.p);
     if (P.out.p) host_free(P.out.p);
     P.prog = DevBuf();
     P.ltab = DevBuf();
-    P.partial = DevBuf();
     P.misc = DevBuf();
     P.out = HostBuf();
 }
@@ -1162,7 +1213,7 @@ static int execute(CxtLik *lik, int prec, double *lnL, double *site) {
         S.last_valid = false;
         return rc;
     }
-    S.last_d2h = 32 + (site ? (size_t)P.npat * 8 : 0);
+    S.last_d2h = kResultRead + (site ? (size_t)P.npat * 8 : 0);
     rc = finish(S, P, lnL, site);
     if (rc) S.last_valid = false;
     return rc;
@@ -1491,10 +1542,8 @@ struct cxgBatch {
     std::vector<Plan *> plans;
     DevBuf jobs, items, pmats, prefix, results;
     HostBuf out;
-    // Jobs that stage their leaves and jobs that stream them run as two
-    // persistent launches (each walker is built for one of the two).
-    BatchArgs args[2];
-    unsigned grid[2] = {0, 0}, nitems = 0;
+    BatchArgs args;
+    unsigned grid = 0, nitems = 0;
     uint32_t pmat_total = 0;
     double updates = 0.0, alg_bytes = 0.0;
     unsigned long long launches = 0;
@@ -1519,15 +1568,13 @@ static void free_batch(cxgBatch *b) {
 static int batch_enqueue(State &S, cxgBatch *b, cudaEvent_t e0 = nullptr,
                          cudaEvent_t e1 = nullptr) {
     const size_t n = b->plans.size();
-    CXG_CUDA(cudaMemsetAsync(b->results.p, 0, n * 32 + 32, S.stream));
+    CXG_CUDA(cudaMemsetAsync(b->results.p, 0, n * kResultBytes + 16, S.stream));
     CXG_CUDA(launch_pmat_batch(static_cast<const PmatArgs *>(b->pmats.p),
                                static_cast<const uint32_t *>(b->prefix.p),
                                (uint32_t)n, b->pmat_total, S.stream));
     if (e0) CXG_CUDA(cudaEventRecord(e0, S.stream));
     if (!b->per_node) {
-        for (int gi = 0; gi < 2; ++gi)
-            if (b->args[gi].nitems)
-                CXG_CUDA(launch_batch(b->prec, b->args[gi], b->grid[gi], S.stream));
+        CXG_CUDA(launch_batch(b->prec, b->args, b->grid, S.stream));
     } else {
         // The plain comparison: one launch per node update.
         for (Plan *P : b->plans) {
@@ -1543,7 +1590,7 @@ static int batch_enqueue(State &S, cxgBatch *b, cudaEvent_t e0 = nullptr,
         }
     }
     if (e1) CXG_CUDA(cudaEventRecord(e1, S.stream));
-    CXG_CUDA(cudaMemcpyAsync(b->out.p, b->results.p, n * 32,
+    CXG_CUDA(cudaMemcpyAsync(b->out.p, b->results.p, n * kResultBytes,
                              cudaMemcpyDeviceToHost, S.stream));
     return 0;
 }
@@ -1554,9 +1601,9 @@ static int batch_finish(State &S, cxgBatch *b, double *lnLs) {
     for (size_t j = 0; j < b->plans.size(); ++j) {
         uint32_t ninf, err;
         double tot[2];
-        memcpy(&ninf, o + j * 32 + 4, 4);
-        memcpy(&err, o + j * 32 + 8, 4);
-        memcpy(tot, o + j * 32 + 16, 16);
+        memcpy(&ninf, o + j * kResultBytes + 4, 4);
+        memcpy(&err, o + j * kResultBytes + 8, 4);
+        memcpy(tot, o + j * kResultBytes + 16, 16);
         for (DevCL *p : b->plans[j]->parents) p->computed = (err == 0);
         if (err)
             return fail(CXG_ETIMEOUT,
@@ -1605,7 +1652,8 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
     for (unsigned j = 0; j < n; ++j) {
         Plan *P = new Plan();
         b->plans.push_back(P);
-        rc = translate(S, liks[j], precision, *P, !b->per_node, false, patterns);
+        rc = translate(S, liks[j], precision, *P, !b->per_node, false, patterns,
+                       b->per_node ? 1 : n);
         if (rc) {
             free_batch(b);
             return rc;
@@ -1621,10 +1669,9 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
         b->alg_bytes += P->alg_bytes;
         b->launches += P->nops;
     }
-    // Per-job results live side by side: [ticket ninf err pad total] x n,
-    // then the work counters of the two launches (16 bytes apart).
-    if ((rc = b->results.ensure((size_t)n * 32 + 32)) ||
-        (rc = b->out.ensure((size_t)n * 32)) ||
+    // Per-job result words side by side, then the walker's work counter.
+    if ((rc = b->results.ensure((size_t)n * kResultBytes + 16)) ||
+        (rc = b->out.ensure((size_t)n * kResultBytes)) ||
         (rc = b->jobs.ensure((size_t)n * sizeof(PlanArgs))) ||
         (rc = b->pmats.ensure((size_t)n * sizeof(PmatArgs))) ||
         (rc = b->prefix.ensure((size_t)(n + 1) * 4))) {
@@ -1638,10 +1685,11 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
     char *res = static_cast<char *>(b->results.p);
     for (unsigned j = 0; j < n; ++j) {
         PlanArgs a = b->plans[j]->a;
-        a.ticket = (unsigned *)(res + (size_t)j * 32);
-        a.ninf = (uint32_t *)(res + (size_t)j * 32 + 4);
-        a.err = (uint32_t *)(res + (size_t)j * 32 + 8);
-        a.total = (double *)(res + (size_t)j * 32 + 16);
+        a.ticket = (unsigned *)(res + (size_t)j * kResultBytes);
+        a.ninf = (uint32_t *)(res + (size_t)j * kResultBytes + 4);
+        a.err = (uint32_t *)(res + (size_t)j * kResultBytes + 8);
+        a.total = (double *)(res + (size_t)j * kResultBytes + 16);
+        a.acc = (uint64_t *)(res + (size_t)j * kResultBytes + 32);
         a.site = nullptr;
         b->plans[j]->a = a;
         jobs[j] = a;
@@ -1649,18 +1697,10 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
         prefix[j + 1] = prefix[j] + pm[j].nchild * pm[j].kact;
         for (unsigned t = 0; t < a.ntiles; ++t) items.push_back(WalkItem{j, t});
     }
-    // The two-pattern walker is built for staged or streamed leaves: jobs
-    // that stage them first, then the others (two launches; the lean walker
-    // takes all in the second).  Each group longest jobs first, so its
-    // persistent grid ends together.
-    const bool lean = b->plans[0]->ppt == 1;
-    auto streams = [&](const WalkItem &x) { return lean || jobs[x.job].lmax != 0; };
-    std::stable_sort(items.begin(), items.end(),
-                     [&](const WalkItem &x, const WalkItem &y) {
-                         const bool sx = streams(x), sy = streams(y);
-                         if (sx != sy) return sy;
-                         return jobs[x.job].nops > jobs[y.job].nops;
-                     });
+    // Longest jobs first, so that the persistent grid ends together.
+    std::stable_sort(items.begin(), items.end(), [&](const WalkItem &x, const WalkItem &y) {
+        return jobs[x.job].nops > jobs[y.job].nops;
+    });
     b->nitems = (unsigned)items.size();
     b->pmat_total = prefix[n];
     if ((rc = b->items.ensure(items.size() * sizeof(WalkItem)))) {
@@ -1679,55 +1719,38 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
         free_batch(b);
         return cuda_fail(e, "cxgBatchCreate upload");
     }
-    unsigned nstaged = 0;
-    while (nstaged < items.size() && !streams(items[nstaged])) ++nstaged;
-    for (int gi = 0; gi < 2; ++gi) {
-        BatchArgs &ba = b->args[gi];
-        memset(&ba, 0, sizeof(ba));
-        const unsigned i0 = gi == 0 ? 0 : nstaged;
-        const unsigned i1 = gi == 0 ? nstaged : (unsigned)items.size();
-        ba.jobs = static_cast<const PlanArgs *>(b->jobs.p);
-        ba.items = static_cast<const WalkItem *>(b->items.p) + i0;
-        ba.nitems = i1 - i0;
-        ba.counter = (unsigned *)(res + (size_t)n * 32 + 16 * gi);
-        ba.tile = b->plans[0]->tile;
-        ba.tpp = b->plans[0]->tpp;
-        ba.ppt = b->plans[0]->ppt;
-        ba.ring = kRing;
-        ba.kact = kact;
-        ba.max_rstride = 16;
-        for (unsigned i = i0; i < i1; ++i) {
-            const PlanArgs &a = jobs[items[i].job];
-            ba.max_nslot = std::max(ba.max_nslot, a.nslot);
-            ba.max_rstride = std::max(ba.max_rstride, a.rstride);
-            ba.max_lmax = std::max(ba.max_lmax, a.lmax);
-            ba.max_nleaf = std::max(ba.max_nleaf, a.nleaf);
-        }
-        // One ring for all: every job's group fits the stage of the widest.
-        WalkShape w = b->plans[0]->shape;
-        fit_ring(w, ba.max_rstride, ba.max_lmax);
-        ba.ring = w.ring;
+    BatchArgs &ba = b->args;
+    memset(&ba, 0, sizeof(ba));
+    ba.jobs = static_cast<const PlanArgs *>(b->jobs.p);
+    ba.items = static_cast<const WalkItem *>(b->items.p);
+    ba.nitems = b->nitems;
+    ba.counter = (unsigned *)(res + (size_t)n * kResultBytes);
+    ba.tile = b->plans[0]->tile;
+    ba.tpp = b->plans[0]->tpp;
+    ba.ppt = b->plans[0]->ppt;
+    ba.kact = kact;
+    ba.max_rstride = 16;
+    for (const PlanArgs &a : jobs) {
+        ba.max_nslot = std::max(ba.max_nslot, a.nslot);
+        ba.max_rstride = std::max(ba.max_rstride, a.rstride);
+        ba.max_lmax = std::max(ba.max_lmax, a.lmax);
     }
+    // One ring for all: every job's group fits the stage of the widest.
+    WalkShape w = b->plans[0]->shape;
+    fit_ring(w, ba.max_rstride, ba.max_lmax);
+    ba.ring = w.ring;
     if (!b->per_node) {
         int dev = 0, nsm = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        b->launches = 0;
-        for (int gi = 0; gi < 2; ++gi) {
-            const BatchArgs &ba = b->args[gi];
-            if (ba.nitems == 0) continue;
-            WalkShape w = b->plans[0]->shape;
-            w.ring = ba.ring;
-            const size_t smem = walk_smem_bytes(w, ba.max_nslot, ba.max_rstride, ba.max_lmax,
-                                                ba.max_nleaf);
-            const int per = batch_ctas_per_sm(w, gi == 0, smem);
-            if (per <= 0 || nsm <= 0) {
-                free_batch(b);
-                return fail(CXG_EINVAL, "cxgBatchCreate: walker does not fit an SM");
-            }
-            b->grid[gi] = (unsigned)(per * nsm);
-            b->launches += 1;
+        b->launches = 1;
+        const size_t smem = walk_smem_bytes(w, ba.max_nslot, ba.max_rstride, ba.max_lmax, 0);
+        const int per = batch_ctas_per_sm(w, smem);
+        if (per <= 0 || nsm <= 0) {
+            free_batch(b);
+            return fail(CXG_EINVAL, "cxgBatchCreate: walker does not fit an SM");
         }
+        b->grid = (unsigned)(per * nsm);
         // Capture one run as a CUDA graph.
         cudaGraph_t graph = nullptr;
         bool began = false;
@@ -1821,7 +1844,7 @@ int cxgBatchInfo(const cxgBatch *b, double *updates, double *alg_bytes,
     if (updates) *updates = b->updates;
     if (alg_bytes) *alg_bytes = b->alg_bytes;
     if (nitems) *nitems = b->nitems;
-    if (grid) *grid = b->grid[0] + b->grid[1];
+    if (grid) *grid = b->grid;
     if (launches_per_run) *launches_per_run = b->launches + 1;  // + P kernel
     return 0;
 }

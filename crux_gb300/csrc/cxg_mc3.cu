@@ -156,7 +156,7 @@ struct Mc3Dev {
     int32_t *kid_tab;     // [c][maxkids]
     uint32_t *nkids;      // [c]
     double *ltab;         // [c][maxkids][16][kact][4] (FP64 chains)
-    char *results;        // [c][32]
+    char *results;        // [c][kResultBytes]
     unsigned *counter;
     double wcdf[kMoves];
     double brlen_lambda, brlen_prior, rate_conc, alpha_lambda, alpha_prior;
@@ -177,7 +177,6 @@ struct Mc3Dev {
     uint64_t trace_cap;
     uint32_t *status;     // nonzero: a model could not be decomposed
     uint32_t nslot_cap;   // shared-memory stack slots of the walker
-    uint32_t staged;      // leaves staged per tile (else streamed)
 };
 
 // wNorm and the root weights of a mixture whose members' eigensystems and
@@ -652,11 +651,12 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
         Philox rng;
         philox_init(rng, d.seed, c, g);
         if (c == 0) *d.counter = 0;
-        char *res = d.results + (size_t)c * 32;
+        char *res = d.results + (size_t)c * kResultBytes;
         // A walker tile that gave up on a bounded wait leaves the ticket
         // counted short; the error word stays set until the run reports it.
         *(uint32_t *)(res + 0) = 0;  // ticket
         *(uint32_t *)(res + 4) = 0;  // ninf
+        for (int i = 0; i < 4; ++i) ((uint64_t *)(res + 32))[i] = 0;  // sum
 
         const Mc3Model &m0 = d.model[c * 2 + d.curmodel[c]];
         Mc3Model &m1 = d.model[c * 2 + (1 - d.curmodel[c])];
@@ -1502,7 +1502,7 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
         hd.nchild = nch;
         hd.slot = op_slot[o];
         hd.flags = 0;
-        hd.next_bytes = 0;
+        hd.pad = 0;
         int kcls[3] = {1, 1, 1};
         unsigned ci = 0, nkid = kid0[o], nl = 0;
         size_t area = sizeof(RecHead) + nch * sizeof(RecChild);
@@ -1514,7 +1514,7 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
             memset(&ch, 0, sizeof(ch));
             if (u < (int)N) {
                 ch.data = d.leafmask[u];
-                ch.idx = (uint32_t)u;  // staged row (leaf u is taxon u)
+                ch.idx = (uint32_t)u;
                 lr[nl++] = d.leafmask[u];
                 ch.src = SRC_LEAF;
                 ch.tab = nkid;
@@ -1609,7 +1609,7 @@ __global__ void mc3_accept_kernel(Mc3Dev d) {
     const unsigned N = d.ntaxa, NN = d.nnodes;
     for (unsigned c = threadIdx.x; c < d.nchains; c += blockDim.x) {
         Mc3Prop &pr = d.prop[c];
-        const char *res = d.results + (size_t)c * 32;
+        const char *res = d.results + (size_t)c * kResultBytes;
         const uint32_t ninf = *(const uint32_t *)(res + 4);
         const double lnL1 = ninf ? -INFINITY
                                  : ((const double *)(res + 16))[0] +
@@ -1845,15 +1845,11 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
                                           child_area_bytes(cfg->precision, K, false))) +
                             15) &
                            ~(size_t)15);
-    WalkShape w = choose_shape(cfg->precision, K, (size_t)C * d.ppad, false);
+    WalkShape w = choose_shape(cfg->precision, K, (size_t)C * d.ppad, C, false);
     const unsigned tile = w.tile;
     d.ntiles = plan_blocks(d.ppad, tile);
-    // Leaves staged per tile or streamed with the op records; stack slots
-    // within the tuned shared-memory budget.
-    d.staged = stages_leaves(w, N);
-    const unsigned lm = d.staged ? 0 : 3, nl = d.staged ? N : 0;
-    fit_ring(w, d.rstride, lm);
-    d.nslot_cap = stack_slots(w, d.rstride, lm, nl);
+    fit_ring(w, d.rstride, 3);
+    d.nslot_cap = stack_slots(w, d.rstride, 3, 0);
     d.seed = cfg->seed;
     d.swap_stride = cfg->swap_stride ? cfg->swap_stride : 1;
     // Without a +I component the +I weight move has nothing to change
@@ -2012,7 +2008,7 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
                                  cfg->precision == CXG_FP64
                                      ? (size_t)C * d.maxkids * 16 * K * 4
                                      : 2)) ||
-        (rc = mc3_upload<char>(h, &d.results, nullptr, (size_t)C * 32 + 16)) ||
+        (rc = mc3_upload<char>(h, &d.results, nullptr, (size_t)C * kResultBytes + 16)) ||
         (rc = mc3_upload<uint32_t>(h, &d.acc, nullptr, (size_t)C * kMoves)) ||
         (rc = mc3_upload<uint32_t>(h, &d.rej, nullptr, (size_t)C * kMoves)) ||
         (rc = mc3_upload<uint32_t>(h, &d.nswap, nullptr, C)) ||
@@ -2031,7 +2027,7 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
         mc3_free(h);
         return rc;
     }
-    d.counter = (unsigned *)(d.results + (size_t)C * 32);
+    d.counter = (unsigned *)(d.results + (size_t)C * kResultBytes);
     {
         void *slab_cl = nullptr, *slab_sc = nullptr;
         if ((rc = mc3_alloc(h, &slab_cl, cl.size() * cl_bytes)) ||
@@ -2050,11 +2046,6 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
         return rc;
     }
     // Walk jobs: one per chain.
-    double *partial = nullptr;
-    if ((rc = mc3_upload<double>(h, &partial, nullptr, (size_t)C * d.ntiles * 2))) {
-        mc3_free(h);
-        return rc;
-    }
     std::vector<PlanArgs> jobs(C);
     std::vector<WalkItem> items;
     for (unsigned c = 0; c < C; ++c) {
@@ -2062,9 +2053,7 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
         memset(&a, 0, sizeof(a));
         a.rec = d.rec + (size_t)c * M * d.rstride;
         a.lrows = d.lrows + (size_t)c * M * 3;
-        a.lmax = d.staged ? 0 : 3;
-        a.leaves = d.staged ? d.leafmask : nullptr;
-        a.nleaf = d.staged ? N : 0;
+        a.lmax = 3;
         a.rstride = d.rstride;
         a.ring = w.ring;
         a.nops = 0;
@@ -2077,11 +2066,11 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
         a.ppad = d.ppad;
         a.root_last = 1;
         a.freqs = dfreq;
-        a.partial = partial + (size_t)c * d.ntiles * 2;
-        a.ticket = (unsigned *)(d.results + (size_t)c * 32);
-        a.ninf = (uint32_t *)(d.results + (size_t)c * 32 + 4);
-        a.err = (uint32_t *)(d.results + (size_t)c * 32 + 8);
-        a.total = (double *)(d.results + (size_t)c * 32 + 16);
+        a.acc = (uint64_t *)(d.results + (size_t)c * kResultBytes + 32);
+        a.ticket = (unsigned *)(d.results + (size_t)c * kResultBytes);
+        a.ninf = (uint32_t *)(d.results + (size_t)c * kResultBytes + 4);
+        a.err = (uint32_t *)(d.results + (size_t)c * kResultBytes + 8);
+        a.total = (double *)(d.results + (size_t)c * kResultBytes + 16);
         a.ltab = d.ltab + (cfg->precision == CXG_FP64 ? (size_t)c * d.maxkids * 16 * K * 4 : 0);
         a.ntiles = d.ntiles;
         a.no_root = 0;
@@ -2107,14 +2096,12 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
     ba.kact = K;
     ba.max_nslot = d.nslot_cap;
     ba.max_rstride = d.rstride;
-    ba.max_lmax = d.staged ? 0 : 3;
-    ba.max_nleaf = d.staged ? N : 0;
-    const size_t smem =
-        walk_smem_bytes(w, d.nslot_cap, d.rstride, ba.max_lmax, ba.max_nleaf);
+    ba.max_lmax = 3;
+    const size_t smem = walk_smem_bytes(w, d.nslot_cap, d.rstride, ba.max_lmax, 0);
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const int per = batch_ctas_per_sm(w, d.staged != 0, smem);
+    const int per = batch_ctas_per_sm(w, smem);
     if (per <= 0) {
         mc3_free(h);
         return fail(CXG_EINVAL, "cxgMc3Create: walker does not fit an SM");
@@ -2200,7 +2187,7 @@ extern "C" int cxgMc3Run(cxgMc3 *h, unsigned long long ngen, double *seconds) {
     cudaEventDestroy(t1);
     if (seconds) *seconds = ms / 1e3;
     uint32_t st = 0;
-    std::vector<char> res((size_t)h->d.nchains * 32);
+    std::vector<char> res((size_t)h->d.nchains * kResultBytes);
     CXG_CUDA(cudaMemcpyAsync(&st, h->d.status, 4, cudaMemcpyDeviceToHost, h->stream));
     CXG_CUDA(cudaMemcpyAsync(res.data(), h->d.results, res.size(), cudaMemcpyDeviceToHost,
                              h->stream));
@@ -2211,7 +2198,7 @@ extern "C" int cxgMc3Run(cxgMc3 *h, unsigned long long ngen, double *seconds) {
     if (st & 2u) return fail(CXG_EINVAL, "MC3: an eTBR move met a malformed tree");
     // Any bounded wait that gave up?
     for (unsigned c = 0; c < h->d.nchains; ++c)
-        if (*(const uint32_t *)(res.data() + (size_t)c * 32 + 8))
+        if (*(const uint32_t *)(res.data() + (size_t)c * kResultBytes + 8))
             return fail(CXG_ETIMEOUT, "MC3 walker: a record copy timed out");
     return 0;
 }
@@ -2409,10 +2396,10 @@ extern "C" int cxgMc3Resume(cxgMc3 *h, unsigned long long generation) {
     CXG_CUDA(cudaMemcpyAsync(&st, d.status, 4, cudaMemcpyDeviceToHost, h->stream));
     CXG_CUDA(cudaStreamSynchronize(h->stream));
     if (st & 1u) return fail(CXG_EINVAL, "cxgMc3Resume: a model cannot be decomposed");
-    std::vector<char> res((size_t)d.nchains * 32);
+    std::vector<char> res((size_t)d.nchains * kResultBytes);
     CXG_CUDA(cudaMemcpy(res.data(), d.results, res.size(), cudaMemcpyDeviceToHost));
     for (unsigned c = 0; c < d.nchains; ++c)
-        if (*(const uint32_t *)(res.data() + (size_t)c * 32 + 8))
+        if (*(const uint32_t *)(res.data() + (size_t)c * kResultBytes + 8))
             return fail(CXG_ETIMEOUT, "MC3 walker: a record copy timed out");
     CXG_CUDA(cudaMemcpy(d.gen, &generation, 8, cudaMemcpyHostToDevice));
     return 0;

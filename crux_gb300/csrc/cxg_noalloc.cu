@@ -189,7 +189,7 @@ extern "C" int cxgLikExecuteNoAlloc(const CxtLik *lik, int precision,
 
     // Scratch layout (same offsets on host and device):
     //   misc 256 | records | elen | cmult | rmult | model | cube | eig | dst |
-    //   tab | pn | leaf rows | ltab | partial
+    //   tab | pn | leaf rows | ltab
     const size_t o_misc = 0;
     const size_t o_rec = 256;
     const size_t o_elen = al16(o_rec + (size_t)(nops ? nops : 1) * rstride);
@@ -217,12 +217,12 @@ extern "C" int cxgLikExecuteNoAlloc(const CxtLik *lik, int precision,
         if (ltab_bytes > kNaTabBudget)
             return fail(CXG_EINVAL, "cxgLikExecuteNoAlloc: leaf tables above 1.5 MiB");
     }
-    const size_t o_part = al16(o_ltab + (ltab_bytes ? ltab_bytes : 16));
-    WalkShape w = choose_shape(prec, kact, ppad, false);
+    const size_t o_end = al16(o_ltab + (ltab_bytes ? ltab_bytes : 16));
+    WalkShape w = choose_shape(prec, kact, ppad, 1, false);
     const unsigned tile = w.tile;
     fit_ring(w, (unsigned)rstride, lmax);
     const unsigned nb = plan_blocks(ppad, tile);
-    if (o_part + (size_t)nb * 16 > kNaScratchBytes)
+    if (o_end > kNaScratchBytes)
         return fail(CXG_EINVAL, "cxgLikExecuteNoAlloc: scratch too small");
     const size_t upload = o_ltab;  // host-packed prefix (misc..root weights)
 
@@ -393,7 +393,7 @@ extern "C" int cxgLikExecuteNoAlloc(const CxtLik *lik, int precision,
     a.rootsc = lik->rootCLC->lnScale;
     a.freqs = dFreqs;
     a.site = dSiteLnL;
-    a.partial = reinterpret_cast<double *>(dev + o_part);
+    a.acc = reinterpret_cast<uint64_t *>(dev + o_misc + 32);
     a.ticket = reinterpret_cast<unsigned *>(dev + o_misc);
     a.ninf = reinterpret_cast<uint32_t *>(dev + o_misc + 4);
     a.err = reinterpret_cast<uint32_t *>(dev + o_misc + 8);

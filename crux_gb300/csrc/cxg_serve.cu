@@ -133,7 +133,6 @@ struct HostPlan {
     unsigned K = 0, ppad = 0, ntiles = 0, nops = 0, nk = 0, nslot = 0, nhbm = 0;
     WalkShape w;
     unsigned lmax = 0;
-    bool staged = false;  // leaves staged per tile (else streamed)
     size_t rstride = 0, job_bytes = 0, data_bytes = 0;
     size_t up_bytes = 0;  // records .. model: the job's one upload
     std::vector<int> order, slot, hbm;
@@ -306,7 +305,7 @@ struct cxgServer {
     std::map<unsigned long long, SrvSession> sessions;
     uint64_t use_clock = 0;
     std::unordered_map<uint64_t, SrvDataset *> datasets;
-    char *pinned = nullptr;  // [kResultSlots][max_active * 32]
+    char *pinned = nullptr;  // [kResultSlots][max_active * kResultBytes]
     bool slot_busy[kResultSlots] = {};
     StagePool stage;  // likelihood worker's upload staging
 };
@@ -328,7 +327,10 @@ void plan_request(SrvRequest &rq, int prec) {
     const unsigned N = r.ntaxa, NN = 2 * N - 2;
     P.K = r.ncat + (r.pinv > 0.0 ? 1 : 0);
     P.ppad = pad_patterns(r.npat);
-    P.w = choose_shape(prec, P.K, P.ppad, false);
+    P.w = choose_shape(prec, P.K, P.ppad, 2, false);
+    // Results kept on the stack need no HBM copy here (a request's CLs are
+    // not kept), and a request with fewer copies is admitted sooner.
+    if (P.w.budget == 0) P.w.budget = 24 * 1024;
     P.ntiles = plan_blocks(P.ppad, P.w.tile);
     const size_t elt = prec == CXG_FP32 ? 4 : 8;
     const unsigned K = P.K;
@@ -364,10 +366,8 @@ void plan_request(SrvRequest &rq, int prec) {
         for (int j = 0; j < 3; ++j) n += (child[v * 3 + j] >= 0 && child[v * 3 + j] < (int)N);
         if (n > P.lmax) P.lmax = n;
     }
-    P.staged = stages_leaves(P.w, N);
-    const unsigned s_lmax = P.staged ? 0 : P.lmax, s_nleaf = P.staged ? N : 0;
-    fit_ring(P.w, (unsigned)P.rstride, s_lmax);
-    const unsigned cap = stack_slots(P.w, (unsigned)P.rstride, s_lmax, s_nleaf);
+    fit_ring(P.w, (unsigned)P.rstride, P.lmax);
+    const unsigned cap = stack_slots(P.w, (unsigned)P.rstride, P.lmax, 0);
     std::vector<int> owner(cap, -1), op_of(NN, -1);
     std::vector<char> need_hbm(nops, 0);
     P.slot.assign(nops, -1);
@@ -430,11 +430,10 @@ void plan_request(SrvRequest &rq, int prec) {
     b += al256((size_t)nops * P.rstride);                // records
     b += al256((size_t)nops * (P.lmax ? P.lmax : 1) * 8);  // leaf rows
     b += al256(kids * (8 + 8 + 4));                      // lens, dsts, tabs
-    b += al256((size_t)P.ntiles * 16);                   // partial sums
     b += al256(sizeof(SrvModel));
     P.up_bytes = al256((size_t)nops * P.rstride) +
                  al256((size_t)nops * (P.lmax ? P.lmax : 1) * 8) + al256(kids * (8 + 8 + 4)) +
-                 al256((size_t)P.ntiles * 16) + sizeof(SrvModel);
+                 sizeof(SrvModel);
     if (prec == CXG_FP64) b += al256(kids * 16 * K * 4 * 8);
     P.job_bytes = b;
     P.data_bytes = dataset_bytes(N, r.npat);
@@ -604,7 +603,6 @@ int prepare_job(cxgServer *S, SrvJob &J, char *stage) {
     const uint8_t **lrows =
         (const uint8_t **)take((size_t)P.nops * (P.lmax ? P.lmax : 1) * sizeof(void *));
     char *kidarr = take((size_t)P.nk * (8 + 8 + 4));
-    double *partial = (double *)take((size_t)P.ntiles * 16);
     SrvModel *model = (SrvModel *)take(sizeof(SrvModel));
     double *ltab = prec == CXG_FP64 ? (double *)take((size_t)P.nk * 16 * K * 4 * 8) : nullptr;
     double *klen = (double *)kidarr;
@@ -649,7 +647,7 @@ int prepare_job(cxgServer *S, SrvJob &J, char *stage) {
             ch.off = (uint32_t)area;
             if (k.src == SRC_LEAF) {
                 ch.data = J.ds->masks + (size_t)k.idx * J.ds->stride;  // taxon's masks
-                ch.idx = (uint32_t)k.idx;                       // its staged row
+                ch.idx = (uint32_t)k.idx;
                 const uint8_t **lr = hlr + (size_t)o * P.lmax;
                 unsigned j = 0;
                 while (lr[j] != nullptr) ++j;
@@ -683,8 +681,6 @@ int prepare_job(cxgServer *S, SrvJob &J, char *stage) {
     hmod.alpha = r.alpha;
     hmod.pinv = r.pinv;
     hmod.ncat = (int32_t)r.ncat;
-    // The partial sums between the kid tables and the model go up too
-    // (unset; the walker writes them before it reads them).
     CXG_CUDA(cudaMemcpyAsync(rec, stage, P.up_bytes, cudaMemcpyHostToDevice, S->s_prep));
     J.model = model;
 
@@ -692,9 +688,7 @@ int prepare_job(cxgServer *S, SrvJob &J, char *stage) {
     memset(&a, 0, sizeof(a));
     a.rec = rec;
     a.lrows = lrows;
-    a.lmax = P.staged ? 0 : P.lmax;
-    a.leaves = P.staged ? J.ds->leaves : nullptr;
-    a.nleaf = P.staged ? N : 0;
+    a.lmax = P.lmax;
     a.rstride = (uint32_t)rstride;
     a.ring = P.w.ring;
     a.nops = P.nops;
@@ -708,7 +702,6 @@ int prepare_job(cxgServer *S, SrvJob &J, char *stage) {
     a.root_last = 1;
     a.pn = model->pn;
     a.freqs = J.ds->weights;
-    a.partial = partial;
     a.ltab = ltab;
     a.ntiles = J.ntiles;
     PmatArgs &pa = J.pa;
@@ -741,20 +734,20 @@ int launch_batch_of(cxgServer *S, SrvBatch &B, cudaStream_t st) {
     std::vector<PmatArgs> pm(n);
     std::vector<uint32_t> prefix(n + 1, 0);
     std::vector<WalkItem> items;
-    unsigned max_nslot = 0, max_rstride = 16, max_lmax = 0, max_nleaf = 0;
+    unsigned max_nslot = 0, max_rstride = 16, max_lmax = 0;
     size_t nitems = 0;
     for (size_t j = 0; j < n; ++j) nitems += B.jobs[j]->ntiles;
     const size_t o_jobs = 0, o_items = al256(n * sizeof(PlanArgs));
     const size_t o_pm = o_items + al256(nitems * sizeof(WalkItem));
     const size_t o_pre = o_pm + al256(n * sizeof(PmatArgs));
     const size_t o_res = o_pre + al256((n + 1) * 4);
-    B.bytes = o_res + al256(n * 32 + 16);
+    B.bytes = o_res + al256(n * kResultBytes + 16);
     B.slot = -1;
     for (int k = 0; k < kResultSlots && B.slot < 0; ++k)
         if (!S->slot_busy[k]) B.slot = k;
     if (B.slot < 0) return fail(CXG_EBUSY, "server: no free result slot");
     S->slot_busy[B.slot] = true;
-    B.host = S->pinned + (size_t)B.slot * S->cfg.max_active * 32;
+    B.host = S->pinned + (size_t)B.slot * S->cfg.max_active * kResultBytes;
     if (const cudaError_t e = dev_malloc_async((void **)&B.mem, B.bytes, st)) {
         B.mem = nullptr;
         return cuda_fail(e, "dev_malloc_async(server batch)");
@@ -763,10 +756,11 @@ int launch_batch_of(cxgServer *S, SrvBatch &B, cudaStream_t st) {
     for (size_t j = 0; j < n; ++j) {
         SrvJob *J = B.jobs[j];
         PlanArgs a = J->a;
-        a.ticket = (unsigned *)(res + j * 32);
-        a.ninf = (uint32_t *)(res + j * 32 + 4);
-        a.err = (uint32_t *)(res + j * 32 + 8);
-        a.total = (double *)(res + j * 32 + 16);
+        a.ticket = (unsigned *)(res + j * kResultBytes);
+        a.ninf = (uint32_t *)(res + j * kResultBytes + 4);
+        a.err = (uint32_t *)(res + j * kResultBytes + 8);
+        a.total = (double *)(res + j * kResultBytes + 16);
+        a.acc = (uint64_t *)(res + j * kResultBytes + 32);
         jobs[j] = a;
         pm[j] = J->pa;
         prefix[j + 1] = prefix[j] + J->nchild * J->kact;
@@ -774,7 +768,6 @@ int launch_batch_of(cxgServer *S, SrvBatch &B, cudaStream_t st) {
         max_nslot = std::max(max_nslot, a.nslot);
         max_rstride = std::max(max_rstride, a.rstride);
         max_lmax = std::max(max_lmax, a.lmax);
-        max_nleaf = std::max(max_nleaf, a.nleaf);
     }
     std::stable_sort(items.begin(), items.end(), [&](const WalkItem &x, const WalkItem &y) {
         return jobs[x.job].nops > jobs[y.job].nops;
@@ -789,7 +782,7 @@ int launch_batch_of(cxgServer *S, SrvBatch &B, cudaStream_t st) {
     const cudaError_t ce = cudaMemcpyAsync(B.mem, host, o_res, cudaMemcpyHostToDevice, st);
     S->stage.hand_off(sb, st);
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemcpyAsync(server batch)");
-    CXG_CUDA(cudaMemsetAsync(res, 0, n * 32 + 16, st));
+    CXG_CUDA(cudaMemsetAsync(res, 0, n * kResultBytes + 16, st));
     CXG_CUDA(launch_pmat_batch((const PmatArgs *)(B.mem + o_pm),
                                (const uint32_t *)(B.mem + o_pre), (uint32_t)n,
                                prefix[n], st));
@@ -797,7 +790,7 @@ int launch_batch_of(cxgServer *S, SrvBatch &B, cudaStream_t st) {
     ba.jobs = (const PlanArgs *)(B.mem + o_jobs);
     ba.items = (const WalkItem *)(B.mem + o_items);
     ba.nitems = (uint32_t)items.size();
-    ba.counter = (unsigned *)(res + n * 32);
+    ba.counter = (unsigned *)(res + n * kResultBytes);
     ba.tile = B.jobs[0]->a.tile;
     ba.tpp = B.jobs[0]->a.tpp;
     ba.ppt = B.jobs[0]->a.ppt;
@@ -805,21 +798,20 @@ int launch_batch_of(cxgServer *S, SrvBatch &B, cudaStream_t st) {
     ba.max_nslot = max_nslot;
     ba.max_rstride = max_rstride;
     ba.max_lmax = max_lmax;
-    ba.max_nleaf = max_nleaf;
     const int prec = S->cfg.precision;
     // One ring for all: every job's group fits the stage of the widest.
     WalkShape w = B.jobs[0]->rq->plan.w;
     fit_ring(w, max_rstride, max_lmax);
     ba.ring = w.ring;
-    const size_t smem = walk_smem_bytes(w, max_nslot, max_rstride, max_lmax, max_nleaf);
+    const size_t smem = walk_smem_bytes(w, max_nslot, max_rstride, max_lmax, 0);
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const int per = batch_ctas_per_sm(w, max_lmax == 0, smem);
+    const int per = batch_ctas_per_sm(w, smem);
     if (per <= 0) return fail(CXG_EINVAL, "server: walker does not fit an SM");
     cudaError_t e = launch_batch(prec, ba, (unsigned)(per * nsm), st);
     if (e != cudaSuccess) return cuda_fail(e, "walk_batch_kernel (server)");
-    CXG_CUDA(cudaMemcpyAsync(B.host, res, n * 32, cudaMemcpyDeviceToHost, st));
+    CXG_CUDA(cudaMemcpyAsync(B.host, res, n * kResultBytes, cudaMemcpyDeviceToHost, st));
     CXG_CUDA(cudaEventCreateWithFlags(&B.done, cudaEventDisableTiming));
     CXG_CUDA(cudaEventRecord(B.done, st));
     B.stream = st;
@@ -832,9 +824,9 @@ void retire(cxgServer *S, SrvBatch &B) {
         SrvJob *J = B.jobs[j];
         uint32_t ninf, err;
         double tot[2];
-        memcpy(&ninf, B.host + j * 32 + 4, 4);
-        memcpy(&err, B.host + j * 32 + 8, 4);
-        memcpy(tot, B.host + j * 32 + 16, 16);
+        memcpy(&ninf, B.host + j * kResultBytes + 4, 4);
+        memcpy(&err, B.host + j * kResultBytes + 8, 4);
+        memcpy(tot, B.host + j * kResultBytes + 16, 16);
         const double v = ninf ? -INFINITY : tot[0] + tot[1];
         if (err) fail(CXG_ETIMEOUT, "walk_batch_kernel (server): record wait timed out");
         complete(S, J->rq->ticket, err ? CXG_ETIMEOUT : 0, v, J->rq->t_submit);
@@ -1018,11 +1010,10 @@ void lnl_loop(cxgServer *S) {
         if (!ready.empty() && inflight.size() < 2) {
             // A failed launch must give its slot back.
             // One launch per walker shape: components, tile, threads per
-            // pattern, staged or streamed leaves.
-            std::map<std::array<unsigned, 5>, std::vector<SrvJob *>> byk;
+            // pattern, patterns per thread.
+            std::map<std::array<unsigned, 4>, std::vector<SrvJob *>> byk;
             for (SrvJob *J : ready)
-                byk[{J->kact, J->a.tile, J->a.tpp, J->a.ppt, J->rq->plan.staged ? 0u : 1u}]
-                    .push_back(J);
+                byk[{J->kact, J->a.tile, J->a.tpp, J->a.ppt}].push_back(J);
             ready.clear();
             for (auto &kv : byk) {
                 SrvBatch B;
@@ -1204,7 +1195,7 @@ extern "C" int cxgServerCreate(const cxgServerConfig *cfg, cxgServer **out) {
     }
     S->budget = cfg->hbm_budget ? (size_t)cfg->hbm_budget : (size_t)(fr * 0.8);
     if ((e = host_alloc((void **)&S->pinned,
-                        (size_t)kResultSlots * S->cfg.max_active * 32)) != cudaSuccess) {
+                        (size_t)kResultSlots * S->cfg.max_active * kResultBytes)) != cudaSuccess) {
         delete S;
         return cuda_fail(e, "cudaHostAlloc(server results)");
     }
