@@ -99,160 +99,108 @@ __device__ inline void pmat_one(const PmatArgs &a, unsigned idx, unsigned q) {
 // [73] status (0 ok, 1 bad input, 2 no convergence).
 // ---------------------------------------------------------------------------
 
-// Pick entry r (0..3) without indexing a register array by a run-time value.
-__device__ __forceinline__ double sel4(int r, double a, double b, double c, double d) {
-    return r == 0 ? a : r == 1 ? b : r == 2 ? c : d;
-}
-
-// The eigensystem of qdecomp4 on four lanes of a warp (lanes base .. base+3,
-// all four calling; out in memory those lanes can all reach, as for
-// qdecomp4).  Lane base+r holds row r of S = Pi^1/2 Q Pi^-1/2 and of the
+// One warp, all 32 lanes calling; out in memory they can all reach.  Lane
+// 4 i + j holds entry (i, j) of S, lane 16 + 4 i + j entry (i, j) of the
 // rotations U.  Jacobi by rounds: each round applies two disjoint rotations,
 // (0,1)(2,3), then (0,2)(1,3), then (0,3)(1,2).  Disjoint rotations commute
 // and neither changes the entries the other's angle is computed from, so
 // taking both angles from the round's starting matrix is the same as
-// applying them one after the other.  Both lanes of a pair use the lower
-// lane's off-diagonal entry, so they compute the same rotation.  Each FP64
-// instruction of a warp costs the same with one lane active or four, so the
-// four lanes do in one instruction stream what qdecomp4 does in four.
-__device__ inline void qdecomp4_warp(const double *rtri, const double *pi, double *out,
-                                     unsigned base) {
+// applying them one after the other.
+//
+// A warp's FP64 instruction takes its SM quarter 64 cycles whether one lane
+// or 32 are active, so what counts is the instructions of one lane: an entry
+// a lane needs 4 per rotation for S and U (a row a lane: 24), the angle comes
+// from two reciprocal square roots (five divisions and roots before), and
+// convergence is read from exponents on the integer pipe.
+__device__ inline void qdecomp_warp(const double *rtri, const double *pi, double *out) {
+    constexpr unsigned kAll = 0xffffffffu;
     const unsigned lane = threadIdx.x & 31u;
-    const int r = (int)(lane - base);
-    const unsigned mask = 0xFu << base;
-    double pn[4];
+    const int i = (int)(lane >> 2) & 3, j = (int)lane & 3;
+    const bool in_s = lane < 16;
     double psum = 0.0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) psum += pi[i];
-    bool ok = true;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        pn[i] = pi[i] / psum;
-        ok = ok && (pn[i] > 0.0);
-    }
-    if (!ok) {  // the same on the four lanes
-        if (r == 0) out[73] = 1.0;
+    for (int k = 0; k < 4; ++k) psum += pi[k];
+    const double pnj = pi[j] / psum;
+    if (!__all_sync(kAll, pnj > 0.0)) {
+        if (lane == 0) out[73] = 1.0;
         return;
     }
-    double rt[6];
-#pragma unroll
-    for (int i = 0; i < 6; ++i) rt[i] = rtri[i];
+    const double pni = __shfl_sync(kAll, pnj, i);
+    const double sqj = sqrt(pnj), sqi = __shfl_sync(kAll, sqj, i);
     // Upper-triangle order of rtri: (0,1) (0,2) (0,3) (1,2) (1,3) (2,3).
-    const int tri[4][4] = {{-1, 0, 1, 2}, {0, -1, 3, 4}, {1, 3, -1, 5},
-                           {2, 4, 5, -1}};
-    double q[16];
-    double qscale = 0.0;
+    const int lo = min(i, j), hi = max(i, j);
+    const double rt = i == j ? 0.0 : rtri[lo == 0 ? hi - 1 : lo + hi];
+    // Q = R Pi with zero row sums; qscale = sum over j < i of 2 Q_ij pi_i.
+    const double q = rt * pnj, qp = q * pni * 2.0;
+    double qscale = 0.0, diag = 0.0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int r = 1; r < 4; ++r)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (i == j) continue;
-            q[i * 4 + j] = rt[tri[i][j]] * pn[j];
-            if (j < i) qscale += q[i * 4 + j] * pn[i] * 2.0;
-        }
+        for (int c = 0; c < r; ++c) qscale += __shfl_sync(kAll, qp, r * 4 + c);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        double d = 0.0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (j != i) d -= q[i * 4 + j];
-        q[i * 4 + i] = d;
+    for (int c = 0; c < 4; ++c) {
+        const double x = __shfl_sync(kAll, q, i * 4 + c);
+        if (c != i) diag -= x;
     }
-    const double sqr = sqrt(sel4(r, pn[0], pn[1], pn[2], pn[3]));
-    double sq[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) sq[j] = __shfl_sync(mask, sqr, base + j);
-    // Row r of S and of U.
-    double s[4], u[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        double e[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            e[i] = (i == j) ? q[i * 4 + i] : rt[tri[i][j]] * sq[i] * sq[j];
-        s[j] = sel4(r, e[0], e[1], e[2], e[3]);
-        u[j] = (j == r) ? 1.0 : 0.0;
-    }
+    const double slo = i < j ? sqi : sqj, shi = i < j ? sqj : sqi;
+    double v = in_s ? (i == j ? diag : rt * slo * shi) : (i == j ? 1.0 : 0.0);
     int conv = 0;
-    for (int sweep = 0; sweep < 64 && !conv; ++sweep) {
-        double offr = 0.0, dgr = 0.0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (j == r) dgr = s[j] * s[j];
-            if (j > r) offr += s[j] * s[j];
-        }
-        // Butterfly sums: every lane adds the same pairs, so all agree.
-        offr += __shfl_xor_sync(mask, offr, 1);
-        offr += __shfl_xor_sync(mask, offr, 2);
-        dgr += __shfl_xor_sync(mask, dgr, 1);
-        dgr += __shfl_xor_sync(mask, dgr, 2);
-        if (offr == 0.0 || offr <= 1e-40 * dgr) {
+    for (int sweep = 0; sweep < 64; ++sweep) {
+        // Off-diagonal entries below 2^-62 of the largest on the diagonal
+        // (by their exponents; a NaN never converges).
+        const unsigned e = (unsigned)__double2hiint(v) & 0x7ff00000u;
+        const unsigned off = __reduce_max_sync(kAll, in_s && i != j ? e : 0u);
+        const unsigned dg = __reduce_max_sync(kAll, in_s && i == j ? e : 0u);
+        if (off == 0u || (off != 0x7ff00000u && off + (62u << 20) <= dg)) {
             conv = 1;
             break;
         }
 #pragma unroll
-        for (int X = 1; X <= 3; ++X) {  // partner of row r: r ^ X
-            const int pr = r ^ X;
-            const int lo = r < pr ? r : pr;
-            // The pair's entries: the diagonals from their own lanes, the
-            // off-diagonal from the lower lane.
-            const double dr = sel4(r, s[0], s[1], s[2], s[3]);
-            const double dp = __shfl_sync(mask, dr, base + pr);
-            const double opr = sel4(pr, s[0], s[1], s[2], s[3]);
-            const double apq = __shfl_sync(mask, opr, base + lo);
-            const double app = r == lo ? dr : dp, aqq = r == lo ? dp : dr;
+        for (int X = 1; X <= 3; ++X) {  // partner of index a: a ^ X
+            const int a = min(j, j ^ X), b = max(j, j ^ X);
+            const double app = __shfl_sync(kAll, v, a * 5);
+            const double aqq = __shfl_sync(kAll, v, b * 5);
+            const double apq2 = 2.0 * __shfl_sync(kAll, v, a * 4 + b);
+            // tan 2 phi = 2 apq / (aqq - app), |phi| <= pi / 4:
+            // c^2 = (1 + |d| / h) / 2, s = 2 apq sign(d) / (2 c h).
             double c = 1.0, sn = 0.0;
-            if (apq != 0.0) {
-                const double th = (aqq - app) / (2.0 * apq);
-                const double t = (th >= 0.0 ? 1.0 : -1.0) /
-                                 (fabs(th) + sqrt(th * th + 1.0));
-                c = 1.0 / sqrt(t * t + 1.0);
-                sn = t * c;
+            const double d = aqq - app, h2 = fma(d, d, apq2 * apq2);
+            if (h2 > 0.0) {
+                const double rh = rsqrt(h2);
+                const double c2 = fma(0.5 * fabs(d), rh, 0.5);
+                const double rc = rsqrt(c2);
+                c = c2 * rc;
+                sn = 0.5 * apq2 * rh * rc;
+                if (d < 0.0) sn = -sn;
+                // To unit length: the rotations stay orthogonal.
+                const double dl = -0.5 * fma(c, c, fma(sn, sn, -1.0));
+                c = fma(c, dl, c);
+                sn = fma(sn, dl, sn);
             }
-            // The other pair's rotation, from one of its lanes.
-            const int ol = r ^ (X == 1 ? 2 : 1);
-            const double co = __shfl_sync(mask, c, base + ol);
-            const double so = __shfl_sync(mask, sn, base + ol);
-            // Columns: row r of S J and of U J.  Column j pairs with j ^ X.
-            double ns[4], nu[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int jp = j ^ X;
-                const bool mine = (j == r) || (j == pr);
-                const double cj = mine ? c : co, sj = mine ? sn : so;
-                if (j < jp) {
-                    ns[j] = cj * s[j] - sj * s[jp];
-                    nu[j] = cj * u[j] - sj * u[jp];
-                } else {
-                    ns[j] = sj * s[jp] + cj * s[j];
-                    nu[j] = sj * u[jp] + cj * u[j];
-                }
-            }
-            // Rows: row r of J^T (S J) mixes with the partner's row.
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const double o = __shfl_sync(mask, ns[j], base + pr);
-                s[j] = (r == lo) ? c * ns[j] - sn * o : sn * o + c * ns[j];
-                u[j] = nu[j];
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (j == pr) s[j] = 0.0;
+            // Columns: (lo, hi) -> (c lo - s hi, s lo + c hi).
+            double o = __shfl_sync(kAll, v, lane ^ X);
+            v = fma(c, v, (j == a ? -sn : sn) * o);
+            // Rows of S, with the rotation of row i's pair.
+            const double ci = __shfl_sync(kAll, c, i), si = __shfl_sync(kAll, sn, i);
+            o = __shfl_sync(kAll, v, lane ^ (X << 2));
+            const double w = fma(ci, v, ((i ^ X) < i ? si : -si) * o);
+            if (in_s) v = (i ^ j) == X ? 0.0 : w;
         }
     }
-    out[r] = sel4(r, pn[0], pn[1], pn[2], pn[3]);
-    if (r == 0) out[4] = 1.0 / qscale;
-    // cube[r][j][k] = V[r][k] V^-1[k][j] with V = Pi^-1/2 U, V^-1 = U^T Pi^1/2.
-    const double isq = 1.0 / sel4(r, sq[0], sq[1], sq[2], sq[3]);
+    if (lane < 4) out[lane] = pnj;
+    if (lane == 0) out[4] = 1.0 / qscale;
+    // cube[i][j][k] = V[i][k] V^-1[k][j] with V = Pi^-1/2 U, V^-1 = U^T Pi^1/2:
+    // two k a lane.
+    const double isq = 1.0 / sqi;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const double ujk = __shfl_sync(mask, u[k], base + j);
-            out[5 + r * 16 + j * 4 + k] = (u[k] * isq) * (ujk * sq[j]);
-        }
-    out[69 + r] = sel4(r, s[0], s[1], s[2], s[3]);
-    if (r == 0) out[73] = conv ? 0.0 : 2.0;
+    for (int t = 0; t < 2; ++t) {
+        const int k = (in_s ? 0 : 2) + t;
+        const double uik = __shfl_sync(kAll, v, 16 + i * 4 + k);
+        const double ujk = __shfl_sync(kAll, v, 16 + j * 4 + k);
+        out[5 + i * 16 + j * 4 + k] = (uik * isq) * (ujk * sqj);
+    }
+    if (in_s && i == j) out[69 + i] = v;
+    if (lane == 0) out[73] = conv ? 0.0 : 2.0;
 }
 
 }  // namespace cxg

@@ -277,6 +277,9 @@ struct WalkItem {
 struct BatchArgs {
     const PlanArgs *jobs;
     const WalkItem *items;
+    // Instead of items: ntiles tiles of each job, in the order of order[].
+    const uint32_t *order;
+    uint32_t ntiles;
     uint32_t nitems;
     unsigned *counter;
     uint32_t tile, ring, kact;

@@ -1529,7 +1529,9 @@ __global__ void __launch_bounds__(CtaOf<T, KT, G, N>::threads, CtaOf<T, KT, G, N
             __syncthreads();
         }
         if (item >= b.nitems) break;
-        const WalkItem it = b.items[item];
+        const WalkItem it = b.order != nullptr
+                                ? WalkItem{b.order[item / b.ntiles], item % b.ntiles}
+                                : b.items[item];
         if (it.job != job) {
             load_job(s_job, b.jobs + it.job);
             job = it.job;
@@ -1722,7 +1724,7 @@ int batch_ctas_per_sm(const WalkShape &w, size_t smem) {
 
 __global__ void qdecomp_kernel(const double *rtri, const double *pi,
                                double *out) {
-    if (blockIdx.x == 0 && threadIdx.x < 4) qdecomp4_warp(rtri, pi, out, 0);
+    if (blockIdx.x == 0) qdecomp_warp(rtri, pi, out);
 }
 
 cudaError_t launch_qdecomp(const double *rtri, const double *pi, double *out,

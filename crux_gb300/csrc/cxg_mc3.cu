@@ -158,6 +158,7 @@ struct Mc3Dev {
     double *ltab;         // [c][maxkids][16][kact][4] (FP64 chains)
     char *results;        // [c][kResultBytes]
     unsigned *counter;
+    uint32_t *order;      // [c] chains, longest walk of the generation first
     double wcdf[kMoves];
     double brlen_lambda, brlen_prior, rate_conc, alpha_lambda, alpha_prior;
     double freq_conc, etbr_pext, invar_lambda, invar_prior;
@@ -186,48 +187,52 @@ struct Mc3Dev {
 // their sum; across members, by weight / (sum of the members' weights).
 // wNorm = 1 / sum of weightScaled * rmult / qNorm over components with
 // non-zero weight and rate; the +I components stay out of it.
+//
+// One warp, lane c the component c; the sums run in component order.
 __device__ void mc3_model_weights(Mc3Model &m, unsigned ncat, unsigned invar,
                                   unsigned mmax) {
-    const unsigned kper = ncat + (invar ? 1u : 0u);
-    double wsum = 0.0;
-    for (int mi = 0; mi < m.nmodels; ++mi) wsum += m.q[mi].weight;
-    double qmean = 0.0;
-    for (unsigned mi = 0; mi < mmax; ++mi) {
+    const unsigned kper = ncat + (invar ? 1u : 0u), K = mmax * kper;
+    const unsigned c = threadIdx.x & 31u;
+    double ws = 0.0, rate = 0.0;  // this component's part of 1 / wNorm
+    bool in_sum = false;
+    if (c < K) {
+        double wsum = 0.0;
+        for (int mi = 0; mi < m.nmodels; ++mi) wsum += m.q[mi].weight;
+        const unsigned mi = c / kper, k = c % kper;
         const bool on = (int)mi < m.nmodels;
         const unsigned src = on ? mi : 0u;
         const Mc3Sub &s = m.q[src];
-        double cw[kMaxComps], cm[kMaxComps], cwsum = 0.0;
-        for (unsigned k = 0; k < ncat; ++k) {
-            cw[k] = s.wvar / ncat;
-            cm[k] = ncat == 1 ? 1.0 : s.gcat[k];
-        }
-        if (ncat > 1 && !s.gamma_on) {
-            // Lik.setAlpha(INFINITY), Lik.pyx:1264-1273: the first category
-            // takes all the variable weight at rate 1, the others weight 0.
-            cw[0] = s.wvar;
-            cm[0] = 1.0;
-            for (unsigned k = 1; k < ncat; ++k) {
-                cw[k] = 0.0;
-                cm[k] = 0.0;
-            }
-        }
-        if (invar) {
-            cw[ncat] = s.winvar;
-            cm[ncat] = 0.0;
-        }
-        for (unsigned k = 0; k < kper; ++k) cwsum += cw[k];
-        for (unsigned k = 0; k < kper; ++k) {
-            const unsigned c = mi * kper + k;
-            const double ws = on ? (s.weight / wsum) * (cw[k] / cwsum) : 0.0;
-            m.cmult[c] = cm[k];
-            m.rmult[c] = s.rmult;
-            m.midx[c] = (int32_t)src;
-            if (ws != 0.0 && cm[k] != 0.0) qmean += ws * (s.rmult / m.qnorm[src]);
-            for (int i = 0; i < 4; ++i) m.pn[c * 4 + i] = m.pinorm[src * 4 + i] * ws;
-        }
+        // Lik.setAlpha(INFINITY), Lik.pyx:1264-1273, with Gamma off: the
+        // first category takes all the variable weight at rate 1, the others
+        // weight 0.
+        const bool off = ncat > 1 && !s.gamma_on;
+        const double each = s.wvar / ncat;
+        auto weight_of = [&](unsigned q) {
+            return q == ncat ? s.winvar : off ? (q == 0 ? s.wvar : 0.0) : each;
+        };
+        double cwsum = 0.0;
+        for (unsigned q = 0; q < kper; ++q) cwsum += weight_of(q);
+        const double cm = k == ncat ? 0.0
+                          : off     ? (k == 0 ? 1.0 : 0.0)
+                          : ncat == 1 ? 1.0 : s.gcat[k];
+        ws = on ? (s.weight / wsum) * (weight_of(k) / cwsum) : 0.0;
+        m.cmult[c] = cm;
+        m.rmult[c] = s.rmult;
+        m.midx[c] = (int32_t)src;
+        in_sum = ws != 0.0 && cm != 0.0;
+        rate = s.rmult / m.qnorm[src];
+        for (int i = 0; i < 4; ++i) m.pn[c * 4 + i] = m.pinorm[src * 4 + i] * ws;
     }
-    m.wnorm = 1.0 / qmean;
-    m.ok = 1;
+    double qmean = 0.0;
+    for (unsigned q = 0; q < K; ++q) {
+        const double wq = __shfl_sync(0xffffffffu, ws, q);
+        const double rq = __shfl_sync(0xffffffffu, rate, q);
+        if (__shfl_sync(0xffffffffu, (int)in_sum, q)) qmean = fma(wq, rq, qmean);
+    }
+    if (c == 0) {
+        m.wnorm = 1.0 / qmean;
+        m.ok = 1;
+    }
 }
 
 // Parts of a model to derive again: FIN_EIG (rates or frequencies changed),
@@ -238,60 +243,91 @@ enum : unsigned { FIN_EIG = 1, FIN_GAMMA = 2, FIN_ALL = 3, FIN_WEIGHTS = 4 };
 // Derived quantities of mixture member `mi`: its Q eigensystem (FP64
 // Jacobi on the device) and Gamma category rates, then wNorm and the root
 // weights of the whole mixture (Lik.pyx:1603-1665); the parts `what` does
-// not name are kept.  One warp: lanes 0..ncat-2 compute the Gamma category
-// cuts while lanes 28..31 form the eigensystem; lane 0 finishes.  All 32
-// lanes of the warp call it; the result (true: decomposed) is lane 0's.
-__device__ bool mc3_model_finish_warp(Mc3Model &m, unsigned ncat, unsigned invar,
-                                      unsigned mmax, unsigned what, unsigned mi) {
+// not name are kept.  Three warps, threads 32..127 of a block: a warp's FP64
+// instruction holds its SM quarter for 64 cycles, so the Gamma cuts go to
+// one warp each (their series run different lengths) and the eigensystem to
+// the third.  The result (true: decomposed) is thread 32's.
+__device__ bool mc3_model_finish(Mc3Model &m, unsigned ncat, unsigned invar, unsigned mmax,
+                                 unsigned what, unsigned mi) {
     __shared__ double s_cut[kMaxComps];
     __shared__ double s_eig[74];
     __shared__ int s_bad;
     Mc3Sub &q = m.q[mi];
-    const unsigned lane = threadIdx.x & 31u;
-    if (lane == 0) s_bad = 0;
-    __syncwarp();
-    if ((what & FIN_GAMMA) && ncat > 1 && q.gamma_on && lane < ncat - 1) {
-        const double cut = d_gamma_cut(q.alpha, (int)ncat, (int)lane);
+    const unsigned lane = threadIdx.x & 31u, w = (threadIdx.x >> 5) - 1u;
+    const bool gamma = (what & FIN_GAMMA) && ncat > 1 && q.gamma_on;
+    if (threadIdx.x == 32) s_bad = 0;
+    asm volatile("bar.sync 1, 96;" ::: "memory");
+    if (gamma && w + 3 * lane < ncat - 1) {
+        const double cut = d_gamma_cut(q.alpha, (int)ncat, (int)(w + 3 * lane));
         if (cut == -1.0)
             s_bad = 1;
         else
-            s_cut[lane] = cut;
+            s_cut[w + 3 * lane] = cut;
     }
-    if ((what & FIN_EIG) && lane >= 28) qdecomp4_warp(q.rates, q.freqs, s_eig, 28);
     __syncwarp();
-    if ((what & FIN_EIG) && lane == 31) {
-        const double *tmp = s_eig;
-        if (tmp[73] != 0.0) {
-            s_bad = 1;
+    if ((what & FIN_EIG) && w == 2) {
+        qdecomp_warp(q.rates, q.freqs, s_eig);
+        __syncwarp();
+        if (s_eig[73] != 0.0) {
+            if (lane == 0) s_bad = 1;
         } else {
-            for (int i = 0; i < 4; ++i) m.pinorm[mi * 4 + i] = tmp[i];
-            m.qnorm[mi] = tmp[4];
-            for (int i = 0; i < 64; ++i) m.cube[mi * 64 + i] = tmp[5 + i];
-            for (int i = 0; i < 4; ++i) m.eig[mi * 4 + i] = tmp[69 + i];
+            if (lane < 4) {
+                m.pinorm[mi * 4 + lane] = s_eig[lane];
+                m.eig[mi * 4 + lane] = s_eig[69 + lane];
+            }
+            if (lane == 0) m.qnorm[mi] = s_eig[4];
+            m.cube[mi * 64 + lane] = s_eig[5 + lane];
+            m.cube[mi * 64 + 32 + lane] = s_eig[37 + lane];
         }
     }
-    __syncwarp();
-    if (lane != 0) return false;
-    if (s_bad) return false;
-    if ((what & FIN_GAMMA) && ncat > 1 && q.gamma_on) {
-        for (unsigned i = 0; i + 1 < ncat; ++i) q.gcat[i] = s_cut[i];
-        d_gamma_rates_from_cuts((int)ncat, q.gcat);
+    asm volatile("bar.sync 1, 96;" ::: "memory");
+    const bool ok = s_bad == 0;
+    if (w == 0 && ok) {
+        if (gamma && lane == 0) {
+            for (unsigned i = 0; i + 1 < ncat; ++i) q.gcat[i] = s_cut[i];
+            d_gamma_rates_from_cuts((int)ncat, q.gcat);
+        }
+        __syncwarp();
+        mc3_model_weights(m, ncat, invar, mmax);
     }
-    mc3_model_weights(m, ncat, invar, mmax);
-    return true;
+    asm volatile("bar.sync 1, 96;" ::: "memory");  // the shared words are free
+    return ok;
 }
 
 __global__ void mc3_init_kernel(Mc3Dev d) {
     const unsigned c = blockIdx.x;
-    if (c >= d.nchains || threadIdx.x >= 32) return;
+    if (c >= d.nchains || threadIdx.x < 32) return;
     Mc3Model &m = d.model[c * 2 + d.curmodel[c]];
     bool ok = true;
     for (int mi = 0; mi < m.nmodels; ++mi)
-        ok &= mc3_model_finish_warp(m, d.ncat, d.invar, d.mmax, FIN_ALL, (unsigned)mi);
-    if (threadIdx.x == 0 && !ok) atomicOr(d.status, 1u);
+        ok &= mc3_model_finish(m, d.ncat, d.invar, d.mmax, FIN_ALL, (unsigned)mi);
+    if (threadIdx.x == 32 && !ok) atomicOr(d.status, 1u);
 }
 
-// log density of Dirichlet(alpha) at x (both length n).
+// Terms of two log Dirichlet densities, ln D(alpha0; x0) - ln D(alpha1; x1)
+// of n values each, computed by a warp (a logarithm and a log gamma a lane:
+// one thread took 60 us over 14 of them) and added in index order.
+struct DirichletPair {
+    int n;  // 0: none
+    double alpha[2][6], x[2][6];
+};
+__device__ double ln_dirichlet_ratio(const DirichletPair &p) {
+    const unsigned lane = threadIdx.x & 31u;
+    const int side = (int)(lane >> 3) & 1, i = (int)lane & 7;
+    double s = 0.0;
+    for (int k = 0; k < p.n; ++k) s += p.alpha[side][k];
+    double lg = 0.0, term = 0.0;
+    if (lane < 16 && (i < p.n || i == 7)) {
+        const double al = i == 7 ? s : p.alpha[side][i];
+        lg = lgamma(al);
+        if (i < p.n) term = (al - 1.0) * log(p.x[side][i]) - lg;
+    }
+    double r = 0.0;
+    for (int k = 0; k < p.n; ++k) r += __shfl_sync(0xffffffffu, term, (side << 3) + k);
+    r += __shfl_sync(0xffffffffu, lg, (side << 3) + 7);
+    return __shfl_sync(0xffffffffu, r, 0) - __shfl_sync(0xffffffffu, r, 8);
+}
+
 // Partitions of the six exchangeabilities into k classes, k = 1..6
 // (Stirling numbers of the second kind S(6, k)).
 __constant__ double kStirling6[7] = {0.0, 1.0, 31.0, 90.0, 65.0, 15.0, 1.0};
@@ -303,15 +339,6 @@ __device__ void rgs_normalize(int32_t *rc) {
         if (map[rc[i]] < 0) map[rc[i]] = next++;
         rc[i] = map[rc[i]];
     }
-}
-
-__device__ double ln_dirichlet(const double *alpha, const double *x, int n) {
-    double s = 0.0, r = 0.0;
-    for (int i = 0; i < n; ++i) {
-        s += alpha[i];
-        r += (alpha[i] - 1.0) * log(x[i]) - lgamma(alpha[i]);
-    }
-    return r + lgamma(s);
 }
 
 // Mixture members.  A member's prior density (in log) is the product of
@@ -645,9 +672,21 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
     __shared__ int s_nd, s_lowest, s_fl;
     __shared__ unsigned s_fin, s_fin_mi;
     __shared__ bool s_full, s_etbr;
+    __shared__ DirichletPair s_dir;  // a move's Hastings ratio, taken by a warp below
     if (threadIdx.x == 0) {
         s_fin = 0;
         s_etbr = false;
+        s_dir.n = 0;
+        auto keep_dirichlet = [&](const double *al0, const double *x0, const double *al1,
+                                  const double *x1, int n) {
+            for (int i = 0; i < n; ++i) {
+                s_dir.alpha[0][i] = al0[i];
+                s_dir.x[0][i] = x0[i];
+                s_dir.alpha[1][i] = al1[i];
+                s_dir.x[1][i] = x1[i];
+            }
+            s_dir.n = n;
+        };
         Philox rng;
         philox_init(rng, d.seed, c, g);
         if (c == 0) *d.counter = 0;
@@ -1136,7 +1175,7 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
                 }
                 Mc3Sub &q1 = m1.q[mi];
                 for (int i = 0; i < 4; ++i) q1.freqs[i] = f1[i];
-                pr.lnHast = ln_dirichlet(a1, f0, 4) - ln_dirichlet(a0, f1, 4);
+                keep_dirichlet(a1, f0, a0, f1, 4);
                 pr.model_changed = 1;
                 s_fin = FIN_EIG;
                 full = true;
@@ -1162,7 +1201,7 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
                 }
                 Mc3Sub &q1 = m1.q[mi];
                 for (int i = 0; i < 6; ++i) q1.rates[i] = r1[q0.rclass[i]] * s0;
-                pr.lnHast = ln_dirichlet(a1, r0, k) - ln_dirichlet(a0, r1, k);
+                keep_dirichlet(a1, r0, a0, r1, k);
                 pr.model_changed = 1;
                 s_fin = FIN_EIG;
                 full = true;
@@ -1328,11 +1367,16 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
         }
         __syncthreads();
     }
-    // The proposed model's derived quantities (a second warp) while thread
-    // 0 lists the dirty nodes and assigns stack slots.
-    if (threadIdx.x >= 32 && threadIdx.x < 64 && s_fin) {
+    // The proposed model's derived quantities and a Dirichlet move's Hastings
+    // ratio (the other warps) while thread 0 lists the dirty nodes and
+    // assigns stack slots.
+    if (threadIdx.x >= 32 && threadIdx.x < 64 && s_dir.n > 0) {
+        const double h = ln_dirichlet_ratio(s_dir);
+        if (threadIdx.x == 32) pr.lnHast = h;
+    }
+    if (threadIdx.x >= 32 && s_fin) {
         Mc3Model &m1 = d.model[c * 2 + (1 - d.curmodel[c])];
-        const bool ok = mc3_model_finish_warp(m1, d.ncat, d.invar, d.mmax, s_fin, s_fin_mi);
+        const bool ok = mc3_model_finish(m1, d.ncat, d.invar, d.mmax, s_fin, s_fin_mi);
         if (threadIdx.x == 32 && !ok) {
             // A model that cannot be decomposed is rejected outright.
             pr.lnPrior = -INFINITY;
@@ -1575,6 +1619,19 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
 
 // P matrices of every chain's child edges.
 __global__ void mc3_pmat_kernel(Mc3Dev d) {
+    // The walker takes the chains with the longest walks first (a model move
+    // walks every node, a branch move one path), so that no long tile starts
+    // when the others have ended.
+    if (blockIdx.x == 0)
+        for (unsigned c = threadIdx.x; c < d.nchains; c += blockDim.x) {
+            const uint32_t n = d.jobs[c].nops;
+            unsigned rank = 0;
+            for (unsigned q = 0; q < d.nchains; ++q) {
+                const uint32_t m = d.jobs[q].nops;
+                rank += m > n || (m == n && q < c);
+            }
+            d.order[rank] = c;
+        }
     // Four lanes per (chain, kid, comp), see pmat_one.
     const unsigned t = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
     const unsigned per = d.maxkids * d.kact;
@@ -2004,6 +2061,7 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
         (rc = mc3_upload<uint64_t>(h, &d.kid_dst, nullptr, (size_t)C * d.maxkids)) ||
         (rc = mc3_upload<int32_t>(h, &d.kid_tab, nullptr, (size_t)C * d.maxkids)) ||
         (rc = mc3_upload<uint32_t>(h, &d.nkids, nullptr, C)) ||
+        (rc = mc3_upload<uint32_t>(h, &d.order, nullptr, C)) ||
         (rc = mc3_upload<double>(h, &d.ltab, nullptr,
                                  cfg->precision == CXG_FP64
                                      ? (size_t)C * d.maxkids * 16 * K * 4
@@ -2047,7 +2105,6 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
     }
     // Walk jobs: one per chain.
     std::vector<PlanArgs> jobs(C);
-    std::vector<WalkItem> items;
     for (unsigned c = 0; c < C; ++c) {
         PlanArgs a;
         memset(&a, 0, sizeof(a));
@@ -2076,18 +2133,17 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
         a.no_root = 0;
         jobs[c] = a;
     }
-    for (unsigned t = 0; t < d.ntiles; ++t)
-        for (unsigned c = 0; c < C; ++c) items.push_back(WalkItem{c, t});
-    WalkItem *ditems = nullptr;
     e = cudaMemcpy(d.jobs, jobs.data(), C * sizeof(PlanArgs), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess || (rc = mc3_upload(h, &ditems, items.data(), items.size()))) {
+    if (e != cudaSuccess) {
         mc3_free(h);
-        return rc ? rc : cuda_fail(e, "cudaMemcpy(jobs)");
+        return cuda_fail(e, "cudaMemcpy(jobs)");
     }
     BatchArgs &ba = h->ba;
     ba.jobs = d.jobs;
-    ba.items = ditems;
-    ba.nitems = (uint32_t)items.size();
+    ba.items = nullptr;
+    ba.order = d.order;
+    ba.ntiles = d.ntiles;
+    ba.nitems = C * d.ntiles;
     ba.counter = d.counter;
     ba.tile = tile;
     ba.tpp = w.tpp;
@@ -2117,7 +2173,7 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
         }
     }
     // Derived model quantities, then generation 0 (full evaluation).
-    mc3_init_kernel<<<C, 32, 0, h->stream>>>(d);
+    mc3_init_kernel<<<C, 128, 0, h->stream>>>(d);
     if ((e = cudaGetLastError()) != cudaSuccess) {
         mc3_free(h);
         return cuda_fail(e, "mc3_init_kernel");
@@ -2388,7 +2444,7 @@ extern "C" int cxgMc3Resume(cxgMc3 *h, unsigned long long generation) {
     CXG_CUDA(cudaMemcpy(d.gen, &g0, 8, cudaMemcpyHostToDevice));
     const uint32_t st0 = 0;
     CXG_CUDA(cudaMemcpy(d.status, &st0, 4, cudaMemcpyHostToDevice));
-    mc3_init_kernel<<<d.nchains, 32, 0, h->stream>>>(d);
+    mc3_init_kernel<<<d.nchains, 128, 0, h->stream>>>(d);
     CXG_CHECK_LAUNCH("mc3_init_kernel");
     int rc = mc3_enqueue_gen(h);
     if (rc) return rc;

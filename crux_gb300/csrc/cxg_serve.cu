@@ -73,26 +73,34 @@ __global__ void srv_model_kernel(SrvModelList list, unsigned n) {
     __shared__ double tmp[74];
     __shared__ double cut[kMaxComps];
     __shared__ int bad;
-    const unsigned lane = threadIdx.x;
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const int ncat = m->ncat;
-    if (lane == 0) bad = 0;
-    __syncwarp();
-    if (ncat > 1 && (int)lane < ncat - 1) {
-        const double c = d_gamma_cut(m->alpha, ncat, (int)lane);
-        if (c == -1.0)
-            bad = 1;
-        else
-            cut[lane] = c;
+    if (threadIdx.x == 0) bad = 0;
+    __syncthreads();
+    // One Gamma cut to a warp at a time (each on its own FP64 pipe), the
+    // eigensystem on the fourth.
+    if (warp < 3) {
+        const int i = (int)(warp + 3 * lane);
+        if (ncat > 1 && i < ncat - 1) {
+            const double c = d_gamma_cut(m->alpha, ncat, i);
+            if (c == -1.0)
+                bad = 1;
+            else
+                cut[i] = c;
+        }
+    } else {
+        qdecomp_warp(m->rates, m->freqs, tmp);
     }
-    if (lane >= 28) qdecomp4_warp(m->rates, m->freqs, tmp, 28);
-    __syncwarp();
-    if (lane != 0) return;
+    __syncthreads();
+    if (tmp[73] == 0.0 && !bad) {
+        if (threadIdx.x < 64) m->cube[threadIdx.x] = tmp[5 + threadIdx.x];
+    }
+    if (threadIdx.x != 0) return;
     m->ok = 0;
     if (tmp[73] != 0.0 || bad) return;
     double pin[4];
     for (int i = 0; i < 4; ++i) pin[i] = tmp[i];
     const double qnorm = tmp[4];
-    for (int i = 0; i < 64; ++i) m->cube[i] = tmp[5 + i];
     for (int i = 0; i < 4; ++i) m->eig[i] = tmp[69 + i];
     if (ncat > 1) {
         for (int i = 0; i + 1 < ncat; ++i) m->cmult[i] = cut[i];
@@ -977,7 +985,7 @@ void lnl_loop(cxgServer *S) {
                     (unsigned)std::min<size_t>(kModelsPerLaunch, prepared.size() - i);
                 SrvModelList ml;
                 for (unsigned j = 0; j < nm; ++j) ml.m[j] = prepared[i + j]->model;
-                srv_model_kernel<<<nm, 32, 0, S->s_prep>>>(ml, nm);
+                srv_model_kernel<<<nm, 128, 0, S->s_prep>>>(ml, nm);
                 const cudaError_t e = cudaGetLastError();
                 for (unsigned j = 0; j < nm; ++j) {
                     SrvJob *J = prepared[i + j];
