@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 
 #include <mutex>
@@ -30,8 +31,8 @@ constexpr unsigned kPatternQuantum = 128;
 constexpr unsigned kBlock = 128;
 // Largest CTA a caller may tune: tile patterns x threads per pattern.
 constexpr unsigned kTuneThreads = 256;
-// Largest CTA of the plan walkers.  18 warps: 80,000 patterns on 152 SMs are
-// 17 warps an SM, which one CTA of 112 registers a thread holds.
+// Largest CTA of the plan walkers (the wide build: the 20 warps that an SM's
+// registers hold at 96 a thread).
 constexpr unsigned kMaxThreads = 640;
 // Largest CTA of the op-lane walker: 2 lanes x tile patterns (tile <= 64).
 constexpr unsigned kLaneThreads = 128;
@@ -56,11 +57,26 @@ inline unsigned pad_patterns(unsigned p) {
     return (p + kPatternQuantum - 1) / kPatternQuantum * kPatternQuantum;
 }
 
-// A job's result words, cleared before its walk: ticket, -inf count, error
-// word, pad (4 bytes each), total [2 doubles], sum limbs [4 x 8].
-constexpr size_t kResultBytes = 64;
-// Those read back.
-constexpr size_t kResultRead = 32;
+// A job's result, cleared before its walk: how many sites are at -inf, the
+// error word (nonzero: a bounded wait gave up), and the sum of the other site
+// lnLs in fixed point with 64 fraction bits, as four 32-bit limbs in 64-bit
+// accumulators (the top one signed).
+struct WalkResult {
+    uint32_t ninf, err, pad[2];
+    uint64_t acc[4];
+    __host__ __device__ double lnL() const {
+        if (ninf) return -INFINITY;
+        typedef unsigned __int128 u128;
+        u128 t = (u128)(__int128)(long long)acc[3] << 96;
+        for (int i = 0; i < 3; ++i) t += (u128)acc[i] << (32 * i);
+        const bool neg = (t >> 127) != 0;
+        if (neg) t = (u128)0 - t;
+        const double v = (double)(uint64_t)(t >> 64) +
+                         (double)(uint64_t)t * 0x1p-64;
+        return neg ? -v : v;
+    }
+};
+static_assert(sizeof(WalkResult) == 48, "cleared and copied in 16-byte units");
 
 // Where a child's CL comes from during a plan walk.
 enum : uint32_t {
@@ -195,17 +211,15 @@ struct PlanArgs {
     const void *rootsc;   // root scaler
     const uint32_t *freqs;// [npat] pattern weights (charFreqs + cbase)
     double *site;         // [npat] site lnL out (may be null)
-    uint64_t *acc;        // [4] limbs of the sum of site lnLs, cleared before
-    uint32_t *ninf;       // count of -inf sites
-    unsigned *ticket;     // last-block counter
-    double *total;        // [2] the sum: integer and fraction part
-    uint32_t *err;        // nonzero: a bounded wait gave up
+    WalkResult *res;      // cleared before the walk
     const double *ltab;   // FP64 plans: [ntab][16 masks][kact][4]
     uint32_t ntiles;      // tiles of this job (ppad / tile, rounded up)
     uint32_t no_root;     // 1: stop after the ops (per-node launches)
     uint32_t tpp;         // threads per pattern (each holds kact / tpp
                           // components); 0 is read as 1
     uint32_t ppt;         // patterns per thread (1 or 2); 0 is read as 1
+    uint32_t wide;        // WalkShape::wide
+    uint32_t pad;
 };
 
 // Threads per pattern and patterns per thread a walker is built for with
@@ -234,16 +248,21 @@ inline bool walker_shape_ok(int precision, unsigned kact, unsigned tpp,
 struct WalkShape {
     int precision = CXG_FP64;
     unsigned kact = 1, tile = kTile, tpp = 1, ppt = 1, lanes = 1, ring = kRing;
+    bool wide = false;  // the 96-register build of the walker
     size_t budget = 0;  // bytes of the CL stack
+    size_t ring_bytes = 42 * 1024;
+    // Threads of a CTA (of one op lane).
+    unsigned threads() const { return tile / ppt * tpp; }
 };
 
-// Largest CTA the walker of KT components a thread, G threads per pattern and
-// N patterns per thread is built for.  The wide FP32 walkers are held to the
-// registers of one CTA of 576 threads, the others to 128 (two of 256).
-__host__ __device__ constexpr unsigned walker_threads(int precision, unsigned KT, unsigned G,
-                                                      unsigned N) {
-    return precision == CXG_FP32 && G == 1 && N == 1 && KT <= 5 ? kMaxThreads : kTuneThreads;
+// The wide build of the FP32 walker (single plans of up to five components):
+// 96 registers a thread and CTAs of up to kMaxThreads, so that 20 warps run
+// on an SM where the 128-register build keeps 16.
+inline bool wide_shape_ok(const WalkShape &w) {
+    return w.precision == CXG_FP32 && w.tpp == 1 && w.ppt == 1 && w.lanes == 1 && w.kact <= 5;
 }
+// Largest CTA the walkers of this shape are built for.
+inline unsigned walker_threads(const WalkShape &w) { return w.wide ? kMaxThreads : kTuneThreads; }
 
 // The walker's shared memory: barriers and counts, the ring's stages,
 // the CL stack and its scalers.
@@ -329,8 +348,8 @@ struct PmatArgs {
     const double *wnorm_dev;   // if set, wNorm is read here (model built on the GPU)
     unsigned char *rec;
     double *ltab;              // FP64 plans: leaf-message tables
-    uint64_t *zero = nullptr;  // pmat_kernel: kResultBytes cleared before the
-                               // walker that follows it runs (its result)
+    WalkResult *zero = nullptr;  // pmat_kernel: cleared before the walker that
+                                 // follows it runs (its result)
 };
 
 // Allocations of the library (cxg_lik.cu); each fails as an out-of-memory

@@ -50,10 +50,9 @@ __device__ __forceinline__ void pdl_wait() {
 
 __global__ void pmat_kernel(PmatArgs a) {
     pdl_launch_dependents();
-    // The walker's result words (ticket, counts, sum): it reads them only
-    // after this grid has completed (stream order, or griddepcontrol.wait).
-    if (a.zero != nullptr && blockIdx.x == 0 && threadIdx.x < kResultBytes / 8)
-        a.zero[threadIdx.x] = 0;
+    // The walker's result: it adds to it only after this grid has completed (stream order, or griddepcontrol.wait).
+    if (a.zero != nullptr && blockIdx.x == 0 && threadIdx.x < sizeof(WalkResult) / 8)
+        reinterpret_cast<uint64_t *>(a.zero)[threadIdx.x] = 0;
     const unsigned idx = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
     if (idx >= a.nchild * a.kact) return;  // the same for all four lanes
     pmat_one(a, idx, threadIdx.x & 3u);
@@ -126,8 +125,8 @@ __device__ __forceinline__ fixed128 warp_sum(fixed128 f) {
 }
 
 // Add the CTA's site values (finite ones; -inf sites are counted) to the
-// job's sum, four 32-bit limbs in 64-bit accumulators a.acc (cleared with the
-// job's result words); the last tile of the job to finish writes the total.
+// job's result.  No tile waits to be the last: whoever reads the result puts
+// the limbs together.
 template <int NV>
 __device__ void reduce_sites(const PlanArgs &a, const double (&v)[NV],
                              const bool (&neg_inf)[NV]) {
@@ -143,43 +142,22 @@ __device__ void reduce_sites(const PlanArgs &a, const double (&v)[NV],
         ninf += __popc(__ballot_sync(0xffffffffu, neg_inf[h]));
     }
     f = warp_sum(f);
-    if (lane < 4) {
-        // The top limb keeps the sign.
-        const uint64_t w = (uint64_t)(f >> (32 * lane));
-        s_limb[warp][lane] = lane == 3 ? (uint64_t)(long long)(int)(uint32_t)w : (uint32_t)w;
-        if (lane == 0) s_ninf[warp] = ninf;
+    // The top limb keeps the sign.
+    const uint64_t w = (uint64_t)(f >> (32 * (lane & 3u)));
+    uint64_t limb = lane == 3 ? (uint64_t)(long long)(int)(uint32_t)w : (uint32_t)w;
+    if (nwarp > 1) {
+        if (lane < 4) s_limb[warp][lane] = limb;
+        if (lane == 4) s_ninf[warp] = ninf;
+        __syncthreads();
+        if (warp == 0 && lane < 4)
+            for (unsigned q = 1; q < nwarp; ++q) limb += s_limb[q][lane];
+        if (warp == 0 && lane == 4)
+            for (unsigned q = 1; q < nwarp; ++q) ninf += s_ninf[q];
     }
-    __syncthreads();
     if (warp == 0) {
-        uint64_t sum = 0;
-        ninf = 0;
         if (lane < 4)
-            for (unsigned w = 0; w < nwarp; ++w) sum += s_limb[w][lane];
-        if (lane == 4)
-            for (unsigned w = 0; w < nwarp; ++w) ninf += s_ninf[w];
-        if (lane < 4) atomicAdd(reinterpret_cast<unsigned long long *>(a.acc) + lane, sum);
-        if (lane == 4 && ninf) atomicAdd(a.ninf, ninf);
-        __threadfence();
-        __syncwarp();
-        unsigned t = 0;
-        if (lane == 0) t = atomicAdd(a.ticket, 1u);
-        if (__shfl_sync(0xffffffffu, t, 0) == a.ntiles - 1) {
-            __threadfence();
-            if (lane == 0) {
-                const volatile uint64_t *q = a.acc;
-                fixed128 T = 0;
-                for (int i = 0; i < 4; ++i)
-                    T += (i == 3 ? (fixed128)(__int128)(long long)q[i] : (fixed128)q[i])
-                         << (32 * i);
-                const bool neg = (T >> 127) != 0;
-                if (neg) T = (fixed128)0 - T;
-                const double hi = (double)(uint64_t)(T >> 64);
-                const double lo = (double)(uint64_t)T * 5.421010862427522e-20;  // 2^-64
-                a.total[0] = neg ? -hi : hi;
-                a.total[1] = neg ? -lo : lo;
-                *a.ticket = 0;
-            }
-        }
+            atomicAdd(reinterpret_cast<unsigned long long *>(a.res->acc) + lane, limb);
+        if (lane == 4 && ninf) atomicAdd(&a.res->ninf, ninf);
     }
     __syncthreads();  // s_limb is reused by the next item
 }
@@ -1106,7 +1084,7 @@ __device__ bool walk_tile(const PlanArgs &a, unsigned tile_idx, const LeanLayout
         ring.phase ^= 1u << ring.stage;
         if (!ok) {
             if (lane == 0) {
-                atomicOr(a.err, 1u);
+                atomicOr(&a.res->err, 1u);
                 *(volatile uint32_t *)&hd.abort = 1u;
             }
             break;
@@ -1377,7 +1355,7 @@ __device__ bool walk_tile_lanes(const PlanArgs &a, unsigned tile_idx, const Smem
         // waits for the copies still in flight into the ring.
         if (!cta_hand_off(ok, nthr)) {
             if (tid == 0) {
-                atomicOr(a.err, 1u);
+                atomicOr(&a.res->err, 1u);
                 drain_ring(bars, phase ^ (1u << stage), o, nsteps, R_);
             }
             return false;
@@ -1471,17 +1449,18 @@ __device__ __forceinline__ void init_lean() {
     __syncthreads();
 }
 
-// Launch bounds of the walkers (see walker_threads).
-template <typename T, int KT, int G, int N>
+// Launch bounds of the walkers (see walker_threads): up to five components a
+// thread fit 128 registers (two CTAs of 256), the others take what they need.
+template <typename T, int KT, int G, int N, bool WIDE>
 struct CtaOf {
-    static constexpr int threads =
-        walker_threads(sizeof(T) == 4 ? CXG_FP32 : CXG_FP64, KT, G, N);
-    static constexpr int per_sm = 1;
+    static constexpr int threads = WIDE ? kMaxThreads : kTuneThreads;
+    static constexpr int per_sm = !WIDE && sizeof(T) == 4 && KT * N <= 5 ? 2 : 1;
 };
 
 // One plan: one CTA per tile.
-template <typename T, int KT, int G, int N>
-__global__ void __launch_bounds__(CtaOf<T, KT, G, N>::threads, CtaOf<T, KT, G, N>::per_sm)
+template <typename T, int KT, int G, int N, bool WIDE>
+__global__ void __launch_bounds__(CtaOf<T, KT, G, N, WIDE>::threads,
+                                  CtaOf<T, KT, G, N, WIDE>::per_sm)
     walk_kernel(PlanArgs a) {
     const LeanLayout Lay = lean_layout(sizeof(T) == 4 ? CXG_FP32 : CXG_FP64, KT * G,
                                        blockDim.x / G * N, a.nslot, a.ring, a.rstride,
@@ -1508,7 +1487,8 @@ __global__ void __launch_bounds__(NT, MINB) walk_kernel_lanes(PlanArgs a) {
 // Many jobs: a persistent grid claims (job, tile) items in the host's order
 // (longest first).
 template <typename T, int KT, int G, int N>
-__global__ void __launch_bounds__(CtaOf<T, KT, G, N>::threads, CtaOf<T, KT, G, N>::per_sm)
+__global__ void __launch_bounds__(CtaOf<T, KT, G, N, false>::threads,
+                                  CtaOf<T, KT, G, N, false>::per_sm)
     walk_batch_kernel(BatchArgs b) {
     __shared__ unsigned s_item;
     __shared__ __align__(16) PlanArgs s_job;
@@ -1569,11 +1549,11 @@ static cudaError_t ensure_smem(Kern k, size_t sm, size_t &optin) {
 #define CXG_SHAPES_G(X) X(1, 2, 1) X(2, 2, 1) X(3, 2, 1) X(4, 2, 1) X(1, 4, 1) X(2, 4, 1)
 #define CXG_SHAPES_N(X) X(1, 1, 2) X(2, 1, 2) X(3, 1, 2) X(4, 1, 2) X(5, 1, 2)
 
-template <typename T, int KT, int G, int N>
+template <typename T, int KT, int G, int N, bool WIDE>
 static cudaError_t walk_fn(size_t sm, void (**fn)(PlanArgs)) {
     static size_t optin = 0;
-    *fn = walk_kernel<T, KT, G, N>;
-    return ensure_smem(walk_kernel<T, KT, G, N>, sm, optin);
+    *fn = walk_kernel<T, KT, G, N, WIDE>;
+    return ensure_smem(walk_kernel<T, KT, G, N, WIDE>, sm, optin);
 }
 template <typename T, int KT, int G, int N>
 static cudaError_t batch_fn(size_t sm, void (**fn)(BatchArgs)) {
@@ -1587,21 +1567,40 @@ static cudaError_t lanes_fn(size_t sm, void (**fn)(PlanArgs)) {
     *fn = walk_kernel_lanes<K, NT, MINB>;
     return ensure_smem(walk_kernel_lanes<K, NT, MINB>, sm, optin);
 }
-// The walker of shape w, with its dynamic shared memory limit raised to `sm`
-// bytes.
-template <typename T, typename Fn>
-static cudaError_t pick_walker(const WalkShape &w, size_t sm, Fn *fn, bool batch) {
-#define CXG_X(KT, GG, NN)                                                                     \
-    if (w.kact == (KT) * (GG) && w.tpp == (GG) && w.ppt == (NN))                              \
-        return batch ? batch_fn<T, KT, GG, NN>(sm, reinterpret_cast<void (**)(BatchArgs)>(fn)) \
-                     : walk_fn<T, KT, GG, NN>(sm, reinterpret_cast<void (**)(PlanArgs)>(fn));
+// The walkers of shape w, with their dynamic shared memory limit raised to
+// `sm` bytes.
+template <typename T>
+static cudaError_t pick_walker(const WalkShape &w, size_t sm, void (**fn)(PlanArgs)) {
+#define CXG_X(KT, GG, NN)                                             \
+    if (w.kact == (KT) * (GG) && w.tpp == (GG) && w.ppt == (NN))      \
+        return walk_fn<T, KT, GG, NN, false>(sm, fn);
+#define CXG_W(KT) \
+    if (w.kact == (KT)) return walk_fn<T, KT, 1, 1, true>(sm, fn);
+    if constexpr (sizeof(T) == 4) {
+        if (w.wide) {
+            CXG_W(1) CXG_W(2) CXG_W(3) CXG_W(4) CXG_W(5)
+            return cudaErrorInvalidValue;
+        }
+        CXG_SHAPES_N(CXG_X)
+    }
     CXG_SHAPES_1(CXG_X)
     CXG_SHAPES_G(CXG_X)
+#undef CXG_W
+    return cudaErrorInvalidValue;
+#undef CXG_X
+}
+template <typename T>
+static cudaError_t pick_batch_walker(const WalkShape &w, size_t sm, void (**fn)(BatchArgs)) {
+#define CXG_X(KT, GG, NN)                                             \
+    if (w.kact == (KT) * (GG) && w.tpp == (GG) && w.ppt == (NN))      \
+        return batch_fn<T, KT, GG, NN>(sm, fn);
     if constexpr (sizeof(T) == 4) {
         CXG_SHAPES_N(CXG_X)
     }
-#undef CXG_X
+    CXG_SHAPES_1(CXG_X)
+    CXG_SHAPES_G(CXG_X)
     return cudaErrorInvalidValue;
+#undef CXG_X
 }
 
 // The op-lane walker for kact (FP32), with its dynamic shared memory limit
@@ -1633,10 +1632,11 @@ static bool shape_launches(const WalkShape &w) {
     if (w.lanes == 2)
         return lanes_shape_ok(w.precision, w.kact, w.tpp, w.ppt) && w.ring <= 8 &&
                w.tile * 2 <= kLaneThreads;
-    return w.lanes == 1 && w.tile / w.ppt >= 32 &&
-           w.tile / w.ppt * w.tpp <=
-               walker_threads(w.precision, w.kact / w.tpp, w.tpp, w.ppt) &&
-           (w.tpp == 1 || w.tile <= kBlock) && (w.ppt == 1 || kPatternQuantum % w.tile == 0 || w.tile % 64 == 0);
+    // (Only whole warps of a tile may pass a job's patterns: two patterns a
+    // thread need tiles that divide them.)
+    return w.lanes == 1 && w.tile / w.ppt >= 32 && w.threads() <= walker_threads(w) &&
+           (!w.wide || wide_shape_ok(w)) &&
+           (w.ppt == 1 || kPatternQuantum % w.tile == 0);
 }
 
 static WalkShape shape_of(int precision, unsigned kact, unsigned tile, unsigned tpp,
@@ -1654,7 +1654,8 @@ static WalkShape shape_of(int precision, unsigned kact, unsigned tile, unsigned 
 
 cudaError_t launch_plan(int precision, const PlanArgs &a, cudaStream_t s, unsigned lanes,
                         bool pdl) {
-    const WalkShape w = shape_of(precision, a.kact, a.tile, a.tpp, a.ppt, lanes, a.ring);
+    WalkShape w = shape_of(precision, a.kact, a.tile, a.tpp, a.ppt, lanes, a.ring);
+    w.wide = a.wide;
     if (!shape_launches(w) || a.rstride % 16 || a.rstride == 0 ||
         a.ntiles != plan_blocks(a.ppad, a.tile) || (lanes == 1 && w.ring * a.lmax > 32) ||
         (lanes == 2 && (a.lmax != 0 || a.nops % 2 || a.ppad % a.tile)))
@@ -1662,10 +1663,10 @@ cudaError_t launch_plan(int precision, const PlanArgs &a, cudaStream_t s, unsign
     const size_t sm = walk_smem_bytes(w, a.nslot, a.rstride, a.lmax, a.nleaf);
     void (*fn)(PlanArgs) = nullptr;
     cudaError_t e = lanes == 2              ? pick_walker_lanes(a.kact, a.tile, sm, &fn)
-                    : precision == CXG_FP32 ? pick_walker<float>(w, sm, &fn, false)
-                                            : pick_walker<double>(w, sm, &fn, false);
+                    : precision == CXG_FP32 ? pick_walker<float>(w, sm, &fn)
+                                            : pick_walker<double>(w, sm, &fn);
     if (e != cudaSuccess) return e;
-    const unsigned nb = a.ntiles, nt = a.tile * w.tpp * lanes / w.ppt;
+    const unsigned nb = a.ntiles, nt = w.threads() * lanes;
     if (pdl) {
         // A dependent of the P kernel just before it on the stream.
         cudaLaunchConfig_t cfg = {};
@@ -1685,8 +1686,9 @@ cudaError_t launch_plan(int precision, const PlanArgs &a, cudaStream_t s, unsign
 }
 
 static cudaError_t pick_batch(const WalkShape &w, size_t sm, void (**fn)(BatchArgs)) {
-    return w.precision == CXG_FP32 ? pick_walker<float>(w, sm, fn, true)
-                                   : pick_walker<double>(w, sm, fn, true);
+    if (w.wide) return cudaErrorInvalidValue;
+    return w.precision == CXG_FP32 ? pick_batch_walker<float>(w, sm, fn)
+                                   : pick_batch_walker<double>(w, sm, fn);
 }
 
 cudaError_t launch_batch(int precision, const BatchArgs &b_in, unsigned grid,
@@ -1707,7 +1709,7 @@ cudaError_t launch_batch(int precision, const BatchArgs &b_in, unsigned grid,
     void (*fn)(BatchArgs) = nullptr;
     const cudaError_t e = pick_batch(w, sm, &fn);
     if (e != cudaSuccess) return e;
-    fn<<<grid, b.tile * w.tpp / w.ppt, sm, s>>>(b);
+    fn<<<grid, w.threads(), sm, s>>>(b);
     return cudaGetLastError();
 }
 
@@ -1717,7 +1719,7 @@ int batch_ctas_per_sm(const WalkShape &w, size_t smem) {
     cudaError_t e = pick_batch(w, smem, &fn);
     int n = 0;
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, (int)(w.tile * w.tpp / w.ppt),
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, (int)w.threads(),
                                                           smem);
     return e == cudaSuccess ? n : 0;
 }

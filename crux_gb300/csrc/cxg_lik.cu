@@ -406,6 +406,7 @@ static int internal_child(State &S, const CxtLik *lik, const CxtLikCL *cl,
 // A translated plan: the device program of one lik->steps list at one
 // precision, runnable any number of times.  CL buffers it references must
 // outlive it.
+constexpr size_t kSiteOffset = 64;  // site lnLs after the result in Plan::misc
 struct Plan {
     int prec = CXG_FP64;
     unsigned npat = 0, ppad = 0, kact = 0, nops = 0, nchild = 0;
@@ -488,17 +489,23 @@ static bool g_tuned = false;  // cxgTune was called: its shape is used as it is
 // SMs of the GPU these kernels are built for.
 constexpr unsigned kSMs = 152;
 
-// Shape for work no caller has tuned.  Measured on the 128-taxon tree over
+// Shape for work no caller has tuned: a plan (jobs 0), or a batch of `jobs`
+// (the batched walkers have no wide build).  Measured on the 128-taxon tree over
 // 81,664 patterns (2,552 warps), the 32-job batch and the small trees:
 //
-// FP32.  A walker of 96 registers keeps 20 warps on an SM, and a warp that
-// starts late ends late (65 us of latency for 127 ops): so a plan whose warps
-// all fit gets one wave of equal CTAs, two to an SM (tile 288: 144 us; 128,
-// 4.2 CTAs to an SM: 155; 32, which streams the records 9 times as often: 267),
-// and a larger one as few equal waves.  Below four warps an SM the walk is
-// bound by one warp's op after op; two warps a CTA spread it (64: 41.5 us, 32:
-// 44, 128: 42 on 17,018 patterns of 8 components).  Many jobs take tiles of
-// 128 (525 us; 64: 562).
+// FP32.  A warp's walk is a chain of ops (65 us for 127 of four components,
+// alone or with seven others on its SM), so CTAs are of equal size and evenly
+// spread.  Up to eight warps an SM that chain is all there is: small tiles (32
+// up to a warp an SM, 64 up to four, then 128: 246 us against 252 with 64 on
+// 509 taxa x 5,003 sites; 41 us against 44 with 32 on 17,018 patterns) with a
+// deep ring (41 us against 45), and with one component, whose op is too short
+// to hide a read through L2, stack slots (170 us against 188; with two or
+// more nothing).  Up to the 16 warps an SM keeps, two CTAs an SM (101 us with
+// 192 on 49,000 patterns; 128, 2.6 CTAs an SM: 105; 256: 119).  Where all
+// warps fit the wide build but not this one, the wide build saves a second
+// wave (142 us against 187); above that it does not, and fills the waves with
+// fewer warps (214 us with tiles of 128 against 229 at 100,000 patterns, 346
+// against 375 at 200,000).  Many jobs take tiles of 128 (530 us; 64: 564).
 //
 // FP64.  Each SM quarter issues one FP64 instruction a warp in 64 cycles and a
 // pattern's components are independent, so two threads a pattern halve the
@@ -525,13 +532,20 @@ static WalkShape auto_shape(int precision, unsigned kact, size_t patterns, unsig
         w.tile = 128;
         return w;
     }
-    const unsigned most = walker_threads(precision, kact, 1, 1) / 32;  // warps an SM holds
-    if (warps <= 4 * (size_t)kSMs) {
-        w.tile = 64;
-    } else {
-        const size_t waves = (warps + (size_t)kSMs * most - 1) / ((size_t)kSMs * most);
-        const size_t ctas = 2 * kSMs * waves;
-        w.tile = 32 * (unsigned)std::min<size_t>((warps + ctas - 1) / ctas, most / 2);
+    if (warps <= 8 * (size_t)kSMs) {
+        w.tile = warps <= kSMs ? 32 : warps <= 4 * (size_t)kSMs ? 64 : 128;
+        // At most two CTAs an SM: a ring and slots of half its shared memory.
+        w.ring_bytes = 88 * 1024;
+        w.budget = kact == 1 ? 20 * 1024 : 0;
+        return w;
+    }
+    w.tile = 128;
+    if (!wide_shape_ok(w)) return w;
+    const unsigned half = (unsigned)((warps + 2 * kSMs - 1) / (2 * kSMs));
+    if (half <= (jobs ? kTuneThreads : kMaxThreads / 2) / 32) {
+        w.tile = 32 * half;
+        w.wide = w.tile > kTuneThreads;
+        w.ring_bytes = 60 * 1024;
     }
     return w;
 }
@@ -566,11 +580,9 @@ void fit_ring(WalkShape &w, unsigned rstride, unsigned lmax) {
         w.ring = kRing / 2;  // a stage holds a step's two records
         return;
     }
-    // Ring bytes: shared by the CTA's warps, so that the CTAs an SM's
-    // registers hold fit its shared memory (five of 128 threads, two of 288).
-    const unsigned threads = w.tile * w.tpp / w.ppt;
-    size_t bytes = threads > 128 ? 60 * 1024 : 42 * 1024;
-    size_t n = bytes / (kStages * ((size_t)rstride + (size_t)lmax * w.tile));
+    // (Ring bytes are shared by the CTA's warps: the CTAs an SM's registers
+    // hold fit its shared memory.)
+    size_t n = w.ring_bytes / (kStages * ((size_t)rstride + (size_t)lmax * w.tile));
     if (n > 16) n = 16;
     if (lmax && n > 32 / lmax) n = 32 / lmax;
     w.ring = n ? (unsigned)n : 1;
@@ -591,11 +603,11 @@ unsigned stack_slots(const WalkShape &w, unsigned rstride, unsigned lmax, unsign
     return cap > kMaxSlots ? kMaxSlots : (unsigned)cap;
 }
 
-// `patterns`: padded patterns of all the njobs jobs this plan is launched
-// with (0: its own).
+// `patterns`: padded patterns of all the `njobs` jobs of a batch this plan is
+// one of (njobs 0: it is launched by itself; patterns 0: its own).
 static int translate(State &S, CxtLik *lik, int prec, Plan &P,
                      bool use_slots = true, bool allow_lanes = false, size_t patterns = 0,
-                     unsigned njobs = 1) {
+                     unsigned njobs = 0) {
     int rc;
     if (lik == nullptr) return fail(CXG_EINVAL, "lik is NULL");
     if (lik->dim != 4)
@@ -1000,10 +1012,10 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
     pa.ltab = (double *)P.ltab.p;
 
     const unsigned nb = plan_blocks(ppad, tile);
-    // misc: result words | site
-    rc = P.misc.ensure(kResultBytes + (size_t)ppad * 8);
+    // misc: result | site
+    rc = P.misc.ensure(kSiteOffset + (size_t)ppad * 8);
     if (rc) return rc;
-    rc = P.out.ensure(kResultRead);
+    rc = P.out.ensure(sizeof(WalkResult));
     if (rc) return rc;
     char *mp = static_cast<char *>(P.misc.p);
     PlanArgs &a = P.a;
@@ -1018,6 +1030,7 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
     a.tile = tile;
     a.tpp = w.tpp;
     a.ppt = w.ppt;
+    a.wide = w.wide;
     a.root_last = root_last ? 1u : 0u;
     a.nops = (uint32_t)order.size();  // records, empty lanes included
     a.kact = kact;
@@ -1028,11 +1041,7 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
     a.rootsc = P.root->scaler;
     a.freqs = (const uint32_t *)dfreqs;
     a.site = nullptr;
-    a.acc = (uint64_t *)(mp + 32);
-    a.ticket = (unsigned *)mp;
-    a.ninf = (uint32_t *)(mp + 4);
-    a.err = (uint32_t *)(mp + 8);
-    a.total = (double *)(mp + 16);
+    a.res = reinterpret_cast<WalkResult *>(mp);
     a.ltab = (const double *)P.ltab.p;
     a.ntiles = nb;
     a.no_root = 0;
@@ -1062,40 +1071,35 @@ static int enqueue(State &S, Plan &P, bool want_site,
                    cudaEvent_t e0 = nullptr, cudaEvent_t e1 = nullptr,
                    bool pdl = false) {
     char *mp = static_cast<char *>(P.misc.p);
-    P.a.site = want_site ? (double *)(mp + kResultBytes) : nullptr;
+    P.a.site = want_site ? (double *)(mp + kSiteOffset) : nullptr;
     // The P kernel clears the walker's result words; a plan with no P
     // matrices clears them with a memset.
     const bool pmat = P.pa.nchild * P.pa.kact > 0;
-    P.pa.zero = pmat ? reinterpret_cast<uint64_t *>(mp) : nullptr;
-    if (!pmat) CXG_CUDA(cudaMemsetAsync(mp, 0, kResultBytes, S.stream));
+    P.pa.zero = pmat ? P.a.res : nullptr;
+    if (!pmat) CXG_CUDA(cudaMemsetAsync(mp, 0, sizeof(WalkResult), S.stream));
     CXG_CUDA(launch_pmat(P.pa, S.stream));
     if (e0) CXG_CUDA(cudaEventRecord(e0, S.stream));
     CXG_CUDA(launch_plan(P.prec, P.a, S.stream, P.lanes,
                          pdl && e0 == nullptr && P.pa.nchild > 0));
     if (e1) CXG_CUDA(cudaEventRecord(e1, S.stream));
-    CXG_CUDA(cudaMemcpyAsync(P.out.p, mp, kResultRead, cudaMemcpyDeviceToHost, S.stream));
+    CXG_CUDA(cudaMemcpyAsync(P.out.p, mp, sizeof(WalkResult), cudaMemcpyDeviceToHost, S.stream));
     return 0;
 }
 
 static int finish(State &S, Plan &P, double *lnL, double *site) {
     if (site)
-        CXG_CUDA(cudaMemcpyAsync(site, static_cast<char *>(P.misc.p) + kResultBytes,
+        CXG_CUDA(cudaMemcpyAsync(site, static_cast<char *>(P.misc.p) + kSiteOffset,
                                  (size_t)P.npat * 8, cudaMemcpyDeviceToHost,
                                  S.stream));
     CXG_CUDA(cudaStreamSynchronize(S.stream));
-    const char *o = static_cast<const char *>(P.out.p);
-    uint32_t ninf, err;
-    double tot[2];
-    memcpy(&ninf, o + 4, 4);
-    memcpy(&err, o + 8, 4);
-    memcpy(tot, o + 16, 16);
+    const WalkResult r = *static_cast<const WalkResult *>(P.out.p);
     // A walk that gave up leaves its parents partly written: a later plan
     // may not read them as children until they are recomputed.
-    for (DevCL *p : P.parents) p->computed = (err == 0);
-    if (err)
+    for (DevCL *p : P.parents) p->computed = (r.err == 0);
+    if (r.err)
         return fail(CXG_ETIMEOUT,
                     "plan walker: an op-record copy did not complete in time");
-    if (lnL) *lnL = ninf ? -INFINITY : tot[0] + tot[1];
+    if (lnL) *lnL = r.lnL();
     return 0;
 }
 
@@ -1213,7 +1217,7 @@ static int execute(CxtLik *lik, int prec, double *lnL, double *site) {
         S.last_valid = false;
         return rc;
     }
-    S.last_d2h = kResultRead + (site ? (size_t)P.npat * 8 : 0);
+    S.last_d2h = sizeof(WalkResult) + (site ? (size_t)P.npat * 8 : 0);
     rc = finish(S, P, lnL, site);
     if (rc) S.last_valid = false;
     return rc;
@@ -1568,7 +1572,7 @@ static void free_batch(cxgBatch *b) {
 static int batch_enqueue(State &S, cxgBatch *b, cudaEvent_t e0 = nullptr,
                          cudaEvent_t e1 = nullptr) {
     const size_t n = b->plans.size();
-    CXG_CUDA(cudaMemsetAsync(b->results.p, 0, n * kResultBytes + 16, S.stream));
+    CXG_CUDA(cudaMemsetAsync(b->results.p, 0, n * sizeof(WalkResult) + 16, S.stream));
     CXG_CUDA(launch_pmat_batch(static_cast<const PmatArgs *>(b->pmats.p),
                                static_cast<const uint32_t *>(b->prefix.p),
                                (uint32_t)n, b->pmat_total, S.stream));
@@ -1590,25 +1594,20 @@ static int batch_enqueue(State &S, cxgBatch *b, cudaEvent_t e0 = nullptr,
         }
     }
     if (e1) CXG_CUDA(cudaEventRecord(e1, S.stream));
-    CXG_CUDA(cudaMemcpyAsync(b->out.p, b->results.p, n * kResultBytes,
+    CXG_CUDA(cudaMemcpyAsync(b->out.p, b->results.p, n * sizeof(WalkResult),
                              cudaMemcpyDeviceToHost, S.stream));
     return 0;
 }
 
 static int batch_finish(State &S, cxgBatch *b, double *lnLs) {
     CXG_CUDA(cudaStreamSynchronize(S.stream));
-    const char *o = static_cast<const char *>(b->out.p);
     for (size_t j = 0; j < b->plans.size(); ++j) {
-        uint32_t ninf, err;
-        double tot[2];
-        memcpy(&ninf, o + j * kResultBytes + 4, 4);
-        memcpy(&err, o + j * kResultBytes + 8, 4);
-        memcpy(tot, o + j * kResultBytes + 16, 16);
-        for (DevCL *p : b->plans[j]->parents) p->computed = (err == 0);
-        if (err)
+        const WalkResult r = static_cast<const WalkResult *>(b->out.p)[j];
+        for (DevCL *p : b->plans[j]->parents) p->computed = (r.err == 0);
+        if (r.err)
             return fail(CXG_ETIMEOUT,
                         "batched walker: an op-record copy did not complete");
-        if (lnLs) lnLs[j] = ninf ? -INFINITY : tot[0] + tot[1];
+        if (lnLs) lnLs[j] = r.lnL();
     }
     return 0;
 }
@@ -1653,7 +1652,7 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
         Plan *P = new Plan();
         b->plans.push_back(P);
         rc = translate(S, liks[j], precision, *P, !b->per_node, false, patterns,
-                       b->per_node ? 1 : n);
+                       b->per_node ? 0 : n);
         if (rc) {
             free_batch(b);
             return rc;
@@ -1669,9 +1668,9 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
         b->alg_bytes += P->alg_bytes;
         b->launches += P->nops;
     }
-    // Per-job result words side by side, then the walker's work counter.
-    if ((rc = b->results.ensure((size_t)n * kResultBytes + 16)) ||
-        (rc = b->out.ensure((size_t)n * kResultBytes)) ||
+    // The jobs' results side by side, then the walker's work counter.
+    if ((rc = b->results.ensure((size_t)n * sizeof(WalkResult) + 16)) ||
+        (rc = b->out.ensure((size_t)n * sizeof(WalkResult))) ||
         (rc = b->jobs.ensure((size_t)n * sizeof(PlanArgs))) ||
         (rc = b->pmats.ensure((size_t)n * sizeof(PmatArgs))) ||
         (rc = b->prefix.ensure((size_t)(n + 1) * 4))) {
@@ -1685,11 +1684,7 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
     char *res = static_cast<char *>(b->results.p);
     for (unsigned j = 0; j < n; ++j) {
         PlanArgs a = b->plans[j]->a;
-        a.ticket = (unsigned *)(res + (size_t)j * kResultBytes);
-        a.ninf = (uint32_t *)(res + (size_t)j * kResultBytes + 4);
-        a.err = (uint32_t *)(res + (size_t)j * kResultBytes + 8);
-        a.total = (double *)(res + (size_t)j * kResultBytes + 16);
-        a.acc = (uint64_t *)(res + (size_t)j * kResultBytes + 32);
+        a.res = reinterpret_cast<WalkResult *>(res) + j;
         a.site = nullptr;
         b->plans[j]->a = a;
         jobs[j] = a;
@@ -1724,7 +1719,7 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
     ba.jobs = static_cast<const PlanArgs *>(b->jobs.p);
     ba.items = static_cast<const WalkItem *>(b->items.p);
     ba.nitems = b->nitems;
-    ba.counter = (unsigned *)(res + (size_t)n * kResultBytes);
+    ba.counter = (unsigned *)(res + (size_t)n * sizeof(WalkResult));
     ba.tile = b->plans[0]->tile;
     ba.tpp = b->plans[0]->tpp;
     ba.ppt = b->plans[0]->ppt;

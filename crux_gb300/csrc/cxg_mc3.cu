@@ -156,7 +156,7 @@ struct Mc3Dev {
     int32_t *kid_tab;     // [c][maxkids]
     uint32_t *nkids;      // [c]
     double *ltab;         // [c][maxkids][16][kact][4] (FP64 chains)
-    char *results;        // [c][kResultBytes]
+    WalkResult *results;  // [c], then the walker's work counter
     unsigned *counter;
     uint32_t *order;      // [c] chains, longest walk of the generation first
     double wcdf[kMoves];
@@ -690,12 +690,10 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
         Philox rng;
         philox_init(rng, d.seed, c, g);
         if (c == 0) *d.counter = 0;
-        char *res = d.results + (size_t)c * kResultBytes;
-        // A walker tile that gave up on a bounded wait leaves the ticket
-        // counted short; the error word stays set until the run reports it.
-        *(uint32_t *)(res + 0) = 0;  // ticket
-        *(uint32_t *)(res + 4) = 0;  // ninf
-        for (int i = 0; i < 4; ++i) ((uint64_t *)(res + 32))[i] = 0;  // sum
+        // The error word stays set until the run reports it.
+        WalkResult &res = d.results[c];
+        res.ninf = 0;
+        for (int i = 0; i < 4; ++i) res.acc[i] = 0;
 
         const Mc3Model &m0 = d.model[c * 2 + d.curmodel[c]];
         Mc3Model &m1 = d.model[c * 2 + (1 - d.curmodel[c])];
@@ -1666,11 +1664,7 @@ __global__ void mc3_accept_kernel(Mc3Dev d) {
     const unsigned N = d.ntaxa, NN = d.nnodes;
     for (unsigned c = threadIdx.x; c < d.nchains; c += blockDim.x) {
         Mc3Prop &pr = d.prop[c];
-        const char *res = d.results + (size_t)c * kResultBytes;
-        const uint32_t ninf = *(const uint32_t *)(res + 4);
-        const double lnL1 = ninf ? -INFINITY
-                                 : ((const double *)(res + 16))[0] +
-                                       ((const double *)(res + 16))[1];
+        const double lnL1 = d.results[c].lnL();
         bool accept;
         if (pr.type == MV_INIT) {
             accept = true;
@@ -2066,7 +2060,7 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
                                  cfg->precision == CXG_FP64
                                      ? (size_t)C * d.maxkids * 16 * K * 4
                                      : 2)) ||
-        (rc = mc3_upload<char>(h, &d.results, nullptr, (size_t)C * kResultBytes + 16)) ||
+        (rc = mc3_upload<WalkResult>(h, &d.results, nullptr, (size_t)C + 1)) ||
         (rc = mc3_upload<uint32_t>(h, &d.acc, nullptr, (size_t)C * kMoves)) ||
         (rc = mc3_upload<uint32_t>(h, &d.rej, nullptr, (size_t)C * kMoves)) ||
         (rc = mc3_upload<uint32_t>(h, &d.nswap, nullptr, C)) ||
@@ -2085,7 +2079,7 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
         mc3_free(h);
         return rc;
     }
-    d.counter = (unsigned *)(d.results + (size_t)C * kResultBytes);
+    d.counter = reinterpret_cast<unsigned *>(d.results + C);
     {
         void *slab_cl = nullptr, *slab_sc = nullptr;
         if ((rc = mc3_alloc(h, &slab_cl, cl.size() * cl_bytes)) ||
@@ -2123,11 +2117,7 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
         a.ppad = d.ppad;
         a.root_last = 1;
         a.freqs = dfreq;
-        a.acc = (uint64_t *)(d.results + (size_t)c * kResultBytes + 32);
-        a.ticket = (unsigned *)(d.results + (size_t)c * kResultBytes);
-        a.ninf = (uint32_t *)(d.results + (size_t)c * kResultBytes + 4);
-        a.err = (uint32_t *)(d.results + (size_t)c * kResultBytes + 8);
-        a.total = (double *)(d.results + (size_t)c * kResultBytes + 16);
+        a.res = d.results + c;
         a.ltab = d.ltab + (cfg->precision == CXG_FP64 ? (size_t)c * d.maxkids * 16 * K * 4 : 0);
         a.ntiles = d.ntiles;
         a.no_root = 0;
@@ -2243,9 +2233,9 @@ extern "C" int cxgMc3Run(cxgMc3 *h, unsigned long long ngen, double *seconds) {
     cudaEventDestroy(t1);
     if (seconds) *seconds = ms / 1e3;
     uint32_t st = 0;
-    std::vector<char> res((size_t)h->d.nchains * kResultBytes);
+    std::vector<WalkResult> res(h->d.nchains);
     CXG_CUDA(cudaMemcpyAsync(&st, h->d.status, 4, cudaMemcpyDeviceToHost, h->stream));
-    CXG_CUDA(cudaMemcpyAsync(res.data(), h->d.results, res.size(), cudaMemcpyDeviceToHost,
+    CXG_CUDA(cudaMemcpyAsync(res.data(), h->d.results, res.size() * sizeof(WalkResult), cudaMemcpyDeviceToHost,
                              h->stream));
     CXG_CUDA(cudaStreamSynchronize(h->stream));
     // Undecomposable proposed models are rejected, not errors (bit 0 is
@@ -2254,7 +2244,7 @@ extern "C" int cxgMc3Run(cxgMc3 *h, unsigned long long ngen, double *seconds) {
     if (st & 2u) return fail(CXG_EINVAL, "MC3: an eTBR move met a malformed tree");
     // Any bounded wait that gave up?
     for (unsigned c = 0; c < h->d.nchains; ++c)
-        if (*(const uint32_t *)(res.data() + (size_t)c * kResultBytes + 8))
+        if (res[c].err)
             return fail(CXG_ETIMEOUT, "MC3 walker: a record copy timed out");
     return 0;
 }
@@ -2452,10 +2442,10 @@ extern "C" int cxgMc3Resume(cxgMc3 *h, unsigned long long generation) {
     CXG_CUDA(cudaMemcpyAsync(&st, d.status, 4, cudaMemcpyDeviceToHost, h->stream));
     CXG_CUDA(cudaStreamSynchronize(h->stream));
     if (st & 1u) return fail(CXG_EINVAL, "cxgMc3Resume: a model cannot be decomposed");
-    std::vector<char> res((size_t)d.nchains * kResultBytes);
-    CXG_CUDA(cudaMemcpy(res.data(), d.results, res.size(), cudaMemcpyDeviceToHost));
+    std::vector<WalkResult> res(d.nchains);
+    CXG_CUDA(cudaMemcpy(res.data(), d.results, res.size() * sizeof(WalkResult), cudaMemcpyDeviceToHost));
     for (unsigned c = 0; c < d.nchains; ++c)
-        if (*(const uint32_t *)(res.data() + (size_t)c * kResultBytes + 8))
+        if (res[c].err)
             return fail(CXG_ETIMEOUT, "MC3 walker: a record copy timed out");
     CXG_CUDA(cudaMemcpy(d.gen, &generation, 8, cudaMemcpyHostToDevice));
     return 0;

@@ -52,7 +52,7 @@ static __device__ __align__(256) unsigned char g_na_scratch[kNaScratchBytes];
 
 static void *g_na_dev[kNaMaxDevices];
 static unsigned char g_na_host[kNaScratchBytes];  // packing area (static)
-static unsigned char g_na_result[32];
+static WalkResult g_na_result;
 static std::mutex g_na_mu;
 
 // Device address of the scratch array on the current device; the first call
@@ -218,7 +218,7 @@ extern "C" int cxgLikExecuteNoAlloc(const CxtLik *lik, int precision,
             return fail(CXG_EINVAL, "cxgLikExecuteNoAlloc: leaf tables above 1.5 MiB");
     }
     const size_t o_end = al16(o_ltab + (ltab_bytes ? ltab_bytes : 16));
-    WalkShape w = choose_shape(prec, kact, ppad, 1, false);
+    WalkShape w = choose_shape(prec, kact, ppad, 0, false);
     const unsigned tile = w.tile;
     fit_ring(w, (unsigned)rstride, lmax);
     const unsigned nb = plan_blocks(ppad, tile);
@@ -227,7 +227,7 @@ extern "C" int cxgLikExecuteNoAlloc(const CxtLik *lik, int precision,
     const size_t upload = o_ltab;  // host-packed prefix (misc..root weights)
 
     unsigned char *h = g_na_host;
-    memset(h, 0, upload);  // ticket, ninf, err and records start at zero
+    memset(h, 0, upload);  // the result and the records start at zero
 
     // Pass 2: records and children.  Each op's parent is the CxtLikCL of
     // its Compute step; every pointer is the caller's device memory (a leaf
@@ -384,6 +384,7 @@ extern "C" int cxgLikExecuteNoAlloc(const CxtLik *lik, int precision,
     a.tile = tile;
     a.tpp = w.tpp;
     a.ppt = w.ppt;
+    a.wide = w.wide;
     a.kact = kact;
     a.npat = npat;
     a.ppad = ppad;
@@ -393,28 +394,20 @@ extern "C" int cxgLikExecuteNoAlloc(const CxtLik *lik, int precision,
     a.rootsc = lik->rootCLC->lnScale;
     a.freqs = dFreqs;
     a.site = dSiteLnL;
-    a.acc = reinterpret_cast<uint64_t *>(dev + o_misc + 32);
-    a.ticket = reinterpret_cast<unsigned *>(dev + o_misc);
-    a.ninf = reinterpret_cast<uint32_t *>(dev + o_misc + 4);
-    a.err = reinterpret_cast<uint32_t *>(dev + o_misc + 8);
-    a.total = reinterpret_cast<double *>(dev + o_misc + 16);
+    a.res = reinterpret_cast<WalkResult *>(dev + o_misc);
     a.ltab = reinterpret_cast<const double *>(dev + o_ltab);
     a.ntiles = nb;
     a.no_root = 0;
     e = launch_plan(prec, a, st);
     if (e != cudaSuccess) return cuda_fail(e, "walk_kernel");
-    e = cudaMemcpyAsync(g_na_result, dev + o_misc, 32, cudaMemcpyDeviceToHost, st);
+    e = cudaMemcpyAsync(&g_na_result, dev + o_misc, sizeof(WalkResult), cudaMemcpyDeviceToHost,
+                        st);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpyAsync(result)");
     e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamSynchronize");
-    uint32_t ninf, err;
-    double tot[2];
-    memcpy(&ninf, g_na_result + 4, 4);
-    memcpy(&err, g_na_result + 8, 4);
-    memcpy(tot, g_na_result + 16, 16);
-    if (err)
+    if (g_na_result.err)
         return fail(CXG_ETIMEOUT,
                     "plan walker: an op-record copy did not complete in time");
-    *lnL = ninf ? -INFINITY : tot[0] + tot[1];
+    *lnL = g_na_result.lnL();
     return 0;
 }

@@ -313,7 +313,7 @@ struct cxgServer {
     std::map<unsigned long long, SrvSession> sessions;
     uint64_t use_clock = 0;
     std::unordered_map<uint64_t, SrvDataset *> datasets;
-    char *pinned = nullptr;  // [kResultSlots][max_active * kResultBytes]
+    char *pinned = nullptr;  // [kResultSlots][max_active] results
     bool slot_busy[kResultSlots] = {};
     StagePool stage;  // likelihood worker's upload staging
 };
@@ -749,13 +749,13 @@ int launch_batch_of(cxgServer *S, SrvBatch &B, cudaStream_t st) {
     const size_t o_pm = o_items + al256(nitems * sizeof(WalkItem));
     const size_t o_pre = o_pm + al256(n * sizeof(PmatArgs));
     const size_t o_res = o_pre + al256((n + 1) * 4);
-    B.bytes = o_res + al256(n * kResultBytes + 16);
+    B.bytes = o_res + al256(n * sizeof(WalkResult) + 16);
     B.slot = -1;
     for (int k = 0; k < kResultSlots && B.slot < 0; ++k)
         if (!S->slot_busy[k]) B.slot = k;
     if (B.slot < 0) return fail(CXG_EBUSY, "server: no free result slot");
     S->slot_busy[B.slot] = true;
-    B.host = S->pinned + (size_t)B.slot * S->cfg.max_active * kResultBytes;
+    B.host = S->pinned + (size_t)B.slot * S->cfg.max_active * sizeof(WalkResult);
     if (const cudaError_t e = dev_malloc_async((void **)&B.mem, B.bytes, st)) {
         B.mem = nullptr;
         return cuda_fail(e, "dev_malloc_async(server batch)");
@@ -764,11 +764,7 @@ int launch_batch_of(cxgServer *S, SrvBatch &B, cudaStream_t st) {
     for (size_t j = 0; j < n; ++j) {
         SrvJob *J = B.jobs[j];
         PlanArgs a = J->a;
-        a.ticket = (unsigned *)(res + j * kResultBytes);
-        a.ninf = (uint32_t *)(res + j * kResultBytes + 4);
-        a.err = (uint32_t *)(res + j * kResultBytes + 8);
-        a.total = (double *)(res + j * kResultBytes + 16);
-        a.acc = (uint64_t *)(res + j * kResultBytes + 32);
+        a.res = reinterpret_cast<WalkResult *>(res) + j;
         jobs[j] = a;
         pm[j] = J->pa;
         prefix[j + 1] = prefix[j] + J->nchild * J->kact;
@@ -790,7 +786,7 @@ int launch_batch_of(cxgServer *S, SrvBatch &B, cudaStream_t st) {
     const cudaError_t ce = cudaMemcpyAsync(B.mem, host, o_res, cudaMemcpyHostToDevice, st);
     S->stage.hand_off(sb, st);
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemcpyAsync(server batch)");
-    CXG_CUDA(cudaMemsetAsync(res, 0, n * kResultBytes + 16, st));
+    CXG_CUDA(cudaMemsetAsync(res, 0, n * sizeof(WalkResult) + 16, st));
     CXG_CUDA(launch_pmat_batch((const PmatArgs *)(B.mem + o_pm),
                                (const uint32_t *)(B.mem + o_pre), (uint32_t)n,
                                prefix[n], st));
@@ -798,7 +794,7 @@ int launch_batch_of(cxgServer *S, SrvBatch &B, cudaStream_t st) {
     ba.jobs = (const PlanArgs *)(B.mem + o_jobs);
     ba.items = (const WalkItem *)(B.mem + o_items);
     ba.nitems = (uint32_t)items.size();
-    ba.counter = (unsigned *)(res + n * kResultBytes);
+    ba.counter = (unsigned *)(res + n * sizeof(WalkResult));
     ba.tile = B.jobs[0]->a.tile;
     ba.tpp = B.jobs[0]->a.tpp;
     ba.ppt = B.jobs[0]->a.ppt;
@@ -819,7 +815,7 @@ int launch_batch_of(cxgServer *S, SrvBatch &B, cudaStream_t st) {
     if (per <= 0) return fail(CXG_EINVAL, "server: walker does not fit an SM");
     cudaError_t e = launch_batch(prec, ba, (unsigned)(per * nsm), st);
     if (e != cudaSuccess) return cuda_fail(e, "walk_batch_kernel (server)");
-    CXG_CUDA(cudaMemcpyAsync(B.host, res, n * kResultBytes, cudaMemcpyDeviceToHost, st));
+    CXG_CUDA(cudaMemcpyAsync(B.host, res, n * sizeof(WalkResult), cudaMemcpyDeviceToHost, st));
     CXG_CUDA(cudaEventCreateWithFlags(&B.done, cudaEventDisableTiming));
     CXG_CUDA(cudaEventRecord(B.done, st));
     B.stream = st;
@@ -830,14 +826,10 @@ void retire(cxgServer *S, SrvBatch &B) {
     const size_t n = B.jobs.size();
     for (size_t j = 0; j < n; ++j) {
         SrvJob *J = B.jobs[j];
-        uint32_t ninf, err;
-        double tot[2];
-        memcpy(&ninf, B.host + j * kResultBytes + 4, 4);
-        memcpy(&err, B.host + j * kResultBytes + 8, 4);
-        memcpy(tot, B.host + j * kResultBytes + 16, 16);
-        const double v = ninf ? -INFINITY : tot[0] + tot[1];
-        if (err) fail(CXG_ETIMEOUT, "walk_batch_kernel (server): record wait timed out");
-        complete(S, J->rq->ticket, err ? CXG_ETIMEOUT : 0, v, J->rq->t_submit);
+        const WalkResult r = reinterpret_cast<const WalkResult *>(B.host)[j];
+        const double v = r.lnL();
+        if (r.err) fail(CXG_ETIMEOUT, "walk_batch_kernel (server): record wait timed out");
+        complete(S, J->rq->ticket, r.err ? CXG_ETIMEOUT : 0, v, J->rq->t_submit);
         {
             std::lock_guard<std::mutex> g(S->mu);
             S->updates_done += J->updates;
@@ -1203,7 +1195,7 @@ extern "C" int cxgServerCreate(const cxgServerConfig *cfg, cxgServer **out) {
     }
     S->budget = cfg->hbm_budget ? (size_t)cfg->hbm_budget : (size_t)(fr * 0.8);
     if ((e = host_alloc((void **)&S->pinned,
-                        (size_t)kResultSlots * S->cfg.max_active * kResultBytes)) != cudaSuccess) {
+                        (size_t)kResultSlots * S->cfg.max_active * sizeof(WalkResult))) != cudaSuccess) {
         delete S;
         return cuda_fail(e, "cudaHostAlloc(server results)");
     }

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from crux_gb300 import Alignment, Lik, TaxaMap, Tree, synth, tune
+from crux_gb300.batch import Batch
 from crux_gb300.plan import Plan
 
 pytestmark = pytest.mark.gpu
@@ -15,7 +16,8 @@ pytestmark = pytest.mark.gpu
 TOL = {"fp64": 1e-11, "fp32": 1e-6}
 
 # taxa, sites (not compacted: as many patterns, padded by the Lik).
-SIZES = [(9, 5), (17, 129), (70, 1000), (5, 20011), (4, 98304), (4, 200001)]
+SIZES = [(9, 5), (17, 129), (70, 1000), (5, 20011), (4, 47003), (4, 84000), (4, 98304),
+         (4, 200001)]
 # Gamma categories, +I: 1, 2, 3, 4, 5, 6, 7 and 8 components.
 MODELS = [(1, 0.0), (2, 0.0), (3, 0.0), (4, 0.0), (4, 0.2), (6, 0.0), (6, 0.2),
           (8, 0.0)]
@@ -39,7 +41,7 @@ def make(ntaxa, nsites, ncat, pinv, lib, precision):
 
 def sizes_of(model):
     # The largest walks with the benchmark's components and with one.
-    return [s for s in SIZES if s[1] < 50000 or model in ((1, 0.0), (4, 0.0))]
+    return [s for s in SIZES if s[1] < 40000 or model in ((1, 0.0), (4, 0.0))]
 
 
 @pytest.mark.parametrize("precision", ["fp32", "fp64"])
@@ -62,6 +64,19 @@ def test_chosen_shape_matches_oracle(gpu, port, model, precision):
         plan.close()
 
 
+@pytest.mark.parametrize("nsites", [129, 84000])
+def test_batch_of_one_takes_a_batched_shape(gpu, port, nsites):
+    """A batch of one job, at sizes where a plan takes the small tiles and
+    where it takes the wide build, which batches do not have."""
+    lik = make(5, nsites, 4, 0.0, gpu, "fp32")
+    ref = make(5, nsites, 4, 0.0, port, "fp64")
+    lik.prepare_plan()
+    b = Batch([lik], "fp32")
+    got, want = b.run()[0], ref.lnL()
+    b.close()
+    assert abs(got - want) <= TOL["fp32"] * abs(want)
+
+
 def test_chosen_shapes_differ_and_tuned_ones_give_their_bits(gpu):
     """Runs after the choices above: the process is tuned from here on."""
     if not SEEN:
@@ -69,7 +84,7 @@ def test_chosen_shapes_differ_and_tuned_ones_give_their_bits(gpu):
     shapes = {(s["tile"], s["threads_per_pattern"]) for _, _, _, s in SEEN.values()}
     assert len(shapes) >= 4, shapes
     for (model, precision, ntaxa, nsites), (got, site, path, _) in SEEN.items():
-        if nsites > 50000:
+        if nsites > 40000:
             continue
         for shape in ((64, 1, 1, 24 << 10), (32, 1, 1, 0), (128, 1, 1, 48 << 10)):
             tune.set_shape(gpu, *shape)
