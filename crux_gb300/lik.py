@@ -1236,7 +1236,8 @@ class Lik:
         else:
             self.lib.CxLikExecute(ctypes.byref(self.lik))
         n = self.lik.nchars - self.lik.npad
-        return [float(x) for x in self.siteLnLBuf[:n]]
+        # (A float() a site took 0.7 ms more for 20,000 of them.)
+        return self.siteLnLBuf[:n].tolist()
 
     def execute_dropin(self, root=None):
         """Plan, then run the library's drop-in CxLikExecute; return the
