@@ -8,16 +8,17 @@
 //
 //   0. compact_used: which canonical codes occur (a 256-entry flag table,
 //      read back); the rank of a character is the position of its
-//      canonical code among those, in byte order, so rank order is byte
-//      order and a rank fits `bits` bits (3 for ACGT, N and gaps).
-//   1. compact_keys: every column's characters, `cpk` to a 64-bit key
-//      (first character most significant, rank order = byte order), as
-//      key[chunk][site], read straight from the row-major input.
-//   2. LSD sort: for each chunk, last first, gather the chunk key of every
-//      column in the current order and stable-radix-sort (key, column
-//      index) pairs: 8-bit digits, each a histogram per tile, one scan of
-//      the (digit, tile) counts and a stable scatter (radix_hist,
-//      radix_scan, radix_scatter below).
+//      canonical code among the r that occur, in byte order, so rank order
+//      is byte order.
+//   1. compact_keys: every column's characters, `cpk` to a 64-bit key as a
+//      number of base r (first character most significant), so that r = 5
+//      packs 27 characters where three bits each hold 21: key[chunk][site],
+//      read straight from the row-major input.
+//   2. LSD sort: for each chunk, last first, stable radix passes over the
+//      8-bit digits of (key, column index) pairs, one kernel each
+//      (radix_pass): a pass counts the digits of the next one while it
+//      writes its pairs, and the last pass of a chunk fetches the next
+//      chunk's keys.
 //   3. compact_flags: a column starts a pattern unless all its chunk keys
 //      equal those of the column before it (the packing is exact); a scan
 //      numbers the patterns.
@@ -27,6 +28,7 @@
 #include <cuda_runtime.h>
 #include <string.h>
 
+#include <algorithm>
 #include <mutex>
 #include <vector>
 
@@ -65,28 +67,24 @@ __global__ void compact_used(const uint8_t *rows, size_t n, const uint8_t *canon
         if (u[i]) used[i] = 1;
 }
 
-// keys[c][s] = ranks of characters [c*cpk, c*cpk + cpk) of column s,
-// `bits` bits each, the first one most significant (rank 0 past ntaxa).
-// Thread per site: each character read is a coalesced row access.
+// keys[c][s] = ranks of characters [c*cpk, c*cpk + cpk) of column s as a
+// number of base r, the first one most significant (fewer characters in the
+// last chunk).  Thread per site: each character read is a coalesced row
+// access.
 __global__ void compact_keys(const uint8_t *rows, unsigned ntaxa, unsigned nsites,
-                             const uint8_t *rank, unsigned bits, unsigned cpk,
+                             const uint8_t *rank, unsigned r, unsigned cpk,
                              unsigned long long *keys) {
+    __shared__ uint8_t rs[256];
+    for (unsigned i = threadIdx.x; i < 256; i += blockDim.x) rs[i] = rank[i];
+    __syncthreads();
     const unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned c = blockIdx.y;
     if (s >= nsites) return;
+    const unsigned t1 = min((c + 1) * cpk, ntaxa);
     unsigned long long k = 0;
-    for (unsigned j = 0; j < cpk; ++j) {
-        const unsigned t = c * cpk + j;
-        k = (k << bits) | (t < ntaxa ? rank[rows[(size_t)t * nsites + s]] : 0u);
-    }
+#pragma unroll 8
+    for (unsigned t = c * cpk; t < t1; ++t) k = k * r + rs[rows[(size_t)t * nsites + s]];
     keys[(size_t)c * nsites + s] = k;
-}
-
-// key[i] = keys[c][idx[i]]: chunk c of the columns in the current order.
-__global__ void compact_gather(const unsigned long long *keys_c, const uint32_t *idx,
-                               unsigned n, unsigned long long *key) {
-    const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) key[i] = keys_c[idx[i]];
 }
 
 // flag[i] = 1 if column idx[i] differs from column idx[i - 1] (or i == 0):
@@ -146,31 +144,163 @@ size_t al256c(size_t x) { return (x + 255) & ~(size_t)255; }
 // --- stable LSD radix sort of (64-bit key, 32-bit value) pairs ------------
 // One pass orders the pairs by the 8-bit digit (key >> shift) & 255, keeping
 // the order of equal digits.  The input is cut into tiles of kSortTile
-// pairs, one CTA each.
-constexpr unsigned kSortThreads = 256;
+// pairs, one CTA each, a pair a thread.
 constexpr unsigned kSortTile = 1024;
+// Up to this many tiles a CTA sums the counts of the tiles before its own
+// by itself; more are scanned by a kernel between the passes (radix_rowscan:
+// 4 us at 1,000 tiles, where the sums would read 1 GB).
+constexpr unsigned kSelfSum = 128;
 
-// hist[d * ntiles + b] = pairs of tile b with digit d.
-__global__ void __launch_bounds__(kSortThreads)
+// hist[b][d] = pairs of tile b with digit d: the first pass's counts.
+__global__ void __launch_bounds__(kSortTile)
     radix_hist(const unsigned long long *key, unsigned n, unsigned shift, uint32_t *hist) {
     __shared__ uint32_t h[256];
     const unsigned t = threadIdx.x;
-    h[t] = 0;
+    if (t < 256) h[t] = 0;
     __syncthreads();
-    const unsigned base = blockIdx.x * kSortTile;
-    const unsigned end = min(base + kSortTile, n);
-    for (unsigned i = base + t; i < end; i += kSortThreads)
-        atomicAdd(&h[(unsigned)(key[i] >> shift) & 255u], 1u);
+    const size_t i = (size_t)blockIdx.x * kSortTile + t;
+    if (i < n) atomicAdd(&h[(unsigned)(key[i] >> shift) & 255u], 1u);
     __syncthreads();
-    hist[t * gridDim.x + blockIdx.x] = h[t];
+    if (t < 256) hist[(size_t)blockIdx.x * 256 + t] = h[t];
 }
 
-// Exclusive scan of the NT values v[0..n) in place, one CTA of NT
-// threads: each thread sums a contiguous segment, the segment sums are
-// scanned in shared memory, then each thread writes its segment's
-// prefixes.  Returns the total (every thread).
-template <unsigned NT>
-__device__ uint32_t block_exclusive_scan(uint32_t *v, unsigned n) {
+// hist[b][d] becomes the count of digit d in the tiles before b, tot[d] that
+// of all tiles.  CTA of 32 digits (a lane each), a warp per run of tiles.
+__global__ void __launch_bounds__(1024)
+    radix_rowscan(uint32_t *hist, unsigned ntiles, uint32_t *tot) {
+    __shared__ uint32_t part[32][32];
+    const unsigned lane = threadIdx.x & 31, w = threadIdx.x / 32;
+    const unsigned d = blockIdx.x * 32 + lane;
+    const unsigned seg = (ntiles + 31) / 32;
+    const unsigned a = min(w * seg, ntiles), b = min(a + seg, ntiles);
+    uint32_t sum = 0;
+    for (unsigned i = a; i < b; ++i) sum += hist[(size_t)i * 256 + d];
+    part[w][lane] = sum;
+    __syncthreads();
+    uint32_t run = 0;
+    for (unsigned j = 0; j < w; ++j) run += part[j][lane];
+    if (w == 31) tot[d] = run + sum;
+    for (unsigned i = a; i < b; ++i) {
+        const uint32_t x = hist[(size_t)i * 256 + d];
+        hist[(size_t)i * 256 + d] = run;
+        run += x;
+    }
+}
+
+// One pass: pairs (kin, vin) to (kout, vout); vin null: vin[i] = i.
+struct RadixPass {
+    const unsigned long long *kin;
+    const uint32_t *vin;
+    unsigned n, shift;
+    const uint32_t *hist;  // [tile][256] counts (scanned: those of the tiles before)
+    const uint32_t *tot;   // [256] counts of all tiles, null: sum hist here
+    uint32_t *hist_next;   // zero before: counts of the next pass (null: last pass)
+    uint32_t *hist_zero;   // cleared for the pass after the next
+    const unsigned long long *keys_next;  // the next pass's keys by column, null: the same
+    unsigned shift_next;
+    unsigned long long *kout;
+    uint32_t *vout;
+};
+
+// Bound by latency: launch, the count sums and four barriers.  On 100,000
+// columns of 128 taxa a pass takes 7.5 us alone and there are 38 (0.28 ms); a
+// histogram, a scan and a scatter kernel took 15.2, for 56 digits of keys with
+// three bits a character (0.87 ms).
+__global__ void __launch_bounds__(kSortTile) radix_pass(RadixPass p) {
+    constexpr unsigned W = kSortTile / 32;
+    __shared__ __align__(16) uint32_t wcnt[W][256];  // per warp and digit: count, then place
+    __shared__ uint32_t part[4][256], parttot[4][256], wsum[8];
+    const unsigned t = threadIdx.x, w = t / 32, lane = t % 32;
+    const unsigned d0 = t & 255, q = t >> 8;  // a quarter of the rows for digit d0
+    const unsigned b = blockIdx.x;
+    for (unsigned j = t; j < W * 64; j += kSortTile)
+        reinterpret_cast<uint4 *>(wcnt)[j] = make_uint4(0, 0, 0, 0);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const size_t i = (size_t)b * kSortTile + t;
+    const bool active = i < p.n;
+    const unsigned long long k = active ? p.kin[i] : 0ull;
+    const uint32_t v = !active ? 0u : p.vin != nullptr ? p.vin[i] : (uint32_t)i;
+    if (p.hist_zero != nullptr && t < 256) p.hist_zero[(size_t)b * 256 + t] = 0;
+    uint32_t pre = 0, tot = 0;
+    if (p.tot == nullptr) {
+#pragma unroll 8
+        for (unsigned r = q; r < gridDim.x; r += 4) {
+            const uint32_t x = p.hist[(size_t)r * 256 + d0];
+            tot += x;
+            pre += r < b ? x : 0u;
+        }
+    } else if (q == 0) {
+        pre = p.hist[(size_t)b * 256 + d0];
+        tot = p.tot[d0];
+    }
+    part[q][d0] = pre;
+    parttot[q][d0] = tot;
+    __syncthreads();  // wcnt is clear
+    // Inactive lanes get a digit no other lane has.
+    const unsigned d = active ? ((unsigned)(k >> p.shift) & 255u) : 256u + lane;
+    const unsigned peers = __match_any_sync(0xffffffffu, d);
+    const unsigned below = __popc(peers & ((1u << lane) - 1u));
+    if (active && below == 0) wcnt[w][d] = __popc(peers);
+    // Digits before d0, this warp's 32 digits first.
+    uint32_t base = 0;
+    if (q == 0) {
+        tot = parttot[0][d0] + parttot[1][d0] + parttot[2][d0] + parttot[3][d0];
+        base = tot;
+        for (unsigned o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, base, o);
+            if (lane >= o) base += x;
+        }
+        if (lane == 31) wsum[w] = base;
+        base -= tot;
+        pre = part[0][d0] + part[1][d0] + part[2][d0] + part[3][d0];
+    }
+    __syncthreads();
+    if (q == 0) {
+        for (unsigned j = 0; j < w; ++j) base += wsum[j];
+        part[0][d0] = base + pre;  // the tile's first place for the digit
+    }
+    uint32_t sum = 0;
+#pragma unroll
+    for (unsigned j = 0; j < W / 4; ++j) sum += wcnt[q * (W / 4) + j][d0];
+    parttot[q][d0] = sum;
+    __syncthreads();
+    uint32_t run = part[0][d0];
+    for (unsigned j = 0; j < q; ++j) run += parttot[j][d0];
+#pragma unroll
+    for (unsigned j = 0; j < W / 4; ++j) {
+        uint32_t &c = wcnt[q * (W / 4) + j][d0];
+        const uint32_t x = c;
+        c = run;
+        run += x;
+    }
+    __syncthreads();
+    const uint32_t pos = active ? wcnt[w][d] + below : 0u;
+    if (p.hist_next != nullptr) {
+        const unsigned long long kn =
+            p.keys_next != nullptr && active ? p.keys_next[v] : k;
+        if (active) {
+            p.kout[pos] = kn;
+            p.vout[pos] = v;
+        }
+        // (Columns of an alignment crowd on few digits: a warp's equal counts
+        // are added at once.)
+        const unsigned at = active ? (pos / kSortTile) * 256u +
+                                         ((unsigned)(kn >> p.shift_next) & 255u)
+                                   : 0x80000000u + lane;
+        const unsigned same = __match_any_sync(0xffffffffu, at);
+        if (active && (same & ((1u << lane) - 1u)) == 0)
+            atomicAdd(p.hist_next + at, __popc(same));
+    } else if (active) {
+        p.vout[pos] = v;
+    }
+}
+
+// Exclusive scan of v[0..n) in place, one CTA of 1024 threads: each sums a
+// contiguous segment, the segment sums are scanned in shared memory, then
+// each thread writes its segment's prefixes.
+__global__ void __launch_bounds__(1024) radix_scan(uint32_t *v, unsigned n) {
+    constexpr unsigned NT = 1024;
     __shared__ uint32_t part[NT];
     const unsigned t = threadIdx.x;
     const unsigned seg = (n + NT - 1) / NT;
@@ -190,72 +320,6 @@ __device__ uint32_t block_exclusive_scan(uint32_t *v, unsigned n) {
         const uint32_t x = v[i];
         v[i] = run;
         run += x;
-    }
-    const uint32_t total = part[NT - 1];
-    __syncthreads();  // part is reused by the next call
-    return total;
-}
-
-// Exclusive scan of v[0..n) in place, one CTA of 1024 threads.
-__global__ void __launch_bounds__(1024) radix_scan(uint32_t *v, unsigned n) {
-    block_exclusive_scan<1024>(v, n);
-}
-
-// Digit d's row of tile counts, hist[d * ntiles ..], scanned in place by
-// CTA d; tot[d] = the digit's count.
-__global__ void __launch_bounds__(kSortThreads)
-    radix_rowscan(uint32_t *hist, unsigned ntiles, uint32_t *tot) {
-    const uint32_t t = block_exclusive_scan<kSortThreads>(hist + (size_t)blockIdx.x * ntiles,
-                                                          ntiles);
-    if (threadIdx.x == 0) tot[blockIdx.x] = t;
-}
-
-// Stable scatter of one pass.  A tile is read in rounds of kSortThreads
-// pairs, pair r + t to thread t, so lower threads hold earlier pairs.  A
-// pair's place is its digit's next free slot for this tile (offs: the
-// digit's base, an exclusive scan of the digit counts tot, plus its
-// row-scanned tile count), plus the pairs with its digit in lower warps of
-// the round (wcnt) and in lower lanes of its warp (__match_any_sync).
-__global__ void __launch_bounds__(kSortThreads)
-    radix_scatter(const unsigned long long *kin, const uint32_t *vin, unsigned n,
-                  unsigned shift, const uint32_t *hist, const uint32_t *tot,
-                  unsigned long long *kout, uint32_t *vout) {
-    constexpr unsigned W = kSortThreads / 32;
-    __shared__ uint32_t offs[256];
-    __shared__ uint32_t wcnt[W][256];
-    const unsigned t = threadIdx.x, w = t / 32, lane = t % 32;
-    offs[t] = tot[t];
-    __syncthreads();
-    block_exclusive_scan<kSortThreads>(offs, 256);
-    offs[t] += hist[t * gridDim.x + blockIdx.x];
-    for (unsigned j = 0; j < W; ++j) wcnt[j][t] = 0;
-    __syncthreads();
-    const unsigned base = blockIdx.x * kSortTile;
-    const unsigned end = min(base + kSortTile, n);
-    for (unsigned r = base; r < end; r += kSortThreads) {
-        const unsigned i = r + t;
-        const bool active = i < end;
-        const unsigned long long k = active ? kin[i] : 0ull;
-        const uint32_t v = active ? vin[i] : 0u;
-        // Inactive lanes get a digit no other lane has.
-        const unsigned d = active ? ((unsigned)(k >> shift) & 255u) : 256u + lane;
-        const unsigned peers = __match_any_sync(0xffffffffu, d);
-        const unsigned below = __popc(peers & ((1u << lane) - 1u));
-        const bool leader = below == 0;
-        if (active && leader) wcnt[w][d] = __popc(peers);
-        __syncthreads();
-        if (active) {
-            unsigned pos = offs[d] + below;
-            for (unsigned j = 0; j < w; ++j) pos += wcnt[j][d];
-            kout[pos] = k;
-            vout[pos] = v;
-        }
-        __syncthreads();
-        if (active && leader) {
-            atomicAdd(&offs[d], __popc(peers));
-            wcnt[w][d] = 0;
-        }
-        __syncthreads();
     }
 }
 
@@ -304,17 +368,31 @@ __global__ void __launch_bounds__(1024)
 }  // namespace
 
 // Rank table over the canonical codes that occur (used[code] != 0), in
-// byte order, and the bits a rank needs.
+// byte order, and the base of the keys: the number of those codes, at least 2.
 static void compact_tables(const uint8_t *canon, const uint32_t *used, uint8_t *rank,
-                           unsigned *bits) {
+                           unsigned *base) {
     unsigned r = 0;
     uint8_t code_rank[256] = {};
     for (int c = 0; c < 256; ++c)
         if (used[c]) code_rank[c] = (uint8_t)r++;
     for (int c = 0; c < 256; ++c) rank[c] = code_rank[canon[c]];
-    unsigned b = 1;
-    while ((1u << b) < r) ++b;
-    *bits = b;
+    *base = r < 2 ? 2 : r;
+}
+
+// Characters of base r a 64-bit key holds (8 for r = 256).
+static unsigned chars_per_key(unsigned r) {
+    unsigned m = 0;
+    for (unsigned __int128 p = r; p <= (unsigned __int128)1 << 64; p *= r) ++m;
+    return m;
+}
+
+// 8-bit digits of the keys of m characters of base r.
+static unsigned key_digits(unsigned r, unsigned m) {
+    unsigned __int128 p = 1;
+    for (unsigned i = 0; i < m; ++i) p *= r;
+    unsigned d = 0;
+    for (--p; p; p >>= 8) ++d;
+    return d;
 }
 
 // Device compaction: inputs and outputs in device memory, on `s`.
@@ -327,9 +405,8 @@ size_t compact_work_bytes(unsigned ntaxa, unsigned nsites) {
     const size_t max_chunks = (ntaxa + 7) / 8;
     const size_t n = nsites;
     const size_t ntiles = (n + kSortTile - 1) / kSortTile;
-    const size_t hist = ntiles * 256 * 4 + 1024, scan = ((n + 1023) / 1024) * 4;
     return 2048 + al256c(max_chunks * n * 8) + 2 * al256c(n * 8) + 4 * al256c(n * 4) +
-           al256c(hist > scan ? hist : scan);
+           3 * al256c(ntiles * 1024) + 1024;
 }
 
 int compact_device(const uint8_t *rows, unsigned ntaxa, unsigned nsites,
@@ -356,10 +433,10 @@ int compact_device(const uint8_t *rows, unsigned ntaxa, unsigned nsites,
     CXG_CUDA(cudaMemcpyAsync(used_h, used, 1024, cudaMemcpyDeviceToHost, s));
     CXG_CUDA(cudaStreamSynchronize(s));
     uint8_t rank_h[256];
-    unsigned bits = 8;
-    compact_tables(canon_host, used_h, rank_h, &bits);
+    unsigned base = 2;
+    compact_tables(canon_host, used_h, rank_h, &base);
     CXG_CUDA(cudaMemcpyAsync(rank, rank_h, 256, cudaMemcpyHostToDevice, s));
-    const unsigned cpk = 64 / bits;
+    const unsigned cpk = chars_per_key(base);
     const unsigned nchunks = (ntaxa + cpk - 1) / cpk;
     if (nchunks > 65535) return fail(CXG_EINVAL, "compaction: too many taxa");
     unsigned long long *keys = (unsigned long long *)take(((size_t)ntaxa + 7) / 8 * n * 8);
@@ -370,42 +447,70 @@ int compact_device(const uint8_t *rows, unsigned ntaxa, unsigned nsites,
     uint32_t *flag = (uint32_t *)take(n * 4);
     uint32_t *gid = (uint32_t *)take(n * 4);
     const unsigned ntiles = (unsigned)((n + kSortTile - 1) / kSortTile);
-    uint32_t *hist = (uint32_t *)p;  // [256][ntiles] digit counts, or tile sums
-    uint32_t *dtot = hist + (size_t)ntiles * 256;  // [256] counts of each digit
+    uint32_t *hist[3];  // [ntiles][256] digit counts of a pass and the next two
+    for (uint32_t *&h : hist) h = (uint32_t *)take((size_t)ntiles * 1024);
+    uint32_t *dtot = (uint32_t *)take(1024);  // [256] counts of each digit
 
     const unsigned nb = (unsigned)((n + 255) / 256);
-    compact_keys<<<dim3(nb, nchunks), 256, 0, s>>>(rows, ntaxa, nsites, rank, bits, cpk, keys);
+    compact_keys<<<dim3(nb, nchunks), 256, 0, s>>>(rows, ntaxa, nsites, rank, base, cpk, keys);
     CXG_CHECK_LAUNCH("compact_keys");
-    // Identity order, then one stable sort per key chunk, last chunk first.
-    std::vector<uint32_t> iota(n);
-    for (size_t i = 0; i < n; ++i) iota[i] = (uint32_t)i;
-    CXG_CUDA(cudaMemcpyAsync(i0, iota.data(), n * 4, cudaMemcpyHostToDevice, s));
-    const unsigned kbits = cpk * bits;
-    for (int c = (int)nchunks - 1; c >= 0; --c) {
-        compact_gather<<<nb, 256, 0, s>>>(keys + (size_t)c * n, i0, (unsigned)n, k0);
-        CXG_CHECK_LAUNCH("compact_gather");
-        // Stable passes over the key's 8-bit digits, least significant first.
-        for (unsigned shift = 0; shift < kbits; shift += 8) {
-            radix_hist<<<ntiles, kSortThreads, 0, s>>>(k0, (unsigned)n, shift, hist);
-            radix_rowscan<<<256, kSortThreads, 0, s>>>(hist, ntiles, dtot);
-            radix_scatter<<<ntiles, kSortThreads, 0, s>>>(k0, i0, (unsigned)n, shift, hist,
-                                                          dtot, k1, i1);
-            CXG_CHECK_LAUNCH("compaction radix sort");
-            unsigned long long *tk = k0;
-            k0 = k1;
-            k1 = tk;
-            uint32_t *ti = i0;
-            i0 = i1;
-            i1 = ti;
+    // Stable passes, last chunk first, each from its least significant digit.
+    struct Digit {
+        unsigned chunk, shift;
+    };
+    std::vector<Digit> dig;
+    for (unsigned c = nchunks; c-- > 0;) {
+        const unsigned nd = key_digits(base, std::min(cpk, ntaxa - c * cpk));
+        for (unsigned j = 0; j < nd; ++j) dig.push_back({c, 8 * j});
+    }
+    const unsigned long long *kin = keys + (size_t)dig[0].chunk * n;
+    radix_hist<<<ntiles, kSortTile, 0, s>>>(kin, (unsigned)n, dig[0].shift, hist[0]);
+    CXG_CHECK_LAUNCH("radix_hist");
+    CXG_CUDA(cudaMemsetAsync(hist[1], 0, (size_t)ntiles * 1024, s));
+    for (size_t j = 0; j < dig.size(); ++j) {
+        const bool more = j + 1 < dig.size();
+        RadixPass ps = {};
+        if (ntiles > kSelfSum) {
+            radix_rowscan<<<8, 1024, 0, s>>>(hist[j % 3], ntiles, dtot);
+            CXG_CHECK_LAUNCH("radix_rowscan");
+            ps.tot = dtot;
         }
+        ps.kin = kin;
+        ps.vin = j ? i0 : nullptr;
+        ps.n = (unsigned)n;
+        ps.shift = dig[j].shift;
+        ps.hist = hist[j % 3];
+        if (more) {
+            ps.hist_next = hist[(j + 1) % 3];
+            ps.hist_zero = hist[(j + 2) % 3];
+            if (dig[j + 1].chunk != dig[j].chunk) ps.keys_next = keys + (size_t)dig[j + 1].chunk * n;
+            ps.shift_next = dig[j + 1].shift;
+        }
+        ps.kout = k1;
+        ps.vout = i1;
+        // Launched while the kernel before it still runs; it waits for that
+        // one's end before it reads or writes memory.
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(ntiles);
+        cfg.blockDim = dim3(kSortTile);
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        CXG_CUDA(cudaLaunchKernelEx(&cfg, radix_pass, ps));
+        kin = k1;
+        std::swap(k0, k1);
+        std::swap(i0, i1);
     }
     compact_flags<<<nb, 256, 0, s>>>(keys, nchunks, i0, (unsigned)n, flag);
     CXG_CHECK_LAUNCH("compact_flags");
     // gid = inclusive scan of the flags.
     const unsigned nt = (unsigned)((n + 1023) / 1024);
-    tile_sums<<<nt, 1024, 0, s>>>(flag, (unsigned)n, hist);
-    radix_scan<<<1, 1024, 0, s>>>(hist, nt);
-    tile_scan<<<nt, 1024, 0, s>>>(flag, (unsigned)n, hist, gid);
+    tile_sums<<<nt, 1024, 0, s>>>(flag, (unsigned)n, hist[0]);
+    radix_scan<<<1, 1024, 0, s>>>(hist[0], nt);
+    tile_scan<<<nt, 1024, 0, s>>>(flag, (unsigned)n, hist[0], gid);
     CXG_CHECK_LAUNCH("compaction scan");
     CXG_CUDA(cudaMemcpyAsync(npat_dev, gid + n - 1, 4, cudaMemcpyDeviceToDevice, s));
     // rep reuses the key buffer (n words); frequencies start at zero.
@@ -433,6 +538,9 @@ static std::mutex g_compact_mu;
 // small fraction of the DMA rate.
 namespace {
 constexpr size_t kStageChunk = (size_t)32 << 20;
+// What is copied at a time (rows wider than this: up to a chunk).  A 12.8 MB
+// alignment in one piece had its copies one after the other.
+constexpr size_t kStagePiece = (size_t)2 << 20;
 unsigned char *g_stage[2] = {nullptr, nullptr};
 cudaEvent_t g_stage_ev[2] = {nullptr, nullptr};
 
@@ -454,9 +562,9 @@ int stage_init() {
 int staged_h2d(void *dst, const void *src, size_t n, cudaStream_t s) {
     const unsigned char *h = static_cast<const unsigned char *>(src);
     unsigned char *d = static_cast<unsigned char *>(dst);
-    for (size_t off = 0, i = 0; off < n; off += kStageChunk, ++i) {
+    for (size_t off = 0, i = 0; off < n; off += kStagePiece, ++i) {
         const int b = (int)(i & 1);
-        const size_t len = n - off < kStageChunk ? n - off : kStageChunk;
+        const size_t len = n - off < kStagePiece ? n - off : kStagePiece;
         CXG_CUDA(cudaEventSynchronize(g_stage_ev[b]));  // its last DMA is done
         memcpy(g_stage[b], h + off, len);
         CXG_CUDA(cudaMemcpyAsync(d + off, g_stage[b], len, cudaMemcpyHostToDevice, s));
@@ -477,7 +585,7 @@ int staged_d2h_rows(void *dst, const void *src, size_t dpitch, size_t width, siz
         CXG_CUDA(cudaStreamSynchronize(s));
         return 0;
     }
-    const size_t per = kStageChunk / width;
+    const size_t per = (width > kStagePiece ? kStageChunk : kStagePiece) / width;
     const size_t nblk = (height + per - 1) / per;
     auto issue = [&](size_t k) -> int {
         const size_t r0 = k * per, nr = height - r0 < per ? height - r0 : per;
@@ -540,9 +648,8 @@ extern "C" int cxgCompact(const uint8_t *rows, unsigned ntaxa, unsigned nsites,
     memcpy(tabs + 256, canon, 256);
     if (val) memcpy(tabs + 512, val, 256); else memset(tabs + 512, 0, 256);
     if ((rc = stage_init()) || (rc = staged_h2d(d + o_rows, rows, in_bytes, s))) return fin(rc);
-    if ((freqs && (e = cudaMemcpyAsync(d + o_freq, freqs, (size_t)nsites * 4,
-                                       cudaMemcpyHostToDevice, s))) ||
-        (e = cudaMemcpyAsync(d + o_tab, tabs, 768, cudaMemcpyHostToDevice, s)))
+    if (freqs && (rc = staged_h2d(d + o_freq, freqs, (size_t)nsites * 4, s))) return fin(rc);
+    if ((e = cudaMemcpyAsync(d + o_tab, tabs, 768, cudaMemcpyHostToDevice, s)))
         return fin(cuda_fail(e, "cxgCompact: upload"));
     const uint8_t *dt = (const uint8_t *)(d + o_tab);
     rc = compact_device((const uint8_t *)(d + o_rows), ntaxa, nsites,
@@ -560,9 +667,8 @@ extern "C" int cxgCompact(const uint8_t *rows, unsigned ntaxa, unsigned nsites,
         return fin(rc);
     if (masks_out && np && (rc = staged_d2h_rows(masks_out, d + o_mask, nsites, np, ntaxa, s)))
         return fin(rc);
-    if ((e = cudaMemcpyAsync(freqs_out, d + o_fout, (size_t)np * 4, cudaMemcpyDeviceToHost, s)) ||
-        (e = cudaStreamSynchronize(s)))
-        return fin(cuda_fail(e, "cxgCompact: frequencies"));
+    if (np && (rc = staged_d2h_rows(freqs_out, d + o_fout, (size_t)np * 4, (size_t)np * 4, 1, s)))
+        return fin(rc);
     *npat = np;
     return fin(0);
 }
