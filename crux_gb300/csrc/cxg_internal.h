@@ -350,6 +350,10 @@ struct PmatArgs {
     double *ltab;              // FP64 plans: leaf-message tables
     WalkResult *zero = nullptr;  // pmat_kernel: cleared before the walker that
                                  // follows it runs (its result)
+    // pmat_kernel: root weights copied for the walker that follows it, when
+    // the values are read from pinned host memory (null: they are in place).
+    const double *pn_src = nullptr;  // [kact][4]
+    double *pn_dst = nullptr;
 };
 
 // Allocations of the library (cxg_lik.cu); each fails as an out-of-memory
@@ -400,7 +404,12 @@ cudaError_t launch_pmat_batch(const PmatArgs *jobs, const uint32_t *prefix,
 // before it on `s` (the walker stages its leaves while the P kernel runs).
 cudaError_t launch_plan(int precision, const PlanArgs &a, cudaStream_t s,
                         unsigned lanes = 1, bool pdl = false);
-cudaError_t launch_qdecomp(const double *rtri, const double *pi, double *out,
+// Eigensystem of a model given by value; out (74 doubles) may be pinned host
+// memory.
+struct QModel {
+    double rtri[6], pi[4];
+};
+cudaError_t launch_qdecomp(const QModel &m, double *out,
                            cudaStream_t s);
 unsigned plan_blocks(unsigned ppad, unsigned tile);
 // try_wait attempts of the walkers' record waits on the current device

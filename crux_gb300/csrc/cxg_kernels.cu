@@ -50,9 +50,12 @@ __device__ __forceinline__ void pdl_wait() {
 
 __global__ void pmat_kernel(PmatArgs a) {
     pdl_launch_dependents();
-    // The walker's result: it adds to it only after this grid has completed (stream order, or griddepcontrol.wait).
+    // The walker adds to its result only after this grid has completed
+    // (stream order, or griddepcontrol.wait).
     if (a.zero != nullptr && blockIdx.x == 0 && threadIdx.x < sizeof(WalkResult) / 8)
         reinterpret_cast<uint64_t *>(a.zero)[threadIdx.x] = 0;
+    if (a.pn_src != nullptr && blockIdx.x == 0 && threadIdx.x < a.kact * 4)
+        a.pn_dst[threadIdx.x] = a.pn_src[threadIdx.x];
     const unsigned idx = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
     if (idx >= a.nchild * a.kact) return;  // the same for all four lanes
     pmat_one(a, idx, threadIdx.x & 3u);
@@ -1213,7 +1216,7 @@ __device__ bool walk_tile(const PlanArgs &a, unsigned tile_idx, const LeanLayout
             for (int i = 0; i < KT * 4; ++i) {
                 T x = acc[h].get(i / 4, i % 4);
                 if (G > 1) x = __shfl_sync(0xffffffffu, x, lead + gg);
-                L = fma(__ldg(a.pn + gg * KT * 4 + i), (double)x, L);
+                L = fma(__ldcg(a.pn + gg * KT * 4 + i), (double)x, L);
             }
         }
         v[h] = 0.0;
@@ -1395,7 +1398,7 @@ __device__ bool walk_tile_lanes(const PlanArgs &a, unsigned tile_idx, const Smem
     double Lsum = 0.0;
 #pragma unroll
     for (int q = 0; q < KT * 4; ++q)
-        Lsum = fma(__ldg(a.pn + q), (double)acc[0].get(q / 4, q % 4), Lsum);
+        Lsum = fma(__ldcg(a.pn + q), (double)acc[0].get(q / 4, q % 4), Lsum);
     double v[1] = {0.0};
     bool ninf[1] = {false};
     if (lane == 0 && p < a.npat) {
@@ -1724,14 +1727,12 @@ int batch_ctas_per_sm(const WalkShape &w, size_t smem) {
     return e == cudaSuccess ? n : 0;
 }
 
-__global__ void qdecomp_kernel(const double *rtri, const double *pi,
-                               double *out) {
-    if (blockIdx.x == 0) qdecomp_warp(rtri, pi, out);
+__global__ void qdecomp_kernel(const __grid_constant__ QModel m, double *out) {
+    if (blockIdx.x == 0) qdecomp_warp(m.rtri, m.pi, out);
 }
 
-cudaError_t launch_qdecomp(const double *rtri, const double *pi, double *out,
-                           cudaStream_t s) {
-    qdecomp_kernel<<<1, 32, 0, s>>>(rtri, pi, out);
+cudaError_t launch_qdecomp(const QModel &m, double *out, cudaStream_t s) {
+    qdecomp_kernel<<<1, 32, 0, s>>>(m, out);
     return cudaGetLastError();
 }
 

@@ -240,8 +240,7 @@ struct State {
     std::unordered_map<uintptr_t, DevCL> cls;
     size_t cl_bytes = 0;
     size_t last_h2d = 0, last_d2h = 0;  // bytes copied by the last execute
-    DevBuf misc;         // CxLikQDecomp in/out
-    HostBuf stage, out;  // program staging, CxLikQDecomp staging
+    HostBuf stage, out;  // program staging, CxLikQDecomp results
     // Recorded after each program upload from `stage`: the next translation
     // waits on it before it rewrites the staging buffer, so no upload has
     // to be waited for on the launch path.
@@ -1006,6 +1005,7 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
     pa.tab = (const int32_t *)(d + o_tab);
     pa.wnorm = lik->wNorm;
     pa.wnorm_dev = nullptr;
+    pa.pn_src = nullptr;
     pa.rec = (unsigned char *)(d + o_rec);
     rc = P.ltab.ensure((size_t)(ntab ? ntab : 1) * 16 * kact * 4 * 8);
     if (rc) return rc;
@@ -1156,9 +1156,11 @@ static void plan_key(const State &S, const CxtLik *lik, int prec,
     }
 }
 
-// Reuse the scratch plan's translation for a call with the same key:
-// write the values into the staging image and upload only them (the
-// records, child descriptors and tables on the device are unchanged).
+// Reuse the scratch plan's translation for a call with the same key: the
+// records, child descriptors and tables on the device are unchanged, and the
+// P kernel reads the values from the pinned staging image itself (two copies
+// and an event less).  The caller waits for the stream before the image is
+// written again.
 static int refresh_values(State &S, CxtLik *lik, Plan &P) {
     const void *dfreqs = nullptr;
     int rc = pattern_weights(S, lik, &dfreqs);
@@ -1172,15 +1174,22 @@ static int refresh_values(State &S, CxtLik *lik, Plan &P) {
     if (rc) return rc;
     char *h = static_cast<char *>(S.stage.p);
     pack_values(lik, P, h);
-    char *d = static_cast<char *>(P.prog.p);
-    CXG_CUDA(cudaMemcpyAsync(d + P.o_elen, h + P.o_elen, P.o_dst - P.o_elen,
-                             cudaMemcpyHostToDevice, S.stream));
-    CXG_CUDA(cudaMemcpyAsync(d + P.o_pn, h + P.o_pn, pn_bytes, cudaMemcpyHostToDevice,
-                             S.stream));
-    CXG_CUDA(cudaEventRecord(S.stage_ev, S.stream));
-    S.stage_pending = true;
+    PmatArgs &pa = P.pa;
+    pa.edge_len = (const double *)(h + P.o_elen);
+    pa.cmult = (const double *)(h + P.o_cm);
+    pa.rmult = (const double *)(h + P.o_rm);
+    pa.model = (const int32_t *)(h + P.o_mod);
+    pa.cube = (const double *)(h + P.o_cube);
+    pa.eig = (const double *)(h + P.o_eig);
+    pa.wnorm = lik->wNorm;
+    char *pn = static_cast<char *>(P.prog.p) + P.o_pn;
+    if (pa.nchild) {
+        pa.pn_src = (const double *)(h + P.o_pn);
+        pa.pn_dst = (double *)pn;
+    } else {  // nothing but the root to evaluate: no P kernel
+        CXG_CUDA(cudaMemcpyAsync(pn, h + P.o_pn, pn_bytes, cudaMemcpyHostToDevice, S.stream));
+    }
     S.last_h2d = (P.o_dst - P.o_elen) + pn_bytes;
-    P.pa.wnorm = lik->wNorm;
     P.a.freqs = static_cast<const uint32_t *>(dfreqs);
     return 0;
 }
@@ -1213,13 +1222,14 @@ static int execute(CxtLik *lik, int prec, double *lnL, double *site) {
         return rc;
     }
     rc = enqueue(S, P, site != nullptr, nullptr, nullptr, true);
+    if (rc == 0) {
+        S.last_d2h = sizeof(WalkResult) + (site ? (size_t)P.npat * 8 : 0);
+        rc = finish(S, P, lnL, site);
+    }
     if (rc) {
         S.last_valid = false;
-        return rc;
+        cudaStreamSynchronize(S.stream);  // what was launched reads the staging image
     }
-    S.last_d2h = sizeof(WalkResult) + (site ? (size_t)P.npat * 8 : 0);
-    rc = finish(S, P, lnL, site);
-    if (rc) S.last_valid = false;
     return rc;
 }
 
@@ -1862,18 +1872,14 @@ bool CxLikQDecomp(int n, double *RTri, double *PiDiag, double *PiDiagNorm,
     State &S = state();
     std::lock_guard<std::mutex> g(S.mu);
     if (ensure_ready(S)) return true;
-    if (S.out.ensure(74 * 8 + 10 * 8)) return true;
-    if (S.misc.ensure(32 + 128 * 8 + 84 * 8)) return true;
+    // The kernel takes the model by value and writes pinned memory: with a
+    // copy each way a call took 42 us, 20 of them the kernel's.
+    if (S.out.ensure(74 * 8)) return true;
     double *h = static_cast<double *>(S.out.p);
-    for (int i = 0; i < 6; ++i) h[i] = RTri[i];
-    for (int i = 0; i < 4; ++i) h[6 + i] = PiDiag[i];
-    double *din = (double *)((char *)S.misc.p + 32);
-    double *dout = din + 10;
-    if (cudaMemcpyAsync(din, h, 10 * 8, cudaMemcpyHostToDevice, S.stream) !=
-            cudaSuccess ||
-        launch_qdecomp(din, din + 6, dout, S.stream) != cudaSuccess ||
-        cudaMemcpyAsync(h, dout, 74 * 8, cudaMemcpyDeviceToHost, S.stream) !=
-            cudaSuccess ||
+    QModel m;
+    for (int i = 0; i < 6; ++i) m.rtri[i] = RTri[i];
+    for (int i = 0; i < 4; ++i) m.pi[i] = PiDiag[i];
+    if (launch_qdecomp(m, h, S.stream) != cudaSuccess ||
         cudaStreamSynchronize(S.stream) != cudaSuccess) {
         set_error("CxLikQDecomp: CUDA failure");
         return true;
