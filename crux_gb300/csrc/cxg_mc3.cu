@@ -245,8 +245,7 @@ enum : unsigned { FIN_EIG = 1, FIN_GAMMA = 2, FIN_ALL = 3, FIN_WEIGHTS = 4 };
 // weights of the whole mixture (Lik.pyx:1603-1665); the parts `what` does
 // not name are kept.  Three warps, threads 32..127 of a block: a warp's FP64
 // instruction holds its SM quarter for 64 cycles, so the Gamma cuts go to
-// one warp each (their series run different lengths) and the eigensystem to
-// the third.  The result (true: decomposed) is thread 32's.
+// half a warp each and the eigensystem to the third warp.  The result (true: decomposed) is thread 32's.
 __device__ bool mc3_model_finish(Mc3Model &m, unsigned ncat, unsigned invar, unsigned mmax,
                                  unsigned what, unsigned mi) {
     __shared__ double s_cut[kMaxComps];
@@ -257,13 +256,7 @@ __device__ bool mc3_model_finish(Mc3Model &m, unsigned ncat, unsigned invar, uns
     const bool gamma = (what & FIN_GAMMA) && ncat > 1 && q.gamma_on;
     if (threadIdx.x == 32) s_bad = 0;
     asm volatile("bar.sync 1, 96;" ::: "memory");
-    if (gamma && w + 3 * lane < ncat - 1) {
-        const double cut = d_gamma_cut(q.alpha, (int)ncat, (int)(w + 3 * lane));
-        if (cut == -1.0)
-            s_bad = 1;
-        else
-            s_cut[w + 3 * lane] = cut;
-    }
+    if (gamma && !gamma_cuts(q.alpha, (int)ncat, w, s_cut)) s_bad = 1;
     __syncwarp();
     if ((what & FIN_EIG) && w == 2) {
         qdecomp_warp(q.rates, q.freqs, s_eig);
@@ -601,6 +594,25 @@ __device__ EtbrEnd etbr_end(int n0, int eA, int32_t *inc, int32_t *ex, Philox &r
     return r;
 }
 
+// The k-th v < n (from 0) with ok(v), -1 if there are fewer: eight at a time,
+// whose loads go out together.
+template <typename F>
+__device__ inline int kth_node(unsigned n, unsigned k, F ok) {
+    for (unsigned v0 = 0; v0 < n; v0 += 8) {
+        unsigned m = 0;
+#pragma unroll
+        for (unsigned j = 0; j < 8; ++j)
+            if (v0 + j < n && ok(v0 + j)) m |= 1u << j;
+        const unsigned c = (unsigned)__popc(m);
+        if (k < c) {
+            for (; k; --k) m &= m - 1;
+            return (int)v0 + __ffs((int)m) - 1;
+        }
+        k -= c;
+    }
+    return -1;
+}
+
 // Shared memory of one chain's proposal: the tree (parent, child, len,
 // cur), dirty flags, DFS stack, dirty list, the per-op prefix of
 // children, and the stack slot of each op and of each op's children.
@@ -612,8 +624,12 @@ __host__ __device__ inline size_t mc3_propose_smem(unsigned NN, unsigned M) {
 // One block per chain.  The chain's tree is staged in shared memory; one
 // thread draws and applies the move and lists the dirty nodes there (the
 // serial part: pointer chasing at shared-memory latency), then the block
-// writes the op records and the tree back in parallel.
-__global__ void mc3_propose_kernel(Mc3Dev d) {
+// writes the op records and the tree back in parallel.  Bound by the serial
+// part and by FP64 latency: the slowest of eight chains takes 83 us on average
+// (102 with 128 threads, an op's record to a thread and SPR's nodes listed by
+// a walk over the whole tree).  The model's warps are threads 32..127.
+constexpr unsigned kProposeThreads = 256;
+__global__ void __launch_bounds__(kProposeThreads) mc3_propose_kernel(Mc3Dev d) {
     const unsigned c = blockIdx.x;
     if (c >= d.nchains) return;
     const uint64_t g = *d.gen;
@@ -669,7 +685,7 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
         }
         __syncthreads();
     }
-    __shared__ int s_nd, s_lowest, s_fl;
+    __shared__ int s_nd, s_lowest, s_lowest2, s_fl;
     __shared__ unsigned s_fin, s_fin_mi;
     __shared__ bool s_full, s_etbr;
     __shared__ DirichletPair s_dir;  // a move's Hastings ratio, taken by a warp below
@@ -704,7 +720,7 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
         bool full = false;
         bool topo = false;  // a topology move under polytomy jumps
         double lnr0 = 0.0;  // ln NR of the current tree (topo)
-        int lowest = -1;  // lowest dirty node of a path move
+        int lowest = -1, lowest2 = -1;  // lowest dirty nodes of a path move
         if (g == 0) {
             pr.type = MV_INIT;
             full = true;
@@ -786,11 +802,9 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
                 // the root (the root keeps its three children).
                 const unsigned ns = NN - 1 - 3;
                 unsigned k = philox_below(rng, ns);
-                int s = -1;
-                for (unsigned v = 0; v < NN && s < 0; ++v) {
-                    if (v == d.root || parent[v] == (int)d.root) continue;
-                    if (k-- == 0) s = (int)v;
-                }
+                const int s = kth_node(NN, k, [&](unsigned v) {
+                    return v != d.root && parent[v] != (int)d.root;
+                });
                 const int p = parent[s], g = parent[p];
                 int jb = -1, jg = -1;
                 for (int j = 0; j < 3; ++j) {
@@ -824,11 +838,9 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
                 // subtree: not the root, not p, not marked.
                 const unsigned ne = NN - 2 - nsub;
                 k = philox_below(rng, ne);
-                int x = -1;
-                for (unsigned v = 0; v < NN && x < 0; ++v) {
-                    if (v == d.root || (int)v == p || dflag[v] == 2) continue;
-                    if (k-- == 0) x = (int)v;
-                }
+                const int x = kth_node(NN, k, [&](unsigned v) {
+                    return v != d.root && (int)v != p && dflag[v] != 2;
+                });
                 {
                     int sp = 0;
                     stack[sp++] = s;
@@ -871,8 +883,8 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
                 // reverse meets the same edges).
                 if (coll[p] || coll[b] || coll[x]) pr.lnPrior = -INFINITY;
                 // Dirty: both paths to the root (p's new place, g's old child).
-                for (int v = p; v >= 0; v = parent[v]) dflag[v] = 1;
-                for (int v = g; v >= 0; v = parent[v]) dflag[v] = 1;
+                lowest = p;
+                lowest2 = g;
             } else if (t == MV_ETBR) {
                 // Edges are named by the node below them in the current
                 // rooting; len[] holds their lengths.  child[] becomes the
@@ -1330,6 +1342,7 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
         if (pr.type != MV_MIXJ) s_fin_mi = mi;
         s_full = full;
         s_lowest = lowest;
+        s_lowest2 = lowest2;
     }
     __syncthreads();
     if (s_etbr) {
@@ -1372,7 +1385,7 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
         const double h = ln_dirichlet_ratio(s_dir);
         if (threadIdx.x == 32) pr.lnHast = h;
     }
-    if (threadIdx.x >= 32 && s_fin) {
+    if (threadIdx.x >= 32 && threadIdx.x < 128 && s_fin) {
         Mc3Model &m1 = d.model[c * 2 + (1 - d.curmodel[c])];
         const bool ok = mc3_model_finish(m1, d.ncat, d.invar, d.mmax, s_fin, s_fin_mi);
         if (threadIdx.x == 32 && !ok) {
@@ -1394,7 +1407,7 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
                 for (int u = parent[v]; u >= 0 && dflag[u] != 1; u = parent[u]) dflag[u] = 1;
             }
         }
-        if (pr.type == MV_SPR || s_etbr) {
+        if (s_etbr) {
             // The nodes flagged above, in reversed pre-order of the new tree.
             int sp = 0;
             stack[sp++] = (int)d.root;
@@ -1434,6 +1447,11 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
             }
             nd = top;
         } else {
+            if (s_lowest2 >= 0) {
+                // The second path up to where it meets the first.
+                for (int v = lowest; v >= 0; v = parent[v]) dflag[v] = 1;
+                for (int v = s_lowest2; !dflag[v]; v = parent[v]) dirty[nd++] = v;
+            }
             for (int v = lowest; v >= 0; v = parent[v]) dirty[nd++] = v;
         }
         pr.ndirty = nd;
@@ -1523,9 +1541,11 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
         }
         __syncthreads();
     }
-    // Op records, one op per thread: parent -> its spare buffer; children
-    // -> spare buffer if dirty (computed earlier in this walk), else
-    // current.  A leaf child points at the leaf's mask array.
+    // Op records, an op's head and each of its children to a thread (an op a
+    // thread, one load waiting for another, took 17 us of a full walk's
+    // proposal): parent -> its spare buffer; children -> spare buffer if dirty
+    // (computed earlier in this walk), else current.  A leaf child points at
+    // the leaf's mask array.
     const Mc3Model &mm = pr.model_changed ? d.model[c * 2 + (1 - d.curmodel[c])]
                                           : d.model[c * 2 + d.curmodel[c]];
     unsigned char *rec = d.rec + (size_t)c * M * d.rstride;
@@ -1533,61 +1553,71 @@ __global__ void mc3_propose_kernel(Mc3Dev d) {
     double *klen = d.kid_len + (size_t)c * d.maxkids;
     uint64_t *kdst = d.kid_dst + (size_t)c * d.maxkids;
     int32_t *ktab = d.kid_tab + (size_t)c * d.maxkids;
-    for (int o = threadIdx.x; o < nd; o += blockDim.x) {
+    for (int it = threadIdx.x; it < 4 * nd; it += blockDim.x) {
+        const int o = it >> 2, j = it & 3;
         const int v = dirty[o];
-        const int mi = v - (int)N;
         unsigned char *r = rec + (size_t)o * d.rstride;
-        RecHead hd;
-        hd.data = d.cl_data[((size_t)c * M + mi) * 2 + (1 - cur[v])];
-        hd.scaler = d.cl_sc[((size_t)c * M + mi) * 2 + (1 - cur[v])];
-        const unsigned nch = kid0[o + 1] - kid0[o];
-        hd.nchild = nch;
-        hd.slot = op_slot[o];
-        hd.flags = 0;
-        hd.pad = 0;
-        int kcls[3] = {1, 1, 1};
-        unsigned ci = 0, nkid = kid0[o], nl = 0;
-        size_t area = sizeof(RecHead) + nch * sizeof(RecChild);
         const uint8_t **lr = lrows + (size_t)o * 3;
-        for (int j = 0; j < 3; ++j) {
-            const int u = child[v * 3 + j];
-            if (u < 0) continue;
-            RecChild ch;
-            memset(&ch, 0, sizeof(ch));
-            if (u < (int)N) {
-                ch.data = d.leafmask[u];
-                ch.idx = (uint32_t)u;
-                lr[nl++] = d.leafmask[u];
-                ch.src = SRC_LEAF;
-                ch.tab = nkid;
-                // FP64: table index; FP32: >= 0, the table goes in the record.
-                ktab[nkid] = (int32_t)nkid;
-            } else if (kid_slot[o * 3 + ci] >= 0) {
-                ch.src = SRC_SLOT;
-                ch.idx = (uint32_t)kid_slot[o * 3 + ci];
-                ktab[nkid] = -1;
-            } else {
-                const int ui = u - (int)N;
-                const int b = dflag[u] ? 1 - cur[u] : cur[u];
-                ch.data = d.cl_data[((size_t)c * M + ui) * 2 + b];
-                ch.scaler = d.cl_sc[((size_t)c * M + ui) * 2 + b];
-                ch.src = SRC_GLOBAL;
-                ktab[nkid] = -1;
-            }
-            ch.off = (uint32_t)area;
-            memcpy(r + sizeof(RecHead) + ci * sizeof(RecChild), &ch, sizeof(ch));
+        const unsigned nch = kid0[o + 1] - kid0[o];
+        // Children and leaf children before slot j, and where j's area is.
+        unsigned ci = 0, nl = 0;
+        size_t area = sizeof(RecHead) + nch * sizeof(RecChild);
+        int kcls[3] = {1, 1, 1};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const int u = child[v * 3 + q];
+            if (q >= j || u < 0) continue;
             // Class for the op kind: dirty node o - 1 is F (its result is
             // still in the walker's registers).
-            kcls[ci] = u < (int)N ? 0 : (o > 0 && u == dirty[o - 1] ? 2 : 1);
-            klen[nkid] = len[u];
-            kdst[nkid] = (size_t)o * d.rstride + area;
+            const int cls = u < (int)N ? 0 : (o > 0 && u == dirty[o - 1] ? 2 : 1);
+            if (ci == 0) kcls[0] = cls;
+            if (ci == 1) kcls[1] = cls;
             area += child_area_bytes((int)d.prec, d.kact, u < (int)N);
-            ++nkid;
             ++ci;
+            nl += u < (int)N;
         }
-        for (unsigned j = nl; j < 3; ++j) lr[j] = nullptr;
-        if (nch == 2) hd.flags |= op_kind_of_classes(kcls[0], kcls[1]);
-        memcpy(r, &hd, sizeof(hd));
+        if (j == 3) {
+            const size_t at = ((size_t)c * M + (v - (int)N)) * 2 + (1 - cur[v]);
+            RecHead hd;
+            hd.data = d.cl_data[at];
+            hd.scaler = d.cl_sc[at];
+            hd.nchild = nch;
+            hd.slot = op_slot[o];
+            hd.flags = nch == 2 ? op_kind_of_classes(kcls[0], kcls[1]) : 0;
+            hd.pad = 0;
+            memcpy(r, &hd, sizeof(hd));
+            for (; nl < 3; ++nl) lr[nl] = nullptr;
+            continue;
+        }
+        const int u = child[v * 3 + j];
+        if (u < 0) continue;
+        const unsigned nkid = kid0[o] + ci;
+        RecChild ch;
+        memset(&ch, 0, sizeof(ch));
+        int32_t tab = -1;
+        if (u < (int)N) {
+            ch.data = d.leafmask[u];
+            ch.idx = (uint32_t)u;
+            lr[nl] = d.leafmask[u];
+            ch.src = SRC_LEAF;
+            ch.tab = nkid;
+            // FP64: table index; FP32: >= 0, the table goes in the record.
+            tab = (int32_t)nkid;
+        } else if (kid_slot[o * 3 + ci] >= 0) {
+            ch.src = SRC_SLOT;
+            ch.idx = (uint32_t)kid_slot[o * 3 + ci];
+        } else {
+            const size_t at = ((size_t)c * M + (u - (int)N)) * 2 +
+                              (dflag[u] ? 1 - cur[u] : cur[u]);
+            ch.data = d.cl_data[at];
+            ch.scaler = d.cl_sc[at];
+            ch.src = SRC_GLOBAL;
+        }
+        ch.off = (uint32_t)area;
+        memcpy(r + sizeof(RecHead) + ci * sizeof(RecChild), &ch, sizeof(ch));
+        ktab[nkid] = tab;
+        klen[nkid] = len[u];
+        kdst[nkid] = (size_t)o * d.rstride + area;
     }
     // The tree (moved) and the dirty list back to HBM; an eTBR result goes
     // to the spare tree buffer, which the accept kernel makes current.
@@ -1820,7 +1850,7 @@ static void mc3_free(cxgMc3 *h) {
 
 static int mc3_enqueue_gen(cxgMc3 *h) {
     const Mc3Dev &d = h->d;
-    mc3_propose_kernel<<<d.nchains, 128, h->propose_smem, h->stream>>>(d);
+    mc3_propose_kernel<<<d.nchains, kProposeThreads, h->propose_smem, h->stream>>>(d);
     CXG_CHECK_LAUNCH("mc3_propose_kernel");
     mc3_pmat_kernel<<<h->pmat_grid, 128, 0, h->stream>>>(d);
     CXG_CHECK_LAUNCH("mc3_pmat_kernel");

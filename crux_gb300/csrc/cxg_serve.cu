@@ -59,9 +59,9 @@ struct SrvModel {
 // Model of one request, FP64 on the GPU: mixture of ncat Gamma categories
 // with weight (1 - pinv)/ncat each and, if pinv > 0, an invariant component
 // (cmult 0) of weight pinv; wNorm and root weights as Lik.prep
-// (Lik.pyx:1603-1665).  One warp per request (block b builds m[b]): lanes
-// 0..ncat-2 compute the Gamma category cuts while lanes 28..31 form the
-// eigensystem; lane 0 finishes.
+// (Lik.pyx:1603-1665).  Four warps per request (block b builds m[b]): three
+// compute the Gamma category cuts while the fourth forms the eigensystem;
+// thread 0 finishes.
 constexpr unsigned kModelsPerLaunch = 128;
 struct SrvModelList {
     SrvModel *m[kModelsPerLaunch];
@@ -73,21 +73,14 @@ __global__ void srv_model_kernel(SrvModelList list, unsigned n) {
     __shared__ double tmp[74];
     __shared__ double cut[kMaxComps];
     __shared__ int bad;
-    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const unsigned warp = threadIdx.x >> 5;
     const int ncat = m->ncat;
     if (threadIdx.x == 0) bad = 0;
     __syncthreads();
-    // One Gamma cut to a warp at a time (each on its own FP64 pipe), the
+    // The Gamma cuts on three warps (each its own FP64 pipe), the
     // eigensystem on the fourth.
     if (warp < 3) {
-        const int i = (int)(warp + 3 * lane);
-        if (ncat > 1 && i < ncat - 1) {
-            const double c = d_gamma_cut(m->alpha, ncat, i);
-            if (c == -1.0)
-                bad = 1;
-            else
-                cut[i] = c;
-        }
+        if (ncat > 1 && !gamma_cuts(m->alpha, ncat, warp, cut)) bad = 1;
     } else {
         qdecomp_warp(m->rates, m->freqs, tmp);
     }
