@@ -354,6 +354,14 @@ struct PmatArgs {
     // the values are read from pinned host memory (null: they are in place).
     const double *pn_src = nullptr;  // [kact][4]
     double *pn_dst = nullptr;
+    // pmat_kernel: a program image in pinned host memory, copied to the
+    // device by further blocks (null: it is there): of each of nrec records
+    // the head and its children, at most img_units 16-byte units, and
+    // img_tail units from img_off on.
+    const char *img_src = nullptr;
+    char *img_dst = nullptr;
+    uint32_t nrec = 0, rstride = 0, img_units = 0, img_tail = 0;
+    size_t img_off = 0;
 };
 
 // Allocations of the library (cxg_lik.cu); each fails as an out-of-memory

@@ -48,6 +48,36 @@ __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Blocks of four lanes per (child edge, component).
+__host__ __device__ inline unsigned pmat_blocks(const PmatArgs &a) {
+    return (a.nchild * a.kact + 31) / 32;
+}
+__host__ __device__ inline unsigned image_units(const PmatArgs &a) {
+    return a.nrec * a.img_units + a.img_tail;
+}
+
+// Unit t of a plan's program image, read from pinned host memory.  (A copy
+// and an event before the P kernel took 2 us more of every evaluation whose
+// path is new.)
+__device__ inline void copy_image(const PmatArgs &a, unsigned t) {
+    if (t >= image_units(a)) return;
+    size_t off = 0;
+    bool mine = true;
+    if (t < a.nrec * a.img_units) {
+        const unsigned u = t % a.img_units;
+        const size_t rec = (size_t)(t / a.img_units) * a.rstride;
+        // (The areas behind a record's children are the P blocks' to write.)
+        const uint32_t nchild =
+            reinterpret_cast<const RecHead *>(a.img_src + rec)->nchild;
+        mine = u < 2 + 2 * nchild;
+        off = rec + u * 16;
+    } else {
+        off = a.img_off + (size_t)(t - a.nrec * a.img_units) * 16;
+    }
+    const uint4 v = *reinterpret_cast<const uint4 *>(a.img_src + off);
+    if (mine) *reinterpret_cast<uint4 *>(a.img_dst + off) = v;
+}
+
 __global__ void pmat_kernel(PmatArgs a) {
     pdl_launch_dependents();
     // The walker adds to its result only after this grid has completed
@@ -56,6 +86,11 @@ __global__ void pmat_kernel(PmatArgs a) {
         reinterpret_cast<uint64_t *>(a.zero)[threadIdx.x] = 0;
     if (a.pn_src != nullptr && blockIdx.x == 0 && threadIdx.x < a.kact * 4)
         a.pn_dst[threadIdx.x] = a.pn_src[threadIdx.x];
+    const unsigned nblk = pmat_blocks(a);
+    if (blockIdx.x >= nblk) {
+        copy_image(a, (blockIdx.x - nblk) * blockDim.x + threadIdx.x);
+        return;
+    }
     const unsigned idx = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
     if (idx >= a.nchild * a.kact) return;  // the same for all four lanes
     pmat_one(a, idx, threadIdx.x & 3u);
@@ -83,9 +118,9 @@ cudaError_t launch_pmat_batch(const PmatArgs *jobs, const uint32_t *prefix,
 }
 
 cudaError_t launch_pmat(const PmatArgs &a, cudaStream_t s) {
-    const unsigned n = a.nchild * a.kact;
-    if (n == 0) return cudaSuccess;
-    pmat_kernel<<<(n + 31) / 32, 128, 0, s>>>(a);
+    if (a.nchild * a.kact == 0) return cudaSuccess;
+    const unsigned copies = a.img_src != nullptr ? (image_units(a) + 127) / 128 : 0;
+    pmat_kernel<<<pmat_blocks(a) + copies, 128, 0, s>>>(a);
     return cudaGetLastError();
 }
 

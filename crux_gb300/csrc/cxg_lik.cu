@@ -424,7 +424,7 @@ struct Plan {
     // lengths [stepsLen], cmult, rmult, model index [kact], cube and
     // eigenvalues [models], root weights pn [kact][4]; and what they are
     // read from (active components, their models).
-    size_t o_elen = 0, o_cm = 0, o_rm = 0, o_mod = 0, o_cube = 0, o_eig = 0,
+    size_t o_elen = 0, o_cm = 0, o_tab = 0, o_rm = 0, o_mod = 0, o_cube = 0, o_eig = 0,
            o_dst = 0, o_pn = 0;
     std::vector<unsigned> act;
     std::vector<const CxtLikModel *> models;
@@ -604,9 +604,11 @@ unsigned stack_slots(const WalkShape &w, unsigned rstride, unsigned lmax, unsign
 
 // `patterns`: padded patterns of all the `njobs` jobs of a batch this plan is
 // one of (njobs 0: it is launched by itself; patterns 0: its own).
+// upload false: the first run's P kernel fetches the program from the pinned
+// staging image, which the caller keeps until that run has ended.
 static int translate(State &S, CxtLik *lik, int prec, Plan &P,
                      bool use_slots = true, bool allow_lanes = false, size_t patterns = 0,
-                     unsigned njobs = 0) {
+                     unsigned njobs = 0, bool upload = true) {
     int rc;
     if (lik == nullptr) return fail(CXG_EINVAL, "lik is NULL");
     if (lik->dim != 4)
@@ -966,6 +968,7 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
     P.o_cube = o_cube;
     P.o_eig = o_eig;
     P.o_dst = o_dst;
+    P.o_tab = o_tab;
     P.o_pn = o_pn;
     P.act = act;
     P.models = models;
@@ -984,28 +987,44 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
         if (s_nleaf) memcpy(h + o_leaf, leaf_ptrs.data(), s_nleaf * sizeof(void *));
     }
     char *d = static_cast<char *>(P.prog.p);
-    CXG_CUDA(cudaMemcpyAsync(d, h, total, cudaMemcpyHostToDevice, S.stream));
-    S.last_h2d = total;
-    if (S.stage_ev == nullptr)
-        CXG_CUDA(cudaEventCreateWithFlags(&S.stage_ev, cudaEventDisableTiming));
-    CXG_CUDA(cudaEventRecord(S.stage_ev, S.stream));
-    S.stage_pending = true;
-
     PmatArgs &pa = P.pa;
     pa.nchild = nchild;
     pa.kact = kact;
     pa.precision = prec;
-    pa.edge_len = (const double *)(d + o_elen);
-    pa.cmult = (const double *)(d + o_cm);
-    pa.rmult = (const double *)(d + o_rm);
-    pa.model = (const int32_t *)(d + o_mod);
-    pa.cube = (const double *)(d + o_cube);
-    pa.eig = (const double *)(d + o_eig);
-    pa.dst = (const uint64_t *)(d + o_dst);
-    pa.tab = (const int32_t *)(d + o_tab);
+    pa.img_src = nullptr;
+    pa.pn_src = nullptr;
+    const char *from = d;  // what the P kernel reads its inputs from
+    if (upload || nchild == 0) {
+        CXG_CUDA(cudaMemcpyAsync(d, h, total, cudaMemcpyHostToDevice, S.stream));
+        S.last_h2d = total;
+        if (S.stage_ev == nullptr)
+            CXG_CUDA(cudaEventCreateWithFlags(&S.stage_ev, cudaEventDisableTiming));
+        CXG_CUDA(cudaEventRecord(S.stage_ev, S.stream));
+        S.stage_pending = true;
+    } else {
+        unsigned most = 0;
+        for (const HostOp &o : ops) most = std::max(most, (unsigned)o.nchild);
+        from = h;
+        pa.img_src = h;
+        pa.img_dst = d;
+        pa.nrec = (uint32_t)order.size();
+        pa.rstride = (uint32_t)rstride;
+        pa.img_units = (uint32_t)((sizeof(RecHead) + most * sizeof(RecChild)) / 16);
+        pa.img_off = o_dst;
+        pa.img_tail = (uint32_t)((total - o_dst) / 16);
+        S.last_h2d = order.size() * pa.img_units * 16 + (total - o_elen);
+    }
+
+    pa.edge_len = (const double *)(from + o_elen);
+    pa.cmult = (const double *)(from + o_cm);
+    pa.rmult = (const double *)(from + o_rm);
+    pa.model = (const int32_t *)(from + o_mod);
+    pa.cube = (const double *)(from + o_cube);
+    pa.eig = (const double *)(from + o_eig);
+    pa.dst = (const uint64_t *)(from + o_dst);
+    pa.tab = (const int32_t *)(from + o_tab);
     pa.wnorm = lik->wNorm;
     pa.wnorm_dev = nullptr;
-    pa.pn_src = nullptr;
     pa.rec = (unsigned char *)(d + o_rec);
     rc = P.ltab.ensure((size_t)(ntab ? ntab : 1) * 16 * kact * 4 * 8);
     if (rc) return rc;
@@ -1182,7 +1201,10 @@ static int refresh_values(State &S, CxtLik *lik, Plan &P) {
     pa.cube = (const double *)(h + P.o_cube);
     pa.eig = (const double *)(h + P.o_eig);
     pa.wnorm = lik->wNorm;
-    char *pn = static_cast<char *>(P.prog.p) + P.o_pn;
+    char *d = static_cast<char *>(P.prog.p), *pn = d + P.o_pn;
+    pa.img_src = nullptr;  // (its first run copied the rest)
+    pa.dst = (const uint64_t *)(d + P.o_dst);
+    pa.tab = (const int32_t *)(d + P.o_tab);
     if (pa.nchild) {
         pa.pn_src = (const double *)(h + P.o_pn);
         pa.pn_dst = (double *)pn;
@@ -1211,7 +1233,7 @@ static int execute(CxtLik *lik, int prec, double *lnL, double *site) {
         rc = refresh_values(S, lik, P);
     } else {
         S.last_valid = false;
-        rc = translate(S, lik, prec, P, true, true);
+        rc = translate(S, lik, prec, P, true, true, 0, 0, false);
         if (rc == 0) {
             plan_key(S, lik, prec, S.last_key);  // translating may allocate
             S.last_valid = true;
