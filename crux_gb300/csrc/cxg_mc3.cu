@@ -1781,6 +1781,39 @@ __global__ void mc3_accept_kernel(Mc3Dev d) {
     *d.gen = g + 1;
 }
 
+// A chain's state in pinned host memory: len[nnodes], parent[nnodes] and
+// coll[nnodes] follow.
+struct Mc3State {
+    double lnL, heat;
+    Mc3Model model;
+    __host__ __device__ double *len() { return reinterpret_cast<double *>(this + 1); }
+    __host__ __device__ int32_t *parent(unsigned nn) {
+        return reinterpret_cast<int32_t *>(len() + nn);
+    }
+    __host__ __device__ uint8_t *coll(unsigned nn) {
+        return reinterpret_cast<uint8_t *>(parent(nn) + nn);
+    }
+};
+
+// Written by one block.  (Eight copies a chain, each waited for because the
+// next one's address came with it, took 60 us.)
+__global__ void mc3_state_kernel(Mc3Dev d, unsigned c, Mc3State *out) {
+    const unsigned NN = d.nnodes;
+    const size_t t = ((size_t)d.curtree[c] * d.nchains + c) * NN;
+    for (unsigned i = threadIdx.x; i < NN; i += blockDim.x) {
+        out->len()[i] = d.len[t + i];
+        out->parent(NN)[i] = d.parent[t + i];
+        out->coll(NN)[i] = d.coll[t + i];
+    }
+    const uint64_t *m = reinterpret_cast<const uint64_t *>(&d.model[c * 2 + d.curmodel[c]]);
+    for (unsigned i = threadIdx.x; i < sizeof(Mc3Model) / 8; i += blockDim.x)
+        reinterpret_cast<uint64_t *>(&out->model)[i] = m[i];
+    if (threadIdx.x == 0) {
+        out->lnL = d.lnL[c];
+        out->heat = d.heat[c];
+    }
+}
+
 }  // namespace cxg
 
 using namespace cxg;
@@ -1799,6 +1832,7 @@ struct cxgMc3 {
     BatchArgs ba;
     unsigned grid = 0, pmat_grid = 0;
     size_t propose_smem = 0;
+    Mc3State *state = nullptr;  // pinned: one chain's state as last fetched
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;
     unsigned graph_gens = 0;
@@ -1844,6 +1878,7 @@ static void mc3_free(cxgMc3 *h) {
     if (h->exec) cudaGraphExecDestroy(h->exec);
     if (h->graph) cudaGraphDestroy(h->graph);
     for (void *p : h->allocs) dev_free(p);
+    if (h->state) host_free(h->state);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
 }
@@ -2054,6 +2089,13 @@ extern "C" int cxgMc3Create(const cxgMc3Config *cfg, cxgMc3 **out) {
             const uint8_t v = cfg->masks[(size_t)t * cfg->npat + p] & 15;
             masks[(size_t)t * d.ppad + p] = v ? v : 15;
         }
+    {
+        const cudaError_t se = host_alloc((void **)&h->state, sizeof(Mc3State) + (size_t)NN * 13);
+        if (se != cudaSuccess) {
+            mc3_free(h);
+            return cuda_fail(se, "cxgMc3Create: host memory");
+        }
+    }
     uint8_t *dmask = nullptr;
     uint32_t *dfreq = nullptr;
     const uint8_t **leafptr_host = new const uint8_t *[N];
@@ -2295,28 +2337,27 @@ int cxg::mc3_cold_lnl(cxgMc3 *h, double *out) {
     return 0;
 }
 
+// Chain c's state into h->state (the caller holds h->mu).
+static int mc3_fetch(cxgMc3 *h, unsigned c) {
+    mc3_state_kernel<<<1, 256, 0, h->stream>>>(h->d, c, h->state);
+    CXG_CHECK_LAUNCH("mc3_state_kernel");
+    CXG_CUDA(cudaStreamSynchronize(h->stream));
+    return 0;
+}
+
 extern "C" int cxgMc3Chain(cxgMc3 *h, unsigned chain, double *lnL, double *heat,
                            int32_t *parent, double *len, double *rates,
                            double *freqs, double *alpha) {
     if (h == nullptr || chain >= h->d.nchains) return fail(CXG_EINVAL, "cxgMc3Chain: bad chain");
     std::lock_guard<std::mutex> lk(h->mu);
     const Mc3Dev &d = h->d;
-    CXG_CUDA(cudaStreamSynchronize(h->stream));
-    if (lnL) CXG_CUDA(cudaMemcpy(lnL, d.lnL + chain, 8, cudaMemcpyDeviceToHost));
-    if (heat) CXG_CUDA(cudaMemcpy(heat, d.heat + chain, 8, cudaMemcpyDeviceToHost));
-    uint8_t tb = 0;
-    CXG_CUDA(cudaMemcpy(&tb, d.curtree + chain, 1, cudaMemcpyDeviceToHost));
-    const size_t t = (size_t)tb * d.nchains + chain;
-    if (parent)
-        CXG_CUDA(cudaMemcpy(parent, d.parent + t * d.nnodes, d.nnodes * 4,
-                            cudaMemcpyDeviceToHost));
-    if (len)
-        CXG_CUDA(cudaMemcpy(len, d.len + t * d.nnodes, d.nnodes * 8,
-                            cudaMemcpyDeviceToHost));
-    uint8_t cm = 0;
-    CXG_CUDA(cudaMemcpy(&cm, d.curmodel + chain, 1, cudaMemcpyDeviceToHost));
-    Mc3Model m;
-    CXG_CUDA(cudaMemcpy(&m, d.model + chain * 2 + cm, sizeof(m), cudaMemcpyDeviceToHost));
+    if (int rc = mc3_fetch(h, chain)) return rc;
+    Mc3State &st = *h->state;
+    if (lnL) *lnL = st.lnL;
+    if (heat) *heat = st.heat;
+    if (parent) memcpy(parent, st.parent(d.nnodes), (size_t)d.nnodes * 4);
+    if (len) memcpy(len, st.len(), (size_t)d.nnodes * 8);
+    const Mc3Model &m = st.model;
     const Mc3Sub &q = m.q[0];
     if (rates) memcpy(rates, q.rates, 48);
     if (freqs) memcpy(freqs, q.freqs, 32);
@@ -2485,12 +2526,8 @@ extern "C" int cxgMc3ChainCollapsed(cxgMc3 *h, unsigned chain, uint8_t *out) {
     if (h == nullptr || chain >= h->d.nchains || out == nullptr)
         return fail(CXG_EINVAL, "cxgMc3ChainCollapsed: bad arguments");
     std::lock_guard<std::mutex> lk(h->mu);
-    const Mc3Dev &d = h->d;
-    CXG_CUDA(cudaStreamSynchronize(h->stream));
-    uint8_t tb = 0;
-    CXG_CUDA(cudaMemcpy(&tb, d.curtree + chain, 1, cudaMemcpyDeviceToHost));
-    const size_t t = (size_t)tb * d.nchains + chain;
-    CXG_CUDA(cudaMemcpy(out, d.coll + t * d.nnodes, d.nnodes, cudaMemcpyDeviceToHost));
+    if (int rc = mc3_fetch(h, chain)) return rc;
+    memcpy(out, h->state->coll(h->d.nnodes), h->d.nnodes);
     return 0;
 }
 
@@ -2500,11 +2537,8 @@ extern "C" int cxgMc3ChainModel(cxgMc3 *h, unsigned chain, unsigned model,
         return fail(CXG_EINVAL, "cxgMc3ChainModel: bad chain or model");
     std::lock_guard<std::mutex> lk(h->mu);
     const Mc3Dev &d = h->d;
-    CXG_CUDA(cudaStreamSynchronize(h->stream));
-    uint8_t cm = 0;
-    CXG_CUDA(cudaMemcpy(&cm, d.curmodel + chain, 1, cudaMemcpyDeviceToHost));
-    Mc3Model m;
-    CXG_CUDA(cudaMemcpy(&m, d.model + chain * 2 + cm, sizeof(m), cudaMemcpyDeviceToHost));
+    if (int rc = mc3_fetch(h, chain)) return rc;
+    const Mc3Model &m = h->state->model;
     if (nmodels) *nmodels = (unsigned)m.nmodels;
     if (out == nullptr) return 0;
     if ((int)model >= m.nmodels) return fail(CXG_EINVAL, "cxgMc3ChainModel: no such model");
@@ -2526,12 +2560,8 @@ extern "C" int cxgMc3ChainWeights(cxgMc3 *h, unsigned chain, double *wvar, doubl
     if (h == nullptr || chain >= h->d.nchains)
         return fail(CXG_EINVAL, "cxgMc3ChainWeights: bad chain");
     std::lock_guard<std::mutex> lk(h->mu);
-    const Mc3Dev &d = h->d;
-    CXG_CUDA(cudaStreamSynchronize(h->stream));
-    uint8_t cm = 0;
-    CXG_CUDA(cudaMemcpy(&cm, d.curmodel + chain, 1, cudaMemcpyDeviceToHost));
-    Mc3Model m;
-    CXG_CUDA(cudaMemcpy(&m, d.model + chain * 2 + cm, sizeof(m), cudaMemcpyDeviceToHost));
+    if (int rc = mc3_fetch(h, chain)) return rc;
+    const Mc3Model &m = h->state->model;
     if (wvar) *wvar = m.q[0].wvar;
     if (winvar) *winvar = m.q[0].winvar;
     return 0;
