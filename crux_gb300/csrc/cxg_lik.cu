@@ -529,6 +529,7 @@ static WalkShape auto_shape(int precision, unsigned kact, size_t patterns, unsig
     }
     if (jobs > 1) {
         w.tile = 128;
+        w.ring_bytes = 50 * 1024;  // four CTAs an SM: 523 us, with 42 KB 531
         return w;
     }
     if (warps <= 8 * (size_t)kSMs) {

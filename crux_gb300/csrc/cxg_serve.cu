@@ -332,6 +332,7 @@ void plan_request(SrvRequest &rq, int prec) {
     // Results kept on the stack need no HBM copy here (a request's CLs are
     // not kept), and a request with fewer copies is admitted sooner.
     if (P.w.budget == 0) P.w.budget = 24 * 1024;
+    P.w.ring_bytes = 42 * 1024;
     P.ntiles = plan_blocks(P.ppad, P.w.tile);
     const size_t elt = prec == CXG_FP32 ? 4 : 8;
     const unsigned K = P.K;
