@@ -90,6 +90,57 @@ __device__ inline void pmat_one(const PmatArgs &a, unsigned idx, unsigned q) {
     }
 }
 
+// The same by sixteen lanes, lane 4 i + j the entry (i, j) and four masks of
+// row i's messages: the same products and sums in the same order.
+__device__ inline void pmat_one16(const PmatArgs &a, unsigned idx, unsigned l) {
+    const unsigned c = idx / a.kact, k = idx % a.kact;
+    const int m = a.model[k];
+    const double wn = a.wnorm_dev ? *a.wnorm_dev : a.wnorm;
+    const double t = __dmul_rn(__dmul_rn(__dmul_rn(a.edge_len[c], a.cmult[k]),
+                                         a.rmult[k]), wn);
+    const int i = (int)(l >> 2), j = (int)(l & 3u);
+    const double *cube = a.cube + (size_t)m * 64 + l * 4;
+    const double exq = exp(__dmul_rn(a.eig[(size_t)m * 4 + j], t));
+    const unsigned gmask = 0xffffu << (threadIdx.x & 16u);
+    double s = 0.0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+        s = __dadd_rn(s, __dmul_rn(cube[r], __shfl_sync(gmask, exq, r, 4)));
+    const double p = s < 0.0 ? 0.0 : s;
+    const int tb = a.tab[c];
+    unsigned char *dst = a.rec + a.dst[c];
+    const bool lone = (a.kact & 1u) && k + 1 == a.kact;
+    if (tb >= 0) {
+        double P[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) P[q] = __shfl_sync(gmask, p, q, 4);
+        // Masks j, j + 4, j + 8, j + 12.
+        double T[4];
+        T[0] = j & 1 ? P[0] : 0.0;
+        if (j & 2) T[0] = __dadd_rn(T[0], P[1]);
+        T[1] = __dadd_rn(T[0], P[2]);
+        T[2] = __dadd_rn(T[0], P[3]);
+        T[3] = __dadd_rn(T[1], P[3]);
+        if (a.precision == CXG_FP32) {
+            float *o = reinterpret_cast<float *>(dst) +
+                       (lone ? (size_t)k * 64 + i
+                             : (size_t)(k >> 1) * 128 + (i >> 1) * 64 + (i & 1) * 2 + (k & 1u));
+#pragma unroll
+            for (int h = 0; h < 4; ++h) o[(size_t)(j + 4 * h) * 4] = (float)T[h];
+            return;
+        }
+        double *tt = a.ltab + ((size_t)tb * 16 * a.kact + k) * 4 + i;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) tt[(size_t)(j + 4 * h) * a.kact * 4] = T[h];
+    }
+    if (a.precision == CXG_FP32) {
+        float *o = reinterpret_cast<float *>(dst) +
+                   (lone ? (size_t)k * 16 + i : (size_t)(k >> 1) * 32 + i * 2 + (k & 1u));
+        o[j * (lone ? 4 : 8)] = (float)p;
+    } else {
+        reinterpret_cast<double *>(dst)[(size_t)k * 16 + l] = p;
+    }
+}
 
 // ---------------------------------------------------------------------------
 // FP64 eigensystem of Q = R Pi (reversible, 4 states): Q is similar to the

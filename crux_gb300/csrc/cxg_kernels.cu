@@ -1,7 +1,7 @@
 // Device kernels of the pruning likelihood on sm_103a.
 //
 // Layout in HBM: a CL buffer of K active components over ppad patterns is
-// [K][U][ppad] 16-byte units (FP32: U = 1, a float4 of the four states;
+// [K][U][ppad] 16-byte units (FP32: U = 1, components in pairs, see Rows;
 // FP64: U = 2, two double2), so that the threads of a warp, one pattern
 // each, move 512 contiguous bytes per instruction.  Leaves are one uint8
 // state mask per pattern.  Scalers are one FP64 log scale (plain form) or
@@ -11,16 +11,14 @@
 //   pmat_kernel     P(t) = V diag(exp(lambda r t)) V^-1 per (child edge,
 //                   component), FP64, clipped at 0 (CxLik.c:258-292), plus
 //                   the 16-entry message table of every leaf child.
-//   walk_kernel<T>  one CTA per tile of patterns, one thread per pattern,
-//                   walks the whole node-update list (patterns are
-//                   independent through the entire post-order,
-//                   CxLik.c:314-596, so no grid-wide sync is needed).  CLs
-//                   produced and consumed within the walk stay in a
-//                   shared-memory stack (slots assigned by the host), so HBM
-//                   sees the write-through of every parent, the staged leaf
-//                   masks and CLs cached by earlier runs.  Then it
-//                   aggregates the root (CxLik.c:598-632) and reduces the
-//                   weighted site lnLs with a compensated sum.
+//   walk_kernel     one CTA per tile of patterns walks the whole node-update
+//                   list (patterns are independent through the entire
+//                   post-order, CxLik.c:314-596, so no grid-wide sync is
+//                   needed): records and leaf masks come in groups through a
+//                   ring in shared memory, the previous op's result stays in
+//                   registers, every parent is written through to HBM.  Then
+//                   it aggregates the root (CxLik.c:598-632) and adds the
+//                   weighted site lnLs in fixed point.
 //   qdecomp_kernel  FP64 eigensystem of a reversible 4x4 Q by Jacobi
 //                   rotations of the symmetrised matrix (CxLik.c:59-250).
 #include <math.h>
@@ -48,9 +46,17 @@ __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// Blocks of four lanes per (child edge, component).
+// Lanes per (child edge, component): a warp's FP64 instruction takes its SM
+// quarter 64 cycles whatever its lanes do, and sixteen lanes need 39 of them
+// where four need 73.  So sixteen while the warps have the chip's 608 quarters
+// almost to themselves and the edges are few (an evaluation of one path on 64
+// taxa: 3 us less; 250 taxa, two components: 135 -> 131; 300: 152 -> 157; 509
+// taxa, one component: 200 -> 209).
+__host__ __device__ inline unsigned pmat_lanes(const PmatArgs &a) {
+    return a.nchild <= 512 && a.nchild * a.kact <= 1024 ? 16 : 4;
+}
 __host__ __device__ inline unsigned pmat_blocks(const PmatArgs &a) {
-    return (a.nchild * a.kact + 31) / 32;
+    return (a.nchild * a.kact * pmat_lanes(a) + 127) / 128;
 }
 __host__ __device__ inline unsigned image_units(const PmatArgs &a) {
     return a.nrec * a.img_units + a.img_tail;
@@ -91,9 +97,13 @@ __global__ void pmat_kernel(PmatArgs a) {
         copy_image(a, (blockIdx.x - nblk) * blockDim.x + threadIdx.x);
         return;
     }
-    const unsigned idx = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
-    if (idx >= a.nchild * a.kact) return;  // the same for all four lanes
-    pmat_one(a, idx, threadIdx.x & 3u);
+    const unsigned lanes = pmat_lanes(a);
+    const unsigned idx = (blockIdx.x * blockDim.x + threadIdx.x) / lanes;
+    if (idx >= a.nchild * a.kact) return;  // the same for all its lanes
+    if (lanes == 16)
+        pmat_one16(a, idx, threadIdx.x & 15u);
+    else
+        pmat_one(a, idx, threadIdx.x & 3u);
 }
 
 // P matrices of many jobs in one launch: (edge, component) t belongs to
@@ -201,10 +211,9 @@ __device__ void reduce_sites(const PlanArgs &a, const double (&v)[NV],
 }
 
 // ---------------------------------------------------------------------------
-// Plan walker.  T = double: plain form, the reference's scaler (max over
-// child messages, CxLik.c:390-403 and 577-588).  T = float: FP32 form, scale
-// by the power of two that puts the largest parent entry in [0.5, 1); the
-// exponent is an exact integer.
+// Plan walker.  T = double: plain form; T = float: FP32 form.  Both scale by
+// powers of two (rescale), where the reference divides by the largest child
+// message (CxLik.c:390-403 and 577-588).
 // ---------------------------------------------------------------------------
 template <typename T>
 struct Prec;
@@ -231,13 +240,10 @@ __device__ __forceinline__ float pow2f(int n) {  // n in [-126, 127]
     return __int_as_float((n + 127) << 23);
 }
 
-// Shared memory of one CTA: mbarriers [ring]; the stage ring [ring] of
-// `stage` bytes, each an op record (rstride) followed, for a job that
-// streams its leaves, by this tile's mask rows of the op's leaf children
-// (lmax rows of tile bytes); stack slots [nslot][K][U][tile] units; slot
-// scalers [nslot][tile]; and, for a job that stages its leaves, every
-// leaf's mask row [nleaf][tile], loaded once per tile.  A batched launch
-// lays it out for its largest job; every job uses a prefix of each region.
+// Shared memory of an op-lane CTA: mbarriers [ring]; the stage ring [ring] of
+// `stage` bytes, each the op records of a step; stack slots
+// [nslot][K][U][tile] units; slot scalers [nslot][tile]; and every leaf's
+// mask row [nleaf][tile], loaded once per tile.
 struct SmemLayout {
     size_t bars, ring, stage, slots, slot_sc, masks, total;
 };
