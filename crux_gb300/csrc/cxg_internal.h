@@ -181,8 +181,8 @@ static_assert(sizeof(RecHead) == 32, "record header is 32 bytes");
 static_assert(sizeof(RecChild) == 32, "record child is 32 bytes");
 
 // Per-call constants of a plan execution.  CL buffers in HBM are
-// [K][U][ppad] 16-byte units (U = 1 for FP32: states 0-3; U = 2 for FP64:
-// states 0-1, 2-3), so that one thread per pattern moves whole units and a
+// [K][U][ppad] 16-byte units (U = 1 for FP32, components in pairs: see Rows in
+// cxg_kernels.cu; U = 2 for FP64: states 0-1, 2-3), so that one thread per pattern moves whole units and a
 // warp writes 512 contiguous bytes per store.
 struct PlanArgs {
     const unsigned char *rec;      // [nops][rstride] op records
@@ -249,7 +249,7 @@ struct WalkShape {
     int precision = CXG_FP64;
     unsigned kact = 1, tile = kTile, tpp = 1, ppt = 1, lanes = 1, ring = kRing;
     bool wide = false;  // the 96-register build of the walker
-    size_t budget = 0;  // bytes of the CL stack
+    size_t budget = 0;  // bytes of a CTA's ring and CL stack
     size_t ring_bytes = 42 * 1024;
     // Threads of a CTA (of one op lane).
     unsigned threads() const { return tile / ppt * tpp; }

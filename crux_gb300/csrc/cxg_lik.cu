@@ -536,7 +536,7 @@ static WalkShape auto_shape(int precision, unsigned kact, size_t patterns, unsig
         w.tile = warps <= kSMs ? 32 : warps <= 4 * (size_t)kSMs ? 64 : 128;
         // At most two CTAs an SM: a ring and slots of half its shared memory.
         w.ring_bytes = 88 * 1024;
-        w.budget = kact == 1 ? 20 * 1024 : 0;
+        w.budget = kact == 1 ? 110 * 1024 : 0;
         return w;
     }
     w.tile = 128;
@@ -565,6 +565,9 @@ WalkShape choose_shape(int precision, unsigned kact, size_t patterns, unsigned j
             w.tpp = g_tpp;
         if (walker_shape_ok(precision, kact, w.tpp, g_ppt) && g_tile / g_ppt >= 32)
             w.ppt = g_ppt;
+        // The ring in proportion to the CTA: as many warps fit an SM's shared
+        // memory with small CTAs as with large ones.
+        w.ring_bytes = std::max(w.ring_bytes * w.threads() / 128, (size_t)10 * 1024);
     }
     if (lanes_ok && g_lanes == 2 && lanes_shape_ok(precision, kact, w.tpp, w.ppt) &&
         g_tile * 2 <= kLaneThreads) {
@@ -591,15 +594,8 @@ void fit_ring(WalkShape &w, unsigned rstride, unsigned lmax) {
 unsigned stack_slots(const WalkShape &w, unsigned rstride, unsigned lmax, unsigned nleaf) {
     const size_t base = walk_smem_bytes(w, 0, rstride, lmax, nleaf);
     const size_t slot = walk_smem_bytes(w, 1, rstride, lmax, nleaf) - base;
-    size_t cap = 0;
-    if (w.lanes == 1) {
-        // The budget is the stack's; the CTA as a whole stays launchable.
-        cap = w.budget / slot;
-        const size_t most = 200 * 1024;
-        if (base + cap * slot > most) cap = base < most ? (most - base) / slot : 0;
-    } else if (w.budget > base) {
-        cap = (w.budget - base) / slot;
-    }
+    // (The budget is the CTA's: what the ring leaves of it.)
+    const size_t cap = w.budget > base ? (w.budget - base) / slot : 0;
     return cap > kMaxSlots ? kMaxSlots : (unsigned)cap;
 }
 

@@ -140,14 +140,12 @@ struct HostPlan {
     std::vector<std::vector<HostKid>> kids;
 };
 
-// Patterns on the device: leaf masks, pattern weights and the table of the
-// leaves' mask arrays (for jobs that stage their leaves).
+// Patterns on the device: leaf masks and pattern weights.
 // A registered dataset also keeps its host copy (MC3 requests build their
 // chains from it) and a count of the admitted requests that use it.
 struct SrvDataset {
     uint8_t *masks = nullptr;      // [ntaxa][ppad]
     uint32_t *weights = nullptr;   // [npat]
-    const uint8_t **leaves = nullptr;  // [ntaxa] mask array of each taxon
     size_t stride = 0;  // mask row stride (>= the padded pattern count)
     char *mem = nullptr;
     size_t bytes = 0;
@@ -317,8 +315,7 @@ size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 size_t dataset_bytes(unsigned ntaxa, unsigned npat) {
     const size_t ppad = pad_patterns(npat);
-    return al256((size_t)ntaxa * ppad) + al256((size_t)npat * 4) +
-           al256((size_t)ntaxa * sizeof(void *));
+    return al256((size_t)ntaxa * ppad) + al256((size_t)npat * 4);
 }
 
 // Plan a likelihood request on the host (no device work).
@@ -331,8 +328,12 @@ void plan_request(SrvRequest &rq, int prec) {
     P.w = choose_shape(prec, P.K, P.ppad, 2, false);
     // Results kept on the stack need no HBM copy here (a request's CLs are
     // not kept), and a request with fewer copies is admitted sooner.
-    if (P.w.budget == 0) P.w.budget = 24 * 1024;
-    P.w.ring_bytes = 42 * 1024;
+    // A quarter of an SM's shared memory for a CTA of 128 threads: sixteen warps
+    // an SM whatever shape is tuned (on one plan, where slots cost nothing;
+    // a tuned 48 KB for CTAs of one warp served 2,860 of 5,000 requests a
+    // second, this 4,990).
+    P.w.ring_bytes = std::min(P.w.ring_bytes, (size_t)42 * 1024 * P.w.threads() / 128);
+    P.w.budget = (size_t)54 * 1024 * P.w.threads() / 128;
     P.ntiles = plan_blocks(P.ppad, P.w.tile);
     const size_t elt = prec == CXG_FP32 ? 4 : 8;
     const unsigned K = P.K;
@@ -456,7 +457,6 @@ int upload_dataset(unsigned N, unsigned npat, const uint8_t *masks,
     }
     ds.masks = (uint8_t *)ds.mem;
     ds.weights = (uint32_t *)(ds.mem + al256((size_t)N * ppad));
-    ds.leaves = (const uint8_t **)(ds.mem + al256((size_t)N * ppad) + al256((size_t)npat * 4));
     std::vector<uint8_t> hm((size_t)N * ppad, 15);
     for (unsigned t = 0; t < N; ++t) {
         const uint8_t *src = masks + (size_t)t * npat;
@@ -468,10 +468,6 @@ int upload_dataset(unsigned N, unsigned npat, const uint8_t *masks,
     }
     CXG_CUDA(cudaMemcpyAsync(ds.masks, hm.data(), hm.size(), cudaMemcpyHostToDevice, s));
     CXG_CUDA(cudaMemcpyAsync(ds.weights, pfreqs, (size_t)npat * 4,
-                             cudaMemcpyHostToDevice, s));
-    std::vector<const uint8_t *> hl(N);
-    for (unsigned t = 0; t < N; ++t) hl[t] = ds.masks + (size_t)t * ppad;
-    CXG_CUDA(cudaMemcpyAsync(ds.leaves, hl.data(), N * sizeof(void *),
                              cudaMemcpyHostToDevice, s));
     return 0;
 }
@@ -1339,13 +1335,12 @@ extern "C" int cxgServerAddDatasetRaw(cxgServer *S, unsigned long long id, unsig
         if (S->datasets.count(id)) return fail(CXG_EINVAL, "cxgServerAddDatasetRaw: id in use");
     }
     // The dataset keeps masks with row stride pad(nsites) >= pad(npat)
-    // (pad patterns are "any"), weights and the leaf table; the raw rows
-    // and the compaction scratch are freed afterwards.
+    // (pad patterns are "any") and weights; the raw rows and the compaction
+    // scratch are freed afterwards.
     const unsigned N = ntaxa;
     const size_t stride = pad_patterns(nsites);
     auto ds = std::make_unique<SrvDataset>();
-    ds->bytes = al256((size_t)N * stride) + al256((size_t)nsites * 4) +
-                al256((size_t)N * sizeof(void *));
+    ds->bytes = al256((size_t)N * stride) + al256((size_t)nsites * 4);
     ds->ntaxa = N;
     ds->stride = stride;
     cudaStream_t s = S->s_prep;
@@ -1363,8 +1358,6 @@ extern "C" int cxgServerAddDatasetRaw(cxgServer *S, unsigned long long id, unsig
     }
     ds->masks = (uint8_t *)ds->mem;
     ds->weights = (uint32_t *)(ds->mem + al256((size_t)N * stride));
-    ds->leaves = (const uint8_t **)(ds->mem + al256((size_t)N * stride) +
-                                    al256((size_t)nsites * 4));
     uint8_t *d_rows = (uint8_t *)tmp;
     uint8_t *d_tab = (uint8_t *)tmp + al256(in_bytes);       // canon | val
     uint32_t *d_np = (uint32_t *)(d_tab + 512 + 256);
@@ -1372,13 +1365,9 @@ extern "C" int cxgServerAddDatasetRaw(cxgServer *S, unsigned long long id, unsig
     uint8_t tabs[512];
     memcpy(tabs, canon, 256);
     memcpy(tabs + 256, val, 256);
-    std::vector<const uint8_t *> hl(N);
-    for (unsigned t = 0; t < N; ++t) hl[t] = ds->masks + (size_t)t * stride;
     uint32_t np = 0;
     if ((e = cudaMemcpyAsync(d_rows, rows, in_bytes, cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(d_tab, tabs, 512, cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(ds->leaves, hl.data(), N * sizeof(void *),
-                             cudaMemcpyHostToDevice, s)))
+        (e = cudaMemcpyAsync(d_tab, tabs, 512, cudaMemcpyHostToDevice, s)))
         rc = cuda_fail(e, "cxgServerAddDatasetRaw: upload");
     if (rc == 0)
         rc = compact_device(d_rows, N, nsites, nullptr, canon, d_tab, d_tab + 256, any_mask,

@@ -2,7 +2,8 @@
 
 The walker's shape is five numbers, set process-wide by ``cxgTune`` and
 ``cxgTuneLanes`` (include/cxlik_gpu.h) and read when a plan, batch, MC3 run
-or server request is translated:
+or server request is translated (until one is set, the library chooses a
+shape by the size of each plan or batch):
 
 * ``tile``: patterns per CTA (32, 64 or 128);
 * ``tpp``: threads per pattern (1, 2 or 4). The FP32 form splits a

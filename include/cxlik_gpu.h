@@ -142,8 +142,8 @@ void CxLikPt(int n, double *P, double *qEigVecCube, double *qEigVals,
              double v);
 
 /* Replaces CxLikExecute (CxLik.h:284-285; CxLik.c:914-968).  Runs the
- * lik->steps plan on the GPU in FP64 with the reference's per-pattern
- * scaler, then writes siteLnL[cbase .. cbase+mschars) and
+ * lik->steps plan on the GPU in FP64 with a per-pattern scaler (by powers of
+ * two; the site lnLs are the reference's), then writes siteLnL[cbase .. cbase+mschars) and
  * stripeLnL[0 .. nstripes).  Failures leave a message in cxgLastError(). */
 void CxLikExecute(CxtLik *lik);
 
@@ -162,7 +162,7 @@ enum {
 
 /* Precision of a plan execution. */
 enum {
-    CXG_FP64 = 0,      /* plain: FP64 CLVs, the reference's scaler */
+    CXG_FP64 = 0,      /* plain: FP64 CLVs, per-pattern log scalers */
     CXG_FP32 = 1       /* FP32 CLVs, per-pattern power-of-two exponents */
 };
 
@@ -196,8 +196,8 @@ int cxgLikReset(void);
 int cxgLikSetPatternWeights(const unsigned *freqs, unsigned n);
 int cxgLikForgetPatternWeights(const unsigned *freqs, unsigned n);
 
-/* Execute lik's plan at the given precision; write the compensated FP64
- * sum of site lnLs to *lnL (one 8-byte device-to-host copy).  If siteLnL is
+/* Execute lik's plan at the given precision; write the sum of the site lnLs
+ * (taken in 128-bit fixed point) to *lnL (one 48-byte device-to-host copy).  If siteLnL is
  * non-NULL also fill it (mschars doubles, pad patterns included). */
 int cxgLikExecuteLnL(CxtLik *lik, int precision, double *lnL,
                      double *siteLnL);
@@ -500,7 +500,8 @@ int cxgCompact(const uint8_t *rows, unsigned ntaxa, unsigned nsites,
  * the FP32 form with one thread per pattern and <= 5 components can give a
  * thread two patterns; tile >= 64) and the shared-memory budget of its CL
  * stack (bytes, <= 200 KiB).  Every shape gives the same bits.  Chosen by
- * the autotuner (crux_gb300.tune). */
+ * the autotuner (crux_gb300.tune).  Until the first call the library takes
+ * a shape by the size of each plan or batch. */
 int cxgTune(unsigned tile, unsigned threads_per_pattern,
             unsigned patterns_per_thread, size_t smem_budget);
 int cxgTuneGet(unsigned *tile, unsigned *threads_per_pattern,
@@ -544,7 +545,10 @@ int cxgDebugCanarySelfTest(int *detected);
  *   - each CxtLikCL in lik->steps and lik->rootCLC holds DEVICE pointers:
  *     internal CL: cLMat -> kact*4*ceil128(mschars) elements of the
  *     precision (double or float) laid out [kact][U][ppad] in 16-byte
- *     units, lnScale -> ppad scalers (double for CXG_FP64, int32 for
+ *     units (FP64: U = 2, states 0-1 and 2-3 of a component; FP32: U = 1,
+ *     components in pairs, units 2m and 2m+1 holding states 0-1 and 2-3 of
+ *     components 2m and 2m+1 interleaved, the last of an odd number alone,
+ *     states 0-3), lnScale -> ppad scalers (double for CXG_FP64, int32 for
  *     CXG_FP32; size the buffer for 8 bytes per pattern); leaf CL: cLMat
  *     -> ppad uint8 state masks (pad patterns set to 15), lnScale unused;
  *     every cLMat 16-byte aligned, as cudaMalloc returns;
