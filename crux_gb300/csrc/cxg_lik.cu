@@ -512,8 +512,8 @@ constexpr unsigned kSMs = 152;
 // 1,535 with four), and four serve a walk of few patterns (27 us against 57
 // on 522).
 //
-// No shape takes stack slots: a result is stored to HBM anyway, and reading
-// it back through L2 costs less than storing it twice.
+// Otherwise no shape takes stack slots: a result is stored to HBM anyway, and
+// reading it back through L2 costs less than storing it twice.
 static WalkShape auto_shape(int precision, unsigned kact, size_t patterns, unsigned jobs) {
     WalkShape w;
     w.precision = precision;
