@@ -1387,6 +1387,8 @@ __device__ bool walk_tile_lanes(const PlanArgs &a, unsigned tile_idx, const Smem
                         acc[0].mul(x[0]);
                         lns[0] += l[0];
                     }
+                    // (As in walk_op: a long product stays inside the range.)
+                    if (ci >= 1 && ci + 1 < nchild) rescale<KT, 1>(acc[0], lns[0], true);
                 }
             }
             ydata = hd->data;
@@ -1412,7 +1414,7 @@ __device__ bool walk_tile_lanes(const PlanArgs &a, unsigned tile_idx, const Smem
         }
         // (An empty lane of a step, with no children, stores nothing.)
         if (nchild != 0) {
-            rescale<KT, 1>(acc[0], lns[0], nchild > 2);
+            rescale<KT, 1>(acc[0], lns[0], false);
             if (yhbm) {
                 acc[0].store_global(reinterpret_cast<uint64_t>(static_cast<float4 *>(ydata) + p),
                                     w.pitch, 0u);
