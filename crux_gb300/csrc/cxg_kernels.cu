@@ -1265,12 +1265,11 @@ __device__ bool walk_tile(const PlanArgs &a, unsigned tile_idx, const LeanLayout
         if (g == 0 && p < a.npat) {
             v[h] = (sizeof(T) == 8 ? log(L) + (double)lns[h] : site_log(L, (int)lns[h])) *
                    (double)a.freqs[p];
-            if (isnan(v[h])) v[h] = -INFINITY;
+            // (NaN, or +inf from rows that left the range: no likelihood.)
+            if (!(v[h] < INFINITY)) v[h] = -INFINITY;
             if (a.site) a.site[p] = v[h];
-            if (isinf(v[h])) {
-                ninf[h] = (v[h] < 0.0);
-                v[h] = 0.0;
-            }
+            ninf[h] = isinf(v[h]);
+            if (ninf[h]) v[h] = 0.0;
         }
     }
     reduce_sites<N>(a, v, ninf);
@@ -1446,12 +1445,10 @@ __device__ bool walk_tile_lanes(const PlanArgs &a, unsigned tile_idx, const Smem
     bool ninf[1] = {false};
     if (lane == 0 && p < a.npat) {
         v[0] = site_log(Lsum, lns[0]) * (double)a.freqs[p];
-        if (isnan(v[0])) v[0] = -INFINITY;
+        if (!(v[0] < INFINITY)) v[0] = -INFINITY;  // as in walk_tile
         if (a.site) a.site[p] = v[0];
-        if (isinf(v[0])) {
-            ninf[0] = (v[0] < 0.0);
-            v[0] = 0.0;
-        }
+        ninf[0] = isinf(v[0]);
+        if (ninf[0]) v[0] = 0.0;
     }
     reduce_sites<1>(a, v, ninf);
     return true;
