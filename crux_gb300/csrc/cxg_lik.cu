@@ -431,8 +431,6 @@ struct Plan {
     std::vector<int32_t> model_of;
 };
 
-// Launch shape of the plan walker: patterns per CTA, threads per pattern
-// and the shared-memory budget of the CL stack (set by cxgTune).
 // Device copy of lik's pattern weights, one per (host pointer, length),
 // uploaded again whenever the host values differ from the kept copy.
 static int pattern_weights(State &S, const CxtLik *lik, const void **out) {
@@ -478,12 +476,16 @@ static void pack_values(const CxtLik *lik, const Plan &P, char *h) {
     }
 }
 
+// Launch shape of the plan walker set by cxgTune: patterns per CTA, threads
+// per pattern, patterns per thread, bytes of ring and CL stack.  While none is
+// set (g_tuned false) the shape follows the size of the work, and these are
+// what plans with op lanes (cxgTuneLanes) take.
 static unsigned g_tile = kTile;
 static unsigned g_tpp = 1;
 static unsigned g_ppt = 1;
 static unsigned g_lanes = 1;
 static size_t g_smem_budget = 24 * 1024;
-static bool g_tuned = false;  // cxgTune was called: its shape is used as it is
+static bool g_tuned = false;
 
 // SMs of the GPU these kernels are built for.
 constexpr unsigned kSMs = 152;
@@ -1337,6 +1339,12 @@ int cxgLikReset(void) {
 }
 
 int cxgTune(unsigned tile, unsigned tpp, unsigned ppt, size_t smem_budget) {
+    const bool set = tile != 0 || tpp != 0 || ppt != 0 || smem_budget != 0;
+    if (!set) {  // back to shapes by size
+        tile = kTile;
+        tpp = ppt = 1;
+        smem_budget = 24 * 1024;
+    }
     if (tile != 32 && tile != 64 && tile != 128)
         return fail(CXG_EINVAL, "cxgTune: tile must be 32, 64 or 128");
     if (tpp != 1 && tpp != 2 && tpp != 4)
@@ -1356,7 +1364,7 @@ int cxgTune(unsigned tile, unsigned tpp, unsigned ppt, size_t smem_budget) {
     g_tpp = tpp;
     g_ppt = ppt;
     g_smem_budget = smem_budget;
-    g_tuned = true;
+    g_tuned = set;
     return 0;
 }
 
@@ -1375,10 +1383,10 @@ int cxgTuneLanesGet(unsigned *lanes) {
 }
 
 int cxgTuneGet(unsigned *tile, unsigned *tpp, unsigned *ppt, size_t *smem_budget) {
-    if (tile) *tile = g_tile;
-    if (tpp) *tpp = g_tpp;
-    if (ppt) *ppt = g_ppt;
-    if (smem_budget) *smem_budget = g_smem_budget;
+    if (tile) *tile = g_tuned ? g_tile : 0;
+    if (tpp) *tpp = g_tuned ? g_tpp : 0;
+    if (ppt) *ppt = g_tuned ? g_ppt : 0;
+    if (smem_budget) *smem_budget = g_tuned ? g_smem_budget : 0;
     return 0;
 }
 

@@ -2,8 +2,7 @@
 
 The walker's shape is five numbers, set process-wide by ``cxgTune`` and
 ``cxgTuneLanes`` (include/cxlik_gpu.h) and read when a plan, batch, MC3 run
-or server request is translated (until one is set, the library chooses a
-shape by the size of each plan or batch):
+or server request is translated:
 
 * ``tile``: patterns per CTA (32, 64 or 128);
 * ``tpp``: threads per pattern (1, 2 or 4). The FP32 form splits a
@@ -19,10 +18,15 @@ shape by the size of each plan or batch):
   leaves runs two independent node updates per step on two thread groups
   over the same patterns. Batches, MC3 and the server keep one lane.
 
+Until one is set, and again after ``set_shape(lib, *AUTO)``, the library
+chooses a shape by the size of each plan or batch (also from shapes that
+``cxgTune`` does not offer, so it is a candidate of its own).
+
 Every shape gives bit-identical results, so the choice is speed alone.
 ``tune_plan`` and ``tune_batch`` time each candidate on the caller's own
 workload with CUDA events (the walker launch, after warm-up), set the
-fastest with ``cxgTune`` and return the whole table.
+fastest with ``cxgTune`` (or leave the choice to the library) and return the
+whole table.
 """
 import ctypes
 import itertools
@@ -33,10 +37,13 @@ PPTS = (1, 2)
 BUDGETS = (0, 12 << 10, 24 << 10, 48 << 10, 96 << 10)
 LANES = (1, 2)
 MAX_THREADS = 256
+# No shape set: the library chooses one.
+AUTO = (0, 0, 0, 0, 1)
 
 
 def get(lib):
-    """The current shape as (tile, tpp, ppt, budget, lanes)."""
+    """The current shape as (tile, tpp, ppt, budget, lanes), the first four 0
+    while the library chooses it."""
     t, g, p = ctypes.c_uint(), ctypes.c_uint(), ctypes.c_uint()
     b = ctypes.c_size_t()
     lanes = ctypes.c_uint()
@@ -55,8 +62,7 @@ def set_shape(lib, tile, tpp, ppt, budget, lanes=1):
 
 def shape_ok(precision, kact, tile, tpp, ppt=1, lanes=1):
     """Whether the library has a walker for this shape (the C rules of
-    walker_shape_ok, lanes_shape_ok and tuned_ppt,
-    crux_gb300/csrc/cxg_internal.h)."""
+    walker_shape_ok and lanes_shape_ok, crux_gb300/csrc/cxg_internal.h)."""
     if tile * tpp * lanes > MAX_THREADS or kact < 1:
         return False
     if lanes == 2:
@@ -78,12 +84,12 @@ def shape_ok(precision, kact, tile, tpp, ppt=1, lanes=1):
 
 def candidates(precision, kact, tiles=TILES, tpps=TPPS, budgets=BUDGETS,
                ppts=PPTS, lanes=LANES):
-    """(tile, tpp, ppt, budget, lanes) shapes the library has a walker for.
-    Lanes apply to single plans only: pass lanes=(1,) for batches, MC3 and
-    the server."""
-    return [(t, g, p, b, n) for t, g, p, b, n in
-            itertools.product(tiles, tpps, ppts, budgets, lanes)
-            if shape_ok(precision, kact, t, g, p, n)]
+    """(tile, tpp, ppt, budget, lanes) shapes the library has a walker for,
+    after AUTO.  Lanes apply to single plans only: pass lanes=(1,) for
+    batches, MC3 and the server."""
+    return [AUTO] + [(t, g, p, b, n) for t, g, p, b, n in
+                     itertools.product(tiles, tpps, ppts, budgets, lanes)
+                     if shape_ok(precision, kact, t, g, p, n)]
 
 
 def active_components(lik):

@@ -500,8 +500,10 @@ int cxgCompact(const uint8_t *rows, unsigned ntaxa, unsigned nsites,
  * the FP32 form with one thread per pattern and <= 5 components can give a
  * thread two patterns; tile >= 64) and the shared-memory budget of its CL
  * stack (bytes, <= 200 KiB).  Every shape gives the same bits.  Chosen by
- * the autotuner (crux_gb300.tune).  Until the first call the library takes
- * a shape by the size of each plan or batch. */
+ * the autotuner (crux_gb300.tune).  Until a shape is set, and again after
+ * cxgTune(0, 0, 0, 0), the library takes a shape by the size of each plan or
+ * batch; cxgTuneGet then reports zeros, so what it reports always restores
+ * the state. */
 int cxgTune(unsigned tile, unsigned threads_per_pattern,
             unsigned patterns_per_thread, size_t smem_budget);
 int cxgTuneGet(unsigned *tile, unsigned *threads_per_pattern,

@@ -1,0 +1,81 @@
+"""No shape set is a state of its own: what tune.get reports restores it, the
+tuner tries it, and a sweep that sets nothing leaves it.  (The shape calls need
+no GPU; the choice itself is looked at on one.)"""
+import pytest
+
+from crux_gb300 import _native, synth, tune
+
+AUTO = (0, 0, 0, 0, 1)
+
+
+@pytest.fixture
+def lib():
+    lib = _native.load()
+    saved = tune.get(lib)
+    tune.set_shape(lib, *AUTO)
+    yield lib
+    tune.set_shape(lib, *saved)
+
+
+def test_get_and_set_restore_the_state(lib):
+    assert tune.get(lib) == AUTO
+    tune.set_shape(lib, 128, 1, 2, 48 << 10, 2)
+    assert tune.get(lib) == (128, 1, 2, 48 << 10, 2)
+    tune.set_shape(lib, *AUTO)
+    assert tune.get(lib) == AUTO
+
+
+@pytest.mark.parametrize("shape", [(0, 1, 1, 0), (0, 0, 0, 1), (64, 0, 1, 0), (64, 1, 0, 0),
+                                   (0, 0, 1, 0), (96, 1, 1, 0)])
+def test_part_of_a_shape_is_refused(lib, shape):
+    for state in (AUTO, (32, 2, 1, 0, 1)):
+        tune.set_shape(lib, *state)
+        assert lib.cxgTune(*shape) == -1
+        assert tune.get(lib) == state
+
+
+def test_sweep_restores_and_keeps_the_fastest(lib):
+    def fails():
+        raise RuntimeError("does not fit")
+
+    with pytest.raises(RuntimeError):
+        tune._sweep(lib, [(64, 1, 1, 0, 1)], fails)
+    assert tune.get(lib) == AUTO
+    ms = {AUTO[:4]: 1.0, (64, 1, 1, 0): 2.0, (32, 1, 1, 0): 3.0}
+    shapes = [AUTO, (64, 1, 1, 0, 1), (32, 1, 1, 0, 1)]
+    for fastest in shapes:
+        best = tune._sweep(lib, shapes, lambda: ms[tune.get(lib)[:4]] *
+                           (0.1 if tune.get(lib) == fastest else 1.0))["best"]
+        assert tune.get(lib) == fastest
+        assert (best["tile"], best["budget"]) == (fastest[0], fastest[3])
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_the_choice_is_a_candidate(precision):
+    for kact in (1, 4, 5, 8):
+        assert tune.candidates(precision, kact)[0] == AUTO
+        assert tune.candidates(precision, kact, budgets=(0,), lanes=(1,)).count(AUTO) == 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_plans_take_the_choice_again(gpu, lib, precision):
+    from crux_gb300.plan import Plan
+    case = synth.Case(12, 3000, 0.1, 6)
+    lik = case.lik(lib=gpu, precision=precision)
+    lik.prepare_plan()
+
+    def shape():
+        plan = Plan(lik, precision)
+        try:
+            return plan.shape(), plan.run()
+        finally:
+            plan.close()
+
+    chosen, v = shape()
+    for s in (128, 1, 1, 48 << 10, 1), (64, 1, 1, 24 << 10, 1):
+        tune.set_shape(gpu, *s)
+        tuned, w = shape()
+        assert tuned["tile"] == s[0] and w == v
+        tune.set_shape(gpu, *AUTO)
+        assert shape() == (chosen, v)
