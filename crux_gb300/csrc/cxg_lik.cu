@@ -516,17 +516,21 @@ constexpr unsigned kSMs = 152;
 //
 // Otherwise no shape takes stack slots: a result is stored to HBM anyway, and
 // reading it back through L2 costs less than storing it twice.
+static unsigned fp64_split(unsigned kact, size_t patterns, unsigned tile) {
+    const size_t warps = (patterns + 31) / 32;
+    const bool few = warps * 4 <= (size_t)kSMs * 16;
+    if (few && walker_shape_ok(CXG_FP64, kact, 4) && tile * 4 <= kTuneThreads) return 4;
+    return walker_shape_ok(CXG_FP64, kact, 2) && tile * 2 <= kTuneThreads ? 2 : 1;
+}
+
 static WalkShape auto_shape(int precision, unsigned kact, size_t patterns, unsigned jobs) {
     WalkShape w;
     w.precision = precision;
     w.kact = kact;
     const size_t warps = (patterns + 31) / 32;
     if (precision == CXG_FP64) {
-        const bool few = warps * 4 <= (size_t)kSMs * 16;
-        w.tile = 32;
-        if (few && walker_shape_ok(precision, kact, 4)) w.tpp = 4;
-        else if (walker_shape_ok(precision, kact, 2)) w.tpp = 2;
-        else w.tile = 64;
+        w.tpp = fp64_split(kact, patterns, 32);
+        w.tile = w.tpp > 1 ? 32 : 64;
         return w;
     }
     if (jobs > 1) {
@@ -562,8 +566,11 @@ WalkShape choose_shape(int precision, unsigned kact, size_t patterns, unsigned j
         w.kact = kact;
         w.tile = g_tile;
         w.budget = g_smem_budget;
-        if (precision == CXG_FP32 && walker_shape_ok(precision, kact, g_tpp) &&
-            g_tile * g_tpp <= kTuneThreads)
+        // (Threads a pattern are tuned for the FP32 form; the FP64 form's follow
+        // the size, so that tuning one does not slow the other.)
+        if (precision == CXG_FP64)
+            w.tpp = fp64_split(kact, patterns, g_tile);
+        else if (walker_shape_ok(precision, kact, g_tpp) && g_tile * g_tpp <= kTuneThreads)
             w.tpp = g_tpp;
         if (walker_shape_ok(precision, kact, w.tpp, g_ppt) && g_tile / g_ppt >= 32)
             w.ppt = g_ppt;

@@ -7,7 +7,7 @@ or server request is translated:
 * ``tile``: patterns per CTA (32, 64 or 128);
 * ``tpp``: threads per pattern (1, 2 or 4). The FP32 form splits a
   pattern's components over that many consecutive threads when the count
-  divides them;
+  divides them. (The FP64 form's follow the size of the work.)
 * ``ppt``: patterns per thread (1 or 2). The FP32 form with one thread per
   pattern and at most five components can give each thread two patterns,
   half a tile apart, for twice the independent arithmetic per thread;

@@ -496,7 +496,8 @@ int cxgCompact(const uint8_t *rows, unsigned ntaxa, unsigned nsites,
 /* Launch shape of the plan walker for plans translated from now on:
  * patterns per CTA (32, 64 or 128), threads per pattern (1, 2 or 4: the
  * FP32 form splits a pattern's components over that many threads when the
- * count divides them; tile x threads <= 256), patterns per thread (1 or 2:
+ * count divides them; tile x threads <= 256; the FP64 form's follow the size
+ * of the work), patterns per thread (1 or 2:
  * the FP32 form with one thread per pattern and <= 5 components can give a
  * thread two patterns; tile >= 64) and the shared-memory budget of its CL
  * stack (bytes, <= 200 KiB).  Every shape gives the same bits.  Chosen by

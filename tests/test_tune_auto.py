@@ -79,3 +79,37 @@ def test_plans_take_the_choice_again(gpu, lib, precision):
         assert tuned["tile"] == s[0] and w == v
         tune.set_shape(gpu, *AUTO)
         assert shape() == (chosen, v)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ncat, sites, split", [(4, 500, 4), (4, 60000, 2), (2, 500, 2), (3, 500, 1),
+                                                (1, 500, 1)])
+def test_tuning_leaves_the_fp64_form_its_threads(gpu, lib, ncat, sites, split):
+    """Under a shape tuned for the FP32 form the FP64 form keeps as many threads
+    a pattern as the library would take, where the tile leaves room for them."""
+    import numpy as np
+    from crux_gb300 import Alignment, Lik, TaxaMap, Tree
+    from crux_gb300.plan import Plan
+    rng = np.random.default_rng(sites)
+    rows = np.frombuffer(b"ACGT", dtype=np.uint8)[rng.integers(4, size=(5, sites))]
+    aln = Alignment(taxaMap=TaxaMap(["T%d" % i for i in range(5)]), rows=rows)
+    tree = Tree("(T0:.1,T1:.2,(T2:.1,(T3:.1,T4:.2):.1):.1);")
+    tree.deroot()
+    tree.canonize(aln.taxaMap)
+    lik = Lik(tree, aln, ncat=ncat, lib=gpu, precision="fp64")
+    if ncat > 1:
+        lik.setAlpha(0, 0.5)
+    lik.prepare_plan()
+
+    def run():
+        plan = Plan(lik, "fp64")
+        try:
+            return plan.shape()["threads_per_pattern"], plan.run()
+        finally:
+            plan.close()
+
+    own, v = run()
+    assert own == split
+    for tile in (32, 64, 128):
+        tune.set_shape(gpu, tile, 1, 1, 24 << 10)
+        assert run() == (min(split, 256 // tile) if split > 1 else 1, v)
