@@ -581,6 +581,7 @@ WalkShape choose_shape(int precision, unsigned kact, size_t patterns, unsigned j
     if (lanes_ok && g_lanes == 2 && lanes_shape_ok(precision, kact, w.tpp, w.ppt) &&
         g_tile * 2 <= kLaneThreads) {
         w.lanes = 2;
+        w.wide = false;
         w.tile = g_tile;
         w.budget = g_smem_budget;
     }
@@ -745,9 +746,8 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
     // Leaves: staged once per tile (each distinct leaf one row, named by
     // kids[c].idx) when they fit kLeafStageBytes, else each op's mask
     // arrays (kids[c].data) travel with its record (lmax rows per stage).
-    WalkShape w = choose_shape(prec, kact, patterns ? patterns : ppad, njobs,
-                               allow_lanes && ops.size() >= 2);
-    const unsigned tile = w.tile;
+    const size_t work = patterns ? patterns : ppad;
+    WalkShape w = choose_shape(prec, kact, work, njobs, allow_lanes && ops.size() >= 2);
     std::vector<const uint8_t *> leaf_ptrs;
     unsigned lmax = 0;
     {
@@ -770,7 +770,9 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
     }
     const unsigned nleaf = (unsigned)leaf_ptrs.size();
     // Op lanes stage the leaves, and run where they fit.
-    if ((size_t)nleaf * tile > kLeafStageBytes) w.lanes = 1;
+    if (w.lanes == 2 && (size_t)nleaf * w.tile > kLeafStageBytes)
+        w = choose_shape(prec, kact, work, njobs, false);
+    const unsigned tile = w.tile;
     const bool stage_leaves = w.lanes == 2;
     const unsigned s_lmax = stage_leaves ? 0 : lmax;
     const unsigned s_nleaf = stage_leaves ? nleaf : 0;

@@ -113,3 +113,29 @@ def test_tuning_leaves_the_fp64_form_its_threads(gpu, lib, ncat, sites, split):
     for tile in (32, 64, 128):
         tune.set_shape(gpu, tile, 1, 1, 24 << 10)
         assert run() == (min(split, 256 // tile) if split > 1 else 1, v)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sites", [300, 60000])
+def test_lanes_that_do_not_fit_change_nothing(gpu, lib, sites):
+    """300 taxa: more leaf masks than a tile of the op lanes stages, so the plan
+    runs one lane, in the shape and with the bits it has without lanes."""
+    import numpy as np
+    from crux_gb300 import Alignment, Lik, TaxaMap, Tree
+    from crux_gb300.plan import Plan
+    rng = np.random.default_rng(sites)
+    rows = np.frombuffer(b"ACGT", dtype=np.uint8)[rng.integers(4, size=(300, sites))]
+    aln = Alignment(taxaMap=TaxaMap(["T%d" % i for i in range(300)]), rows=rows)
+    tree = Tree(synth.yule_newick(300, 0.1, rng))
+    tree.deroot()
+    tree.canonize(aln.taxaMap)
+    lik = Lik(tree, aln, ncat=1, lib=gpu, precision="fp32")
+    lik.prepare_plan()
+    out = []
+    for lanes in (1, 2):
+        tune.set_shape(gpu, 0, 0, 0, 0, lanes)
+        plan = Plan(lik, "fp32")
+        out.append((plan.shape(), plan.run()))
+        plan.close()
+    assert out[0][0]["lanes"] == 1
+    assert out[1] == out[0]
