@@ -195,14 +195,21 @@ __device__ inline void qdecomp_warp(const double *rtri, const double *pi, double
     }
     const double slo = i < j ? sqi : sqj, shi = i < j ? sqj : sqi;
     double v = in_s ? (i == j ? diag : rt * slo * shi) : (i == j ? 1.0 : 0.0);
+    // The angles take squares of entries: S is brought to [1, 2) by a power of
+    // two, so that the units of the rates do not matter, and the eigenvalues
+    // back from it at the end.
+    const unsigned top = __reduce_max_sync(
+        kAll, in_s ? (unsigned)__double2hiint(v) & 0x7ff00000u : 0u) >> 20;
+    const int up = max(2046 - (int)top, 1);
+    if (in_s) v *= __hiloint2double(up << 20, 0);
     int conv = 0;
     for (int sweep = 0; sweep < 64; ++sweep) {
-        // Off-diagonal entries below 2^-62 of the largest on the diagonal
+        // Off-diagonal entries below 2^-67 of the largest on the diagonal
         // (by their exponents; a NaN never converges).
         const unsigned e = (unsigned)__double2hiint(v) & 0x7ff00000u;
         const unsigned off = __reduce_max_sync(kAll, in_s && i != j ? e : 0u);
         const unsigned dg = __reduce_max_sync(kAll, in_s && i == j ? e : 0u);
-        if (off == 0u || (off != 0x7ff00000u && off + (62u << 20) <= dg)) {
+        if (off == 0u || (off != 0x7ff00000u && off + (68u << 20) <= dg)) {
             conv = 1;
             break;
         }
@@ -250,7 +257,7 @@ __device__ inline void qdecomp_warp(const double *rtri, const double *pi, double
         const double ujk = __shfl_sync(kAll, v, 16 + j * 4 + k);
         out[5 + i * 16 + j * 4 + k] = (uik * isq) * (ujk * sqj);
     }
-    if (in_s && i == j) out[69 + i] = v;
+    if (in_s && i == j) out[69 + i] = scalbn(v, 1023 - up);
     if (lane == 0) out[73] = conv ? 0.0 : 2.0;
 }
 
