@@ -483,6 +483,11 @@ __device__ __forceinline__ uint64_t addr_at(uint64_t base, uint32_t a, uint32_t 
     asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(base));
     return r;
 }
+// Unit u of a CL row at `at`; its units are `pitch` patterns apart (counted in
+// patterns: the bytes pass 32 bits from 2^28 patterns on).
+__device__ __forceinline__ uint64_t unit_at(uint64_t at, uint32_t pitch, uint32_t u) {
+    return addr_at(at, pitch, u * 16u);
+}
 template <typename X>
 __device__ __forceinline__ X ld_l2(uint64_t at) {
     return __ldcg(reinterpret_cast<const X *>(at));
@@ -561,7 +566,7 @@ struct Rows<float, KT, G> {
     }
     __device__ __forceinline__ void load_l2(uint64_t at, uint32_t pitch, unsigned k0) {
 #pragma unroll
-        for (int u = 0; u < 2 * NP; ++u) set(u, ld_l2<pairs>(addr_at(at, pitch, k0 + u)));
+        for (int u = 0; u < 2 * NP; ++u) set(u, ld_l2<pairs>(unit_at(at, pitch, k0 + u)));
 #pragma unroll
         for (int i = 0; i < NS; ++i) {
             const unsigned k = k0 + 2 * NP + i;
@@ -569,25 +574,25 @@ struct Rows<float, KT, G> {
 #pragma unroll
                 for (int s = 0; s < 4; ++s)
                     sg[i][s] = __ldcg(reinterpret_cast<const float *>(
-                        addr_at(at, pitch, (k & ~1u) + (s >> 1)) + part(k, s)));
+                        unit_at(at, pitch, (k & ~1u) + (s >> 1)) + part(k, s)));
             } else {
-                unpack(ld_l2<float4>(addr_at(at, pitch, k)), sg[i]);
+                unpack(ld_l2<float4>(unit_at(at, pitch, k)), sg[i]);
             }
         }
     }
     __device__ __forceinline__ void store_global(uint64_t at, uint32_t pitch,
                                                  unsigned k0) const {
 #pragma unroll
-        for (int u = 0; u < 2 * NP; ++u) st_global(addr_at(at, pitch, k0 + u), unit(u));
+        for (int u = 0; u < 2 * NP; ++u) st_global(unit_at(at, pitch, k0 + u), unit(u));
 #pragma unroll
         for (int i = 0; i < NS; ++i) {
             const unsigned k = k0 + 2 * NP + i;
             if (split) {
 #pragma unroll
                 for (int s = 0; s < 4; ++s)
-                    st_global(addr_at(at, pitch, (k & ~1u) + (s >> 1)) + part(k, s), sg[i][s]);
+                    st_global(unit_at(at, pitch, (k & ~1u) + (s >> 1)) + part(k, s), sg[i][s]);
             } else {
-                st_global(addr_at(at, pitch, k),
+                st_global(unit_at(at, pitch, k),
                           make_float4(sg[i][0], sg[i][1], sg[i][2], sg[i][3]));
             }
         }
@@ -686,12 +691,12 @@ struct Rows<double, KT, G> {
     __device__ __forceinline__ void load_l2(uint64_t at, uint32_t pitch, unsigned k0) {
 #pragma unroll
         for (int u = 0; u < 2 * KT; ++u)
-            set(u, ld_l2<double2>(addr_at(at, pitch, 2 * k0 + u)));
+            set(u, ld_l2<double2>(unit_at(at, pitch, 2 * k0 + u)));
     }
     __device__ __forceinline__ void store_global(uint64_t at, uint32_t pitch,
                                                  unsigned k0) const {
 #pragma unroll
-        for (int u = 0; u < 2 * KT; ++u) st_global(addr_at(at, pitch, 2 * k0 + u), unit(u));
+        for (int u = 0; u < 2 * KT; ++u) st_global(unit_at(at, pitch, 2 * k0 + u), unit(u));
     }
     __device__ __forceinline__ void load_smem(const double2 *p, unsigned stride, unsigned k0) {
 #pragma unroll
@@ -936,7 +941,7 @@ struct TileView {
     V *slots;
     S *slot_sc;
     const double *ltab;  // FP64: leaf-message tables
-    uint32_t pitch;      // bytes between a CL's units
+    uint32_t pitch;      // patterns between a CL's units
     unsigned tile, pl, p, k0;
 };
 
@@ -1090,7 +1095,7 @@ __device__ bool walk_tile(const PlanArgs &a, unsigned tile_idx, const LeanLayout
     w.slots = reinterpret_cast<V *>(smem + Lay.slots);
     w.slot_sc = reinterpret_cast<S *>(smem + Lay.slot_sc);
     w.ltab = a.ltab;
-    w.pitch = a.ppad * 16u;
+    w.pitch = a.ppad;
     w.tile = tile;
     w.pl = tid / G;
     w.p = p0 + w.pl;
@@ -1333,7 +1338,7 @@ __device__ bool walk_tile_lanes(const PlanArgs &a, unsigned tile_idx, const Smem
     typedef Rows<float, KT, 1> R;
     R acc[1];
     int lns[1] = {0};
-    const TileView<float> w{slots, slot_sc, nullptr, a.ppad * 16u, tile, pl, p, 0u};
+    const TileView<float> w{slots, slot_sc, nullptr, a.ppad, tile, pl, p, 0u};
     const uint32_t spin = g_spin_limit;
     for (unsigned o = 0, stage = 0; o < nsteps;
          ++o, stage = (stage + 1 == R_) ? 0u : stage + 1) {
