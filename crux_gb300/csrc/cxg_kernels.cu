@@ -869,26 +869,39 @@ __device__ __forceinline__ X group_max(X x) {
 // Rescale a pattern's rows by an exact power of two when their largest
 // entry has fallen low.
 //
-// FP32: when the largest entry of any pattern of the warp has left
-// [2^-16, 2^44), every pattern of it goes to [2^19, 2^20), the exponent added
-// to the integer scaler.  So a warp's patterns fall together and it
-// rescales about once in ten ops; pattern by pattern, at below 2^-16 to
-// [0.5, 1), nearly every op had some lane in the branch.  P has entries of
-// at most 1, so a product of two rows stays far inside the FP32 range, the
-// scaling is exact, and a rescale sooner or later changes no mantissa: the
-// root takes rows and exponent together.  Called by whole warps.
+// FP32: when the largest entry of any of eight consecutive patterns has left
+// [2^-16, 2^44), all eight go to [2^19, 2^20), the exponent added to the
+// integer scaler.  So patterns of a warp fall together, where pattern by
+// pattern, at below 2^-16 to [0.5, 1), nearly every op had some lane in the
+// branch.  Eight are what a warp holds with four threads a pattern: the
+// groups are the same in every shape, and with them the bits also of rows with
+// subnormal entries.  (Groups of a warp's 32, 16 or 8 gave other bits there
+// and rescaled less: 128 taxa x 81,664 patterns, eight proposals 1,837 us and
+// 1,846 now.)  P has entries of at most 1, so a product of two rows stays far
+// inside the FP32 range, and the scaling of normal entries is exact.  Called
+// by whole warps.
 template <int KT, int G>
 __device__ __forceinline__ void rescale(Rows<float, KT, G> &r, int &lns, bool always) {
     constexpr uint32_t kLow = (127 - 16) << 23, kHigh = (127 + 44) << 23;
     const float mx = group_max<G>(r.top());
-    if (!__any_sync(0xffffffffu, (__float_as_uint(mx) - kLow >= kHigh - kLow) | always)) return;
-    if (!(mx > 0.0f && mx <= 3.0e38f)) return;
-    int e;
-    frexpf(mx, &e);
-    const int n = 20 - e;
-    r.scale(pow2f(n < 127 ? n : 127));
-    if (n > 127) r.scale(pow2f(n - 127));
-    lns -= n;
+    unsigned vote =
+        __ballot_sync(0xffffffffu, (__float_as_uint(mx) - kLow >= kHigh - kLow) | always);
+    if (vote == 0) return;
+    if (G < 4) vote &= ((1u << (8 * G % 32)) - 1u) << (threadIdx.x & (32u - 8 * G));
+    if (vote == 0) return;
+    // From its exponent field, 126 more than frexp's exponent; rows below
+    // 2^-108 need two factors, zeros and what is not a number none.
+    const uint32_t b = __float_as_uint(mx) >> 23;
+    if (b - 19u < 255u - 19u) {
+        r.scale(pow2f(146 - (int)b));
+        lns -= 146 - (int)b;
+    } else if (b < 19u && mx > 0.0f) {
+        int e;
+        frexpf(mx, &e);
+        r.scale(pow2f(127));
+        if (20 - e > 127) r.scale(pow2f(20 - e - 127));
+        lns -= 20 - e;
+    }
 }
 // FP64: below 2^-32 (or at 2^511), to [2^200, 2^201), and its exponent times
 // ln 2 joins the log scaler.  The reference divides by the largest child
