@@ -178,13 +178,13 @@ def autotune(lib, prec, args, lik=None, liks=None, lanes=True):
                 "source": "--shape"}
     if liks is not None:
         r = tune.tune_batch(liks, prec, iters=3,
-                            shapes=tune.candidates(
+                            shapes=tune.choices(
                                 prec, tune.active_components(liks[0]),
                                 budgets=(12 << 10, 24 << 10, 48 << 10),
                                 lanes=(1,)))
     else:
         r = tune.tune_plan(lik, prec, iters=10,
-                           shapes=None if lanes else tune.candidates(
+                           shapes=None if lanes else tune.choices(
                                prec, tune.active_components(lik), lanes=(1,)))
     best = dict(r["best"])
     top = sorted(r["table"], key=lambda x: x["ms"])
@@ -220,9 +220,8 @@ def batched_measure(gpu, case, nevals, oracle=None):
         lk.prepare_plan()
         liks.append(lk)
     tr = tune.tune_batch(liks, "fp32", iters=3,
-                         shapes=tune.candidates("fp32", 4,
-                                                budgets=(0, 12 << 10, 24 << 10),
-                                                lanes=(1,)))
+                         shapes=tune.choices("fp32", 4, budgets=(0, 12 << 10, 24 << 10),
+                                             lanes=(1,)))
     b = Batch(liks, "fp32")
     got = b.run()
     b.time(3)

@@ -84,12 +84,17 @@ def shape_ok(precision, kact, tile, tpp, ppt=1, lanes=1):
 
 def candidates(precision, kact, tiles=TILES, tpps=TPPS, budgets=BUDGETS,
                ppts=PPTS, lanes=LANES):
-    """(tile, tpp, ppt, budget, lanes) shapes the library has a walker for,
-    after AUTO.  Lanes apply to single plans only: pass lanes=(1,) for
-    batches, MC3 and the server."""
-    return [AUTO] + [(t, g, p, b, n) for t, g, p, b, n in
-                     itertools.product(tiles, tpps, ppts, budgets, lanes)
-                     if shape_ok(precision, kact, t, g, p, n)]
+    """(tile, tpp, ppt, budget, lanes) shapes the library has a walker for.
+    Lanes apply to single plans only: pass lanes=(1,) for batches, MC3 and
+    the server."""
+    return [(t, g, p, b, n) for t, g, p, b, n in
+            itertools.product(tiles, tpps, ppts, budgets, lanes)
+            if shape_ok(precision, kact, t, g, p, n)]
+
+
+def choices(precision, kact, **kw):
+    """What a sweep times: the library's own choice, then the candidates."""
+    return [AUTO] + candidates(precision, kact, **kw)
 
 
 def active_components(lik):
@@ -128,7 +133,7 @@ def tune_plan(lik, precision="fp32", iters=20, shapes=None):
     """Tune on one Lik's current full plan (``lik._prep`` done); the time is
     the walker kernel's mean over `iters` back-to-back runs."""
     from .plan import Plan
-    shapes = shapes or candidates(precision, active_components(lik))
+    shapes = shapes or choices(precision, active_components(lik))
 
     def measure():
         plan = Plan(lik, precision)
@@ -148,8 +153,8 @@ def tune_mc3(lib, make, precision="fp32", kact=4, gens=32, warm=16, shapes=None)
     walks short dirty paths over many (chain, tile) items, so per-tile
     costs weigh more there than on a full plan, and the two can prefer
     different tiles."""
-    shapes = shapes or candidates(precision, kact, tpps=(1,), ppts=(1,),
-                                  budgets=(0, 24 << 10), lanes=(1,))
+    shapes = shapes or choices(precision, kact, tpps=(1,), ppts=(1,),
+                               budgets=(0, 24 << 10), lanes=(1,))
 
     def measure():
         m = make()
@@ -167,8 +172,8 @@ def tune_batch(liks, precision="fp32", iters=5, shapes=None):
     the walker's mean over `iters` graph replays."""
     from .batch import Batch
     lk = liks[0]
-    shapes = shapes or candidates(precision, active_components(lk),
-                                  lanes=(1,))
+    shapes = shapes or choices(precision, active_components(lk),
+                               lanes=(1,))
 
     def measure():
         b = Batch(liks, precision)

@@ -51,7 +51,7 @@ def test_every_shape_same_bits(gpu, ncat):
     saved = tune.get(gpu)
     try:
         first = None
-        for shape in tune.candidates("fp32", ncat, budgets=(0, 24 << 10)):
+        for shape in tune.choices("fp32", ncat, budgets=(0, 24 << 10)):
             tune.set_shape(gpu, *shape)
             got = make(gpu, ncat).siteLnLs()
             first = first or got

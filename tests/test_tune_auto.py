@@ -51,10 +51,11 @@ def test_sweep_restores_and_keeps_the_fastest(lib):
 
 
 @pytest.mark.parametrize("precision", ["fp32", "fp64"])
-def test_the_choice_is_a_candidate(precision):
+def test_sweeps_time_the_choice_first(precision):
     for kact in (1, 4, 5, 8):
-        assert tune.candidates(precision, kact)[0] == AUTO
-        assert tune.candidates(precision, kact, budgets=(0,), lanes=(1,)).count(AUTO) == 1
+        for kw in {}, {"budgets": (0,), "lanes": (1,)}:
+            assert tune.choices(precision, kact, **kw) == \
+                [AUTO] + tune.candidates(precision, kact, **kw)
 
 
 @pytest.mark.gpu
