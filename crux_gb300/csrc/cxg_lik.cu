@@ -1275,7 +1275,7 @@ int cxgInfo(char *buf, size_t len) {
     int dev = -1, rt = 0;
     cudaRuntimeGetVersion(&rt);
     cudaError_t e = cudaGetDevice(&dev);
-    snprintf(buf, len, "cxlik_gpu 1 sm_103a cudart %d device %d%s", rt, dev,
+    snprintf(buf, len, "cxlik_gpu %d sm_103a cudart %d device %d%s", CXG_VERSION, rt, dev,
              e == cudaSuccess ? "" : " (no device)");
     return 0;
 }

@@ -169,7 +169,11 @@ enum {
 /* Message describing the most recent failure on the calling thread. */
 const char *cxgLastError(void);
 
-/* Library version and build facts: writes "cxlik_gpu <ver> sm_103a ..." */
+/* Library version and build facts: writes "cxlik_gpu <ver> sm_103a ...", ver
+ * being CXG_VERSION.  2: FP32 CLs in a caller's memory (cxgLikExecuteNoAlloc)
+ * hold their components in pairs; a buffer that version 1 wrote, a float4 a
+ * component, has to be computed again. */
+#define CXG_VERSION 2
 int cxgInfo(char *buf, size_t len);
 
 /* Register leaf CL `cl` (identified by cl->cLMat) with n per-pattern state
