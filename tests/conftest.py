@@ -71,3 +71,15 @@ def canaries_intact(request):
                                      ctypes.byref(bad)) == 0
     assert bad.value == 0, "%d of %d canaries overwritten" % (bad.value,
                                                               checked.value)
+
+
+@pytest.fixture(autouse=True)
+def no_shape_left_set(request):
+    """After every GPU test: the library chooses the walker's launch shape
+    again, so that no test runs in a shape that one before it tuned."""
+    yield
+    if request.node.get_closest_marker("gpu") is None or \
+            "gpu" not in request.fixturenames:
+        return
+    from crux_gb300 import tune
+    tune.set_shape(request.getfixturevalue("gpu"), *tune.AUTO)
