@@ -487,14 +487,36 @@ static unsigned g_lanes = 1;
 static size_t g_smem_budget = 24 * 1024;
 static bool g_tuned = false;
 
-// SMs of the GPU these kernels are built for.
-constexpr unsigned kSMs = 152;
+// SMs of the GPU (152 of a GB300; 152 too where none can be asked).
+static unsigned sm_count() {
+    static const unsigned n = [] {
+        int dev = 0, v = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+            v = 0;
+        return v > 0 ? (unsigned)v : 152u;
+    }();
+    return n;
+}
+
+// Threads per pattern of the FP64 form.  Each SM quarter issues one FP64
+// instruction a warp in 64 cycles and a pattern's components are independent, so
+// two threads a pattern halve the unit in which quarters are loaded (1,511 us
+// against 1,681 with one and 1,535 with four on 81,664 patterns), and four serve
+// a walk of few patterns (27 us against 57 on 522).
+static unsigned fp64_split(unsigned kact, size_t patterns, unsigned tile) {
+    const size_t warps = (patterns + 31) / 32;
+    const bool few = warps * 4 <= (size_t)sm_count() * 16;
+    if (few && walker_shape_ok(CXG_FP64, kact, 4) && tile * 4 <= kTuneThreads) return 4;
+    return walker_shape_ok(CXG_FP64, kact, 2) && tile * 2 <= kTuneThreads ? 2 : 1;
+}
 
 // Shape for work no caller has tuned: a plan (jobs 0), or a batch of `jobs`
 // (the batched walkers have no wide build).  Measured on the 128-taxon tree over
 // 81,664 patterns (2,552 warps), the 32-job batch and the small trees:
 //
-// FP32.  A warp's walk is a chain of ops (65 us for 127 of four components,
+// FP64 plans take tiles of 32 with several threads a pattern (fp64_split), or of
+// 64.  FP32: a warp's walk is a chain of ops (65 us for 127 of four components,
 // alone or with seven others on its SM), so CTAs are of equal size and evenly
 // spread.  Up to eight warps an SM that chain is all there is: small tiles (32
 // up to a warp an SM, 64 up to four, then 128: 246 us against 252 with 64 on
@@ -508,26 +530,13 @@ constexpr unsigned kSMs = 152;
 // fewer warps (214 us with tiles of 128 against 229 at 100,000 patterns, 346
 // against 375 at 200,000).  Many jobs take tiles of 128 (530 us; 64: 564).
 //
-// FP64.  Each SM quarter issues one FP64 instruction a warp in 64 cycles and a
-// pattern's components are independent, so two threads a pattern halve the
-// unit in which quarters are loaded (1,511 us against 1,681 with one and
-// 1,535 with four), and four serve a walk of few patterns (27 us against 57
-// on 522).
-//
 // Otherwise no shape takes stack slots: a result is stored to HBM anyway, and
 // reading it back through L2 costs less than storing it twice.
-static unsigned fp64_split(unsigned kact, size_t patterns, unsigned tile) {
-    const size_t warps = (patterns + 31) / 32;
-    const bool few = warps * 4 <= (size_t)kSMs * 16;
-    if (few && walker_shape_ok(CXG_FP64, kact, 4) && tile * 4 <= kTuneThreads) return 4;
-    return walker_shape_ok(CXG_FP64, kact, 2) && tile * 2 <= kTuneThreads ? 2 : 1;
-}
-
 static WalkShape auto_shape(int precision, unsigned kact, size_t patterns, unsigned jobs) {
     WalkShape w;
     w.precision = precision;
     w.kact = kact;
-    const size_t warps = (patterns + 31) / 32;
+    const size_t warps = (patterns + 31) / 32, sms = sm_count();
     if (precision == CXG_FP64) {
         w.tpp = fp64_split(kact, patterns, 32);
         w.tile = w.tpp > 1 ? 32 : 64;
@@ -538,8 +547,8 @@ static WalkShape auto_shape(int precision, unsigned kact, size_t patterns, unsig
         w.ring_bytes = 50 * 1024;  // four CTAs an SM: 523 us, with 42 KB 531
         return w;
     }
-    if (warps <= 8 * (size_t)kSMs) {
-        w.tile = warps <= kSMs ? 32 : warps <= 4 * (size_t)kSMs ? 64 : 128;
+    if (warps <= 8 * sms) {
+        w.tile = warps <= sms ? 32 : warps <= 4 * sms ? 64 : 128;
         // At most two CTAs an SM: a ring and slots of half its shared memory.
         w.ring_bytes = 88 * 1024;
         w.budget = kact == 1 ? 110 * 1024 : 0;
@@ -547,7 +556,7 @@ static WalkShape auto_shape(int precision, unsigned kact, size_t patterns, unsig
     }
     w.tile = 128;
     if (!wide_shape_ok(w)) return w;
-    const unsigned half = (unsigned)((warps + 2 * kSMs - 1) / (2 * kSMs));
+    const unsigned half = (unsigned)((warps + 2 * sms - 1) / (2 * sms));
     if (half <= (jobs ? kTuneThreads : kMaxThreads / 2) / 32) {
         w.tile = 32 * half;
         w.wide = w.tile > kTuneThreads;
