@@ -26,9 +26,6 @@ struct NvtxRange {
 // Patterns are padded to a multiple of this on the device, so that every
 // plane of a CL buffer starts on a 512-byte boundary.
 constexpr unsigned kPatternQuantum = 128;
-// Most patterns per tile a caller may tune (cxgTune), and of a CTA whose
-// patterns have several threads each.
-constexpr unsigned kBlock = 128;
 // Largest CTA a caller may tune: tile patterns x threads per pattern.
 constexpr unsigned kTuneThreads = 256;
 // Largest CTA of the plan walkers (the wide build: the 20 warps that an SM's
@@ -40,8 +37,7 @@ constexpr unsigned kLaneThreads = 128;
 constexpr unsigned kTile = 64;
 // Most shared-memory stack slots per tile.
 constexpr unsigned kMaxSlots = 16;
-// Op records in flight per CTA of the two-pattern and op-lane walkers
-// (bulk-copy ring depth).
+// Op records in flight per CTA of the op-lane walker (bulk-copy ring depth).
 constexpr unsigned kRing = 4;
 // Stages of the plan walker's ring, each a group of ops.
 constexpr unsigned kStages = 3;
@@ -105,7 +101,6 @@ struct RecHead {
     uint32_t nchild;
     int32_t slot;      // stack slot keeping the result for a later op, or -1
     uint32_t flags;    // REC_NO_HBM: the result is not written to HBM
-    uint32_t pad;
 };
 
 // RecHead.flags: the parent is consumed from its stack slot (or is the
@@ -219,7 +214,6 @@ struct PlanArgs {
                           // components); 0 is read as 1
     uint32_t ppt;         // patterns per thread (1 or 2); 0 is read as 1
     uint32_t wide;        // WalkShape::wide
-    uint32_t pad;
 };
 
 // Threads per pattern and patterns per thread a walker is built for with
@@ -409,7 +403,8 @@ cudaError_t launch_pmat_batch(const PmatArgs *jobs, const uint32_t *prefix,
                               uint32_t njobs, uint32_t total, cudaStream_t s);
 // `lanes` 2: the op-lane walker (the plan's records come in steps of two).
 // `pdl`: launch as a programmatic dependent of the P kernel launched just
-// before it on `s` (the walker stages its leaves while the P kernel runs).
+// before it on `s` (the walker's CTAs start while the P kernel runs and wait
+// for it before their first copy).
 cudaError_t launch_plan(int precision, const PlanArgs &a, cudaStream_t s,
                         unsigned lanes = 1, bool pdl = false);
 // Eigensystem of a model given by value; out (74 doubles) may be pinned host

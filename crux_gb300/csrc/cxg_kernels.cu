@@ -33,7 +33,6 @@ namespace cxg {
 // ---------------------------------------------------------------------------
 // P matrices, written into the op records.
 // ---------------------------------------------------------------------------
-// Four lanes per (child edge, component), see pmat_one.
 // Programmatic dependent launch: a walker launched as a dependent of the
 // P kernel may start (be scheduled, set up its shared memory and barriers)
 // once every P block has started; it waits here, before it copies its

@@ -417,9 +417,8 @@ struct Plan {
     PlanArgs a;
     double alg_bytes = 0.0;   // algorithmic bytes of one plan-walker launch
     double updates = 0.0;     // pattern-node updates of one run
-    unsigned tile = kTile, tpp = 1, ppt = 1, nslot = 0, nleaf = 0;
-    unsigned lanes = 1;       // op lanes of the walker (records per step)
-    WalkShape shape;
+    unsigned nslot = 0, nleaf = 0;
+    WalkShape shape;          // of the walker
     // Where the per-call values sit in the program (byte offsets): branch
     // lengths [stepsLen], cmult, rmult, model index [kact], cube and
     // eigenvalues [models], root weights pn [kact][4]; and what they are
@@ -1089,10 +1088,6 @@ static int translate(State &S, CxtLik *lik, int prec, Plan &P,
     P.nchild = nchild;
     P.alg_bytes = bytes * npat;
     P.updates = (double)ops.size() * npat;
-    P.tile = tile;
-    P.tpp = a.tpp;
-    P.ppt = a.ppt;
-    P.lanes = lanes;
     P.shape = w;
     P.nslot = nslot;
     P.nleaf = nleaf;
@@ -1115,7 +1110,7 @@ static int enqueue(State &S, Plan &P, bool want_site,
     if (!pmat) CXG_CUDA(cudaMemsetAsync(mp, 0, sizeof(WalkResult), S.stream));
     CXG_CUDA(launch_pmat(P.pa, S.stream));
     if (e0) CXG_CUDA(cudaEventRecord(e0, S.stream));
-    CXG_CUDA(launch_plan(P.prec, P.a, S.stream, P.lanes,
+    CXG_CUDA(launch_plan(P.prec, P.a, S.stream, P.shape.lanes,
                          pdl && e0 == nullptr && P.pa.nchild > 0));
     if (e1) CXG_CUDA(cudaEventRecord(e1, S.stream));
     CXG_CUDA(cudaMemcpyAsync(P.out.p, mp, sizeof(WalkResult), cudaMemcpyDeviceToHost, S.stream));
@@ -1558,9 +1553,9 @@ int cxgPlanTime(cxgPlan *h, int iters, double *ms_per_run,
 int cxgPlanShape(const cxgPlan *h, unsigned *tile, unsigned *tpp, unsigned *ppt,
                  unsigned *nslot, unsigned *nleaf) {
     if (h == nullptr) return fail(CXG_EINVAL, "cxgPlanShape: NULL plan");
-    if (tile) *tile = h->p.tile;
-    if (tpp) *tpp = h->p.tpp;
-    if (ppt) *ppt = h->p.ppt;
+    if (tile) *tile = h->p.shape.tile;
+    if (tpp) *tpp = h->p.shape.tpp;
+    if (ppt) *ppt = h->p.shape.ppt;
     if (nslot) *nslot = h->p.nslot;
     if (nleaf) *nleaf = h->p.nleaf;
     return 0;
@@ -1568,7 +1563,7 @@ int cxgPlanShape(const cxgPlan *h, unsigned *tile, unsigned *tpp, unsigned *ppt,
 
 int cxgPlanLanes(const cxgPlan *h, unsigned *lanes) {
     if (h == nullptr || lanes == nullptr) return fail(CXG_EINVAL, "cxgPlanLanes: NULL argument");
-    *lanes = h->p.lanes;
+    *lanes = h->p.shape.lanes;
     return 0;
 }
 
@@ -1775,9 +1770,6 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
     ba.items = static_cast<const WalkItem *>(b->items.p);
     ba.nitems = b->nitems;
     ba.counter = (unsigned *)(res + (size_t)n * sizeof(WalkResult));
-    ba.tile = b->plans[0]->tile;
-    ba.tpp = b->plans[0]->tpp;
-    ba.ppt = b->plans[0]->ppt;
     ba.kact = kact;
     ba.max_rstride = 16;
     for (const PlanArgs &a : jobs) {
@@ -1788,6 +1780,9 @@ int cxgBatchCreate(CxtLik *const *liks, unsigned n, int precision,
     // One ring for all: every job's group fits the stage of the widest.
     WalkShape w = b->plans[0]->shape;
     fit_ring(w, ba.max_rstride, ba.max_lmax);
+    ba.tile = w.tile;
+    ba.tpp = w.tpp;
+    ba.ppt = w.ppt;
     ba.ring = w.ring;
     if (!b->per_node) {
         int dev = 0, nsm = 0;

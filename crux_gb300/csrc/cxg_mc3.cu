@@ -1584,7 +1584,6 @@ __global__ void __launch_bounds__(kProposeThreads) mc3_propose_kernel(Mc3Dev d) 
             hd.nchild = nch;
             hd.slot = op_slot[o];
             hd.flags = nch == 2 ? op_kind_of_classes(kcls[0], kcls[1]) : 0;
-            hd.pad = 0;
             memcpy(r, &hd, sizeof(hd));
             for (; nl < 3; ++nl) lr[nl] = nullptr;
             continue;

@@ -961,7 +961,7 @@ void lnl_loop(cxgServer *S) {
                 }
                 prepared.push_back(J);
             }
-            // One model launch per kModelsPerLaunch jobs, a warp per job.
+            // One model launch per kModelsPerLaunch jobs, four warps per job.
             for (size_t i = 0; i < prepared.size(); i += kModelsPerLaunch) {
                 const unsigned nm =
                     (unsigned)std::min<size_t>(kModelsPerLaunch, prepared.size() - i);
