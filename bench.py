@@ -15,8 +15,10 @@ walker; the plain FP64 path is measured beside it on the same plan.
   e2e        the same metric through the public API (Lik.lnL with a full
              re-plan each step: host planning, program upload from pinned
              memory, kernels, result read-back)
-  roofline   plan-walker kernel: algorithmic bytes per launch / event time,
-             against MEASURED_PEAKS.json hbm_gbs
+  roofline   plan-walker kernel: the bytes a launch cannot do without (every
+             CL written once, every leaf's masks read once; the other reads
+             are of CLs it has just written) / event time, against
+             MEASURED_PEAKS.json hbm_gbs
   cpu_baseline  the FP64 oracle CxLikExecute on the host cores (reference
              build when present, else this repository's port)
   batched    the same tree under 32 sets of exchangeabilities in one
@@ -201,11 +203,20 @@ def autotune(lib, prec, args, lik=None, liks=None, lanes=True):
     return best
 
 
+def walk_bytes(liks):
+    """Bytes that walks of the Liks' current full plans (FP32 form) cannot do
+    without: the parents' CLs and scalers written once, the leaves' masks and
+    the pattern weights read once."""
+    from crux_gb300 import synth, tune
+    return sum(synth.nnodes_updates(lk) * (16 * tune.active_components(lk) + 4) +
+               lk.lik.mschars * (lk.alignment.ntaxa + 4) for lk in liks)
+
+
 def batched_measure(gpu, case, nevals, oracle=None):
     """The bench tree under `nevals` different GTR exchangeabilities (the
     work of as many chains' proposals) in one persistent batched launch
     (crux_gb300.batch.Batch): pattern-node updates/s of the walk, its
-    roofline by algorithmic bytes, and two of the lnLs against the FP64
+    roofline (walk_bytes), and two of the lnLs against the FP64
     oracle.  The shape is tuned on this batch."""
     import numpy as np
     from crux_gb300 import tune
@@ -230,7 +241,7 @@ def batched_measure(gpu, case, nevals, oracle=None):
     b.close()
     peaks = measured_peaks()
     hbm = peaks["hbm_gbs"] if peaks else 6800.0
-    achieved = info["alg_bytes"] / (t["walk_ms"] / 1e3) / 1e9
+    achieved = walk_bytes(liks) / (t["walk_ms"] / 1e3) / 1e9
     out = {"evals_per_launch": nevals,
            "value": info["updates"] / (t["walk_ms"] / 1e3), "unit": UNIT,
            "walk_ms": t["walk_ms"], "ms_per_run": t["ms_per_run"],
@@ -421,7 +432,7 @@ def run_ours(args, dist):
     kern_ms = res["fp32"]["t"]["kernel_ms"]
     peaks = measured_peaks()
     hbm = peaks["hbm_gbs"] if peaks else 6800.0
-    achieved = info["alg_bytes"] / (kern_ms / 1e3) / 1e9
+    achieved = walk_bytes([res["fp32"]["lik"]]) / (kern_ms / 1e3) / 1e9
     traffic = profile_traffic("walk_kernel_fp32_128taxa_100ksites.md")
 
     # Oracle check of both forms (FP64 oracle on the same plan).
@@ -592,7 +603,7 @@ def run_batch(args, dist):
     upd = fb["info"]["updates"]
     peaks = measured_peaks()
     hbm = peaks["hbm_gbs"] if peaks else 6800.0
-    achieved = fb["info"]["alg_bytes"] / (fb["t"]["walk_ms"] / 1e3) / 1e9
+    achieved = walk_bytes(liks["fp32"]) / (fb["t"]["walk_ms"] / 1e3) / 1e9
     line = {
         "metric": "CLV pattern-node updates/s (batched FP32-scaled form)",
         "value": upd / (fb["t"]["ms_per_run"] / 1e3), "unit": UNIT,
