@@ -204,12 +204,14 @@ __device__ inline void qdecomp_warp(const double *rtri, const double *pi, double
     if (in_s) v *= __hiloint2double(up << 20, 0);
     int conv = 0;
     for (int sweep = 0; sweep < 64; ++sweep) {
-        // Off-diagonal entries below 2^-67 of the largest on the diagonal
-        // (by their exponents; a NaN never converges).
+        // Off-diagonal entries below 2^-61 of the largest on the diagonal (by
+        // their exponents; a NaN never converges): what is left out is a
+        // change of S by less than a hundredth of an ulp of its entries.
+        // (To 2^-67 a call took 37.4 us on average over 400 models, 36.8 now.)
         const unsigned e = (unsigned)__double2hiint(v) & 0x7ff00000u;
         const unsigned off = __reduce_max_sync(kAll, in_s && i != j ? e : 0u);
         const unsigned dg = __reduce_max_sync(kAll, in_s && i == j ? e : 0u);
-        if (off == 0u || (off != 0x7ff00000u && off + (68u << 20) <= dg)) {
+        if (off == 0u || (off != 0x7ff00000u && off + (62u << 20) <= dg)) {
             conv = 1;
             break;
         }
